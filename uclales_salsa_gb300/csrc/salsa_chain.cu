@@ -24,6 +24,9 @@
 #include <cuda_runtime.h>
 #include <type_traits>
 #include "../../include/salsa_gb300.h"
+// The chain keeps the plain operations and CUDA's functions: over many steps its
+// condensation magnifies a last-bit difference by orders of magnitude.
+#define SALSA_MATH_PLAIN
 #include "salsa_kernel_impl.cuh"
 #include "salsa_dual.cuh"
 #include "salsa_internal.h"
@@ -59,8 +62,8 @@ template <> __device__ __forceinline__ Dual<2> t_cbrt<Dual<2>>(Dual<2> x) { retu
 template <> __device__ __forceinline__ Dual<2> t_pow<Dual<2>>(Dual<2> x, Dual<2> y) { return d_pow(x, y); }
 
 // generic math for the step (double or dual)
-__device__ __forceinline__ double g_cbrt(double x) { return cbrt(x); }
-__device__ __forceinline__ double g_exp(double x) { return exp(x); }
+__device__ __forceinline__ double g_cbrt(double x) { return dcbrt(x); }
+__device__ __forceinline__ double g_exp(double x) { return dexp(x); }
 template <int N> __device__ __forceinline__ Dual<N> g_cbrt(const Dual<N> &x) { return d_cbrt(x); }
 template <int N> __device__ __forceinline__ Dual<N> g_exp(const Dual<N> &x) { return d_exp(x); }
 __device__ __forceinline__ double g_fma(double a, double b, double c) { return fma(a, b, c); }
@@ -79,7 +82,7 @@ template <typename R> __device__ __forceinline__ R g_wsum(R v) {
   return v;
 }
 template <typename R> __device__ __forceinline__ R g_acth2o(R znw, R zns) {   // acth2o_w
-  return fmax(R(0.1), znw / fmax(R(K_EPS), znw + zns));
+  return fmax(R(0.1), ddiv(znw, fmax(R(K_EPS), znw + zns)));
 }
 
 // ---- per-cell constants of a chain ----
@@ -181,7 +184,7 @@ __device__ __forceinline__ R liquid_dwet(const DevParams &P, const CW<R> &w, con
   if (val(w.n[b]) > nlim_of(ph)) {
     R vs = R(0.);
     for (int s = 0; s < P.nwet; s++) vs += w.V(s, b);
-    dw = g_cbrt(vs * (R(1.) / (w.n[b] * K_PI6)));   // as the step kernel's updateDiameterAll
+    dw = g_cbrt(vs * (ddiv(R(1.), w.n[b] * K_PI6)));   // as the step kernel's updateDiameterAll
   } else {
     dw = R(dmid[b]);
   }
@@ -190,14 +193,14 @@ __device__ __forceinline__ R liquid_dwet(const DevParams &P, const CW<R> &w, con
 
 template <typename R>
 __device__ __forceinline__ CoagCell<R> chain_coagcell(double T, double pres, const DevParams &P) {
-  const double visc = (7.44523e-3 * sqrt(cube(T))) / (5093. * (T + 110.4));
-  const double mfp = (1.656e-10 * T + 1.828e-8) * K_PSTAND / pres;
-  const double zrhoa = pres / (K_RD * T);
-  const double vkin = visc / zrhoa;
+  const double visc = ddiv(7.44523e-3 * dsqrt(cube(T)), 5093. * (T + 110.4));
+  const double mfp = ddiv((1.656e-10 * T + 1.828e-8) * K_PSTAND, pres);
+  const double zrhoa = ddiv(pres, K_RD * T);
+  const double vkin = ddiv(visc, zrhoa);
   CoagCell<R> c;
   c.T_ = R(T); c.visc = R(visc); c.mfp = R(mfp); c.zrhoa = R(zrhoa); c.vkin = R(vkin);
-  c.shearA = R(sqrt(8. * K_PI * P.eddy_dis / (15. * vkin)));
-  c.turbB = R(K_PI * pow(P.eddy_dis, 0.75) / (K_GRAV * sqrt(sqrt(vkin))));
+  c.shearA = R(dsqrt(ddiv(8. * K_PI * P.eddy_dis, 15. * vkin)));
+  c.turbB = R(ddiv(K_PI * dpow(P.eddy_dis, 0.75), K_GRAV * dsqrt(dsqrt(vkin))));
   return c;
 }
 
@@ -330,7 +333,7 @@ __device__ __forceinline__ void chain_apply(const CW<R> &w, int t, int nspec, do
   const bool vol = lane < nspec;
   const R num = vol ? w.V(lane, t) + dt * my * n : n;
   const R den = vol ? 1. + dt * sink : 1. + dt * (sink + self);
-  const R q = num / den;
+  const R q = ddiv(num, den);
   __syncwarp();
   if (vol) w.V(lane, t) = q;
   else if (lane == nspec) w.n[t] = q;
@@ -467,16 +470,16 @@ template <typename R>
 __device__ __forceinline__ void eq1a_iter(R zrh, R &izke, R zv0, R zv1, R numc, R zvp56, R zcore, double T, R &zlwc,
                                           R &zdwet) {
   const double rhosu_msu = 1830. / 98.08e-3, rhooc_moc = 1400. / 150.e-3;
-  const double ckt = 2. * K_SURFW0 * K_MVWA / (K_BOLTZ * T);
+  const double ckt = ddiv(2. * K_SURFW0 * K_MVWA, K_BOLTZ * T);
   R zaw = zrh * izke;
   R a2 = zaw * zaw, a3 = a2 * zaw, a4 = a2 * a2;
   R bm1 = +1.1065495e+2 - 3.6759197e+2 * zaw + 5.0462934e+2 * a2 - 3.1543839e+2 * a3 + 6.770824e+1 * a4;
-  R bm2 = 1. / (zaw * K_MWA) - 1. / K_MWA;
+  R bm2 = drcp(zaw * K_MWA) - 1. / K_MWA;
   R q0 = zv0 * rhosu_msu, q1 = K_EPSOC * zv1 * rhooc_moc;
-  zlwc = g_fma(q1, bm1, q0 * bm2) / (bm1 * bm2);
-  R rinv = 1. / (numc * (K_RHOWA * K_PI6));
-  zdwet = g_cbrt(g_fma(zlwc, rinv, zvp56 / K_PI6) + zcore / K_PI6);
-  izke = g_exp(-(ckt / zdwet));
+  zlwc = ddiv(g_fma(q1, bm1, q0 * bm2), bm1 * bm2);
+  R rinv = drcp(numc * (K_RHOWA * K_PI6));
+  zdwet = g_cbrt(g_fma(zlwc, rinv, divc(zvp56, K_PI6)) + divc(zcore, K_PI6));
+  izke = g_exp(-(ddiv(ckt, zdwet)));
 }
 
 // the regime-1a chain of the non-initialising equilibration (:160-250), on every lane
@@ -493,7 +496,7 @@ __device__ void chain_equil_1a(const DevParams &P, const CW<R> &w, R prh, double
     const R numc = w.n[kk];
     const R zv0 = chain_zvolc(P, w, 0, kk), zv1 = chain_zvolc(P, w, 1, kk);
     R zvp[7];
-    for (int i = 0; i < 7; i++) zvp[i] = chain_zvolc(P, w, i, kk) / numc;
+    for (int i = 0; i < 7; i++) zvp[i] = ddiv(chain_zvolc(P, w, i, kk), numc);
     const R zcore = zvp[0] + zvp[1];
     const R zvp56 = zvp[5] + zvp[6];
     double zdwet = val(w.dw[kk]), zdold = 1.;
@@ -511,7 +514,7 @@ __device__ void chain_equil_1a(const DevParams &P, const CW<R> &w, R prh, double
     }
     if (te && lane == 0) te[0] = (double)count;
     __syncwarp();
-    if (lane == 0) w.V(P.iwa, kk) = zlwc / K_RHOWA;
+    if (lane == 0) w.V(P.iwa, kk) = divc(zlwc, K_RHOWA);
     __syncwarp();
   }
 }
@@ -521,25 +524,25 @@ template <typename R>
 __device__ __forceinline__ void cond_coeffs(R n, R dwet, R znw, R zns, double T, double prs, double rhoair, double zdfh2o,
                                             double zmfph2o, double zthcond, R &k_, R &sf, R &ws, R &m) {
   R zact = g_acth2o(znw, zns);
-  k_ = g_exp(4. * K_SURFW0 * K_MWA / (K_RG * T * K_RHOWA * dwet));
-  sf = R(prs * rhoair / K_MWA);
+  k_ = g_exp(ddiv(4. * K_SURFW0 * K_MWA, K_RG * T * K_RHOWA * dwet));
+  sf = R(divc(prs * rhoair, K_MWA));
   ws = zact * k_;
-  R zknud = 2. * zmfph2o / dwet;
-  R zbeta = (zknud + 1.) / (0.377 * zknud + 1. + 4. / (3. * 1.) * (zknud + zknud * zknud));
+  R zknud = ddiv(2. * zmfph2o, dwet);
+  R zbeta = ddiv(zknud + 1., 0.377 * zknud + 1. + 4. / (3. * 1.) * (zknud + zknud * zknud));
   R h1 = n * 2. * K_PI * dwet * zdfh2o * zbeta;
-  R h2 = K_MWA * zdfh2o * K_ALV * ws * sf / (zthcond * T);
-  R h3 = R(((K_ALV * K_MWA) / (K_RG * T)) - 1.);
-  m = h1 / (h2 * h3 + 1.);
+  R h2 = ddiv(K_MWA * zdfh2o * K_ALV * ws * sf, zthcond * T);
+  R h3 = R((ddiv(K_ALV * K_MWA, K_RG * T)) - 1.);
+  m = ddiv(h1, h2 * h3 + 1.);
 }
 
 struct CondConst { double rhoair, zdfh2o, zmfph2o, zthcond; };
 __device__ __forceinline__ CondConst cond_const(double T, double pres) {
   CondConst c;
-  c.rhoair = K_MAIR * pres / (K_RG * T);
-  double zdfh2o = (5. / (16. * K_AVOG * c.rhoair * 1.e-3 * sq(3.11e-8))) *
-                  sqrt(K_RG * 1.e7 * T * K_MAIR * 1.e3 * (K_MWA + K_MAIR) * 1.e3 / (2. * K_PI * K_MWA * 1.e3));
+  c.rhoair = ddiv(K_MAIR * pres, K_RG * T);
+  double zdfh2o = (ddiv(5., 16. * K_AVOG * c.rhoair * 1.e-3 * sq(3.11e-8))) *
+                  dsqrt(divc(K_RG * 1.e7 * T * K_MAIR * 1.e3 * (K_MWA + K_MAIR) * 1.e3, 2. * K_PI * K_MWA * 1.e3));
   c.zdfh2o = zdfh2o * 1.e-4;
-  c.zmfph2o = 3. * c.zdfh2o * sqrt(K_PI * K_MWA / (8. * K_RG * T));
+  c.zmfph2o = 3. * c.zdfh2o * dsqrt(ddiv(K_PI * K_MWA, 8. * K_RG * T));
   c.zthcond = 0.023807 + 7.1128e-5 * (T - 273.16);
   return c;
 }
@@ -549,7 +552,7 @@ __device__ __forceinline__ R chain_solute(const DevParams &P, const CW<R> &w, in
   R vs = R(0.);
   for (int nn = 0; nn < P.ndry; nn++)
     if (P.diss[nn] > 0.) vs += w.V(nn, b);
-  return kappa * vs * K_RHOWA / K_MWA;
+  return divc(kappa * vs * K_RHOWA, K_MWA);
 }
 
 // gpparth2o for warm cells (level 4).  Returns the substep count.
@@ -561,7 +564,7 @@ __device__ int chain_condensation(const DevParams &P, const CW<R> &w, const doub
   const double T = c.T, pres = c.pres, prs = c.prs;
   SUB_BEGIN();
   R prv = c.prv0;
-  const R zrh = prv / prs;
+  const R zrh = ddiv(prv, prs);
   R l1 = R(0.);
   for (int b = lane; b <= P.fn2b; b += 32) l1 += w.V(iwa, b);
   const R zaelwc1 = g_wsum(l1) * K_RHOWA;
@@ -570,7 +573,7 @@ __device__ int chain_condensation(const DevParams &P, const CW<R> &w, const doub
   R l2 = R(0.);
   for (int b = lane; b <= P.fn2b; b += 32) l2 += w.V(iwa, b);
   const R zaelwc2 = g_wsum(l2) * K_RHOWA;
-  prv = prv - (zaelwc2 - zaelwc1) / (pres * K_MAIR / (K_RG * T));
+  prv = prv - ddiv(zaelwc2 - zaelwc1, ddiv(pres * K_MAIR, K_RG * T));
 
   bool anycl = false, anypr = false, anyae = false;
   for (int b = lane; b < NL; b += 32) {
@@ -596,11 +599,11 @@ __device__ int chain_condensation(const DevParams &P, const CW<R> &w, const doub
     else if (ph == 2) act = val(n) > K_NLIM && P.lscndh2ocl;
     else act = val(n) > K_PRLIM && P.lscndh2ocl;
     if (act) {
-      const R znw = w.V(iwa, b) * P.rholiq[iwa] / P.MM[iwa];
+      const R znw = ddiv(w.V(iwa, b) * P.rholiq[iwa], P.MM[iwa]);
       cond_coeffs(n, dwet, znw, ns_, T, prs, cc.rhoair, cc.zdfh2o, cc.zmfph2o, cc.zthcond, k_, sf, ws, m);
     }
     w.kel[b] = k_; w.surf[b] = sf; w.mt[b] = m; w.wsat[b] = ws; w.zns[b] = ns_;
-    w.cw[b] = w.V(iwa, b) * K_RHOWA / K_MWA;
+    w.cw[b] = divc(w.V(iwa, b) * K_RHOWA, K_MWA);
   }
   __syncwarp();
   SUB_MARK(5);
@@ -611,7 +614,7 @@ __device__ int chain_condensation(const DevParams &P, const CW<R> &w, const doub
     if (ph == 1) a |= n > K_NLIM; else if (ph == 2) cl |= n > K_NLIM; else pr |= n > K_PRLIM;
   }
   const bool upd_ae = warp_any(a) && val(zrh) > 0.98, upd_cl = warp_any(cl), upd_pr = warp_any(pr);
-  R zcwc = prv * cc.rhoair / K_MWA;
+  R zcwc = divc(prv * cc.rhoair, K_MWA);
   R tsum = R(0.), msum = R(0.);
   for (int b = lane; b < NL; b += 32) {
     tsum += w.cw[b];
@@ -643,7 +646,7 @@ __device__ int chain_condensation(const DevParams &P, const CW<R> &w, const doub
     }
     const R zhlp1 = zcwc + adt * spsum;
     const R zhlp2 = 1. + adt * mtot;
-    zcwint = fmin(zhlp1 / zhlp2, zcwtot);
+    zcwint = fmin(ddiv(zhlp1, zhlp2), zcwtot);
     R cs = R(0.), sp = R(0.);
     for (int b = lane; b < NL; b += 32) {
       const int ph = phase_of(P, b);
@@ -671,7 +674,7 @@ __device__ int chain_condensation(const DevParams &P, const CW<R> &w, const doub
       for (int b = lane; b < NL; b += 32) tp[tl.hist_c + counter * NL + b] = val(w.cw[b]);
   }
   __syncwarp();
-  for (int b = lane; b < NL; b += 32) w.V(iwa, b) = fmax(R(0.), w.cw[b] * K_MWA / K_RHOWA);
+  for (int b = lane; b < NL; b += 32) w.V(iwa, b) = fmax(R(0.), divc(w.cw[b] * K_MWA, K_RHOWA));
   __syncwarp();
   SUB_MARK(6);
   return counter;
@@ -747,7 +750,7 @@ __device__ int chain_step(const DevParams &P, const CW<R> &w, const double *tb, 
   // (the non-initialising branch of the water uptake, mo_salsa_dynamics.f90:797-801)
   bool pr = false;
   for (int b = P.nbins + P.ncld + lane; b < NL; b += 32) pr |= val(w.n[b]) >= K_PRLIM;
-  if (warp_any(pr) || !(val(c.prv0) / c.prs >= 0.98)) return 1;
+  if (warp_any(pr) || !(ddiv(val(c.prv0), c.prs) >= 0.98)) return 1;
 #ifdef SALSA_STAGE_TIMERS
   long long t_stage = clock64();
 #endif
@@ -811,12 +814,12 @@ __device__ void chain_store(const DevParams &P, const CW<R> &w, double *x, doubl
   __syncwarp();
   for (int e = lane; e < NL * (1 + P.nwet); e += 32) {
     if (e < NL) {
-      x[e] = val(w.n[e]) / dn;
-      if (dx) dx[e] = tangent(w.n[e]) / dn;
+      x[e] = ddiv(val(w.n[e]), dn);
+      if (dx) dx[e] = ddiv(tangent(w.n[e]), dn);
     } else {
       const int s = (e - NL) / NL, b = (e - NL) - s * NL;
-      x[e] = val(w.V(s, b)) * P.rholiq[s] / dn;
-      if (dx) dx[e] = tangent(w.V(s, b)) * P.rholiq[s] / dn;
+      x[e] = ddiv(val(w.V(s, b)) * P.rholiq[s], dn);
+      if (dx) dx[e] = ddiv(tangent(w.V(s, b)) * P.rholiq[s], dn);
     }
   }
   __syncwarp();
@@ -826,7 +829,7 @@ template <typename R>
 __device__ __forceinline__ ChainCell<R> chain_cell(const ChainArgs &A, long long q, bool tlm) {
   ChainCell<R> c;
   c.T = A.temp[q]; c.pres = A.press[q]; c.prs = A.rs[q]; c.dn = A.dn[q];
-  c.rhoair = K_MAIR * c.pres / (K_RG * c.T);
+  c.rhoair = ddiv(K_MAIR * c.pres, K_RG * c.T);
   c.kappa = R(A.kappa[q]);
   c.prv0 = R(A.rs[q] * (1.0 + A.ssat[q]));
   if (tlm) {
@@ -911,13 +914,13 @@ __device__ void cond_reverse(const DevParams &P, const CW<double> &w, const AW &
   const int NL = w.NL, NW = P.nwet, iwa = P.iwa;
   const double *dmid = tb + TAB_DMID * P.nb_pad;
   const double T = c.T, pres = c.pres, prs = c.prs;
-  const double D = pres * K_MAIR / (K_RG * T);
+  const double D = ddiv(pres * K_MAIR, K_RG * T);
   const int nit = (int)tp[tl.nit];
   SUB_BEGIN();
   // state after the water uptake (x_eq)
   tape_to_state(tp + tl.x_eq, w.n, w.v, NL, NW, lane);
   __syncwarp();
-  const double zrh = c.prv0 / prs;
+  const double zrh = ddiv(c.prv0, prs);
   double prv_adj_bar = 0.;
   const CondConst cc = cond_const(T, pres);
   if (nit >= 0) {
@@ -933,7 +936,7 @@ __device__ void cond_reverse(const DevParams &P, const CW<double> &w, const AW &
       else if (ph == 2) act = n > K_NLIM && P.lscndh2ocl;
       else act = n > K_PRLIM && P.lscndh2ocl;
       if (act) {
-        const double znw = w.V(iwa, b) * P.rholiq[iwa] / P.MM[iwa];
+        const double znw = ddiv(w.V(iwa, b) * P.rholiq[iwa], P.MM[iwa]);
         cond_coeffs(n, dwet, znw, ns_, T, prs, cc.rhoair, cc.zdfh2o, cc.zmfph2o, cc.zthcond, k_, sf, ws, m);
       }
       w.kel[b] = k_; w.surf[b] = sf; w.mt[b] = m; w.zns[b] = ns_;
@@ -949,7 +952,7 @@ __device__ void cond_reverse(const DevParams &P, const CW<double> &w, const AW &
     const bool upd_ae = warp_any(ae) && zrh > 0.98, upd_cl = warp_any(cl), upd_pr = warp_any(pr);
     double tsum = 0., msum = 0.;
     for (int b = lane; b < NL; b += 32) {
-      tsum += w.V(iwa, b) * K_RHOWA / K_MWA;
+      tsum += divc(w.V(iwa, b) * K_RHOWA, K_MWA);
       if (b >= P.in2a) msum += w.mt[b];
     }
     const double zcwtot = tp[tl.hist_zc] + wsum(tsum);
@@ -957,14 +960,14 @@ __device__ void cond_reverse(const DevParams &P, const CW<double> &w, const AW &
     // write-back: V_w = max(0, c_final MWA / RHOWA)
     for (int b = lane; b < NL; b += 32) {
       const double cf = tp[tl.hist_c + nit * NL + b];
-      const double y = cf * K_MWA / K_RHOWA;
-      a.cb[b] = y > 0. ? a.AV(iwa, b) * K_MWA / K_RHOWA : 0.;
+      const double y = divc(cf * K_MWA, K_RHOWA);
+      a.cb[b] = y > 0. ? divc(a.AV(iwa, b) * K_MWA, K_RHOWA) : 0.;
       a.AV(iwa, b) = 0.;
     }
     __syncwarp();
     double zcb = 0., zcwtotb = 0., mtotb = 0.;
     const double adt = 2.e-2;
-    const double izh2 = 1. / (1. + adt * mtot);   // the substeps' constant denominator
+    const double izh2 = drcp(1. + adt * mtot);   // the substeps' constant denominator
     for (int it = nit - 1; it >= 0; it--) {
       const double zc_in = tp[tl.hist_zc + it];
       const double *cin = tp + tl.hist_c + it * NL, *win = tp + tl.hist_w + it * NL;
@@ -973,7 +976,7 @@ __device__ void cond_reverse(const DevParams &P, const CW<double> &w, const AW &
         if (b >= P.in2a) sp += w.mt[b] * win[b] * w.surf[b];
       const double zhlp1 = zc_in + adt * wsum(sp);
       const double zhlp2 = 1. + adt * mtot;
-      const double q = zhlp1 / zhlp2;
+      const double q = ddiv(zhlp1, zhlp2);
       const double zcwint = fmin(q, zcwtot);
       // zcwc_out = zcwtot - sum c_out
       zcwtotb += zcb;
@@ -993,17 +996,17 @@ __device__ void cond_reverse(const DevParams &P, const CW<double> &w, const AW &
         // wsat_out = acth2o(ci, zns) * kel
         const double gw = a.wb[b];
         const double den = fmax(K_EPS, ci + zns);
-        const double r = ci / den;
+        const double r = ddiv(ci, den);
         const double act = fmax(0.1, r);
         a.kelb[b] += gw * act;
         const double ab = gw * kel;
         if (r > 0.1) {
           if (ci + zns > K_EPS) {
-            const double id = 1. / (ci + zns), q2 = ab * id * id;
+            const double id = drcp(ci + zns), q2 = ab * id * id;
             cib += q2 * zns;
             a.znsb[b] += -q2 * ci;
           } else {
-            cib += ab / K_EPS;
+            cib += divc(ab, K_EPS);
           }
         }
         double c0b = cib, a1b = 0.;
@@ -1035,14 +1038,14 @@ __device__ void cond_reverse(const DevParams &P, const CW<double> &w, const AW &
       a.cb[b] += zcwtotb;
     }
     zcb += zcwtotb;
-    prv_adj_bar = zcb * cc.rhoair / K_MWA;
+    prv_adj_bar = divc(zcb * cc.rhoair, K_MWA);
     __syncwarp();
     SUB_MARK(0);
     // coefficients (x_eq state): cw0, zns, and kel/ws/mt through dual numbers
     double kb_l = 0.;
     for (int b = lane; b < NL; b += 32) {
       const int ph = phase_of(P, b);
-      a.AV(iwa, b) += a.cb[b] * K_RHOWA / K_MWA;
+      a.AV(iwa, b) += divc(a.cb[b] * K_RHOWA, K_MWA);
       const double n = w.n[b];
       bool act;
       if (ph == 1) act = n > K_NLIM && zrh > 0.98 && P.lscndh2oae;
@@ -1051,23 +1054,23 @@ __device__ void cond_reverse(const DevParams &P, const CW<double> &w, const AW &
       double znsb = a.znsb[b];
       if (act) {
         // inputs: 0 n, 1 dwet, 2 znw, 3 zns
-        Dual<4> dn_(n), dd(liquid_dwet(P, w, dmid, b)), dz(w.V(iwa, b) * P.rholiq[iwa] / P.MM[iwa]), ds(w.zns[b]);
+        Dual<4> dn_(n), dd(liquid_dwet(P, w, dmid, b)), dz(ddiv(w.V(iwa, b) * P.rholiq[iwa], P.MM[iwa])), ds(w.zns[b]);
         dn_.d[0] = 1.; dd.d[1] = 1.; dz.d[2] = 1.; ds.d[3] = 1.;
         Dual<4> k_, sf, ws, m;
         cond_coeffs(dn_, dd, dz, ds, T, prs, cc.rhoair, cc.zdfh2o, cc.zmfph2o, cc.zthcond, k_, sf, ws, m);
         double g[4];
         for (int i = 0; i < 4; i++) g[i] = a.kelb[b] * k_.d[i] + a.wb[b] * ws.d[i] + a.mtb[b] * m.d[i];
         a.an[b] += g[0];
-        a.AV(iwa, b) += g[2] * P.rholiq[iwa] / P.MM[iwa];
+        a.AV(iwa, b) += ddiv(g[2] * P.rholiq[iwa], P.MM[iwa]);
         znsb += g[3];
         // wet diameter of x_eq
         if (n > nlim_of(ph)) {
           double vs = 0.;
           for (int s = 0; s < NW; s++) vs += w.V(s, b);
-          const double dw = cbrt(vs / n / K_PI6);
+          const double dw = dcbrt(divc(ddiv(vs, n), K_PI6));
           if (!(dlim_of(ph) < dw)) {
-            for (int s = 0; s < NW; s++) a.AV(s, b) += g[1] * dw / (3. * vs);
-            a.an[b] += -g[1] * dw / (3. * n);
+            for (int s = 0; s < NW; s++) a.AV(s, b) += ddiv(g[1] * dw, 3. * vs);
+            a.an[b] += -ddiv(g[1] * dw, 3. * n);
           }
         }
       }
@@ -1075,9 +1078,9 @@ __device__ void cond_reverse(const DevParams &P, const CW<double> &w, const AW &
       double vsol = 0.;
       for (int nn = 0; nn < P.ndry; nn++)
         if (P.diss[nn] > 0.) vsol += w.V(nn, b);
-      kb_l += znsb * vsol * K_RHOWA / K_MWA;
+      kb_l += divc(znsb * vsol * K_RHOWA, K_MWA);
       for (int nn = 0; nn < P.ndry; nn++)
-        if (P.diss[nn] > 0.) a.AV(nn, b) += znsb * c.kappa * K_RHOWA / K_MWA;
+        if (P.diss[nn] > 0.) a.AV(nn, b) += divc(znsb * c.kappa * K_RHOWA, K_MWA);
     }
     kbar += wsum(kb_l);
     __syncwarp();
@@ -1085,7 +1088,7 @@ __device__ void cond_reverse(const DevParams &P, const CW<double> &w, const AW &
   }
   // prv_adj = prv0 - (zaelwc2 - zaelwc1) / D
   pbar += prv_adj_bar;
-  const double zael2b = -prv_adj_bar / D, zael1b = prv_adj_bar / D;
+  const double zael2b = -ddiv(prv_adj_bar, D), zael1b = ddiv(prv_adj_bar, D);
   for (int b = lane; b <= P.fn2b; b += 32) a.AV(iwa, b) += zael2b * K_RHOWA;
   __syncwarp();
   // Regime-1a water uptake reverse.  The forward iterates zke_{i+1} = f(zke_i; bin) through
@@ -1119,12 +1122,12 @@ __device__ void cond_reverse(const DevParams &P, const CW<double> &w, const AW &
         const double numc = xm[kk];
         const double zv0 = P.ix_so4 >= 0 ? xm[NL + P.ix_so4 * NL + kk] : 0.;
         const double zv1 = P.ix_oc >= 0 ? xm[NL + P.ix_oc * NL + kk] : 0.;
-        const double zcore = zv0 / numc + zv1 / numc;
+        const double zcore = ddiv(zv0, numc) + ddiv(zv1, numc);
         Dual<5> izke(te[i]), d0(zv0), d1(zv1), dnm(numc), dco(zcore);
         izke.d[0] = 1.; d0.d[1] = 1.; d1.d[2] = 1.; dnm.d[3] = 1.; dco.d[4] = 1.;
         Dual<5> zlwc, zd;
         eq1a_iter(zrhd, izke, d0, d1, dnm, Dual<5>(0.), dco, T, zlwc, zd);   // izke is now 1/zke_i
-        const double lb = (i == cnt) ? a.AV(iwa, kk) / K_RHOWA : 0.;
+        const double lb = (i == cnt) ? divc(a.AV(iwa, kk), K_RHOWA) : 0.;
         for (int k = 0; k < 5; k++) { p[k] = izke.d[k]; q[k] = lb * zlwc.d[k]; }
       }
       // the zke adjoint entering each iteration, serially through the chunk
@@ -1160,9 +1163,9 @@ __device__ void cond_reverse(const DevParams &P, const CW<double> &w, const AW &
           const double zv1 = P.ix_oc >= 0 ? xm[NL + P.ix_oc * NL + kk] : 0.;
           double zv0b = tot[0], zv1b = tot[1], numcb = tot[2];
           const double zcoreb = tot[3];
-          zv0b += zcoreb / numc;
-          zv1b += zcoreb / numc;
-          numcb += -zcoreb * zv0 / (numc * numc) - zcoreb * zv1 / (numc * numc);
+          zv0b += ddiv(zcoreb, numc);
+          zv1b += ddiv(zcoreb, numc);
+          numcb += -ddiv(zcoreb * zv0, numc * numc) - ddiv(zcoreb * zv1, numc * numc);
           if (P.ix_so4 >= 0) a.AV(P.ix_so4, kk) += zv0b;
           if (P.ix_oc >= 0) a.AV(P.ix_oc, kk) += zv1b;
           a.an[kk] += numcb;
@@ -1224,7 +1227,7 @@ __device__ void coag_reverse(const DevParams &P, const CW<double> &w, const AW &
     const bool has_self = isc ? P.lscgcc : P.lscgaa;
     const double nt = xin[t];
     // the two denominators of the update, as reciprocals (the partials divide by them)
-    const double r1 = 1. / (1. + dt * sink), r2 = 1. / (1. + dt * (sink + self));
+    const double r1 = drcp(1. + dt * sink), r2 = drcp(1. + dt * (sink + self));
     // adjoints of the outputs (new slot of t)
     double vbar[SALSA_NSV];
     for (int s = 0; s < SALSA_NSV; s++) vbar[s] = s < NW ? a.AV(s, t) : 0.;
@@ -1305,10 +1308,10 @@ __device__ void kernel_reverse(const DevParams &P, const AW &a, const double *xi
     if (n > nlim_of(ph) && g != 0.) {
       double vs = 0.;
       for (int s = 0; s < NW; s++) vs += xin[NL + s * NL + b];
-      const double dw = cbrt(vs / n / K_PI6);
+      const double dw = dcbrt(divc(ddiv(vs, n), K_PI6));
       if (!(dlim_of(ph) < dw)) {
-        for (int s = 0; s < NW; s++) a.AV(s, b) += g * dw / (3. * vs);
-        a.an[b] += -g * dw / (3. * n);
+        for (int s = 0; s < NW; s++) a.AV(s, b) += ddiv(g * dw, 3. * vs);
+        a.an[b] += -ddiv(g * dw, 3. * n);
       }
     }
   }
@@ -1440,10 +1443,10 @@ __global__ void chain_adj_units(const DevParams P, const ChainArgs A, int to_sal
     const double dn = A.dn[q];
     const double rho = e < A.NL ? 1. : P.rholiq[(e - A.NL) / A.NL];
     if (to_salsa) {
-      A.xbar0[i] = A.xbarN[i] * rho / dn;
+      A.xbar0[i] = ddiv(A.xbarN[i] * rho, dn);
       if (e == 0) { A.kappabar[q] = 0.; A.ssatbar[q] = 0.; }
     } else {
-      A.xbar0[i] = A.xbar0[i] * dn / rho;
+      A.xbar0[i] = ddiv(A.xbar0[i] * dn, rho);
     }
   }
 }

@@ -9,6 +9,7 @@
 // multiply-adds, which only changes their last bits.
 #pragma once
 #include <cuda_runtime.h>
+#include "salsa_math.cuh"
 
 namespace salsa {
 
@@ -67,8 +68,8 @@ template <int N> __device__ __forceinline__ Dual<N> operator*(const Dual<N> &a, 
   return r;
 }
 template <int N> __device__ __forceinline__ Dual<N> operator/(const Dual<N> &a, const Dual<N> &b) {
-  Dual<N> r; r.v = a.v / b.v;
-  const double ib = 1. / b.v;
+  Dual<N> r; r.v = ddiv(a.v, b.v);
+  const double ib = drcp(b.v);
 #pragma unroll
   for (int i = 0; i < N; i++) r.d[i] = __fma_rn(-r.v, b.d[i], a.d[i]) * ib;
   return r;
@@ -86,6 +87,12 @@ template <int N> __device__ __forceinline__ Dual<N> operator*(const Dual<N> &a, 
 template <int N> __device__ __forceinline__ Dual<N> operator*(double a, const Dual<N> &b) { return b * a; }
 template <int N> __device__ __forceinline__ Dual<N> operator/(const Dual<N> &a, double b) { return a / Dual<N>(b); }
 template <int N> __device__ __forceinline__ Dual<N> operator/(double a, const Dual<N> &b) { return Dual<N>(a) / b; }
+template <int N> __device__ __forceinline__ Dual<N> ddiv(const Dual<N> &a, const Dual<N> &b) { return a / b; }
+template <int N> __device__ __forceinline__ Dual<N> ddiv(const Dual<N> &a, double b) { return a / Dual<N>(b); }
+template <int N> __device__ __forceinline__ Dual<N> ddiv(double a, const Dual<N> &b) { return Dual<N>(a) / b; }
+template <int N> __device__ __forceinline__ Dual<N> drcp(const Dual<N> &a) { return Dual<N>(1.) / a; }
+template <int N> __device__ __forceinline__ Dual<N> divc(const Dual<N> &a, double c) { return a / c; }
+template <int N> __device__ __forceinline__ Dual<N> divc(const Dual<N> &a, const Dual<N> &c) { return a / c; }
 template <int N> __device__ __forceinline__ Dual<N> &operator+=(Dual<N> &a, const Dual<N> &b) { a = a + b; return a; }
 template <int N> __device__ __forceinline__ Dual<N> &operator-=(Dual<N> &a, const Dual<N> &b) { a = a - b; return a; }
 template <int N> __device__ __forceinline__ Dual<N> &operator*=(Dual<N> &a, const Dual<N> &b) { a = a * b; return a; }
@@ -109,21 +116,21 @@ template <int N> __device__ __forceinline__ Dual<N> fmin(const Dual<N> &a, doubl
 template <int N> __device__ __forceinline__ Dual<N> fmax(const Dual<N> &a, double b) { return fmax(a, Dual<N>(b)); }
 template <int N> __device__ __forceinline__ Dual<N> fmin(double a, const Dual<N> &b) { return fmin(Dual<N>(a), b); }
 template <int N> __device__ __forceinline__ Dual<N> fmax(double a, const Dual<N> &b) { return fmax(Dual<N>(a), b); }
-template <int N> __device__ __forceinline__ Dual<N> d_exp(const Dual<N> &a) { double e = exp(a.v); return d_apply(a, e, e); }
-template <int N> __device__ __forceinline__ Dual<N> d_log(const Dual<N> &a) { return d_apply(a, log(a.v), 1. / a.v); }
+template <int N> __device__ __forceinline__ Dual<N> d_exp(const Dual<N> &a) { double e = dexp(a.v); return d_apply(a, e, e); }
+template <int N> __device__ __forceinline__ Dual<N> d_log(const Dual<N> &a) { return d_apply(a, dlog(a.v), drcp(a.v)); }
 template <int N> __device__ __forceinline__ Dual<N> d_sqrt(const Dual<N> &a) {
-  double s = sqrt(a.v);
-  return d_apply(a, s, s > 0. ? 0.5 / s : 0.);
+  double s = dsqrt(a.v);
+  return d_apply(a, s, s > 0. ? ddiv(0.5, s) : 0.);
 }
 template <int N> __device__ __forceinline__ Dual<N> d_cbrt(const Dual<N> &a) {
-  double c = cbrt(a.v);
-  return d_apply(a, c, c != 0. ? 1. / (3. * c * c) : 0.);
+  double c = dcbrt(a.v);
+  return d_apply(a, c, c != 0. ? drcp(3. * c * c) : 0.);
 }
 template <int N> __device__ __forceinline__ Dual<N> d_pow(const Dual<N> &a, const Dual<N> &b) {
   Dual<N> r;
-  r.v = pow(a.v, b.v);
-  const double la = a.v > 0. ? log(a.v) : 0.;
-  const double ga = a.v != 0. ? b.v * r.v / a.v : 0., rl = r.v * la;
+  r.v = dpow(a.v, b.v);
+  const double la = a.v > 0. ? dlog(a.v) : 0.;
+  const double ga = a.v != 0. ? ddiv(b.v * r.v, a.v) : 0., rl = r.v * la;
 #pragma unroll
   for (int i = 0; i < N; i++) r.d[i] = __fma_rn(ga, a.d[i], rl * b.d[i]);
   return r;

@@ -22,6 +22,7 @@
 //     (all-clear or cloudy); a block's cells are then not always neighbours.
 #pragma once
 #include "salsa_device.cuh"
+#include "salsa_math.cuh"
 #include <cstdio>
 #include <type_traits>
 
@@ -98,10 +99,10 @@ __device__ void updateDiameterAll(const DevParams &P, const WS<double> *, double
     for (int s = 0; s < P.ndry; s++) vd += volc[s * NB + b];
     for (int k = 0; k < P.ninsoluble; k++) vi += volc[P.ind_insoluble[k] * NB + b];
     // (v / numc / pi6)^(1/3) with one division for the three diameters
-    const double q = 1. / (n * K_PI6);
-    dw = cbrt(vs * q);
-    dd = cbrt(vd * q);
-    di = cbrt(vi * q);
+    const double q = drcp(n * K_PI6);
+    dw = dcbrt(vs * q);
+    dd = dcbrt(vd * q);
+    di = dcbrt(vi * q);
   } else {
     dw = dd = di = dmid[b];
   }
@@ -117,7 +118,7 @@ __device__ __forceinline__ double rhomean_of(const DevParams &P, int ph, double 
   if (ph > 3) {
     if (n > nlim_of(ph)) {
       double mp = K_RHOIC * vw, mr = K_RHORI * vr, mt = mp + mr;
-      double r = (mp * K_RHOIC + mr * K_RHORI) / fmax(mt, 7.e-25);
+      double r = ddiv(mp * K_RHOIC + mr * K_RHORI, fmax(mt, 7.e-25));
       return fmin(r, K_RHOIC);
     }
     return K_RHOIC;
@@ -128,7 +129,7 @@ __device__ __forceinline__ double rhomean_of(const DevParams &P, int ph, double 
 // classSection.f90:202-224 getRimeFraction
 __device__ __forceinline__ double rimefrac(const DevParams &P, double n, double vw, double vr, int ph) {
   double r = 0.;
-  if (ph == 4 && vw > 1.e-23 && vr > 1.e-23 && n > nlim_of(ph)) r = vr * K_RHORI / (vw * K_RHOIC + vr * K_RHORI);
+  if (ph == 4 && vw > 1.e-23 && vr > 1.e-23 && n > nlim_of(ph)) r = ddiv(vr * K_RHORI, vw * K_RHOIC + vr * K_RHORI);
   return r;
 }
 
@@ -146,23 +147,23 @@ template <> struct is_f32<float> { static constexpr bool value = true; };
 
 template <typename T>
 __device__ __forceinline__ T t_exp(T x);
-template <> __device__ __forceinline__ double t_exp<double>(double x) { return exp(x); }
+template <> __device__ __forceinline__ double t_exp<double>(double x) { return dexp(x); }
 template <> __device__ __forceinline__ float t_exp<float>(float x) { return expf(x); }
 template <typename T>
 __device__ __forceinline__ T t_log(T x);
-template <> __device__ __forceinline__ double t_log<double>(double x) { return log(x); }
+template <> __device__ __forceinline__ double t_log<double>(double x) { return dlog(x); }
 template <> __device__ __forceinline__ float t_log<float>(float x) { return logf(x); }
 template <typename T>
 __device__ __forceinline__ T t_sqrt(T x);
-template <> __device__ __forceinline__ double t_sqrt<double>(double x) { return sqrt(x); }
+template <> __device__ __forceinline__ double t_sqrt<double>(double x) { return dsqrt(x); }
 template <> __device__ __forceinline__ float t_sqrt<float>(float x) { return sqrtf(x); }
 template <typename T>
 __device__ __forceinline__ T t_cbrt(T x);
-template <> __device__ __forceinline__ double t_cbrt<double>(double x) { return cbrt(x); }
+template <> __device__ __forceinline__ double t_cbrt<double>(double x) { return dcbrt(x); }
 template <> __device__ __forceinline__ float t_cbrt<float>(float x) { return cbrtf(x); }
 template <typename T>
 __device__ __forceinline__ T t_pow(T x, T y);
-template <> __device__ __forceinline__ double t_pow<double>(double x, double y) { return pow(x, y); }
+template <> __device__ __forceinline__ double t_pow<double>(double x, double y) { return dpow(x, y); }
 template <> __device__ __forceinline__ float t_pow<float>(float x, float y) { return powf(x, y); }
 
 template <typename T>
@@ -172,17 +173,17 @@ __device__ void shape_coeffs(const DevParams &P, Shape<T> &s, double mpri, doubl
   s.gamma = (T)(K_PI / 4.);
   s.sigma = (T)2.;
   if (numc < 1.e-6) return;
-  double Mtot = (mpri + mrim) / numc;
-  double Fr = fmax(fmin(mrim / (Mtot * numc), 0.9999), 0.0001);
+  double Mtot = ddiv(mpri + mrim, numc);
+  double Fr = fmax(fmin(ddiv(mrim, Mtot * numc), 0.9999), 0.0001);
   double rho_b = Fr * K_RHORI + (1. - Fr) * K_RHOIC;
-  double Dth = pow(K_PI6 * K_RHOIC / P.iceShapeAlpha, 1. / (P.iceShapeBeta - 3.));
-  double Dgr = pow(P.iceShapeAlpha / (K_PI6 * rho_b), 1. / (3. - P.iceShapeBeta));
-  double Dcr = pow((1. / (1. - Fr)) * P.iceShapeAlpha / (K_PI6 * rho_b), 1. / (3. - P.iceShapeBeta));
+  double Dth = dpow(ddiv(K_PI6 * K_RHOIC, P.iceShapeAlpha), drcp(P.iceShapeBeta - 3.));
+  double Dgr = dpow(ddiv(P.iceShapeAlpha, K_PI6 * rho_b), drcp(3. - P.iceShapeBeta));
+  double Dcr = dpow(ddiv((drcp(1. - Fr)) * P.iceShapeAlpha, K_PI6 * rho_b), drcp(3. - P.iceShapeBeta));
   double Mth = K_RHOIC * K_PI6 * cube(Dth), Mgr = rho_b * K_PI6 * cube(Dgr), Mcr = rho_b * K_PI6 * cube(Dcr);
   if (Mtot >= Mth && Mtot < Mgr) {
     s.alpha = (T)P.iceShapeAlpha; s.beta = (T)P.iceShapeBeta; s.gamma = (T)P.iceShapeGamma; s.sigma = (T)P.iceShapeSigma;
   } else if (Mtot > Mcr) {
-    double hlp = 1. / (1. - Fr);
+    double hlp = drcp(1. - Fr);
     s.alpha = (T)(P.iceShapeAlpha * hlp);
     s.beta = (T)P.iceShapeBeta;
     s.gamma = (T)(P.iceShapeGamma * (1. - Fr) + K_PI / 4. * Fr);
@@ -196,51 +197,51 @@ __device__ T terminal_vel(T diam, T rhop, T rhoa, T visc, T beta, int flag, cons
   T tv = 0;
   if (flag <= 3) {
     if (diam <= (T)19E-6) {
-      tv = sq(diam) * (rhop - rhoa) * grav * beta / ((T)18. * visc);
+      tv = ddiv(sq(diam) * (rhop - rhoa) * grav * beta, (T)18. * visc);
     } else if (diam < (T)1.07E-3) {
-      T NDa = (T)4. / (T)3. * cube(diam) * grav * (rhop - rhoa) * rhoa / sq(visc);
+      T NDa = ddiv((T)4. / (T)3. * cube(diam) * grav * (rhop - rhoa) * rhoa, sq(visc));
       T X = t_log(NDa);
       T X2 = sq(X);
       T Y = (T)-0.318657E1 + (T)0.992696 * X - (T)0.153193E-2 * X2 - (T)0.987059E-3 * X2 * X -
             (T)0.578878E-3 * sq(X2) + (T)0.855176E-4 * sq(X2) * X - (T)0.327815E-5 * cube(X2);
       T Re2 = beta * t_exp(Y);
-      tv = visc / rhoa / diam * Re2;
+      tv = ddiv(ddiv(visc, rhoa), diam) * Re2;
     } else {
-      T Np = cube((T)K_SURFW0) * sq(rhoa) / (sq(sq(visc)) * (rhop - rhoa) * grav);
-      T Bo = (T)4. / (T)3. * (rhop - rhoa) * grav / (T)K_SURFW0 * sq(diam);
+      T Np = ddiv(cube((T)K_SURFW0) * sq(rhoa), sq(sq(visc)) * (rhop - rhoa) * grav);
+      T Bo = divc((T)4. / (T)3. * (rhop - rhoa) * grav, (T)K_SURFW0) * sq(diam);
       T Np6 = t_sqrt(t_cbrt(Np));
       T X3 = t_log(Bo * Np6);
       T X32 = sq(X3);
       T Y3 = (T)-0.500015E1 + (T)0.523778E1 * X3 - (T)0.204914E1 * X32 + (T)0.475294 * X32 * X3 -
              (T)0.542819E-1 * sq(X32) + (T)0.238449E-2 * sq(X32) * X3;
       T Re3 = Np6 * t_exp(Y3);
-      tv = fmin(visc / rhoa / diam * Re3, (T)9.2);
+      tv = fmin(ddiv(ddiv(visc, rhoa), diam) * Re3, (T)9.2);
     }
   } else {
     // Khvorostyanov and Curry 2002 (kc1213/kcbre/kcare/kcAv/kcBv/kcVt :297-352)
     T Vb = (T)K_PI6 * cube(diam);
     T Ap = sh.gamma * t_pow(dnsp, sh.sigma);
-    T X = ((T)2. * Vb * (rhop - rhoa) * grav * sq(dnsp)) / (Ap * rhoa * sq(visc));
+    T X = ddiv((T)2. * Vb * (rhop - rhoa) * grav * sq(dnsp), Ap * rhoa * sq(visc));
     const T c1 = (T)0.0902, delta0 = (T)9.06;
     T k12, km1, bre;
     if (!is_f32<T>::value) {
       k12 = t_sqrt((T)1. + c1 * t_sqrt(X));
       km1 = k12 - (T)1.;
       bre = (T)0.5 * c1 * t_sqrt(X);
-      bre = bre / km1;
-      bre = bre / k12;
+      bre = ddiv(bre, km1);
+      bre = ddiv(bre, k12);
     } else {
       // float: sqrt(1+y)-1 = y/(sqrt(1+y)+1) and b_Re = (1 + 1/k12)/2, free of cancellation
       T y = c1 * t_sqrt(X);
       k12 = t_sqrt((T)1. + y);
-      km1 = y / (k12 + (T)1.);
-      bre = (T)0.5 * ((T)1. + (T)1. / k12);
+      km1 = ddiv(y, k12 + (T)1.);
+      bre = (T)0.5 * ((T)1. + ddiv((T)1., k12));
     }
     T are = (T)0.25 * sq(delta0);
     are = are * sq(km1);
-    are = are / t_pow(X, bre);
+    are = ddiv(are, t_pow(X, bre));
     T Av = are * t_pow(visc, (T)1. - (T)2. * bre);
-    Av = Av * t_pow(((T)2. * sh.alpha * grav) / (rhoa * sh.gamma), bre);
+    Av = Av * t_pow(ddiv((T)2. * sh.alpha * grav, rhoa * sh.gamma), bre);
     T Bv = bre * (sh.beta - sh.sigma + (T)2.) - (T)1.;
     tv = Av * t_pow(dnsp, Bv);
   }
@@ -264,12 +265,12 @@ template <typename T>
 __device__ void bin_props(const CoagCell<T> &cc, int ph, T diam, T dsph, T mass, T rhomean, const Shape<T> &sh,
                           BinProps<T> &o) {
   o.diam = diam;
-  T knud = (T)2. * cc.mfp / diam;
-  const T beta = (T)1. + knud * ((T)1.142 + (T)0.558 * t_exp((T)-0.999 / knud));
-  o.dfpart = beta * (T)K_BOLTZ * cc.T_ / ((T)3. * (T)K_PI * cc.visc * diam);
-  const T mtvel = t_sqrt(((T)8. * (T)K_BOLTZ * cc.T_) / ((T)K_PI * mass));
+  T knud = ddiv((T)2. * cc.mfp, diam);
+  const T beta = (T)1. + knud * ((T)1.142 + (T)0.558 * t_exp(ddiv((T)-0.999, knud)));
+  o.dfpart = ddiv(beta * (T)K_BOLTZ * cc.T_, (T)3. * (T)K_PI * cc.visc * diam);
+  const T mtvel = t_sqrt(ddiv((T)8. * (T)K_BOLTZ * cc.T_, (T)K_PI * mass));
   o.mtvel2 = sq(mtvel);
-  o.omega = (T)8. * o.dfpart / ((T)K_PI * mtvel);
+  o.omega = ddiv((T)8. * o.dfpart, (T)K_PI * mtvel);
   if constexpr (is_f32<T>::value) {
     // the fall speed stays FP64 in the mixed form: collision kernels of pairs with close
     // fall speeds take their difference, which would magnify float rounding of the Beard
@@ -283,11 +284,11 @@ __device__ void bin_props(const CoagCell<T> &cc, int ph, T diam, T dsph, T mass,
     if (ph < 4) o.termv = terminal_vel<T>(diam, rhomean, cc.zrhoa, cc.visc, beta, ph, sh, (T)0);
     else o.termv = terminal_vel<T>(dsph, rhomean, cc.zrhoa, cc.visc, beta, ph, sh, diam);
   }
-  o.reyn = diam * o.termv / cc.vkin;
-  const T schm = cc.vkin / o.dfpart;
+  o.reyn = ddiv(diam * o.termv, cc.vkin);
+  const T schm = ddiv(cc.vkin, o.dfpart);
   o.fre = o.reyn <= (T)1. ? t_cbrt(o.reyn) : t_sqrt(o.reyn);
   o.cschm = t_cbrt(schm);
-  o.ire = (T)1. / ((T)60. + o.reyn);
+  o.ire = ddiv((T)1., (T)60. + o.reyn);
 }
 
 // ((m+w)^3 - (m^2+w^2)^(3/2)) / (3 m w) - m without cancellation (float form of :305-313):
@@ -313,8 +314,8 @@ __device__ T coag_pair(const CoagCell<T> &cc, const BinProps<T> &a, const BinPro
   if (!is_f32<T>::value) {
     T m2 = sq(mdiam);
     T oa2 = m2 + sq(a.omega), ob2 = m2 + sq(b.omega);
-    tva1 = (cube(mdiam + a.omega) - oa2 * t_sqrt(oa2)) / ((T)3. * mdiam * a.omega) - mdiam;
-    tva2 = (cube(mdiam + b.omega) - ob2 * t_sqrt(ob2)) / ((T)3. * mdiam * b.omega) - mdiam;
+    tva1 = ddiv(cube(mdiam + a.omega) - oa2 * t_sqrt(oa2), (T)3. * mdiam * a.omega) - mdiam;
+    tva2 = ddiv(cube(mdiam + b.omega) - ob2 * t_sqrt(ob2), (T)3. * mdiam * b.omega) - mdiam;
   } else {
     tva1 = flux_match_stable(mdiam, a.omega);
     tva2 = flux_match_stable(mdiam, b.omega);
@@ -324,26 +325,26 @@ __device__ T coag_pair(const CoagCell<T> &cc, const BinProps<T> &a, const BinPro
   const BinProps<T> &L = first_large ? a : b;
   const BinProps<T> &S = first_large ? b : a;
   T dv = fabs(a.termv - b.termv);
-  T stok = (T)2. * S.termv * dv / (L.diam * (T)K_GRAV);
+  T stok = ddiv((T)2. * S.termv * dv, L.diam * (T)K_GRAV);
   // flux1 / (mdiam/(mdiam+fmdist) + flux1/flux2) as one quotient in FP64; the float form
   // keeps the reference's shape (the products would leave float's range)
   T zbrown;
   if (!is_f32<T>::value) {
     const T mf = mdiam + fmdist;
-    zbrown = flux1 * flux2 * mf / (mdiam * flux2 + flux1 * mf);
+    zbrown = ddiv(flux1 * flux2 * mf, mdiam * flux2 + flux1 * mf);
   } else {
-    zbrown = flux1 / (mdiam / (mdiam + fmdist) + flux1 / flux2);
+    zbrown = ddiv(flux1, ddiv(mdiam, mdiam + fmdist) + ddiv(flux1, flux2));
   }
   // Re <= 1: (Re Sc)^(1/3), else Re^(1/2) Sc^(1/3), from the per-bin factors
   const T zbrconv = (T)0.45 * zbrown * L.fre * S.cschm;
   T hd = (T)0.5 * (a.diam + b.diam);
   T ztshear = cc.shearA * cube(hd);
   T zturb = cc.turbB * sq(hd) * dv;
-  T zea = sq(stok) / sq(stok + (T)0.5);
+  T zea = ddiv(sq(stok), sq(stok + (T)0.5));
   T zev = 0;
   if (stok > (T)1.214) {
-    zev = (T)0.75 * t_log((T)2. * stok) / (stok - (T)1.214);
-    zev = (T)1. / sq((T)1. + zev);
+    zev = ddiv((T)0.75 * t_log((T)2. * stok), stok - (T)1.214);
+    zev = ddiv((T)1., sq((T)1. + zev));
   }
   T zecoll = ((T)60. * zev + zea * L.reyn) * L.ire;
   T zgrav = zecoll * (T)K_PI * sq(mdiam);
@@ -423,7 +424,7 @@ __device__ void eval_pairs(const DevParams &P, const WS<KT> &w, const CoagCell<K
     if (P.lcharge) {
       // charging enhancement (:411-416)
       double kd = (double)k;
-      kd = kd + kd * P.chargeCollEnh * 0.5 * (w.ctime[i] + w.ctime[j]) / P.chargeTimeMax;
+      kd = kd + ddiv(kd * P.chargeCollEnh * 0.5 * (w.ctime[i] + w.ctime[j]), P.chargeTimeMax);
       k = (KT)kd;
     }
     w.K[tri(i, j, NB)] = k;
@@ -442,13 +443,13 @@ __device__ void build_kernels(const DevParams &P, const WS<KT> &w, const double 
   const int NB = w.NB;
   CoagCell<double> cd;
   {
-    double visc = (7.44523e-3 * sqrt(cube(T))) / (5093. * (T + 110.4));
-    double mfp = (1.656e-10 * T + 1.828e-8) * K_PSTAND / pres;
-    double zrhoa = pres / (K_RD * T);
-    double vkin = visc / zrhoa;
+    double visc = ddiv(7.44523e-3 * dsqrt(cube(T)), 5093. * (T + 110.4));
+    double mfp = ddiv((1.656e-10 * T + 1.828e-8) * K_PSTAND, pres);
+    double zrhoa = ddiv(pres, K_RD * T);
+    double vkin = ddiv(visc, zrhoa);
     cd.T_ = T; cd.visc = visc; cd.mfp = mfp; cd.zrhoa = zrhoa; cd.vkin = vkin;
-    cd.shearA = sqrt(8. * K_PI * P.eddy_dis / (15. * vkin));
-    cd.turbB = K_PI * pow(P.eddy_dis, 0.75) / (K_GRAV * sqrt(sqrt(vkin)));
+    cd.shearA = dsqrt(ddiv(8. * K_PI * P.eddy_dis, 15. * vkin));
+    cd.turbB = ddiv(K_PI * dpow(P.eddy_dis, 0.75), K_GRAV * dsqrt(dsqrt(vkin)));
   }
   CoagCell<KT> cc;
   cc.T_ = (KT)cd.T_; cc.visc = (KT)cd.visc; cc.mfp = (KT)cd.mfp; cc.zrhoa = (KT)cd.zrhoa; cc.vkin = (KT)cd.vkin;
@@ -871,7 +872,7 @@ __device__ void sip_cap_sink(const DevParams &P, const double *numc, const doubl
   double ssk = 0., sv = 0.;
   for (int s = 0; s < nspec; s++) { ssk += sinkv[s]; sv += volc[s * NB + g]; }
   if (ssk > sv) {
-    const double frconst = 0.99 * sv / ssk;
+    const double frconst = ddiv(0.99 * sv, ssk);
     for (int s = 0; s < nspec; s++) sinkv[s] = sinkv[s] * frconst;
     sinkn = sinkn * frconst;
     sinkn = fmin(sinkn, 0.99 * numc[g]);
@@ -912,7 +913,7 @@ __device__ void sip_bin_geometry(const DevParams &P, const double *tb, SipScr &q
   const int I0 = P.nliquid;
   for (int bb = 0; bb < P.nice; bb++) {
     q.diams[bb] = tb[TAB_DMID * P.nb_pad + I0 + bb];
-    q.bw[bb] = pow(tb[TAB_VHI * P.nb_pad + I0 + bb] / K_PI6, 1. / 3) - pow(tb[TAB_VLO * P.nb_pad + I0 + bb] / K_PI6, 1. / 3);
+    q.bw[bb] = dpow(divc(tb[TAB_VHI * P.nb_pad + I0 + bb], K_PI6), 1. / 3) - dpow(divc(tb[TAB_VLO * P.nb_pad + I0 + bb], K_PI6), 1. / 3);
   }
 }
 // Fragments dN spread over the ice bins 0..npmax-1 as d^-3 in number (DF :131-146, IIBR
@@ -923,9 +924,9 @@ __device__ double sip_spread(const DevParams &P, const double *volc, int NB, int
   const int nspec = P.nused;
   for (int k = 0; k < P.nice; k++) q.dNb[k] = q.dVb[k] = 0.;
   double Nnorm = 0.;
-  for (int k = 0; k < npmax; k++) q.dNb[k] = 1. / cube(q.diams[k]);
+  for (int k = 0; k < npmax; k++) q.dNb[k] = drcp(cube(q.diams[k]));
   for (int k = 0; k < npmax; k++) Nnorm += q.dNb[k] * q.bw[k];
-  for (int k = 0; k < npmax; k++) q.dNb[k] = dN * q.dNb[k] * q.bw[k] / Nnorm;
+  for (int k = 0; k < npmax; k++) q.dNb[k] = ddiv(dN * q.dNb[k] * q.bw[k], Nnorm);
   for (int k = 0; k < npmax; k++) q.dVb[k] = q.dNb[k] * K_PI6 * cube(q.diams[k]);
   double sdv = 0.;
   sv = 0.;
@@ -934,7 +935,7 @@ __device__ double sip_spread(const DevParams &P, const double *volc, int NB, int
   for (int k = 0; k < npmax; k++) {
     q.fragn_loc[k] = q.fragn_loc[k] + q.dNb[k];
     for (int s = 0; s < nspec; s++)
-      q.fragv_loc[k * SALSA_NSV + s] = q.fragv_loc[k * SALSA_NSV + s] + volc[s * NB + g] * (q.dVb[k] / sv);
+      q.fragv_loc[k * SALSA_NSV + s] = q.fragv_loc[k * SALSA_NSV + s] + volc[s * NB + g] * (ddiv(q.dVb[k], sv));
   }
   return sdv;
 }
@@ -971,14 +972,14 @@ __device__ void sip_rimesplintering(const DevParams &P, const WS<KT> &w, double 
       const double nf = t.nrs[cc * nice + bb], mf = t.mrs[cc * nice + bb];
       if (T < 238.15 || T > 273.15 || nf < 1.e-12 || vall < 1.e-15 || w.numc[g] < K_PRLIM || bb + 1 < splbin + 2)
         continue;
-      const double ddmean = pow(mf / nf / K_RHOWA / K_PI6, 1. / 3.);
+      const double ddmean = dpow(divc(divc(ddiv(mf, nf), K_RHOWA), K_PI6), 1. / 3.);
       if (ddmean < SIP_DLLIQ_RS) continue;
       const double dN = P.sip_rs_mode == 1 ? 3.5E8 * mf : 4.0E-3 * nf;
       const double dV = dN * v_i;
       q.fragn[splbin - 1] = q.fragn[splbin - 1] + dN;
       double sv = 0.;
       for (int s = 0; s < nspec; s++) sv += w.v(s, g);
-      const double f = fmin(dV / sv, 1.);
+      const double f = fmin(ddiv(dV, sv), 1.);
       double ss = 0.;
       for (int s = 0; s < nspec; s++) {
         q.fragv[(splbin - 1) * SALSA_NSV + s] = q.fragv[(splbin - 1) * SALSA_NSV + s] + w.v(s, g) * f;
@@ -986,9 +987,9 @@ __device__ void sip_rimesplintering(const DevParams &P, const WS<KT> &w, double 
         sinkv[s] = sinkv[s] + sk;
         ss += sk;
       }
-      q.sinkn[bb] = q.sinkn[bb] + ss / (K_PI6 * pow(ddmean, 3.0));
+      q.sinkn[bb] = q.sinkn[bb] + ddiv(ss, K_PI6 * dpow(ddmean, 3.0));
       t.tr[nice + splbin - 1] = t.tr[nice + splbin - 1] + dN;   // :134-136
-      t.rate[1] += dN / dt;
+      t.rate[1] += ddiv(dN, dt);
     }
     sip_cap_sink(P, w.numc, w.volc, NB, g, q.sinkn[bb], sinkv);
   }
@@ -998,21 +999,21 @@ __device__ void sip_rimesplintering(const DevParams &P, const WS<KT> &w, double 
 // mo_salsa_SIP_DF.f90:370-398 fragments per frozen drop: Lawson (mode 1), Sullivan
 // (mode 2), Phillips' simple form (mode 3)
 __device__ double sip_df_fragments(int mode, double T, double nf, double ddmean) {
-  if (mode == 1) return nf * 2.5e-11 * pow(fmin(ddmean, 3.e-3) * 1.e6, 4.);
+  if (mode == 1) return nf * 2.5e-11 * dpow(fmin(ddmean, 3.e-3) * 1.e6, 4.);
   if (mode == 2) {
     // f_gauss(T, 10, 258) / f_gauss(258, 10, 258)
     const double a = sqrt(2. * K_PI_FULL) * 10.;
     double b = (T - 258.) * (T - 258.);
-    b = b / (10. * 10.);
-    const double hT = ((1. / a) * exp(-0.5 * b)) / ((1. / a) * exp(-0.5 * 0.));
-    return nf * 0.2 * hT * 2.5e-11 * pow(fmin(ddmean, 3.e-3) * 1.e6, 4.);
+    b = divc(b, 10. * 10.);
+    const double hT = ((1. / a) * dexp(-0.5 * b)) / ((1. / a) * exp(-0.5 * 0.));
+    return nf * 0.2 * hT * 2.5e-11 * dpow(fmin(ddmean, 3.e-3) * 1.e6, 4.);
   }
   const double t0 = -24. + 273.15, t1 = -20. + 273.15, t2 = -16. + 273.15, t3 = -10. + 273.15, t4 = -6. + 273.15;
   double hT = 0.;
-  if (T >= t0 && T < t1) hT = (0.24 - 0.6) * ((T - t0) / 4.) + 0.6;
-  else if (T >= t1 && T < t2) hT = (2.6 - 0.24) * ((T - t2) / 4.) + 2.6;
-  else if (T >= t2 && T < t3) hT = (0.43 - 2.6) * ((T - t3) / 6.) + 0.43;
-  else if (T >= t3 && T < t4) hT = (0.35 - 0.43) * ((T - t4) / 4.) + 0.35;
+  if (T >= t0 && T < t1) hT = (0.24 - 0.6) * (divc(T - t0, 4.)) + 0.6;
+  else if (T >= t1 && T < t2) hT = (2.6 - 0.24) * (divc(T - t2, 4.)) + 2.6;
+  else if (T >= t2 && T < t3) hT = (0.43 - 2.6) * (divc(T - t3, 6.)) + 0.43;
+  else if (T >= t3 && T < t4) hT = (0.35 - 0.43) * (divc(T - t4, 4.)) + 0.35;
   return nf * ((4. / 9.) * 1.e4 * hT * ddmean);
 }
 
@@ -1026,34 +1027,34 @@ __device__ __forceinline__ double sip_ph_cubic(double x, double c1, double c2, d
 __device__ double sip_df_phillips_mode1(double d, double T) {
   const double tc = T - 273.15, x = log10(fmax(fmin(d * 1.e3, 1.6), 0.06));
   const double T0 = sip_ph_cubic(x, -1.3999, -5.3285, -3.9847, -15.0332);
-  const double zeta = pow(10., sip_ph_cubic(x, 2.4268, 3.3274, 2.0783, 1.2927));
-  const double eta = pow(10., sip_ph_cubic(x, 0.1242, -0.2316, -0.9874, -0.0827));
+  const double zeta = dpow(10., sip_ph_cubic(x, 2.4268, 3.3274, 2.0783, 1.2927));
+  const double eta = dpow(10., sip_ph_cubic(x, 0.1242, -0.2316, -0.9874, -0.0827));
   double beta = 0.;
   if (!(d < 0.4e-3)) {
     const double xb = log10(fmin(d * 1.e3, 1.6));
     beta = (-0.1839 * sq(xb)) + (-0.2017 * xb) + -0.0512;
   }
-  return beta * tc + (zeta * sq(eta)) / (sq(tc - T0) + sq(eta));
+  return beta * tc + ddiv(zeta * sq(eta), sq(tc - T0) + sq(eta));
 }
 // :479-532 the crystal heavier than the drop (eq. 7): the collision's kinetic energy over
 // the drop's surface energy
 __device__ double sip_df_phillips_mode2(const DevParams &P, double p, double T, double d, double disph, double dinsph,
                                         double mrim, double mpri, double ncice, double rhoip) {
-  const double rhoa = p / (K_RD * T);
-  const double visc = (7.44523e-3 * sqrt(cube(T))) / (5093. * (T + 110.4));
-  const double mfp = (1.656e-10 * T + 1.828e-8) * K_PSTAND / p;
-  double knud = 2. * mfp / dinsph;
-  double beta = 1. + knud * (1.142 + 0.558 * exp(-0.999 / knud));
+  const double rhoa = ddiv(p, K_RD * T);
+  const double visc = ddiv(7.44523e-3 * dsqrt(cube(T)), 5093. * (T + 110.4));
+  const double mfp = ddiv((1.656e-10 * T + 1.828e-8) * K_PSTAND, p);
+  double knud = ddiv(2. * mfp, dinsph);
+  double beta = 1. + knud * (1.142 + 0.558 * dexp(-ddiv(0.999, knud)));
   Shape<double> ish;
   shape_coeffs<double>(P, ish, mpri, mrim, ncice);
   const double vti = terminal_vel<double>(disph, rhoip, rhoa, visc, beta, 4, ish, dinsph);
-  knud = 2. * mfp / d;
-  beta = 1. + knud * (1.142 + 0.558 * exp(-0.999 / knud));
+  knud = ddiv(2. * mfp, d);
+  beta = 1. + knud * (1.142 + 0.558 * dexp(-ddiv(0.999, knud)));
   const double vtd = terminal_vel<double>(d, K_RHOWA, rhoa, visc, beta, 3, ish, d);
-  const double mip = (mrim + mpri) / ncice, mdp = K_RHOWA * K_PI6 * cube(d);
-  const double K0 = 0.5 * (mip * mdp / (mdp + mip)) * sq(vtd - vti);
-  const double DE = K0 / (K_SURFW0 * K_PI * sq(d));
-  const double fT = -4200. * (T - 273.15) / 3.3e5;   // cwa, alf (mo_submctl.f90:268, 281)
+  const double mip = ddiv(mrim + mpri, ncice), mdp = K_RHOWA * K_PI6 * cube(d);
+  const double K0 = 0.5 * (ddiv(mip * mdp, mdp + mip)) * sq(vtd - vti);
+  const double DE = ddiv(K0, K_SURFW0 * K_PI * sq(d));
+  const double fT = -divc(4200. * (T - 273.15), 3.3e5);   // cwa, alf (mo_submctl.f90:268, 281)
   return 3. * fmin(4. * fT, 1.) * (1. - fT) * fmax(DE - 0.2, 0.);
 }
 // :313-372 the regime by the masses of drop and crystal (ice bin g)
@@ -1063,13 +1064,13 @@ __device__ double sip_df_phillips_full(const DevParams &P, const WS<KT> &w, doub
   double sv = 0.;
   for (int s = 0; s < P.nused - 1; s++) sv += w.v(s, g);
   const double mrim = w.v(P.nused - 1, g) * K_RHORI, mpri = sv * K_RHOIC, ncice = w.numc[g];
-  const double mip = (mrim + mpri) / ncice, mdp = K_RHOWA * K_PI6 * cube(d);
+  const double mip = ddiv(mrim + mpri, ncice), mdp = K_RHOWA * K_PI6 * cube(d);
   if (mdp > mip) {
     if (d < 50.e-6 && T > 267.15) return 0.;
     return fmin(sip_df_phillips_mode1(d, T), 100.) * nf;
   }
   if (d < 150.e-6) return 0.;
-  const double rhoip = (mrim * K_RHORI + mpri * K_RHOIC) / (mrim + mpri);
+  const double rhoip = ddiv(mrim * K_RHORI + mpri * K_RHOIC, mrim + mpri);
   return fmin(sip_df_phillips_mode2(P, p, T, d, w.dwet[g], w.dnsp[g], mrim, mpri, ncice, rhoip), 100.) * nf;
 }
 
@@ -1092,7 +1093,7 @@ __device__ void sip_dropfracturing(const DevParams &P, const WS<KT> &w, const do
     for (int cc = 0; cc < nprc; cc++) {
       const double nf = t.ndf[cc * nice + bb], mf = t.mdf[cc * nice + bb];
       if (T < 248.15 || T > 271.15 || nf < 1.e-12 || vall < 1.e-15 || w.numc[g] < K_PRLIM) continue;
-      const double ddmean = pow(mf / nf / K_RHOWA / K_PI6, 1. / 3.);
+      const double ddmean = dpow(divc(divc(ddiv(mf, nf), K_RHOWA), K_PI6), 1. / 3.);
       if (ddmean < SIP_DLLIQ_DF) continue;
       int npmax = 0;
       for (int k = 0; k < nice; k++) npmax += q.diams[k] <= ddmean;
@@ -1104,15 +1105,15 @@ __device__ void sip_dropfracturing(const DevParams &P, const WS<KT> &w, const do
       const double sdv = sip_spread(P, w.volc, NB, g, dN, npmax, q, sv);
       double ss = 0.;
       for (int s = 0; s < nspec; s++) {
-        const double sk = w.v(s, g) * sdv / sv;
+        const double sk = ddiv(w.v(s, g) * sdv, sv);
         sinkv[s] = sinkv[s] + sk;
         ss += sk;
       }
-      q.sinkn[bb] = q.sinkn[bb] + ss / (mf / nf / K_RHOWA);
+      q.sinkn[bb] = q.sinkn[bb] + ddiv(ss, divc(ddiv(mf, nf), K_RHOWA));
       double sdn = 0.;                                           // :165-167
       for (int k = 0; k < npmax; k++) t.tr[k] = t.tr[k] + q.dNb[k];
       for (int k = 0; k < nice; k++) sdn += q.dNb[k];
-      t.rate[0] += sdn / dt;
+      t.rate[0] += ddiv(sdn, dt);
     }
     sip_fold_local(P, q);
     sip_cap_sink(P, w.numc, w.volc, NB, g, q.sinkn[bb], sinkv);
@@ -1125,8 +1126,8 @@ __device__ void sip_dropfracturing(const DevParams &P, const WS<KT> &w, const do
 __device__ double sip_iibr_imf(int mode, double T, double dmin) {
   const double fbr = 280., Tmin = 252., D0 = 0.02;
   double imf;
-  if (mode == 1) imf = T < Tmin ? 0. : fmax(0., fbr * pow(T - Tmin, 1.2) * exp(-(T - Tmin) / 5.));
-  else imf = T <= Tmin ? 0. : fmax(0., fbr * pow(T - Tmin, 1.2) * exp(-(T - Tmin) / 5.) * dmin / D0);
+  if (mode == 1) imf = T < Tmin ? 0. : fmax(0., fbr * dpow(T - Tmin, 1.2) * dexp(-divc(T - Tmin, 5.)));
+  else imf = T <= Tmin ? 0. : fmax(0., divc(fbr * dpow(T - Tmin, 1.2) * dexp(-divc(T - Tmin, 5.)) * dmin, D0));
   return fmin(imf, 100.0);
 }
 
@@ -1143,11 +1144,11 @@ __device__ __forceinline__ void sip_iibr_masses(const DevParams &P, const WS<KT>
 }
 template <typename KT>
 __device__ double sip_iibr_velocity(const DevParams &P, const WS<KT> &w, int g, double visc, double rhoa, double mfp) {
-  const double knud = 2. * mfp / w.dnsp[g];
-  const double beta = 1. + knud * (1.142 + 0.558 * exp(-0.999 / knud));
+  const double knud = ddiv(2. * mfp, w.dnsp[g]);
+  const double beta = 1. + knud * (1.142 + 0.558 * dexp(-ddiv(0.999, knud)));
   double mrim, mpri;
   sip_iibr_masses(P, w, g, mrim, mpri);
-  const double rhoip = (mrim * K_RHORI + mpri * K_RHOIC) / (mrim + mpri);
+  const double rhoip = ddiv(mrim * K_RHORI + mpri * K_RHOIC, mrim + mpri);
   Shape<double> sh;
   shape_coeffs<double>(P, sh, mpri, mrim, w.numc[g]);
   return terminal_vel<double>(w.dwet[g], rhoip, rhoa, visc, beta, 4, sh, w.dnsp[g]);
@@ -1162,11 +1163,11 @@ __device__ double sip_imf_phillips(const DevParams &P, const WS<KT> &w, double p
   const double T0 = 258.15;
   double mrim, mpri;
   sip_iibr_masses(P, w, small, mrim, mpri);
-  const double rimfrac = mrim / (mrim + mpri);
+  const double rimfrac = ddiv(mrim, mrim + mpri);
   double a0, C, gg, Nmax;
   if (rimfrac > 0.5) {
-    a0 = exp(14.74 * ssi + 14.28);
-    C = exp(20.15 * ssi + 13.78);
+    a0 = dexp(14.74 * ssi + 14.28);
+    C = dexp(20.15 * ssi + 13.78);
     gg = ssi + 0.55;
     Nmax = 600.;
   } else {
@@ -1175,19 +1176,19 @@ __device__ double sip_imf_phillips(const DevParams &P, const WS<KT> &w, double p
     gg = 0.78;
     Nmax = 500.;
   }
-  const double Am = a0 / 3. + fmax(2. / 3. * a0 - 1. / 9. * a0 * fabs(T - T0), 0.);
+  const double Am = divc(a0, 3.) + fmax(2. / 3. * a0 - 1. / 9. * a0 * fabs(T - T0), 0.);
   const double alpha = K_PI * sq(disphmin);
-  const double rhoa = p / (K_RD * T);
-  const double visc = (7.44523e-3 * sqrt(cube(T))) / (5093. * (T + 110.4));
-  const double mfp = (1.656e-10 * T + 1.828e-8) * K_PSTAND / p;
+  const double rhoa = ddiv(p, K_RD * T);
+  const double visc = ddiv(7.44523e-3 * dsqrt(cube(T)), 5093. * (T + 110.4));
+  const double mfp = ddiv((1.656e-10 * T + 1.828e-8) * K_PSTAND, p);
   const double v1 = sip_iibr_velocity(P, w, large, visc, rhoa, mfp);
   double mr1, mp1;
   sip_iibr_masses(P, w, large, mr1, mp1);
-  const double m1 = (mr1 + mp1) / w.numc[large];
+  const double m1 = ddiv(mr1 + mp1, w.numc[large]);
   const double v2 = sip_iibr_velocity(P, w, small, visc, rhoa, mfp);
-  const double m2 = (mrim + mpri) / w.numc[small];
-  const double K0 = (m1 * m2 / (m1 + m2)) * (1.7 * sq(v1 - v2) + 0.3 * v1 * v2);
-  return fmin(alpha * Am * (1 - exp(-pow(C * K0 / alpha / Am, gg))), Nmax);
+  const double m2 = ddiv(mrim + mpri, w.numc[small]);
+  const double K0 = (ddiv(m1 * m2, m1 + m2)) * (1.7 * sq(v1 - v2) + 0.3 * v1 * v2);
+  return fmin(alpha * Am * (1 - dexp(-dpow(ddiv(ddiv(C * K0, alpha), Am), gg))), Nmax);
 }
 
 template <typename KT>
@@ -1214,16 +1215,16 @@ __device__ void sip_iceicecollbreak(const DevParams &P, const WS<KT> &w, const d
           vc < 1.e-15 || w.numc[h] < K_PRLIM)
         continue;
       updateDiameterAll(P, nullptr, w.numc, w.volc, w.dwet, w.ddry, w.dins, w.dnsp, dmid, NB, g);
-      const double v_i = mii / nii / w.rhomean[g];
-      const double dinsphmin = pow(v_i / K_PI6, 1. / 3.);
+      const double v_i = ddiv(ddiv(mii, nii), w.rhomean[g]);
+      const double dinsphmin = dpow(divc(v_i, K_PI6), 1. / 3.);
       int npmax = 0;
       for (int k = 0; k < nice; k++) npmax += q.diams[k] <= dinsphmin;
       npmax = npmax - 1;
       if (npmax <= 2) continue;
       double dN;
       if (P.sip_ib_mode == 3) {   // :148-155: bb passes as the larger crystal, as the reference writes it
-        const double disphmin = pow((mii / nii / w.rhomean[g]) / K_PI6, 1. / 3.);
-        const double ssi = fmax(0., rv / rsi - 1.0);
+        const double disphmin = dpow(divc(ddiv(ddiv(mii, nii), w.rhomean[g]), K_PI6), 1. / 3.);
+        const double ssi = fmax(0., ddiv(rv, rsi) - 1.0);
         dN = fmin(sip_imf_phillips<KT>(P, w, pres, T, g, h, disphmin, ssi), 600.0) * nii;
       } else {
         dN = sip_iibr_imf(P.sip_ib_mode, T, dinsphmin) * nii;
@@ -1232,15 +1233,15 @@ __device__ void sip_iceicecollbreak(const DevParams &P, const WS<KT> &w, const d
       const double sdv = sip_spread(P, w.volc, NB, g, dN, npmax, q, sv);
       double ss = 0.;
       for (int s = 0; s < nspec; s++) {
-        const double sk = w.v(s, g) * sdv / sv;
+        const double sk = ddiv(w.v(s, g) * sdv, sv);
         sinkv[s] = sinkv[s] + sk;
         ss += sk;
       }
-      q.sinkn[bb] = q.sinkn[bb] + ss / v_i;
+      q.sinkn[bb] = q.sinkn[bb] + ddiv(ss, v_i);
       double sdn = 0.;                                           // :187-189
       for (int k = 0; k < npmax; k++) t.tr[2 * nice + k] = t.tr[2 * nice + k] + q.dNb[k];
       for (int k = 0; k < nice; k++) sdn += q.dNb[k];
-      t.rate[2] += sdn / dt;
+      t.rate[2] += ddiv(sdn, dt);
     }
     sip_fold_local(P, q);
     sip_cap_sink(P, w.numc, w.volc, NB, g, q.sinkn[bb], sinkv);
@@ -1316,7 +1317,7 @@ __device__ __forceinline__ void apply_coag(const DevParams &P, const WS<KT> &w, 
   const bool vol = lane < nspec;
   const double num = vol ? w.v(lane, t) + dt * my * n : n;
   const double den = vol ? 1. + dt * sink : 1. + dt * (sink + self);
-  const double q = num / den;
+  const double q = ddiv(num, den);
   __syncwarp();
   if (vol) w.v(lane, t) = q;
   else if (lane == nspec) w.numc[t] = q;
@@ -1357,7 +1358,7 @@ __device__ void precip_formation(const DevParams &P, const WS<KT> &w, const doub
     if (lane < np) {
       int ll = c0 + lane, lg = C0 + ll;
       double dt3 = cube(w.dwet[tg]) + cube(w.dwet[lg]);
-      double D_new = cbrt(dt3);
+      double D_new = dcbrt(dt3);
       int cnt = 0;
       for (int i = 0; i < nprc; i++) cnt += (D_new > pbins[i]);
       double klt = (double)kget(w, lg, tg);
@@ -1450,7 +1451,7 @@ __device__ void coag_cloud(const DevParams &P, const WS<KT> &w, const double *tb
       if (P.lscgcc) {
         if (autoc1) {
           double n = w.numc[tg];
-          double fix = fmax(1. - dt * (0.5 * (double)kget(w, tg, tg) * (n * n) / n), 0.1);
+          double fix = fmax(1. - dt * (ddiv(0.5 * (double)kget(w, tg, tg) * (n * n), n)), 0.1);
           precip_formation(P, w, tb, kk, kk, kk, fix, true, a, diag, lane);
         } else if (lane == 0) {
           a.self += (KT)0.5 * kget(w, tg, tg) * w.nk(tg);
@@ -1517,10 +1518,10 @@ __device__ void coag_cloud(const DevParams &P, const WS<KT> &w, const double *tb
         for (int cc = lane; cc < nprc; cc += 32) {
           int g = P0 + cc;
           double nrate = num_prc[cc];
-          double inf = nrate > 0. ? inf_num[cc] / nrate : 0.;
+          double inf = nrate > 0. ? ddiv(inf_num[cc], nrate) : 0.;
           double n = w.numc[g] + dt * nrate;
           w.numc[g] = n;
-          if (n > K_PRLIM) w.indef[g] = (w.indef[g] * (n - dt * nrate) + inf * dt * nrate) / n;
+          if (n > K_PRLIM) w.indef[g] = ddiv(w.indef[g] * (n - dt * nrate) + inf * dt * nrate, n);
         }
         __syncwarp();
         shadow_bin<KT>(P, w, tg, lane);
@@ -1681,7 +1682,7 @@ __device__ void coag_ice(const DevParams &P, const WS<KT> &w, const double *tb, 
           for (int s = 0; s < SALSA_NSV; s++)
             if (s < ndry) a.src[s] += k * w.vk(s, ll);
         }
-        a.add_at(iwa, k * w.vk(iwa, ll) * (KT)K_RHOWA / (KT)K_RHOIC);
+        a.add_at(iwa, divc(k * w.vk(iwa, ll) * (KT)K_RHOWA, (KT)K_RHOIC));
       }
     if (P.lscgic)
       for (int ll = lane; ll < P.ncld; ll += 32) {
@@ -1692,7 +1693,7 @@ __device__ void coag_ice(const DevParams &P, const WS<KT> &w, const double *tb, 
           for (int s = 0; s < SALSA_NSV; s++)
             if (s < ndry) a.src[s] += k * w.vk(s, g);
         }
-        a.add_at(irim, k * w.vk(iwa, g) * (KT)K_RHOWA / (KT)K_RHORI);
+        a.add_at(irim, divc(k * w.vk(iwa, g) * (KT)K_RHOWA, (KT)K_RHORI));
       }
     if (P.lscgip)
       for (int ll = lane; ll < P.nprc; ll += 32) {
@@ -1703,7 +1704,7 @@ __device__ void coag_ice(const DevParams &P, const WS<KT> &w, const double *tb, 
           for (int s = 0; s < SALSA_NSV; s++)
             if (s < ndry) a.src[s] += k * w.vk(s, g);
         }
-        a.add_at(irim, k * w.vk(iwa, g) * (KT)K_RHOWA / (KT)K_RHORI);
+        a.add_at(irim, divc(k * w.vk(iwa, g) * (KT)K_RHOWA, (KT)K_RHORI));
       }
     // accumulateSourceIce (:1385-1427)
     if (P.lscgii && kk > 0)
@@ -1727,7 +1728,7 @@ __device__ void coag_ice(const DevParams &P, const WS<KT> &w, const double *tb, 
 }
 
 template <typename KT, bool SIP>
-__device__ void coagulation(const DevParams &P, const WS<KT> &w, const double *tb, double dt, double T, double pres,
+__device__ __forceinline__ void coagulation(const DevParams &P, const WS<KT> &w, const double *tb, double dt, double T, double pres,
                             bool diag, long long cell, int lane) {
   const double *dmid = tb + TAB_DMID * P.nb_pad;
   // updateDiameter("all") on every bin (:146-152) and rhomean of the kernel categories
@@ -1799,27 +1800,27 @@ __device__ double equil_iterate(const DevParams &P, const WS<KT> &w, int b, doub
   double numc = w.numc[b];
   double zv0 = zvolc_of(P, w, 0, b), zv1 = zvolc_of(P, w, 1, b), zv4 = zvolc_of(P, w, 4, b);
   double zvp[7];
-  for (int i = 0; i < 7; i++) zvp[i] = zvolc_of(P, w, i, b) / numc;
+  for (int i = 0; i < 7; i++) zvp[i] = ddiv(zvolc_of(P, w, i, b), numc);
   double zcore = regime2 ? (zvp[0] + zvp[1] + zvp[2] + zvp[3] + zvp[4]) : (zvp[0] + zvp[1]);
   double zdwet = w.dwet[b];
   double zdold = 1.;
   double zlwc = 0.;
   int count = 0;
   const double rhosu_msu = 1830. / 98.08e-3, rhooc_moc = 1400. / 150.e-3, rhoss_mss = 2165. / 58.44e-3;
-  while (fabs(zdwet / zdold - 1.) > tol) {
+  while (fabs(ddiv(zdwet, zdold) - 1.) > tol) {
     zdold = fmax(zdwet, 1.e-20);
-    double zaw = zrh / zke;
+    double zaw = ddiv(zrh, zke);
     double a2 = zaw * zaw, a3 = a2 * zaw, a4 = a2 * a2;
     double bm1 = +1.1065495e+2 - 3.6759197e+2 * zaw + 5.0462934e+2 * a2 - 3.1543839e+2 * a3 + 6.770824e+1 * a4;
-    double bm2 = 1. / (zaw * K_MWA) - 1. / K_MWA;
+    double bm2 = drcp(zaw * K_MWA) - 1. / K_MWA;
     // nitric acid molality only multiplies a zero NO volume (NO not copied, :148) -> its term is zero
-    zlwc = (zv0 * rhosu_msu) / bm1 + K_EPSOC * zv1 * rhooc_moc / bm2;
+    zlwc = ddiv(zv0 * rhosu_msu, bm1) + ddiv(K_EPSOC * zv1 * rhooc_moc, bm2);
     if (regime2) {
       double bm5 = +5.875248e+1 - 1.8781997e+2 * zaw + 2.7211377e+2 * a2 - 1.8458287e+2 * a3 + 4.153689e+1 * a4;
-      zlwc += (zv4 * rhoss_mss) / bm5;
+      zlwc += ddiv(zv4 * rhoss_mss, bm5);
     }
-    zdwet = cbrt(zlwc / numc / K_RHOWA / K_PI6 + (zvp[5] + zvp[6]) / K_PI6 + zcore / K_PI6);
-    zke = exp(2. * K_SURFW0 * K_MVWA / (K_BOLTZ * T * zdwet));
+    zdwet = dcbrt(divc(divc(ddiv(zlwc, numc), K_RHOWA), K_PI6) + divc(zvp[5] + zvp[6], K_PI6) + divc(zcore, K_PI6));
+    zke = dexp(ddiv(2. * K_SURFW0 * K_MVWA, K_BOLTZ * T * zdwet));
     count++;
     if (count > 100) { nonconv = 1; break; }
   }
@@ -1846,7 +1847,7 @@ __device__ __forceinline__ void eq_load(const DevParams &P, const WS<KT> &w, int
   j.numc = w.numc[b];
   j.zv0 = zvolc_of(P, w, 0, b); j.zv1 = zvolc_of(P, w, 1, b); j.zv4 = zvolc_of(P, w, 4, b);
   double zvp[7];
-  for (int i = 0; i < 7; i++) zvp[i] = zvolc_of(P, w, i, b) / j.numc;
+  for (int i = 0; i < 7; i++) zvp[i] = ddiv(zvolc_of(P, w, i, b), j.numc);
   j.zcore = j.r2 ? (zvp[0] + zvp[1] + zvp[2] + zvp[3] + zvp[4]) : (zvp[0] + zvp[1]);
   j.zvp56 = zvp[5] + zvp[6];
   {
@@ -1854,9 +1855,9 @@ __device__ __forceinline__ void eq_load(const DevParams &P, const WS<KT> &w, int
     j.q0 = j.zv0 * rhosu_msu;
     j.q1 = K_EPSOC * j.zv1 * rhooc_moc;
     j.q4 = j.zv4 * rhoss_mss;
-    j.p56 = j.zvp56 / K_PI6;
-    j.pc = j.zcore / K_PI6;
-    j.rinv = 1. / (j.numc * (K_RHOWA * K_PI6));   // zlwc / numc / rhowa / pi6 as one product
+    j.p56 = divc(j.zvp56, K_PI6);
+    j.pc = divc(j.zcore, K_PI6);
+    j.rinv = drcp(j.numc * (K_RHOWA * K_PI6));   // zlwc / numc / rhowa / pi6 as one product
   }
   j.zdwet = w.dwet[b];
   j.zdold = 1.;
@@ -1873,17 +1874,17 @@ __device__ __forceinline__ void eq_step(EqJob &j, double ckt) {
   double zaw = j.zrh * j.izke;
   double a2 = zaw * zaw, a3 = a2 * zaw, a4 = a2 * a2;
   double bm1 = +1.1065495e+2 - 3.6759197e+2 * zaw + 5.0462934e+2 * a2 - 3.1543839e+2 * a3 + 6.770824e+1 * a4;
-  double bm2 = 1. / (zaw * K_MWA) - 1. / K_MWA;
+  double bm2 = drcp(zaw * K_MWA) - 1. / K_MWA;
   // regime 1a is the same sum with bm5 = 1 and no sea salt term (one code path for the
   // 1a lane and the regime-2 lanes; explicit fmas so the gradient harness's copy of the
   // 1a iteration rounds the same)
   double bm5 = +5.875248e+1 - 1.8781997e+2 * zaw + 2.7211377e+2 * a2 - 1.8458287e+2 * a3 + 4.153689e+1 * a4;
   bm5 = j.r2 ? bm5 : 1.;
   const double q4 = j.r2 ? j.q4 : 0.;
-  const double zlwc = fma(q4, bm1 * bm2, fma(j.q1, bm1 * bm5, j.q0 * (bm2 * bm5))) / (bm1 * bm2 * bm5);
+  const double zlwc = ddiv(fma(q4, bm1 * bm2, fma(j.q1, bm1 * bm5, j.q0 * (bm2 * bm5))), bm1 * bm2 * bm5);
   j.zlwc = zlwc;
-  j.zdwet = cbrt(fma(zlwc, j.rinv, j.p56) + j.pc);
-  j.izke = exp(-(ckt / j.zdwet));
+  j.zdwet = dcbrt(fma(zlwc, j.rinv, j.p56) + j.pc);
+  j.izke = dexp(-(ddiv(ckt, j.zdwet)));
   j.count++;
 }
 
@@ -1922,7 +1923,7 @@ template <typename KT>
 __device__ __forceinline__ void eq_load_f(const DevParams &P, const WS<KT> &w, int b, EqJobF &j) {
   j.kk = b;
   j.count = 0;
-  const float numc = (float)w.numc[b], in = 1.f / numc;
+  const float numc = (float)w.numc[b], in = ddiv(1.f, numc);
   float zv[7];
   for (int i = 0; i < 7; i++) zv[i] = (float)zvolc_of(P, w, i, b);
   const float zcore = j.r2 ? (zv[0] + zv[1] + zv[2] + zv[3] + zv[4]) * in : (zv[0] + zv[1]) * in;
@@ -1944,13 +1945,13 @@ __device__ __forceinline__ void eq_step_f(EqJobF &j, float ckt) {
   const float u = fmaf(j.zrh, j.em, j.omrh);   // 1 - zrh / zke
   const float zaw = 1.f - u;
   const float bm1 = zsr1_u(u);
-  const float bm2 = u / (zaw * (float)K_MWA);   // 1/(aw M) - 1/M
+  const float bm2 = ddiv(u, zaw * (float)K_MWA);   // 1/(aw M) - 1/M
   const float bm5 = j.r2 ? zsr5_u(u) : 1.f;
   const float q4 = j.r2 ? j.q4 : 0.f;
-  const float zlwc = fmaf(q4, bm1 * bm2, fmaf(j.q1, bm1 * bm5, j.q0 * (bm2 * bm5))) / (bm1 * bm2 * bm5);
+  const float zlwc = ddiv(fmaf(q4, bm1 * bm2, fmaf(j.q1, bm1 * bm5, j.q0 * (bm2 * bm5))), bm1 * bm2 * bm5);
   j.zlwc = zlwc;
   j.zdwet = cbrtf(fmaf(zlwc, j.rinv, j.p56) + j.pc);
-  j.em = -expm1f(-(ckt / j.zdwet));
+  j.em = -expm1f(-(ddiv(ckt, j.zdwet)));
   j.count++;
 }
 
@@ -1970,7 +1971,7 @@ __device__ void equilibration(const DevParams &P, const WS<KT> &w, const double 
   const double *dmid = tb + TAB_DMID * P.nb_pad;
   int nonconv = 0;
   const int n2 = init ? P.fn2b - P.in2a + 1 : 0;
-  const double ckt = 2. * K_SURFW0 * K_MVWA / (K_BOLTZ * T);
+  const double ckt = ddiv(2. * K_SURFW0 * K_MVWA, K_BOLTZ * T);
   if (n2 <= 31 && sizeof(KT) == 4) {
     // the mixed form: lane 31 runs the regime-1a chain, lanes 0..n2-1 the regime-2 bins,
     // all in float; then the regime-2 lanes take two FP64 passes from the float result
@@ -2020,10 +2021,10 @@ __device__ void equilibration(const DevParams &P, const WS<KT> &w, const double 
         d.r2 = true; d.tol = 1.e-12; d.zrh = fmin(fmax(prh, 0.37), 0.98);
         eq_load(P, w, r2k, d);
         d.zdwet = (double)j.zdwet;
-        d.izke = exp(-(ckt / d.zdwet));
+        d.izke = dexp(-(ddiv(ckt, d.zdwet)));
         eq_step(d, ckt);
         eq_step(d, ckt);
-        w.v(P.iwa, r2k) = d.zlwc / K_RHOWA;
+        w.v(P.iwa, r2k) = divc(d.zlwc, K_RHOWA);
         w.dwet[r2k] = d.zdwet;
       }
     }
@@ -2053,7 +2054,7 @@ __device__ void equilibration(const DevParams &P, const WS<KT> &w, const double 
           if (j.count > 100) { nonconv = 1; go = false; }
         }
         if (!go) {
-          w.v(P.iwa, j.kk) = j.zlwc / K_RHOWA;
+          w.v(P.iwa, j.kk) = divc(j.zlwc, K_RHOWA);
           if (init) w.dwet[j.kk] = j.zdwet;
           int k = j.r2 ? -1 : eq_next_1a(P, w, dmid, j.kk, init);
           if (k >= 0) eq_load(P, w, k, j);
@@ -2072,7 +2073,7 @@ __device__ void equilibration(const DevParams &P, const WS<KT> &w, const double 
         double zlwc = equil_iterate<KT>(P, w, kk, zrh, T, zke, 1.e-2, false, zd, zc, nonconv);
         __syncwarp();
         if (lane == 0) {
-          w.v(P.iwa, kk) = zlwc / K_RHOWA;
+          w.v(P.iwa, kk) = divc(zlwc, K_RHOWA);
           if (init) w.dwet[kk] = zd;
         }
       } else if (init && lane == 0) {
@@ -2086,7 +2087,7 @@ __device__ void equilibration(const DevParams &P, const WS<KT> &w, const double 
         double zrh = fmin(fmax(prh, 0.37), 0.98);
         double zd, zc;
         double zlwc = equil_iterate<KT>(P, w, kk, zrh, T, zke, 1.e-12, true, zd, zc, nonconv);
-        w.v(P.iwa, kk) = zlwc / K_RHOWA;
+        w.v(P.iwa, kk) = divc(zlwc, K_RHOWA);
         w.dwet[kk] = zd;
       } else {
         w.dwet[kk] = dmid[kk];
@@ -2108,13 +2109,13 @@ __device__ __forceinline__ double solute_moles(const DevParams &P, const WS<KT> 
   if (P.has_kappa) {
     double vs = 0.;
     for (int nn = 0; nn < P.ndry; nn++) if (P.diss[nn] > 0.) vs += w.v(nn, b);
-    zns = kappa * vs * K_RHOWA / K_MWA;
+    zns = divc(kappa * vs * K_RHOWA, K_MWA);
   } else {
-    for (int nn = 0; nn < P.ndry; nn++) zns = zns + P.diss[nn] * w.v(nn, b) * P.rholiq[nn] / P.MM[nn];
+    for (int nn = 0; nn < P.ndry; nn++) zns = zns + ddiv(P.diss[nn] * w.v(nn, b) * P.rholiq[nn], P.MM[nn]);
   }
   return zns;
 }
-__device__ __forceinline__ double acth2o_w(double znw, double zns) { return fmax(0.1, znw / fmax(K_EPS, (znw + zns))); }
+__device__ __forceinline__ double acth2o_w(double znw, double zns) { return fmax(0.1, ddiv(znw, fmax(K_EPS, (znw + zns)))); }
 
 // ----------------------------------------------------------------------------------------
 // Gas condensation: mo_salsa_dynamics.f90:348-685 (condgas).  H2SO4 and the non- and
@@ -2137,9 +2138,9 @@ __device__ __forceinline__ void condgas(const DevParams &P, const WS<KT> &w, con
   const int C0 = P.nbins, P0 = P.nbins + P.ncld, I0 = P.nliquid;
   const int ioc = P.ix_oc, iso4 = P.ix_so4;
   double *cr = w.scr, *dvoc = w.scr + w.NB;
-  const double zvisc = (7.44523e-3 * sqrt(cube(T))) / (5093. * (T + 110.4));
-  const double zdfvap = 5.1111e-10 * pow(T, 1.75) * K_PSTAND / pres;
-  const double zmfp = 3. * zdfvap * sqrt(K_PI * K_MSU / (8. * K_RG * T));
+  const double zvisc = ddiv(7.44523e-3 * dsqrt(cube(T)), 5093. * (T + 110.4));
+  const double zdfvap = ddiv(5.1111e-10 * dpow(T, 1.75) * K_PSTAND, pres);
+  const double zmfp = 3. * zdfvap * dsqrt(ddiv(K_PI * K_MSU, 8. * K_RG * T));
   for (int b = lane; b < ntot; b += 32) {
     // updateDiameter(limit=.TRUE., type="wet") (:446-448)
     const int ph = phase_of(P, b);
@@ -2148,7 +2149,7 @@ __device__ __forceinline__ void condgas(const DevParams &P, const WS<KT> &w, con
     if (n > nlim_of(ph)) {
       double vs = 0.;
       for (int sp = 0; sp < P.nused; sp++) vs += w.v(sp, b);
-      dw = cbrt(vs / n / K_PI6);
+      dw = dcbrt(divc(ddiv(vs, n), K_PI6));
     }
     dw = fmin(dw, dlim_of(ph));
     w.dwet[b] = dw;
@@ -2156,19 +2157,19 @@ __device__ __forceinline__ void condgas(const DevParams &P, const WS<KT> &w, con
     double r = 0.;
     if (ph == 1) {
       const bool small = b <= in1a + 1;   // molecule size and particle diffusion count below 20 nm
-      const double kn = small ? 2. * zmfp / (dw + K_DSA) : 2. * zmfp / dw;
-      const double beta = (kn + 1.) / (0.377 * kn + 1. + 4. / (3. * K_MASSACC) * (kn + sq(kn)));
+      const double kn = small ? ddiv(2. * zmfp, dw + K_DSA) : ddiv(2. * zmfp, dw);
+      const double beta = ddiv(kn + 1., 0.377 * kn + 1. + 4. / (3. * K_MASSACC) * (kn + sq(kn)));
       if (small) {
-        const double zdfpart = K_BOLTZ * T * beta / (3. * K_PI * zvisc * dw);
+        const double zdfpart = ddiv(K_BOLTZ * T * beta, 3. * K_PI * zvisc * dw);
         if (n > K_NLIM) r = 2. * K_PI * (dw + K_DSA) * (zdfvap + zdfpart) * beta * n;
       } else if (n > K_NLIM) {
         r = 2. * K_PI * dw * zdfvap * beta * n;
       }
       dvoc[b] = 0.;
     } else {
-      const double kn = 2. * zmfp / dw;
-      double beta = 1. + kn * (1.33 + (0.71 / kn)) / (1. + (1. / kn));
-      beta = 1. / beta;
+      const double kn = ddiv(2. * zmfp, dw);
+      double beta = 1. + ddiv(kn * (1.33 + (ddiv(0.71, kn))), 1. + (drcp(kn)));
+      beta = drcp(beta);
       if (n > (ph == 2 ? K_NLIM : K_PRLIM)) r = 2. * K_PI * dw * zdfvap * beta * n;
     }
     cr[b] = r;
@@ -2186,11 +2187,11 @@ __device__ __forceinline__ void condgas(const DevParams &P, const WS<KT> &w, con
   // non-volatile organics onto every bin (:552-598)
   if (zg[3] > 1.e-10 && zcs_tot > 1.e-30 && ioc >= 0) {
     const double zcs = zcs_tot;
-    const double cnew = zg[3] / (1. + dt * zcs);
+    const double cnew = ddiv(zg[3], 1. + dt * zcs);
     const double dv = zg[3] - cnew;
     zg[3] = cnew;
     for (int b = lane; b < ntot; b += 32) {
-      const double inc = cr[b] / zcs * K_MVOC * dv;
+      const double inc = ddiv(cr[b], zcs) * K_MVOC * dv;
       if (b <= fn2b) dvoc[b] = inc;
       w.v(ioc, b) = w.v(ioc, b) + inc;
     }
@@ -2199,29 +2200,29 @@ __device__ __forceinline__ void condgas(const DevParams &P, const WS<KT> &w, con
   // update adds the whole increment row, which still holds the non-volatile increments
   const double zcs_ocsv = sa2 + sca + spa + sia;
   if (zg[4] > 1.e-10 && zcs_ocsv > 1.e-30 && ioc >= 0) {
-    const double cnew = zg[4] / (1. + dt * zcs_ocsv);
+    const double cnew = ddiv(zg[4], 1. + dt * zcs_ocsv);
     const double dv = zg[4] - cnew;
     zg[4] = cnew;
     for (int b = lane; b < ntot; b += 32) {
       if (b <= fn2b) {
         double d = dvoc[b];
-        if (b >= in2a) d = d + cr[b] / zcs_ocsv * K_MVOC * dv;
+        if (b >= in2a) d = d + ddiv(cr[b], zcs_ocsv) * K_MVOC * dv;
         w.v(ioc, b) = w.v(ioc, b) + d;
       } else {
-        w.v(ioc, b) = w.v(ioc, b) + cr[b] / zcs_ocsv * K_MVOC * dv;
+        w.v(ioc, b) = w.v(ioc, b) + ddiv(cr[b], zcs_ocsv) * K_MVOC * dv;
       }
     }
   }
   // sulphuric acid onto every bin (:636-679)
   if (zg[0] > 1.e-10 && zcs_tot > 1.e-30 && iso4 >= 0) {
     const double zcs = zcs_tot;
-    const double cnew = zg[0] / (1. + dt * zcs);
+    const double cnew = ddiv(zg[0], 1. + dt * zcs);
     const double dv = zg[0] - cnew;
     zg[0] = cnew;
     for (int b = lane; b < ntot; b += 32) {
-      const double inc = cr[b] / zcs * K_MVSU * dv;
+      const double inc = ddiv(cr[b], zcs) * K_MVSU * dv;
       w.v(iso4, b) = w.v(iso4, b) + inc;
-      if (b == in1a && zxsa > 0.) w.numc[b] = w.numc[b] + zn_vs_c * inc / K_MVSU / (K_N3 * zxsa);
+      if (b == in1a && zxsa > 0.) w.numc[b] = w.numc[b] + ddiv(divc(zn_vs_c * inc, K_MVSU), K_N3 * zxsa);
     }
   }
   __syncwarp();
@@ -2235,7 +2236,7 @@ __device__ void gpparth2o(const DevParams &P, const WS<KT> &w, const double *tb,
   const int nbins = P.nbins, ncld = P.ncld, nprc = P.nprc, nice = P.nice, ntot = P.ntotal;
   const int iwa = P.iwa, irim = P.irim, C0 = nbins, P0 = nbins + ncld, I0 = P.nliquid;
   const double *dmid = tb + TAB_DMID * P.nb_pad;
-  const double zrh = prv / prs;
+  const double zrh = ddiv(prv, prs);
   // aerosol water before/after the equilibrium update
   double l1 = 0.;
   for (int b = lane; b <= P.fn2b; b += 32) l1 += w.v(iwa, b);
@@ -2253,7 +2254,7 @@ __device__ void gpparth2o(const DevParams &P, const WS<KT> &w, const double *tb,
   double l2 = 0.;
   for (int b = lane; b <= P.fn2b; b += 32) l2 += w.v(iwa, b);
   double zaelwc2 = warp_sum(l2) * K_RHOWA;
-  prv = prv - (zaelwc2 - zaelwc1) / (pres * K_MAIR / (K_RG * T));
+  prv = prv - ddiv(zaelwc2 - zaelwc1, ddiv(pres * K_MAIR, K_RG * T));
 
   bool anycl = false, anypr = false, anyic = false, anyae = false;
   for (int b = lane; b < ntot; b += 32) {
@@ -2268,11 +2269,11 @@ __device__ void gpparth2o(const DevParams &P, const WS<KT> &w, const double *tb,
   if (!((anycl || (anypr && P.lscndh2ocl)) || (anyic && P.lscndh2oic) || (anyae && zrh > 0.98 && P.lscndh2oae)))
     return;
 
-  const double rhoair = K_MAIR * pres / (K_RG * T);
-  double zdfh2o = (5. / (16. * K_AVOG * rhoair * 1.e-3 * sq(3.11e-8))) *
-                  sqrt(K_RG * 1.e7 * T * K_MAIR * 1.e3 * (K_MWA + K_MAIR) * 1.e3 / (2. * K_PI * K_MWA * 1.e3));
+  const double rhoair = ddiv(K_MAIR * pres, K_RG * T);
+  double zdfh2o = (ddiv(5., 16. * K_AVOG * rhoair * 1.e-3 * sq(3.11e-8))) *
+                  dsqrt(divc(K_RG * 1.e7 * T * K_MAIR * 1.e3 * (K_MWA + K_MAIR) * 1.e3, 2. * K_PI * K_MWA * 1.e3));
   zdfh2o = zdfh2o * 1.e-4;
-  const double zmfph2o = 3. * zdfh2o * sqrt(K_PI * K_MWA / (8. * K_RG * T));
+  const double zmfph2o = 3. * zdfh2o * dsqrt(ddiv(K_PI * K_MWA, 8. * K_RG * T));
   const double zthcond = 0.023807 + 7.1128e-5 * (T - 273.16);
   const int NB = w.NB;
   double *kel = w.sc(0), *surf = w.sc(1), *mt = w.sc(2), *wsat = w.sc(3), *cw = w.sc(4), *zns = w.sc(5),
@@ -2294,40 +2295,40 @@ __device__ void gpparth2o(const DevParams &P, const WS<KT> &w, const double *tb,
     if (act) {
       if (ph <= 3) {
         double dwet = w.dwet[b];
-        double znw = w.v(iwa, b) * P.rholiq[iwa] / P.MM[iwa];
+        double znw = ddiv(w.v(iwa, b) * P.rholiq[iwa], P.MM[iwa]);
         double zact = acth2o_w(znw, ns_);
-        k_ = exp(4. * K_SURFW0 * K_MWA / (K_RG * T * K_RHOWA * dwet));
-        sf = prs * rhoair / K_MWA;
+        k_ = dexp(ddiv(4. * K_SURFW0 * K_MWA, K_RG * T * K_RHOWA * dwet));
+        sf = divc(prs * rhoair, K_MWA);
         ws = zact * k_;
-        KT zknud = (KT)2. * (KT)zmfph2o / (KT)dwet;
-        KT zbeta = (zknud + (KT)1.) / ((KT)0.377 * zknud + (KT)1. + (KT)4. / ((KT)3. * (KT)1.) * (zknud + zknud * zknud));
+        KT zknud = ddiv((KT)2. * (KT)zmfph2o, (KT)dwet);
+        KT zbeta = ddiv(zknud + (KT)1., (KT)0.377 * zknud + (KT)1. + (KT)4. / ((KT)3. * (KT)1.) * (zknud + zknud * zknud));
         KT h1 = (KT)n * (KT)2. * (KT)K_PI * (KT)dwet * (KT)zdfh2o * zbeta;
-        KT h2 = (KT)K_MWA * (KT)zdfh2o * (KT)K_ALV * (KT)ws * (KT)sf / ((KT)zthcond * (KT)T);
-        KT h3 = (((KT)K_ALV * (KT)K_MWA) / ((KT)K_RG * (KT)T)) - (KT)1.;
-        m = (double)(h1 / (h2 * h3 + (KT)1.));
+        KT h2 = ddiv((KT)K_MWA * (KT)zdfh2o * (KT)K_ALV * (KT)ws * (KT)sf, (KT)zthcond * (KT)T);
+        KT h3 = (ddiv((KT)K_ALV * (KT)K_MWA, (KT)K_RG * (KT)T)) - (KT)1.;
+        m = (double)(ddiv(h1, h2 * h3 + (KT)1.));
       } else {
         double dwet = w.dnsp[b];
         double cap = 0.5 * dwet;
-        k_ = exp(4. * K_SURFI0 * K_MWA / (K_RG * T * K_RHOWA * dwet));
-        sf = prsi * rhoair / K_MWA;
+        k_ = dexp(ddiv(4. * K_SURFI0 * K_MWA, K_RG * T * K_RHOWA * dwet));
+        sf = divc(prsi * rhoair, K_MWA);
         ws = 1.0 * k_;
-        KT zknud = (KT)2. * (KT)zmfph2o / (KT)dwet;
-        KT zbeta = (zknud + (KT)1.) / ((KT)0.377 * zknud + (KT)1. + (KT)4. / (KT)3. * (zknud + zknud * zknud));
+        KT zknud = ddiv((KT)2. * (KT)zmfph2o, (KT)dwet);
+        KT zbeta = ddiv(zknud + (KT)1., (KT)0.377 * zknud + (KT)1. + (KT)4. / (KT)3. * (zknud + zknud * zknud));
         KT h1 = (KT)n * (KT)4. * (KT)K_PI * (KT)cap * (KT)zdfh2o * zbeta;
-        KT h2 = (KT)K_MWA * (KT)zdfh2o * (KT)K_ALS * (KT)ws * (KT)sf / ((KT)zthcond * (KT)T);
-        KT h3 = (((KT)K_ALS * (KT)K_MWA) / ((KT)K_RG * (KT)T)) - (KT)1.;
-        m = (double)(h1 / (h2 * h3 + (KT)1.));
+        KT h2 = ddiv((KT)K_MWA * (KT)zdfh2o * (KT)K_ALS * (KT)ws * (KT)sf, (KT)zthcond * (KT)T);
+        KT h3 = (ddiv((KT)K_ALS * (KT)K_MWA, (KT)K_RG * (KT)T)) - (KT)1.;
+        m = (double)(ddiv(h1, h2 * h3 + (KT)1.));
       }
     }
     kel[b] = k_; surf[b] = sf; mt[b] = m; wsat[b] = ws; zns[b] = ns_;
     if (ph <= 3) {
-      cw[b] = w.v(iwa, b) * K_RHOWA / K_MWA;
+      cw[b] = divc(w.v(iwa, b) * K_RHOWA, K_MWA);
       orgic[b] = orgri[b] = 0.;
     } else {
-      double c1 = w.v(iwa, b) * K_RHOIC / K_MWA;
-      cw[b] = c1 + w.v(irim, b) * K_RHORI / K_MWA;
-      orgic[b] = w.v(iwa, b) * K_RHOIC / K_MWA;
-      orgri[b] = w.v(irim, b) * K_RHORI / K_MWA;
+      double c1 = divc(w.v(iwa, b) * K_RHOIC, K_MWA);
+      cw[b] = c1 + divc(w.v(irim, b) * K_RHORI, K_MWA);
+      orgic[b] = divc(w.v(iwa, b) * K_RHOIC, K_MWA);
+      orgri[b] = divc(w.v(irim, b) * K_RHORI, K_MWA);
     }
   }
   __syncwarp();
@@ -2342,7 +2343,7 @@ __device__ void gpparth2o(const DevParams &P, const WS<KT> &w, const double *tb,
     }
     upd_ae = warp_any(a) && zrh > 0.98; upd_cl = warp_any(c); upd_pr = warp_any(p); upd_ic = warp_any(i);
   }
-  double zcwc = prv * rhoair / K_MWA;
+  double zcwc = divc(prv * rhoair, K_MWA);
   double tsum = 0., msum = 0.;
   for (int b = lane; b < ntot; b += 32) {
     tsum += cw[b];
@@ -2370,7 +2371,7 @@ __device__ void gpparth2o(const DevParams &P, const WS<KT> &w, const double *tb,
   while (ttot < dt) {
     double zhlp1 = zcwc + adt * spsum;
     double zhlp2 = 1. + adt * mtot;
-    zcwint = fmin(zhlp1 / zhlp2, zcwtot);
+    zcwint = fmin(ddiv(zhlp1, zhlp2), zcwtot);
     double cs = 0., sp = 0.;
     for (int b = lane; b < ntot; b += 32) {
       int ph = phase_of(P, b);
@@ -2405,7 +2406,7 @@ __device__ void gpparth2o(const DevParams &P, const WS<KT> &w, const double *tb,
 #ifdef SALSA_STAGE_TIMERS
   if (lane == 0 && P.stage_clocks) atomicAdd(P.stage_clocks + 9, (unsigned long long)(clock64() - t_sub0));
 #endif
-  prv = zcwint * K_MWA / rhoair;
+  prv = ddiv(zcwint * K_MWA, rhoair);
   // Cond_i diagnostic (:1086-1112): vrate(irim) is only assigned on sublimation and keeps
   // its previous value on later deposition bins; the sum follows the ice bins in order.
   double dci = 0.;
@@ -2415,11 +2416,11 @@ __device__ void gpparth2o(const DevParams &P, const WS<KT> &w, const double *tb,
       int b = I0 + k;
       double dvitot = cw[b] - (orgic[b] + orgri[b]);
       if (dvitot > 0.) {
-        dci += dvitot * K_MWA / K_RHOIC * K_RHOIC + vr_last * K_RHORI;
+        dci += divc(dvitot * K_MWA, K_RHOIC) * K_RHOIC + vr_last * K_RHORI;
       } else if (dvitot < 0.) {
-        double f = (cw[b] / (orgic[b] + orgri[b])) - 1.;
-        vr_last = f * orgri[b] * K_MWA / K_RHORI;
-        dci += f * orgic[b] * K_MWA / K_RHOIC * K_RHOIC + vr_last * K_RHORI;
+        double f = (ddiv(cw[b], orgic[b] + orgri[b])) - 1.;
+        vr_last = divc(f * orgri[b] * K_MWA, K_RHORI);
+        dci += divc(f * orgic[b] * K_MWA, K_RHOIC) * K_RHOIC + vr_last * K_RHORI;
       }
     }
   }
@@ -2429,20 +2430,20 @@ __device__ void gpparth2o(const DevParams &P, const WS<KT> &w, const double *tb,
   for (int b = lane; b < ntot; b += 32) {
     int ph = phase_of(P, b);
     if (ph <= 3) {
-      double nv = fmax(0., cw[b] * K_MWA / K_RHOWA);
+      double nv = fmax(0., divc(cw[b] * K_MWA, K_RHOWA));
       double d = nv - w.v(iwa, b);
       if (ph == 1) dca += d; else if (ph == 2) dcc += d; else dcp += d;
       w.v(iwa, b) = nv;
     } else {
       double dvitot = cw[b] - (orgic[b] + orgri[b]);
       if (dvitot > 0.) {
-        double dv = dvitot * K_MWA / K_RHOIC;
+        double dv = divc(dvitot * K_MWA, K_RHOIC);
         w.v(iwa, b) = w.v(iwa, b) + dv;
       } else if (dvitot < 0.) {
-        double f = (cw[b] / (orgic[b] + orgri[b])) - 1.;
+        double f = (ddiv(cw[b], orgic[b] + orgri[b])) - 1.;
         double dvice = f * orgic[b], dvrime = f * orgri[b];
-        w.v(iwa, b) = w.v(iwa, b) + dvice * K_MWA / K_RHOIC;
-        w.v(irim, b) = w.v(irim, b) + dvrime * K_MWA / K_RHORI;
+        w.v(iwa, b) = w.v(iwa, b) + divc(dvice * K_MWA, K_RHOIC);
+        w.v(irim, b) = w.v(irim, b) + divc(dvrime * K_MWA, K_RHORI);
       }
     }
     if (w.numc[b] > nlim_of(ph)) w.rhomean[b] = rhomean_of(P, ph, w.numc[b], w.v(iwa, b), w.v(irim, b));
@@ -2492,8 +2493,8 @@ __device__ __forceinline__ void act_cloudbase(const DevParams &P, const WS<KT> &
   for (int k = lane; k <= fn2b; k += 32) {
     double n_ = 0.;
     if (w.numc[k] > K_NLIM) {
-      for (int nn = 0; nn < ndry; nn++) n_ = n_ + P.diss[nn] * w.v(nn, k) * P.rholiq[nn] / P.MM[nn];
-      n_ = n_ / w.numc[k];
+      for (int nn = 0; nn < ndry; nn++) n_ = n_ + ddiv(P.diss[nn] * w.v(nn, k) * P.rholiq[nn], P.MM[nn]);
+      n_ = ddiv(n_, w.numc[k]);
     }
     ns[k] = n_;
     frac[k] = zdcrit[k] = zdcrlo[k] = zdcrhi[k] = 0.;
@@ -2502,11 +2503,11 @@ __device__ __forceinline__ void act_cloudbase(const DevParams &P, const WS<KT> &
   int bcrita = fn2a;
   double zdcstar = 0.;
   if (wvel > 0.) {
-    const double aa = 4. * K_MWA * K_SURFW0 / (K_RG * K_RHOWA * T);   // Kelvin term [m]
-    const double x = 4. * cube(aa) / (27. * bb);
+    const double aa = ddiv(4. * K_MWA * K_SURFW0, K_RG * K_RHOWA * T);   // Kelvin term [m]
+    const double x = divc(4. * cube(aa), 27. * bb);
     for (int k = in1a + lane; k <= fn2b; k += 32) {
-      const double scrit = exp(sqrt(x / fmax(K_EPS, ns[k]))) - 1.;
-      term[k] = w.numc[k] / pow(scrit, 2. / 3.);
+      const double scrit = dexp(dsqrt(ddiv(x, fmax(K_EPS, ns[k])))) - 1.;
+      term[k] = ddiv(w.numc[k], dpow(scrit, 2. / 3.));
     }
     __syncwarp();
     double ntot = 0., sum1 = 0.;   // part 3, eq. (8)
@@ -2515,31 +2516,31 @@ __device__ __forceinline__ void act_cloudbase(const DevParams &P, const WS<KT> &
     if (!(ntot < K_NLIM)) {
       const double V = wvel;
       const double L = 2.501e6 - 2370. * (T - 273.15);
-      const double a1 = 1. - (373.15 / T);
-      const double ps = 101325. * exp(13.3185 * a1 - 1.976 * sq(a1) - 0.6445 * cube(a1) - 0.1299 * sq(sq(a1)));
-      const double alpha = K_GRAV * K_MWA * L / (K_CPA * K_RG * sq(T)) - K_GRAV * K_MAIR / (K_RG * T);
-      const double gamma = K_RG * T / (ps * K_MWA) + K_MWA * sq(L) / (K_CPA * pres * K_MAIR * T);
-      const double x1 = pres / 101325.;
-      const double dv1 = 1.e-4 * (0.211 / x1) * pow(T / 273., 1.94);
+      const double a1 = 1. - (ddiv(373.15, T));
+      const double ps = 101325. * dexp(13.3185 * a1 - 1.976 * sq(a1) - 0.6445 * cube(a1) - 0.1299 * sq(sq(a1)));
+      const double alpha = ddiv(K_GRAV * K_MWA * L, K_CPA * K_RG * sq(T)) - ddiv(K_GRAV * K_MAIR, K_RG * T);
+      const double gamma = ddiv(K_RG * T, ps * K_MWA) + ddiv(K_MWA * sq(L), K_CPA * pres * K_MAIR * T);
+      const double x1 = divc(pres, 101325.);
+      const double dv1 = 1.e-4 * (ddiv(0.211, x1)) * dpow(divc(T, 273.), 1.94);
       const double ka1 = 1.e-3 * (4.39 + 0.071 * T);
-      const double Gc = 1. / (K_RHOWA * K_RG * T / (ps * dv1 * K_MWA) +
-                              L * K_RHOWA / (ka1 * T) * (L * K_MWA / (T * K_RG) - 1.));
-      const double s_eff = sqrt(cube(ntot / sum1));
-      const double theta = (sqrt(cube(alpha * V / Gc))) / (2. * K_PI * K_RHOWA * gamma * ntot);
-      const double khi = (2. / 3.) * aa * sqrt(alpha * V / Gc);
-      const double s_max = s_eff / sqrt(0.5 * sqrt(cube(khi / theta)) + pow(sq(s_eff) / (theta + 3. * khi), 0.75));
-      zdcstar = 2. * aa / (3. * s_max);
+      const double Gc = drcp(ddiv(K_RHOWA * K_RG * T, ps * dv1 * K_MWA) +
+                              ddiv(L * K_RHOWA, ka1 * T) * (ddiv(L * K_MWA, T * K_RG) - 1.));
+      const double s_eff = dsqrt(cube(ddiv(ntot, sum1)));
+      const double theta = ddiv(dsqrt(cube(ddiv(alpha * V, Gc))), 2. * K_PI * K_RHOWA * gamma * ntot);
+      const double khi = (2. / 3.) * aa * dsqrt(ddiv(alpha * V, Gc));
+      const double s_max = ddiv(s_eff, dsqrt(0.5 * dsqrt(cube(ddiv(khi, theta))) + dpow(ddiv(sq(s_eff), theta + 3. * khi), 0.75)));
+      zdcstar = ddiv(2. * aa, 3. * s_max);
       for (int kk = in1a + lane; kk <= fn2b; kk += 32) {
         if (w.numc[kk] < K_NLIM) continue;
         const double nshi = ns[kk] * vrhi[kk];
-        const double sil = exp(sqrt(x / nshi)) - 1.;
+        const double sil = dexp(dsqrt(ddiv(x, nshi))) - 1.;
         if (s_max < sil) continue;
         const double nslo = ns[kk] * vrlo[kk];
-        const double siu = exp(sqrt(x / nslo)) - 1.;
-        frac[kk] = fmin(1., log(s_max / sil) / log(siu / sil));
-        zdcrlo[kk] = 2. * sqrt(3. * nslo * bb / aa);
-        zdcrhi[kk] = 2. * sqrt(3. * nshi * bb / aa);
-        zdcrit[kk] = 2. * sqrt(3. * ns[kk] * bb / aa);
+        const double siu = dexp(dsqrt(ddiv(x, nslo))) - 1.;
+        frac[kk] = fmin(1., ddiv(dlog(ddiv(s_max, sil)), dlog(ddiv(siu, sil))));
+        zdcrlo[kk] = 2. * dsqrt(ddiv(3. * nslo * bb, aa));
+        zdcrhi[kk] = 2. * dsqrt(ddiv(3. * nshi * bb, aa));
+        zdcrit[kk] = 2. * dsqrt(ddiv(3. * ns[kk] * bb, aa));
       }
       __syncwarp();
       for (int kk = in1a; kk <= fn2a; kk++)   // the critical bin of regime a
@@ -2556,17 +2557,17 @@ __device__ __forceinline__ void act_cloudbase(const DevParams &P, const WS<KT> &
   } else {
     double sd = 0.;
     for (int i = 0; i < ndry; i++) sd += w.v(i, bcrita);
-    Vmid = sd / fmax(K_NLIM, w.numc[bcrita]);
+    Vmid = ddiv(sd, fmax(K_NLIM, w.numc[bcrita]));
   }
   Vhi = vhi[bcrita];
   Vlo = vlo[bcrita];
   double zvcstar = 0.;
   const double dc = zdcrit[bcrita];
   if (zdcstar >= dc) {
-    const double zhlp = (K_PI6 * cube(zdcstar) - K_PI6 * cube(dc)) / fmax(K_EPS, K_PI6 * cube(zdcrhi[bcrita]) - K_PI6 * cube(dc));
+    const double zhlp = ddiv(K_PI6 * cube(zdcstar) - K_PI6 * cube(dc), fmax(K_EPS, K_PI6 * cube(zdcrhi[bcrita]) - K_PI6 * cube(dc)));
     zvcstar = Vmid + zhlp * (Vhi - Vmid);
   } else if (zdcstar < dc) {
-    const double zhlp = (K_PI6 * cube(dc) - K_PI6 * cube(zdcstar)) / fmax(K_EPS, K_PI6 * cube(dc) - K_PI6 * cube(zdcrlo[bcrita]));
+    const double zhlp = ddiv(K_PI6 * cube(dc) - K_PI6 * cube(zdcstar), fmax(K_EPS, K_PI6 * cube(dc) - K_PI6 * cube(zdcrlo[bcrita])));
     zvcstar = Vmid - zhlp * (Vmid - Vlo);
   }
   zvcstar = fmax(zvcstar, vlo[bcrita]);
@@ -2577,16 +2578,16 @@ __device__ __forceinline__ void act_cloudbase(const DevParams &P, const WS<KT> &
     const double Nmid = fmax(w.numc[ab], K_NLIM);
     double sd = 0.;
     for (int i = 0; i < ndry; i++) sd += w.v(i, ab);
-    const double Vm = sd / Nmid, Vl = vlo[ab], Vh = vhi[ab];
+    const double Vm = ddiv(sd, Nmid), Vl = vlo[ab], Vh = vhi[ab];
     double Nim1, Vim1, Vlom1, Vhim1, Nip1, Vip1, Vlop1, Vhip1;
     if (ab == in1a || ab == in2b) {
-      Nim1 = K_NLIM; Vim1 = Vl / 2.; Vlom1 = 0.; Vhim1 = Vl;
+      Nim1 = K_NLIM; Vim1 = divc(Vl, 2.); Vlom1 = 0.; Vhim1 = Vl;
     } else {
       Nim1 = fmax(w.numc[ab - 1], K_NLIM);
       if (Nim1 > K_NLIM) {
         double v = 0.;
         for (int i = 0; i < ndry; i++) v += w.v(i, ab - 1);
-        Vim1 = v / Nim1;
+        Vim1 = ddiv(v, Nim1);
       } else {
         Vim1 = K_PI6 * cube(dmid[ab - 1]);
       }
@@ -2599,7 +2600,7 @@ __device__ __forceinline__ void act_cloudbase(const DevParams &P, const WS<KT> &
       if (Nip1 > K_NLIM) {
         double v = 0.;
         for (int i = 0; i < ndry; i++) v += w.v(i, ab + 1);
-        Vip1 = v / Nip1;
+        Vip1 = ddiv(v, Nip1);
       } else {
         Vip1 = K_PI6 * cube(dmid[ab + 1]);
       }
@@ -2607,8 +2608,8 @@ __device__ __forceinline__ void act_cloudbase(const DevParams &P, const WS<KT> &
     }
     Vip1 = fmax(Vlop1, fmin(Vip1, Vhip1));
     Vim1 = fmax(Vlom1, fmin(Vim1, Vhim1));
-    const double dNim1 = Nim1 / (Vhim1 - Vlom1), dNip1 = Nip1 / (Vhip1 - Vlop1), dNmid = Nmid / (Vh - Vl);
-    const double zs1 = (dNmid - dNim1) / (Vm - Vim1), zs2 = (dNip1 - dNmid) / (Vip1 - Vm);
+    const double dNim1 = ddiv(Nim1, Vhim1 - Vlom1), dNip1 = ddiv(Nip1, Vhip1 - Vlop1), dNmid = ddiv(Nmid, Vh - Vl);
+    const double zs1 = ddiv(dNmid - dNim1, Vm - Vim1), zs2 = ddiv(dNip1 - dNmid, Vip1 - Vm);
     const double N01 = dNmid - zs1 * Vm, N02 = dNip1 - zs2 * Vip1;
     const double Nnorm = intgN(zs1, N01, Vl, Vm) + intgN(zs2, N02, Vm, Vh);
     const double Vnorm = intgV(zs1, N01, Vl, Vm) + intgV(zs2, N02, Vm, Vh);
@@ -2616,36 +2617,36 @@ __device__ __forceinline__ void act_cloudbase(const DevParams &P, const WS<KT> &
     bool set = false;
     if (zvcstar < Vm) {
       const double zvcint = fmax(zvcstar, Vl);
-      nact = (Nmid / Nnorm) * (intgN(zs1, N01, zvcint, Vm) + intgN(zs2, N02, Vm, Vh));
-      zactvol = (Nmid * Vm / Vnorm) * (intgV(zs1, N01, zvcint, Vm) + intgV(zs2, N02, Vm, Vh));
+      nact = (ddiv(Nmid, Nnorm)) * (intgN(zs1, N01, zvcint, Vm) + intgN(zs2, N02, Vm, Vh));
+      zactvol = (ddiv(Nmid * Vm, Vnorm)) * (intgV(zs1, N01, zvcint, Vm) + intgV(zs2, N02, Vm, Vh));
       set = true;
     } else if (zvcstar >= Vm) {
       const double zvcint = fmin(zvcstar, Vh);
-      nact = (Nmid / Nnorm) * (intgN(zs2, N02, zvcint, Vh));
-      zactvol = (Nmid * Vm / Vnorm) * (intgV(zs2, N02, zvcint, Vh));
+      nact = (ddiv(Nmid, Nnorm)) * (intgN(zs2, N02, zvcint, Vh));
+      zactvol = (ddiv(Nmid * Vm, Vnorm)) * (intgV(zs2, N02, zvcint, Vh));
       set = true;
     }
     nact = fmax(0., set ? nact : 0.);
     for (int ss = 0; ss < nwet; ss++) {
-      double v = set ? zactvol * (w.v(ss, ab) / (Vm * Nmid)) : 0.;
+      double v = set ? zactvol * (ddiv(w.v(ss, ab), Vm * Nmid)) : 0.;
       v = fmax(0., v);
       if (ss == iwa)   // the activated droplets' water (:1366-1367)
-        v = nact * K_PI6 * cube(zdcrit[ab]) * fmin(2., sq(3.e-6 / fmax(K_EPS, zdcrit[ab])));
-      raw[P.raw_vact + ss * ncld + cb] = v * P.rholiq[ss] / dn;
+        v = nact * K_PI6 * cube(zdcrit[ab]) * fmin(2., sq(ddiv(3.e-6, fmax(K_EPS, zdcrit[ab]))));
+      raw[P.raw_vact + ss * ncld + cb] = ddiv(v * P.rholiq[ss], dn);
     }
-    raw[P.raw_nact + cb] = nact / dn;
+    raw[P.raw_nact + cb] = ddiv(nact, dn);
   }
 }
 
 template <typename KT>
 __device__ void act_interst(const DevParams &P, const WS<KT> &w, const double *tb, double prv, double prs, double T,
                             bool diag, int lane) {
-  if (prv / prs <= 1.000) return;
+  if (ddiv(prv, prs) <= 1.000) return;
   const int ndry = P.ndry, nwet = P.nwet, iwa = P.iwa, C0 = P.nbins;
   const double *dmid = tb + TAB_DMID * P.nb_pad, *vrlo = tb + TAB_VRLO * P.nb_pad, *vrhi = tb + TAB_VRHI * P.nb_pad;
   const double THvol = 1.e-28;
-  double zkelvin = 4. * K_MWA * K_SURFW0 / (K_RG * K_RHOWA * T);
-  double zdcstar = 2. * zkelvin / (3. * ((prv / prs) - 1.));
+  double zkelvin = ddiv(4. * K_MWA * K_SURFW0, K_RG * K_RHOWA * T);
+  double zdcstar = ddiv(2. * zkelvin, 3. * ((ddiv(prv, prs)) - 1.));
   double zvcstar = K_PI6 * cube(zdcstar);
   double *actn = w.sc(8);        // per cloud bin
   double *actv = w.sc(0);        // [s * NB + cb] (reuses condensation scratch 0..nwet-1)
@@ -2668,14 +2669,14 @@ __device__ void act_interst(const DevParams &P, const WS<KT> &w, const double *t
       double Vlo = Vmid * vrlo[ab], Vhi = Vmid * vrhi[ab];
       double Nim1, Vim1, Vlom1, Vhim1, Vwim1, Nip1, Vip1, Vlop1, Vhip1, Vwip1;
       if (ab == P.in1a || ab == P.in2b) {
-        Nim1 = K_NLIM; Vim1 = Vlo / 2.; Vlom1 = 0.; Vhim1 = Vlo; Vwim1 = Vim1;
+        Nim1 = K_NLIM; Vim1 = divc(Vlo, 2.); Vlom1 = 0.; Vhim1 = Vlo; Vwim1 = Vim1;
       } else {
         Nim1 = w.numc[ab - 1];
         if (Nim1 > K_NLIM) {
           double vd = 0., vw = 0.;
           for (int s = 0; s < ndry; s++) vd += w.v(s, ab - 1);
           for (int s = 0; s < nwet; s++) vw += w.v(s, ab - 1);
-          Vim1 = vd / Nim1; Vwim1 = vw / Nim1;
+          Vim1 = ddiv(vd, Nim1); Vwim1 = ddiv(vw, Nim1);
         } else {
           Vim1 = K_PI6 * cube(dmid[ab - 1]); Vwim1 = K_PI6 * cube(dmid[ab - 1]);
         }
@@ -2689,7 +2690,7 @@ __device__ void act_interst(const DevParams &P, const WS<KT> &w, const double *t
           double vd = 0., vw = 0.;
           for (int s = 0; s < ndry; s++) vd += w.v(s, ab + 1);
           for (int s = 0; s < nwet; s++) vw += w.v(s, ab + 1);
-          Vip1 = vd / Nip1; Vwip1 = vw / Nip1;
+          Vip1 = ddiv(vd, Nip1); Vwip1 = ddiv(vw, Nip1);
         } else {
           Vip1 = K_PI6 * cube(dmid[ab + 1]); Vwip1 = K_PI6 * cube(dmid[ab + 1]);
         }
@@ -2697,8 +2698,8 @@ __device__ void act_interst(const DevParams &P, const WS<KT> &w, const double *t
       }
       Vip1 = fmax(Vhi, Vip1);
       Vim1 = fmin(Vlo, Vim1);
-      double zs1 = (Vwmid - fmax(Vwim1, 0.)) / (Vmid - Vim1);
-      double zs2 = (fmax(Vwip1, 0.) - Vwmid) / (Vip1 - Vmid);
+      double zs1 = ddiv(Vwmid - fmax(Vwim1, 0.), Vmid - Vim1);
+      double zs2 = ddiv(fmax(Vwip1, 0.) - Vwmid, Vip1 - Vmid);
       double V01 = Vwmid - zs1 * Vmid, V02 = Vwmid - zs2 * Vmid;
       double Vwlo = fmax(V01 + zs1 * Vlo, Vlo), Vwhi = fmax(V02 + zs2 * Vhi, Vhi);
       double vint1, vint2;
@@ -2708,25 +2709,25 @@ __device__ void act_interst(const DevParams &P, const WS<KT> &w, const double *t
       } else if (zvcstar > Vwlo && zvcstar > Vwmid && zvcstar > Vwhi) {
         vint1 = 999.; vint2 = 999.; r1 = r2 = r3 = r4 = false;
       } else {
-        double vcut = (zvcstar - V01) / zs1;
+        double vcut = ddiv(zvcstar - V01, zs1);
         vint1 = (vcut < Vlo || vcut > Vmid) ? Vlo : vcut;
-        vcut = (zvcstar - V02) / zs2;
+        vcut = ddiv(zvcstar - V02, zs2);
         vint2 = (vcut < Vmid || vcut > Vhi) ? Vmid : vcut;
         r1 = Vwlo > zvcstar; r2 = Vwmid > zvcstar; r3 = Vwmid > zvcstar; r4 = Vwhi > zvcstar;
       }
-      double dNim1 = Nim1 / (Vhim1 - Vlom1), dNip1 = Nip1 / (Vhip1 - Vlop1), dNmid = Nmid / (Vhi - Vlo);
-      zs1 = (dNmid - dNim1) / (Vmid - Vim1);
-      zs2 = (dNip1 - dNmid) / (Vip1 - Vmid);
+      double dNim1 = ddiv(Nim1, Vhim1 - Vlom1), dNip1 = ddiv(Nip1, Vhip1 - Vlop1), dNmid = ddiv(Nmid, Vhi - Vlo);
+      zs1 = ddiv(dNmid - dNim1, Vmid - Vim1);
+      zs2 = ddiv(dNip1 - dNmid, Vip1 - Vmid);
       double N01 = dNmid - zs1 * Vmid, N02 = dNmid - zs2 * Vmid;
       double Nnorm = intgN(zs1, N01, Vlo, Vmid) + intgN(zs2, N02, Vmid, Vhi);
       double Vnorm = intgV(zs1, N01, Vlo, Vmid) + intgV(zs2, N02, Vmid, Vhi);
       double zactvol = 0., Nact = 0.;
-      if (r1) { Nact += (Nmid / Nnorm) * intgN(zs1, N01, Vlo, vint1); zactvol += (Nmid * Vmid / Vnorm) * intgV(zs1, N01, Vlo, vint1); }
-      if (r2) { Nact += (Nmid / Nnorm) * intgN(zs1, N01, vint1, Vmid); zactvol += (Nmid * Vmid / Vnorm) * intgV(zs1, N01, vint1, Vmid); }
-      if (r3) { Nact += (Nmid / Nnorm) * intgN(zs2, N02, Vmid, vint2); zactvol += (Nmid * Vmid / Vnorm) * intgV(zs2, N02, Vmid, vint2); }
-      if (r4) { Nact += (Nmid / Nnorm) * intgN(zs2, N02, vint2, Vhi); zactvol += (Nmid * Vmid / Vnorm) * intgV(zs2, N02, vint2, Vhi); }
+      if (r1) { Nact += (ddiv(Nmid, Nnorm)) * intgN(zs1, N01, Vlo, vint1); zactvol += (ddiv(Nmid * Vmid, Vnorm)) * intgV(zs1, N01, Vlo, vint1); }
+      if (r2) { Nact += (ddiv(Nmid, Nnorm)) * intgN(zs1, N01, vint1, Vmid); zactvol += (ddiv(Nmid * Vmid, Vnorm)) * intgV(zs1, N01, vint1, Vmid); }
+      if (r3) { Nact += (ddiv(Nmid, Nnorm)) * intgN(zs2, N02, Vmid, vint2); zactvol += (ddiv(Nmid * Vmid, Vnorm)) * intgV(zs2, N02, Vmid, vint2); }
+      if (r4) { Nact += (ddiv(Nmid, Nnorm)) * intgN(zs2, N02, vint2, Vhi); zactvol += (ddiv(Nmid * Vmid, Vnorm)) * intgV(zs2, N02, vint2, Vhi); }
       an = fmin(Nact, Nmid);
-      for (int s = 0; s < nwet; s++) av[s] = fmin(zactvol * (w.v(s, ab) / (Vmid * Nmid)), w.v(s, ab));
+      for (int s = 0; s < nwet; s++) av[s] = fmin(zactvol * (ddiv(w.v(s, ab), Vmid * Nmid)), w.v(s, ab));
     }
     actn[cb] = an;
     for (int s = 0; s < nwet; s++) actv[s * w.NB + cb] = av[s];
@@ -2740,7 +2741,7 @@ __device__ void act_interst(const DevParams &P, const WS<KT> &w, const double *t
   for (int cb = lane; cb < P.ncld; cb += 32) {
     int ab = P.ica_par + cb, cg = C0 + cb;
     double an = actn[cb];
-    if (an > 0.) w.ctime[cg] = (an * P.chargeTimeMax + w.numc[cg] * w.ctime[cg]) / (an + w.numc[cg]);
+    if (an > 0.) w.ctime[cg] = ddiv(an * P.chargeTimeMax + w.numc[cg] * w.ctime[cg], an + w.numc[cg]);
     w.numc[ab] = fmax(0., w.numc[ab] - an);
     double nc = w.numc[cg] + an;
     w.numc[cg] = nc;
@@ -2749,7 +2750,7 @@ __device__ void act_interst(const DevParams &P, const WS<KT> &w, const double *t
       w.v(s, ab) = fmax(0., w.v(s, ab) - av);
       w.v(s, cg) = w.v(s, cg) + av;
     }
-    if (nc > 0.) w.indef[cg] = (w.indef[cg] * (nc - an) + w.indef[ab] * an) / nc;
+    if (nc > 0.) w.indef[cg] = ddiv(w.indef[cg] * (nc - an) + w.indef[ab] * an, nc);
   }
   __syncwarp();
 }
@@ -2767,18 +2768,18 @@ __device__ void autoconv2(const DevParams &P, const WS<KT> &w, double dt, int la
       for (int s = 0; s < P.nwet; s++) Vtot += w.v(s, g);
       if (Ntot > K_NLIM && Vtot > 0.) {
         double ls = log(sigmag);
-        double dvg = cbrt(Vtot / Ntot / K_PI6) * exp((3. * ls * ls) / 2.);
+        double dvg = dcbrt(divc(ddiv(Vtot, Ntot), K_PI6)) * exp((3. * ls * ls) / 2.);
         double dg = dvg * exp(-3. * ls * ls);
         double hlp2 = sqrt(2.) * ls;
-        double Vrem = Vtot * (1. - (0.5 + 0.5 * erf((log(zd0) - log(dvg)) / hlp2)));
-        double Nrem = Ntot * (1. - (0.5 + 0.5 * erf((log(zd0) - log(dg)) / hlp2)));
+        double Vrem = Vtot * (1. - (0.5 + 0.5 * erf(ddiv(log(zd0) - dlog(dvg), hlp2))));
+        double Nrem = Ntot * (1. - (0.5 + 0.5 * erf(ddiv(log(zd0) - dlog(dg), hlp2))));
         if (Vrem > 0. && Nrem > K_PRLIM) {
           for (int s = 0; s < P.ndry; s++) {
-            w.v(s, P0) = w.v(s, P0) + w.v(s, g) * (Nrem / Ntot);
-            w.v(s, g) = w.v(s, g) * (1. - (Nrem / Ntot));
+            w.v(s, P0) = w.v(s, P0) + w.v(s, g) * (ddiv(Nrem, Ntot));
+            w.v(s, g) = w.v(s, g) * (1. - (ddiv(Nrem, Ntot)));
           }
-          w.v(P.iwa, P0) = w.v(P.iwa, P0) + w.v(P.iwa, g) * (Vrem / Vtot);
-          w.v(P.iwa, g) = w.v(P.iwa, g) * (1. - (Vrem / Vtot));
+          w.v(P.iwa, P0) = w.v(P.iwa, P0) + w.v(P.iwa, g) * (ddiv(Vrem, Vtot));
+          w.v(P.iwa, g) = w.v(P.iwa, g) * (1. - (ddiv(Vrem, Vtot)));
           w.numc[P0] = w.numc[P0] + Nrem;
           w.numc[g] = w.numc[g] - Nrem;
           tot = tot + Nrem;
@@ -2816,30 +2817,30 @@ __device__ double erfm1(double x) {   // math_functions.f90:494-510
   const double a = 0.140012;
   double sgn = x < 0. ? -1. : 1.;
   double xx = fmax(1.e-20, 1. - x * x);
-  double t1 = log(xx), t2 = 2. / (K_PI_FULL * a);
-  double t3 = t2 + mrn(0.5, t1), t4 = t1 / a, t5 = t2 + mrn(0.5, t1);
-  return sgn * sqrt(sqrt(mrn(t3, t3) - t4) - t5);
+  double t1 = dlog(xx), t2 = 2. / (K_PI_FULL * a);
+  double t3 = t2 + mrn(0.5, t1), t4 = divc(t1, a), t5 = t2 + mrn(0.5, t1);
+  return sgn * dsqrt(dsqrt(mrn(t3, t3) - t4) - t5);
 }
 // f_gauss (:515-524) with its per-configuration factors 1/(sqrt(2 pi) sig) and 1/sig^2
 // taken once per cell
 struct GaussC { double ra, rs2, mean; };
 __device__ __forceinline__ GaussC gauss_c(double sig, double mean) {
   GaussC g;
-  g.ra = 1. / (sqrt(2. * K_PI_FULL) * sig);
-  g.rs2 = 1. / (sig * sig);
+  g.ra = drcp(sqrt(2. * K_PI_FULL) * sig);
+  g.rs2 = drcp(sig * sig);
   g.mean = mean;
   return g;
 }
 __device__ __forceinline__ double f_gauss(double x, const GaussC &g) {
   double b = (x - g.mean) * (x - g.mean);
   b = b * g.rs2;
-  return g.ra * exp(-0.5 * b);
+  return g.ra * dexp(-0.5 * b);
 }
 __device__ double het_sf(double x, double mis) {   // SE :375-390
-  if (x > 100.) return (cube_rn(mis) - mrn(3., mis) + 2.) / 4.;
-  double fii = sqrt(1. - mrn(mrn(2., mis), x) + mrn(x, x));
-  double fpsi = (x - mis) / fii;
-  return 0.5 * (1. + cube_rn((1. - mrn(mis, x)) / fii) + mrn(2. - mrn(3., fpsi) + cube_rn(fpsi), cube_rn(x)) +
+  if (x > 100.) return divc(cube_rn(mis) - mrn(3., mis) + 2., 4.);
+  double fii = dsqrt(1. - mrn(mrn(2., mis), x) + mrn(x, x));
+  double fpsi = ddiv(x - mis, fii);
+  return 0.5 * (1. + cube_rn(ddiv(1. - mrn(mis, x), fii)) + mrn(2. - mrn(3., fpsi) + cube_rn(fpsi), cube_rn(x)) +
                 mrn(mrn(mrn(mrn(3., mis), fpsi - 1.), x), x));
 }
 
@@ -2849,50 +2850,50 @@ __device__ JimmPre jimm_pre(double Tk, double Seq) {
   JimmPre r;
   const double rho_ice = 900., T0 = 273.15;
   double Tc = Tk - T0;
-  r.act_energy = K_RG * Tk * (347. / (Tk - 177.) - log(4.14 / 349.)) / K_AVOG;
+  r.act_energy = divc(K_RG * Tk * (ddiv(347., Tk - 177.) - log(4.14 / 349.)), K_AVOG);
   r.sigma_is = 28.e-3 + mrn(0.25e-3, Tc);
   double Lefm = (79.7 + mrn(0.708, Tc) - mrn(mrn(2.5e-3, Tc), Tc)) * 4.1868e3;
-  double GG = K_RG * Tk / K_MWA / Lefm;
-  double sg = pow(Seq, GG);
-  r.ok = !((T0 / Tk) * sg < 1.0001);
-  r.d_g = r.ok ? 4. * r.sigma_is / (mrn(mrn(rho_ice, Lefm), log((T0 / Tk) * sg)) - 1.7e10 * 0.) : 0.;
+  double GG = ddiv(divc(K_RG * Tk, K_MWA), Lefm);
+  double sg = dpow(Seq, GG);
+  r.ok = !((ddiv(T0, Tk)) * sg < 1.0001);
+  r.d_g = r.ok ? ddiv(4. * r.sigma_is, mrn(mrn(rho_ice, Lefm), dlog((ddiv(T0, Tk)) * sg)) - 1.7e10 * 0.) : 0.;
   if (r.d_g <= 1e-10) r.ok = false;
   return r;
 }
 // kth = K_BOLTZ * Tk / K_PLANCK, taken once per cell
 __device__ double J_imm(const JimmPre &q, double theta, double Tk, double Din, double kth) {
   if (Din < 1e-10 || !q.ok) return 0.;
-  double costh = cos(theta * K_PI / 180.);
-  double sf = het_sf(Din / q.d_g, costh);
+  double costh = cos(divc(theta * K_PI, 180.));
+  double sf = het_sf(ddiv(Din, q.d_g), costh);
   double crit = mrn(mrn(mrn((K_PI / 3.), q.sigma_is), mrn(q.d_g, q.d_g)), sf) -
                 mrn(mrn(mrn((1. / 4.) * 0.0, (1. - costh)), Din), Din);
-  return kth * 1.e19 * K_PI * (Din * Din) * exp(-(q.act_energy + crit) / (K_BOLTZ * Tk));
+  return kth * 1.e19 * K_PI * (Din * Din) * dexp(-ddiv(q.act_energy + crit, K_BOLTZ * Tk));
 }
 __device__ double J_dep(double theta, double Tk, double Din, double Seq) {   // :282-331
   if (Din < 1e-10 || Seq < 1.0001) return 0.;
   double Tc = Tk - 273.15;
   double sigma_iv = ((76.1 - mrn(0.155, Tc)) + (28.5 + mrn(0.25, Tc))) * 1.e-3;
-  double d_g = 4. * sigma_iv / (mrn(K_RG * K_RHOIC / K_MWA * Tk, log(Seq)) - 1.7e10 * 0.);
+  double d_g = ddiv(4. * sigma_iv, mrn(K_RG * K_RHOIC / K_MWA * Tk, dlog(Seq)) - 1.7e10 * 0.);
   if (d_g <= 1e-10) return 0.;
-  double costh = cos(theta * K_PI / 180.);
-  double sf = het_sf(Din / d_g, costh);
+  double costh = cos(divc(theta * K_PI, 180.));
+  double sf = het_sf(ddiv(Din, d_g), costh);
   double crit = (K_PI / 3.) * sigma_iv * (d_g * d_g) * sf;
-  return (1. / 4.) * 1.e30 * (Din * Din) * exp(-(0. + crit) / (K_BOLTZ * Tk));
+  return (1. / 4.) * 1.e30 * (Din * Din) * dexp(-ddiv(0. + crit, K_BOLTZ * Tk));
 }
 __device__ double J_hf(double Tk, double Sw) {   // :335-371
   const double Nc = 5.85e16, T0 = 273.15;
   double Tc = Tk - T0;
   double act = 0.694e-19 * (1. + mrn(0.027, (Tc + 30.)));
   double Lefm = (79.7 + mrn(0.708, Tc) - mrn(mrn(2.5e-3, Tc), Tc)) * 4.1868e3;
-  double GG = K_RG * Tk / Lefm / K_MWA;
-  double sg = pow(Sw, GG);
-  if ((T0 / Tk) * sg < 1.0001) return 0.;
+  double GG = divc(ddiv(K_RG * Tk, Lefm), K_MWA);
+  double sg = dpow(Sw, GG);
+  if ((ddiv(T0, Tk)) * sg < 1.0001) return 0.;
   double sigma_is = 28.e-3 + mrn(0.25e-3, Tc);
-  double d_g = 4. * sigma_is / (K_RHOIC * Lefm * log((T0 / Tk) * sg));
+  double d_g = ddiv(4. * sigma_is, K_RHOIC * Lefm * dlog((ddiv(T0, Tk)) * sg));
   if (d_g <= 1e-10) return 0.;
   double crit = (K_PI / 3.) * sigma_is * d_g * d_g;
-  return 2.0 * Nc * (K_RHOWA * K_BOLTZ * Tk / K_RHOIC / K_PLANCK) * sqrt(sigma_is / K_BOLTZ / Tk) *
-         exp(-(crit + act) / (K_BOLTZ * Tk));
+  return 2.0 * Nc * (divc(divc(K_RHOWA * K_BOLTZ * Tk, K_RHOIC), K_PLANCK)) * dsqrt(ddiv(divc(sigma_is, K_BOLTZ), Tk)) *
+         dexp(-ddiv(crit + act, K_BOLTZ * Tk));
 }
 
 // calcSweq (mo_particle_external_properties.f90:402-447)
@@ -2902,29 +2903,29 @@ __device__ double calc_sweq(const DevParams &P, const WS<KT> &w, int b, double T
   if (n < nlim_of(phase_of(P, b))) return 0.;
   double vs = 0.;
   for (int s = 0; s < P.nused; s++) vs += w.v(s, b);
-  double dwet = cbrt(vs / n / K_PI6);
-  double znw = w.v(P.iwa, b) * K_RHOWA / K_MWA, zvw = w.v(P.iwa, b);
+  double dwet = dcbrt(divc(ddiv(vs, n), K_PI6));
+  double znw = divc(w.v(P.iwa, b) * K_RHOWA, K_MWA), zvw = w.v(P.iwa, b);
   double zns = 0., zvs = 0., zvtot = 0.;
   for (int i = 0; i < P.ndry; i++) {
-    zns = zns + P.diss[i] * w.v(i, b) * P.rholiq[i] / P.MM[i];
+    zns = zns + ddiv(P.diss[i] * w.v(i, b) * P.rholiq[i], P.MM[i]);
     zvs = zvs + mrn(fmin(1., P.diss[i]), w.v(i, b));
     zvtot = zvtot + w.v(i, b);
   }
   if (P.has_kappa) zns = solute_moles(P, w, b, kappa);
-  double kel = exp(4. * K_SURFW0 * K_MWA / (K_RG * T * K_RHOWA * dwet));
-  if (zvw > 1.e-28 * n || zvs > 1.e-28 * n) return (znw / (zns + znw)) * kel;
+  double kel = dexp(ddiv(4. * K_SURFW0 * K_MWA, K_RG * T * K_RHOWA * dwet));
+  if (zvw > 1.e-28 * n || zvs > 1.e-28 * n) return (ddiv(znw, zns + znw)) * kel;
   if (zvtot - zvs > 1.e-28 * n) return kel;
-  return (znw / (K_EPS + zns + znw)) * kel;
+  return (ddiv(znw, K_EPS + zns + znw)) * kel;
 }
 
 __device__ __forceinline__ int ice_bin_of(const DevParams &P, const double *vlo, double dwet) {   // :542-555
-  double vol = K_PI6 * cube(dwet) * K_RHOWA / K_RHOIC;
+  double vol = divc(K_PI6 * cube(dwet) * K_RHOWA, K_RHOIC);
   int ii = 0;
   for (int k = 0; k < P.nice; k++) ii += (vlo[P.nliquid + k] < vol);
   return min(max(1, ii), P.nice) - 1;
 }
 __device__ __forceinline__ int precip_bin_of(const DevParams &P, const double *vlo, double dwet, double dens) {
-  double vol = K_PI6 * cube(dwet) * dens / K_RHOWA;   // :559-573
+  double vol = divc(K_PI6 * cube(dwet) * dens, K_RHOWA);   // :559-573
   int ii = 0;
   for (int k = 0; k < P.nprc; k++) ii += (vlo[P.nbins + P.ncld + k] < vol);
   return min(max(1, ii), P.nprc) - 1;
@@ -2966,7 +2967,7 @@ __device__ void ice_nucl_SE(const DevParams &P, const WS<KT> &w, const double *t
   // per-bin records in the (now unused) collision-kernel area: 8 doubles per bin
   double *rec = reinterpret_cast<double *>(w.K);
   enum { R_MODE = 0, R_THMIN, R_DIN, R_AE, R_SIG, R_DG, R_FHOM, R_FINT };
-  const double Si = prv / prsi;
+  const double Si = ddiv(prv, prsi);
   // pass A
   for (int kk = lane; kk < nl; kk += 32) {
     double *st = stage + kk * 10;
@@ -2980,14 +2981,14 @@ __device__ void ice_nucl_SE(const DevParams &P, const WS<KT> &w, const double *t
     const bool countable = !(T > 273.15) && !(n < nlim_of(ph));
     const bool hom = dwet - dins_ > dmin && T < tmax_homog && P.lsicehom;
     const bool imm = P.lsiceimm && (ph == 2 || ph == 3) && (w.dins[kk] > dmin) && countable;
-    const bool dep = P.lsicedep && (ph == 1 && prv / prs < 1.0) && (w.dwet[kk] - w.dins[kk] < dmin) &&
+    const bool dep = P.lsicedep && (ph == 1 && ddiv(prv, prs) < 1.0) && (w.dwet[kk] - w.dins[kk] < dmin) &&
                      (w.dins[kk] > dmin) && countable;
     double Seq = 0.;
     if (hom || imm) Seq = calc_sweq(P, w, kk, T, kappa);
     double f_hom = 0.;
     if (hom) {
       double Jh = J_hf(T, Seq);
-      f_hom = 1. - exp(-Jh * K_PI6 * (cube_rn(dwet) - cube_rn(dins_)) * dt);
+      f_hom = 1. - dexp(-Jh * K_PI6 * (cube_rn(dwet) - cube_rn(dins_)) * dt);
     }
     r[R_FHOM] = f_hom;
     r[R_MODE] = imm ? 1. : (dep ? 2. : 0.);
@@ -3024,7 +3025,7 @@ __device__ void ice_nucl_SE(const DevParams &P, const WS<KT> &w, const double *t
     const int grp = lane / 10, node = lane - grp * 10;
     const GaussC g_imm = gauss_c(P.sigma_theta_imm, P.mean_theta_imm);
     const GaussC g_dep = gauss_c(P.sigma_theta_dep, P.mean_theta_dep);
-    const double kth = K_BOLTZ * T / K_PLANCK;
+    const double kth = divc(K_BOLTZ * T, K_PLANCK);
     for (int b0 = 0; b0 < nlist; b0 += 3) {
       const int slot = b0 + grp;
       const bool on = grp < 3 && slot < nlist;
@@ -3044,7 +3045,7 @@ __device__ void ice_nucl_SE(const DevParams &P, const WS<KT> &w, const double *t
           J = J_dep(th1, T, r[R_DIN], Si);
           ft = th1 > thmin ? f_gauss(th1, g_dep) : 0.;
         }
-        term = ft * c_gl_w[node] * (1. - exp(-J * dt));
+        term = ft * c_gl_w[node] * (1. - dexp(-J * dt));
       }
       double acc = 0.;
       const int g10 = (grp < 3 ? grp : 0) * 10;
@@ -3078,13 +3079,13 @@ __device__ void ice_nucl_SE(const DevParams &P, const WS<KT> &w, const double *t
     double vdry = 0.;
     for (int s = 0; s < ndry; s++) vdry += w.v(s, kk);
     double V_tot = frac * vdry;
-    double frac_DU = w.v(idu, kk) / vdry;
+    double frac_DU = ddiv(w.v(idu, kk), vdry);
     double frac2, ncur0;
     if (frac_DU <= 0.1) { frac2 = frac * frac_DU; ncur0 = n * frac_DU; }
     else { frac2 = frac; ncur0 = n; }
     double nnuc = frac2 * n;
     double f1 = nnuc + mrn((ncur0 - nnuc), w.indef[kk]);
-    f1 = f1 / ncur0;
+    f1 = ddiv(f1, ncur0);
     w.indef[kk] = fmin(fmax(f1, 0.), 1. - 1.e-20);
     st[0] = (double)bb;
     st[9] = 1.;
@@ -3099,9 +3100,9 @@ __device__ void ice_nucl_SE(const DevParams &P, const WS<KT> &w, const double *t
       }
     }
     if (ph == 1 || ph == 2) {
-      if (mk) st[1 + iwa] = w.v(iwa, kk) * frac2 * K_RHOWA / K_RHOIC;
+      if (mk) st[1 + iwa] = divc(w.v(iwa, kk) * frac2 * K_RHOWA, K_RHOIC);
     } else {
-      if (mk) st[1 + irim] = w.v(iwa, kk) * frac2 * K_RHOWA / K_RHORI;
+      if (mk) st[1 + irim] = divc(w.v(iwa, kk) * frac2 * K_RHOWA, K_RHORI);
     }
     w.v(iwa, kk) = fmax(0., w.v(iwa, kk) * (1. - frac2));
     if (mk) st[8] = n * frac2;
@@ -3125,44 +3126,44 @@ __device__ double calc_Jhet(double rn, double temp, double Sw) {
   const double rho_ice = 900., c_1s = 1e32, T0 = 273.15, mis = 0.5;
   if (rn < 1e-10) return 0.;
   double Tc = temp - T0;
-  double act = K_RG * temp * (347. / (temp - 177.) - log(4.14 / 349.)) / K_AVOG;
+  double act = divc(K_RG * temp * (ddiv(347., temp - 177.) - log(4.14 / 349.)), K_AVOG);
   double Lefm = (79.7 + mrn(0.708, Tc) - mrn(mrn(2.5e-3, Tc), Tc)) * 4.1868e3;
-  double GG = K_RG * temp / K_MWA / Lefm;
-  double sg = pow(Sw, GG);
-  if ((T0 / temp) * sg < 1.0001) return 0.;
+  double GG = ddiv(divc(K_RG * temp, K_MWA), Lefm);
+  double sg = dpow(Sw, GG);
+  if ((ddiv(T0, temp)) * sg < 1.0001) return 0.;
   double sigma_is = 28.e-3 + mrn(0.25e-3, Tc);
-  double r_g = 4. * sigma_is / (mrn(mrn(rho_ice, Lefm), log((T0 / temp) * sg)) - 1.7e10 * 0.);
+  double r_g = ddiv(4. * sigma_is, mrn(mrn(rho_ice, Lefm), dlog((ddiv(T0, temp)) * sg)) - 1.7e10 * 0.);
   if (r_g <= 1e-10) return 0.;
-  double sf = het_sf(rn / r_g, mis);
+  double sf = het_sf(ddiv(rn, r_g), mis);
   double crit = mrn(mrn(mrn(mrn((K_PI / 3.), sigma_is), r_g), r_g), sf) -
                 mrn(mrn(mrn((1. / 4.) * 0.0, (1. - mis)), rn), rn);
-  return K_BOLTZ * temp / K_PLANCK * c_1s * K_PI * rn * rn * exp((-act - crit) / (K_BOLTZ * temp));
+  return divc(K_BOLTZ * temp, K_PLANCK) * c_1s * K_PI * rn * rn * dexp(ddiv(-act - crit, K_BOLTZ * temp));
 }
 __device__ double calc_Jdep(double rn, double temp, double Si) {
   const double rho_ice = 900., mis = 0.5;
   if (rn < 1e-10 || Si < 1.0001) return 0.;
   double Tc = temp - 273.15;
   double sigma_iv = ((76.1 - mrn(0.155, Tc)) + (28.5 + mrn(0.25, Tc))) * 1e-3;
-  double r_g = 4. * sigma_iv / (mrn(K_RG * rho_ice / K_MWA * temp, log(Si)) - 1.7e10 * 0.);
+  double r_g = ddiv(4. * sigma_iv, mrn(K_RG * rho_ice / K_MWA * temp, dlog(Si)) - 1.7e10 * 0.);
   if (r_g <= 1e-10) return 0.;
-  double sf = het_sf(rn / r_g, mis);
+  double sf = het_sf(ddiv(rn, r_g), mis);
   double crit = (K_PI / 3.) * sigma_iv * r_g * r_g * sf;
-  return (1. / 4.) * 1.e30 * rn * rn * exp((-0. - crit) / (K_BOLTZ * temp));
+  return (1. / 4.) * 1.e30 * rn * rn * dexp(ddiv(-0. - crit, K_BOLTZ * temp));
 }
 __device__ double calc_Jhf(double temp, double Sw) {
   const double Nc = 5.85e16, rho_ice = 900., T0 = 273.15;
   double Tc = temp - T0;
   double act = 0.694e-19 * (1. + mrn(0.027, (Tc + 30.)));
   double Lefm = (79.7 + mrn(0.708, Tc) - mrn(mrn(2.5e-3, Tc), Tc)) * 4.1868e3;
-  double GG = K_RG * temp / Lefm / K_MWA;
-  double sg = pow(Sw, GG);
-  if ((T0 / temp) * sg < 1.0001) return 0.;
+  double GG = divc(ddiv(K_RG * temp, Lefm), K_MWA);
+  double sg = dpow(Sw, GG);
+  if ((ddiv(T0, temp)) * sg < 1.0001) return 0.;
   double sigma_is = 28.e-3 + mrn(0.25e-3, Tc);
-  double r_g = 2. * sigma_is / (rho_ice * Lefm * log((T0 / temp) * sg));
+  double r_g = ddiv(2. * sigma_is, rho_ice * Lefm * dlog((ddiv(T0, temp)) * sg));
   if (r_g <= 1e-10) return 0.;
   double crit = 4. * K_PI / 3. * sigma_is * r_g * r_g;
-  return 2.0 * Nc * (K_RHOWA * K_BOLTZ * temp / rho_ice / K_PLANCK) * sqrt(sigma_is / K_BOLTZ / temp) *
-         exp((-crit - act) / (K_BOLTZ * temp));
+  return 2.0 * Nc * (divc(divc(K_RHOWA * K_BOLTZ * temp, rho_ice), K_PLANCK)) * dsqrt(ddiv(divc(sigma_is, K_BOLTZ), temp)) *
+         dexp(ddiv(-crit - act, K_BOLTZ * temp));
 }
 
 template <typename KT>
@@ -3183,11 +3184,11 @@ __device__ void ice_nucl_classic(const DevParams &P, const WS<KT> &w, const doub
     double dins_ = w.dins[kk], dwet = w.dwet[kk];
     double Sw = calc_sweq(P, w, kk, T, kappa);
     double pf_imm = 0., pf_dep = 0., pf_hom = 0.;
-    if (dins_ > dmin && P.lsiceimm && (ph == 2 || ph == 3)) pf_imm = 1. - exp(-calc_Jhet(dins_, T, Sw) * dt);
-    if (dins_ > dmin && dwet - dins_ < dmin && prv / prs < 1.0 && ph == 1 && P.lsicedep)
-      pf_dep = 1. - exp(-calc_Jdep(dins_, T, prv / prsi) * dt);
+    if (dins_ > dmin && P.lsiceimm && (ph == 2 || ph == 3)) pf_imm = 1. - dexp(-calc_Jhet(dins_, T, Sw) * dt);
+    if (dins_ > dmin && dwet - dins_ < dmin && ddiv(prv, prs) < 1.0 && ph == 1 && P.lsicedep)
+      pf_dep = 1. - dexp(-calc_Jdep(dins_, T, ddiv(prv, prsi)) * dt);
     if (dwet - dins_ > dmin && T < tmax_homog && P.lsicehom)
-      pf_hom = 1. - exp(-calc_Jhf(T, Sw) * K_PI6 * (cube_rn(dwet) - cube_rn(dins_)) * dt);
+      pf_hom = 1. - dexp(-calc_Jhf(T, Sw) * K_PI6 * (cube_rn(dwet) - cube_rn(dins_)) * dt);
     double frac = fmax(0., fmin(0.99, pf_imm + pf_hom + pf_dep - mrn((pf_imm + pf_dep), pf_hom)));
     int bb = ice_bin_of(P, vlo, dwet);
     bool mk = P.st_icenucl;
@@ -3197,8 +3198,8 @@ __device__ void ice_nucl_classic(const DevParams &P, const WS<KT> &w, const doub
       if (mk) st[1 + s] = w.v(s, kk) * frac;
       w.v(s, kk) = fmax(0., w.v(s, kk) * (1. - frac));
     }
-    if (ph == 1 || ph == 2) { if (mk) st[1 + iwa] = w.v(iwa, kk) * frac * K_RHOWA / K_RHOIC; }
-    else { if (mk) st[1 + irim] = w.v(iwa, kk) * frac * K_RHOWA / K_RHORI; }
+    if (ph == 1 || ph == 2) { if (mk) st[1 + iwa] = divc(w.v(iwa, kk) * frac * K_RHOWA, K_RHOIC); }
+    else { if (mk) st[1 + irim] = divc(w.v(iwa, kk) * frac * K_RHOWA, K_RHORI); }
     w.v(iwa, kk) = fmax(0., w.v(iwa, kk) * (1. - frac));
     if (mk) st[8] = w.numc[kk] * frac;
     double nn = fmax(0., w.numc[kk] * (1. - frac));
@@ -3241,7 +3242,7 @@ __device__ void ice_melt(const DevParams &P, const WS<KT> &w, const double *tb, 
     if (n > K_PRLIM) {
       double vs = 0.;
       for (int s = 0; s < P.nused; s++) vs += w.v(s, g);
-      dw = cbrt(vs / n / K_PI6);
+      dw = dcbrt(divc(ddiv(vs, n), K_PI6));
     } else {
       dw = dmid[g];
     }
@@ -3255,7 +3256,7 @@ __device__ void ice_melt(const DevParams &P, const WS<KT> &w, const double *tb, 
       st[1 + s] = maxfrac * w.v(s, g);
       w.v(s, g) = (1. - maxfrac) * w.v(s, g);
     }
-    double liqvol = (w.v(iwa, g) * K_RHOIC + w.v(irim, g) * K_RHORI) / K_RHOWA;
+    double liqvol = divc(w.v(iwa, g) * K_RHOIC + w.v(irim, g) * K_RHORI, K_RHOWA);
     st[8] = maxfrac * n;
     w.numc[g] = (1. - maxfrac) * n;
     st[1 + iwa] = maxfrac * liqvol;
@@ -3315,7 +3316,7 @@ __device__ __forceinline__ void distr_bin(const DevParams &P, const double *tb, 
   for (int s = 0; s < SALSA_NSV; s++) if (s < nsum) sd += v[s];
   if (CAT == DC_AERO) {
     if (!(n > K_NLIM) || g == P.fn2a) return;
-    const double zvpart = sd / n;
+    const double zvpart = ddiv(sd, n);
     if (vlo[g] > zvpart) {
       if (g == P.in1a) return;
       o.dir = -1; o.target = (g == P.in2b) ? P.fn1a : g - 1;
@@ -3325,17 +3326,17 @@ __device__ __forceinline__ void distr_bin(const DevParams &P, const double *tb, 
       return;
     }
     if (zvpart <= K_PI6 * cube(dmid[g])) return;
-    const double zVrat = vhi[g] / vlo[g];
-    const double zVilo = 2. * zvpart / (1. + zVrat);
+    const double zVrat = ddiv(vhi[g], vlo[g]);
+    const double zVilo = ddiv(2. * zvpart, 1. + zVrat);
     const double zVihi = zVrat * zVilo;
     const double zVexc = 0.5 * (zVihi + vhi[g]);
-    const double znfrac = fmin(1., (zVihi - vhi[g]) / (zVihi - zVilo));
-    const double zvfrac = fmin(0.99, znfrac * zVexc / zvpart);
+    const double znfrac = fmin(1., ddiv(zVihi - vhi[g], zVihi - zVilo));
+    const double zvfrac = fmin(0.99, ddiv(znfrac * zVexc, zvpart));
     o.neg = zvfrac < 0.;
     const double f = znfrac * n * zVexc;
 #pragma unroll
     for (int s = 0; s < SALSA_NSV; s++)
-      if (s < nmove) { double mv = f * v[s] / sd; o.push[s] = mv; o.own[s] = v[s] - mv; }
+      if (s < nmove) { double mv = ddiv(f * v[s], sd); o.push[s] = mv; o.own[s] = v[s] - mv; }
     o.dir = 1; o.target = g + 1;
     o.push_n = znfrac * n;
     o.own_n = n * (1. - znfrac);
@@ -3343,26 +3344,26 @@ __device__ __forceinline__ void distr_bin(const DevParams &P, const double *tb, 
       double s2 = 0.;
 #pragma unroll
       for (int s = 0; s < SALSA_NSV; s++) if (s < nsum) s2 += o.own[s];
-      const double zp = s2 / o.own_n;
+      const double zp = ddiv(s2, o.own_n);
       o.check = true; o.within = (vlo[g] < zp && zp < vhi[g]);
     }
     return;
   }
   const double lim = (CAT == DC_CLOUD) ? K_NLIM : K_PRLIM;
   if (!(n > lim) || (CAT == DC_CLOUD && !(sd > 1.e-30))) return;
-  const double zvpart = sd / n;
-  const double zVrat = vhi[g] / vlo[g];
-  const double zVilo = 2. * zvpart / (1. + zVrat);
+  const double zvpart = ddiv(sd, n);
+  const double zVrat = ddiv(vhi[g], vlo[g]);
+  const double zVilo = ddiv(2. * zvpart, 1. + zVrat);
   const double zVihi = zVrat * zVilo;
   double zVexc, znfrac;
   if (CAT == DC_CLOUD) {
     if (zvpart < vlo[g] && (kk != P.ica_cur && kk != P.icb_cur)) {
       zVexc = 0.5 * (zVilo + vlo[g]);
-      znfrac = fmin(1., (vlo[g] - zVilo) / (zVihi - zVilo));
+      znfrac = fmin(1., ddiv(vlo[g] - zVilo, zVihi - zVilo));
       o.dir = -1;
     } else if (zvpart > vhi[g] && (kk != P.fca_cur && kk != P.fcb_cur)) {
       zVexc = 0.5 * (zVihi + vhi[g]);
-      znfrac = fmin(1., (zVihi - vhi[g]) / (zVihi - zVilo));
+      znfrac = fmin(1., ddiv(zVihi - vhi[g], zVihi - zVilo));
       o.dir = 1;
     } else {
       return;
@@ -3373,18 +3374,18 @@ __device__ __forceinline__ void distr_bin(const DevParams &P, const double *tb, 
     const double zvdec = vm - 0.2 * (vm - vlo[g]);
     if (zvpart < zvdec && kk != 0) {
       zVexc = 0.5 * (zVilo + vlo[g]);
-      znfrac = fmin(1., (vlo[g] - zVilo) / (zVihi - zVilo));
+      znfrac = fmin(1., ddiv(vlo[g] - zVilo, zVihi - zVilo));
       o.dir = -1;
     } else if (zvpart > vm && kk != ntop) {
       zVexc = 0.5 * (zVihi + vhi[g]);
-      znfrac = fmin(0.99, (zVihi - vhi[g]) / (zVihi - zVilo));
+      znfrac = fmin(0.99, ddiv(zVihi - vhi[g], zVihi - zVilo));
       o.dir = 1;
     } else {
       return;
     }
   }
   o.target = g + o.dir;
-  const double zvfrac = fmin(0.99, znfrac * zVexc / zvpart);
+  const double zvfrac = fmin(0.99, ddiv(znfrac * zVexc, zvpart));
   o.neg = zvfrac < 0.;
 #pragma unroll
   for (int s = 0; s < SALSA_NSV; s++)
@@ -3396,7 +3397,7 @@ __device__ __forceinline__ void distr_bin(const DevParams &P, const double *tb, 
   for (int s = 0; s < SALSA_NSV; s++) if (s < nsum) s2 += o.own[s];
   const bool chk = (CAT == DC_PRECP) ? (o.own_n > lim) : (o.own_n > lim && s2 > 1.e-30);
   if (chk) {
-    const double zp = s2 / o.own_n;
+    const double zp = ddiv(s2, o.own_n);
     o.check = true; o.within = (vlo[g] < zp && zp < vhi[g]);
   }
 }
@@ -3637,7 +3638,7 @@ __device__ __forceinline__ void cell_step(const DevParams &P, const WS<KT> &w, c
   // (x / dn - old) / dt: one division for 1/dn per cell, and the quotient by dt as a
   // product when dt is a power of two (then it is the same number)
   bool bad = false;
-  const double idn = 1. / dn;
+  const double idn = drcp(dn);
   for (int e = lane; e < nmrow; e += 32) {
     const int r = m0 + e;
     const int icat = (ncat == 4 && r >= P.raw_mbase[3]) ? 3 : (r >= P.raw_mbase[2] ? 2 : (r >= P.raw_mbase[1] ? 1 : 0));
@@ -3645,7 +3646,7 @@ __device__ __forceinline__ void cell_step(const DevParams &P, const WS<KT> &w, c
     const int sp = loc / nbc, b = bstart[icat] + (loc - sp * nbc);
     const double rho = icat < 3 ? P.rholiq[sp] : (sp < nwet ? P.rhoice[sp] : K_RHORI);
     const double d = (w.v(sp, b) * rho * idn) - raw[r];
-    raw[r] = P.inv_dt != 0. ? d * P.inv_dt : d / dt;
+    raw[r] = P.inv_dt != 0. ? d * P.inv_dt : ddiv(d, dt);
   }
   for (int b = lane; b < P.ntotal; b += 32) {
     int icat = phase_of(P, b) - 1;
@@ -3656,44 +3657,44 @@ __device__ __forceinline__ void cell_step(const DevParams &P, const WS<KT> &w, c
     }
     double *on = raw + P.raw_num + b;
     const double d = (w.numc[b] * idn) - *on;
-    *on = P.inv_dt != 0. ? d * P.inv_dt : d / dt;
+    *on = P.inv_dt != 0. ? d * P.inv_dt : ddiv(d, dt);
     bad |= !isfinite(w.numc[b]);
   }
   // interstitial activation leaves the activated-droplet outputs at zero (:879, local pactd);
   // cloud-base activation has written them
   if (!(P.st_activ && P.activ_mode == 2))
     for (int i = lane; i < P.ncld * (1 + nwet); i += 32) raw[P.raw_nact + i] = 0.;
-  if (lane == 0) raw[RW_RV] = (rv - rv_old) / dt;
+  if (lane == 0) raw[RW_RV] = ddiv(rv - rv_old, dt);
   if constexpr (SIP) {
     if (P.st_secice) {   // :345-349 and :412-416
       const SipT s = sip_tallies(P, w.raw);
-      for (int e = lane; e < 3 * P.nice; e += 32) raw[P.raw_sip + e] = s.tr[e] / dn;
-      if (P.raw_diag >= 0 && lane < 3) raw[P.raw_diag + SALSA_DIAG_SIPDRFR_SLOT + lane] = s.rate[lane] / dn;
+      for (int e = lane; e < 3 * P.nice; e += 32) raw[P.raw_sip + e] = ddiv(s.tr[e], dn);
+      if (P.raw_diag >= 0 && lane < 3) raw[P.raw_diag + SALSA_DIAG_SIPDRFR_SLOT + lane] = ddiv(s.rate[lane], dn);
     }
   }
   if (P.raw_gas >= 0 && lane < 5)   // :369-384
-    raw[P.raw_gas + lane] = ((w.misc[M_GAS + lane] / dn) - raw[P.raw_gas + lane]) / dt;
+    raw[P.raw_gas + lane] = ddiv((ddiv(w.misc[M_GAS + lane], dn)) - raw[P.raw_gas + lane], dt);
   if (DIAG && P.raw_diag >= 0 && lane == 0) {
     const double *d = w.misc + M_DIAG;
     double *o = raw + P.raw_diag;
-    o[DG_AUTOC] = d[DG_AUTOC] * K_RHOWA / dn;
-    o[DG_AUTOC80] = d[DG_AUTOC80] * K_RHOWA / dn;
-    o[DG_AUTOC50] = d[DG_AUTOC50] * K_RHOWA / dn;
-    o[DG_ACCR] = d[DG_ACCR] * K_RHOWA / dn;
-    o[DG_ACCR80] = d[DG_ACCR80] * K_RHOWA / dn;
-    o[DG_ACCR50] = d[DG_ACCR50] * K_RHOWA / dn;
-    o[DG_ACCOLL] = d[DG_ACCOLL] / dn;
-    o[DG_APCOLL] = d[DG_APCOLL] / dn;
-    o[DG_ACTIV] = d[DG_ACTIV] / dn;
-    o[DG_CONDA] = d[DG_CONDA] / dn;
-    o[DG_CONDC] = d[DG_CONDC] / dn;
-    o[DG_CONDP] = d[DG_CONDP] / dn;
+    o[DG_AUTOC] = ddiv(d[DG_AUTOC] * K_RHOWA, dn);
+    o[DG_AUTOC80] = ddiv(d[DG_AUTOC80] * K_RHOWA, dn);
+    o[DG_AUTOC50] = ddiv(d[DG_AUTOC50] * K_RHOWA, dn);
+    o[DG_ACCR] = ddiv(d[DG_ACCR] * K_RHOWA, dn);
+    o[DG_ACCR80] = ddiv(d[DG_ACCR80] * K_RHOWA, dn);
+    o[DG_ACCR50] = ddiv(d[DG_ACCR50] * K_RHOWA, dn);
+    o[DG_ACCOLL] = ddiv(d[DG_ACCOLL], dn);
+    o[DG_APCOLL] = ddiv(d[DG_APCOLL], dn);
+    o[DG_ACTIV] = ddiv(d[DG_ACTIV], dn);
+    o[DG_CONDA] = ddiv(d[DG_CONDA], dn);
+    o[DG_CONDC] = ddiv(d[DG_CONDC], dn);
+    o[DG_CONDP] = ddiv(d[DG_CONDP], dn);
     if (P.level == 5) {
       o[DG_AICOLL] = 0.;   // AIcoll%volc is never accumulated on this path (coag_ice uses the phase-change source)
-      o[DG_ICEHOM] = d[DG_ICEHOM] / dn;
-      o[DG_ICEDEP] = d[DG_ICEDEP] / dn;
-      o[DG_ICEIMM] = d[DG_ICEIMM] / dn;
-      o[DG_CONDI] = d[DG_CONDI] / dn;
+      o[DG_ICEHOM] = ddiv(d[DG_ICEHOM], dn);
+      o[DG_ICEDEP] = ddiv(d[DG_ICEDEP], dn);
+      o[DG_ICEIMM] = ddiv(d[DG_ICEIMM], dn);
+      o[DG_CONDI] = ddiv(d[DG_CONDI], dn);
     }
   }
   bad = warp_any(bad);

@@ -61,17 +61,17 @@ struct SedArgs {
 __device__ double ice_diameter(const DevParams &P, double mpri, double mrim, double numc) {
   double res = 1.e-9;
   if (numc < 1.e-6) return res;
-  const double Mtot = (mpri + mrim) / numc;
-  const double Fr = fmax(fmin(mrim / (Mtot * numc), 0.9999), 0.0001);
+  const double Mtot = ddiv(mpri + mrim, numc);
+  const double Fr = fmax(fmin(ddiv(mrim, Mtot * numc), 0.9999), 0.0001);
   const double rho_b = Fr * K_RHORI + (1. - Fr) * K_RHOIC;
-  const double Dth = pow(K_PI6 * K_RHOIC / P.iceShapeAlpha, 1. / (P.iceShapeBeta - 3.));
-  const double Dgr = pow(P.iceShapeAlpha / (K_PI6 * rho_b), 1. / (3. - P.iceShapeBeta));
-  const double Dcr = pow((1. / (1. - Fr)) * P.iceShapeAlpha / (K_PI6 * rho_b), 1. / (3. - P.iceShapeBeta));
+  const double Dth = dpow(ddiv(K_PI6 * K_RHOIC, P.iceShapeAlpha), drcp(P.iceShapeBeta - 3.));
+  const double Dgr = dpow(ddiv(P.iceShapeAlpha, K_PI6 * rho_b), drcp(3. - P.iceShapeBeta));
+  const double Dcr = dpow(ddiv((drcp(1. - Fr)) * P.iceShapeAlpha, K_PI6 * rho_b), drcp(3. - P.iceShapeBeta));
   const double Mth = K_RHOIC * K_PI6 * cube(Dth), Mgr = rho_b * K_PI6 * cube(Dgr), Mcr = rho_b * K_PI6 * cube(Dcr);
-  if (Mtot < Mth) res = cbrt(Mtot / (K_PI6 * K_RHOIC));
-  else if (Mtot >= Mth && Mtot < Mgr) res = pow(Mtot / P.iceShapeAlpha, 1. / P.iceShapeBeta);
-  else if (Mtot >= Mgr && Mtot < Mcr) res = cbrt(Mtot / (K_PI6 * rho_b));
-  else if (Mtot >= Mcr) res = pow(Mtot / ((1. / (1. - Fr)) * P.iceShapeAlpha), 1. / P.iceShapeBeta);
+  if (Mtot < Mth) res = dcbrt(divc(Mtot, K_PI6 * K_RHOIC));
+  else if (Mtot >= Mth && Mtot < Mgr) res = dpow(ddiv(Mtot, P.iceShapeAlpha), drcp(P.iceShapeBeta));
+  else if (Mtot >= Mgr && Mtot < Mcr) res = dcbrt(ddiv(Mtot, K_PI6 * rho_b));
+  else if (Mtot >= Mcr) res = dpow(ddiv(Mtot, (drcp(1. - Fr)) * P.iceShapeAlpha), drcp(P.iceShapeBeta));
   return res;
 }
 
@@ -87,9 +87,9 @@ __device__ __forceinline__ double sed_vel(const SedArgs &A, int flag, int ns, do
       v += m[s] * (flag == 4 ? A.rrhoice[s] : A.rrholiq[s]);
       sm += m[s];
     }
-  const double rn = 1. / n;
-  dwet = n < 1.e-15 ? 0. : cbrt(v * rn * R_PI6);
-  const double rd = 1. / dwet;
+  const double rn = drcp(n);
+  dwet = n < 1.e-15 ? 0. : dcbrt(v * rn * R_PI6);
+  const double rd = drcp(dwet);
   Shape<double> sh{0., 0., 0., 0.};
   double dnsp = 0.;
   if (flag == 4) {
@@ -104,7 +104,7 @@ __device__ __forceinline__ double sed_vel(const SedArgs &A, int flag, int ns, do
   }
   const double zdn = sm * rn * (rd * rd * rd) * R_PI6;
   const double Kn = 2. * lam * rd;                            // 2 lambda / dwet
-  GG = 1. + Kn * (SED_A + SED_B * exp(-SED_C * 0.5 * dwet * ilam));
+  GG = 1. + Kn * (SED_A + SED_B * dexp(-SED_C * 0.5 * dwet * ilam));
   if (flag <= 3 && dwet <= 19E-6) return sq(dwet) * (zdn - ad) * K_GRAV * GG * r18v;   // Stokes, eq. 3.21
   return terminal_vel<double>(dwet, zdn, ad, avis, GG, flag, sh, dnsp);
 }
@@ -164,13 +164,13 @@ __device__ void sed_slow(const SedArgs &A, double *sm, const double *blk, long l
       vc = fmin(vc, vmax_b[k]);
       if (k == 1) {   // the level just above the surface (:1020-1028)
         const double T = A.f.tk[col + 1], us = A.f.ustar[c2], avis = avis_s[1];
-        const double kvis = avis / ad_s[1];
-        const double mdiff = (LES_KB * T * GG) / (3.0 * LES_PI * avis * dwet);
-        const double Sc = kvis / mdiff;
-        double St = vc * (us * us) / LES_G * kvis;
+        const double kvis = ddiv(avis, ad_s[1]);
+        const double mdiff = ddiv(LES_KB * T * GG, 3.0 * LES_PI * avis * dwet);
+        const double Sc = ddiv(kvis, mdiff);
+        double St = divc(vc * (us * us), LES_G) * kvis;
         if (St < 0.01) St = 0.01;
-        const double rt = 1.0 / fmax(EPS_REAL, (us * (pow(Sc, -2.0 / 3.0) + pow(10., -3.0 / St))));
-        vc = (1. / rt) + vc;
+        const double rt = drcp(fmax(EPS_REAL, (us * (dpow(Sc, -2.0 / 3.0) + dpow(10., -ddiv(3.0, St))))));
+        vc = (drcp(rt)) + vc;
       }
       vc_s[k] = vc;
     }
@@ -217,7 +217,7 @@ __device__ void sed_slow(const SedArgs &A, double *sm, const double *blk, long l
       if (kc == 1) sr_s[0] = sr_s[0] - rsum * ad_s[kc] * LES_ALVL;
     }
     const double tsum = ts_s[kc] + wd_s[kc];
-    tlt_s[kc] = tlt_s[kc] + tsum * (LES_ALVL / LES_CP) * A.f.th[col + kc] / A.f.tk[col + kc];
+    tlt_s[kc] = tlt_s[kc] + ddiv(tsum * (LES_ALVL / LES_CP) * A.f.th[col + kc], A.f.tk[col + kc]);
   }
   __syncwarp();
 }
@@ -340,8 +340,8 @@ __device__ void sed_fast(const SedArgs &A, double *sm, const double *blk, long l
           const double v = src[k];
           if (k == L) acc = acc - v;
           if (kf - 1 == L) {
-            if (code & SED_BR) acc = acc + v * dzt_b[kf - 1] / dzt_b[k];
-            else acc = acc + (f1_s[k] * v) * dzt_b[kf - 1] / dzt_b[kf];
+            if (code & SED_BR) acc = acc + ddiv(v * dzt_b[kf - 1], dzt_b[k]);
+            else acc = acc + ddiv((f1_s[k] * v) * dzt_b[kf - 1], dzt_b[kf]);
           } else if (kf == L && !(code & SED_BR)) {
             acc = acc + (1. - f1_s[k]) * v;
           }
@@ -366,7 +366,7 @@ __device__ void sed_fast(const SedArgs &A, double *sm, const double *blk, long l
     const int L = r * 32 + lane;
     if (L > nzp - 2) continue;
     const double S = flag == 4 ? ws_s[L] + wq_s[L] : ws_s[L];
-    tlt_s[L] = tlt_s[L] - (S * A.rdtlt) * (alv / LES_CP) * A.f.th[col + L] / A.f.tk[col + L];
+    tlt_s[L] = tlt_s[L] - ddiv((S * A.rdtlt) * divc(alv, LES_CP) * A.f.th[col + L], A.f.tk[col + L]);
   }
   __syncwarp();
 }
@@ -377,10 +377,10 @@ __global__ void __launch_bounds__(128) sedimentation_kernel(const SedArgs A) {
   // per block: dzt, 1/dzt and the slow fall-speed cap 0.5*(1/dzt)/dtlt (at most 2 m/s)
   double *blk = sed_smem;
   for (int k = threadIdx.x; k < nzp; k += blockDim.x) {
-    const double dz = A.f.dzt[k], dzl = 1. / dz;
+    const double dz = A.f.dzt[k], dzl = drcp(dz);
     blk[k] = dz;
     blk[nzp + k] = dzl;
-    blk[2 * nzp + k] = fmin(0.5 * dzl / A.dtlt, 2.0);
+    blk[2 * nzp + k] = fmin(ddiv(0.5 * dzl, A.dtlt), 2.0);
   }
   __syncthreads();
   const long long c2 = (long long)blockIdx.x * (blockDim.x >> 5) + wib;   // column i + nxp*j
@@ -412,12 +412,12 @@ __global__ void __launch_bounds__(128) sedimentation_kernel(const SedArgs A) {
     ad_s[k] = ad;
     double avis = 0., lam = 0., ilam = 0., r18 = 0., q = 0.;
     if (k >= 1 && k <= nzp - 2) {
-      const double T = A.f.tk[p], x = T / 296.16;
-      avis = 1.8325e-5 * (416.16 / (T + 120.0)) * (x * sqrt(x));
-      const double va = sqrt(8. * LES_KB * T / (LES_PI * SED_M));
-      lam = 2. * avis / (ad * va);
-      ilam = 1. / lam;
-      r18 = 1. / (18. * avis);
+      const double T = A.f.tk[p], x = divc(T, 296.16);
+      avis = 1.8325e-5 * (ddiv(416.16, T + 120.0)) * (x * dsqrt(x));
+      const double va = dsqrt(ddiv(8. * LES_KB * T, LES_PI * SED_M));
+      lam = ddiv(2. * avis, ad * va);
+      ilam = drcp(lam);
+      r18 = drcp(18. * avis);
       q = A.f.dzt[k] / ad;
     }
     avis_s[k] = avis;
