@@ -33,7 +33,44 @@ cudaError_t launch_ds(const DevParams &, cudaStream_t, int);
 cudaError_t launch_fs(const DevParams &, cudaStream_t, int);
 int blocks_per_sm_ds(const DevParams &);
 int blocks_per_sm_fs(const DevParams &);
+// the lane form of the FP64 ones
+cudaError_t launch_lane_d0(const DevParams &, cudaStream_t, int);
+cudaError_t launch_lane_d1(const DevParams &, cudaStream_t, int);
+cudaError_t launch_lane_ds(const DevParams &, cudaStream_t, int);
+int lane_blocks_per_sm_d0(const DevParams &);
+int lane_blocks_per_sm_d1(const DevParams &);
+int lane_blocks_per_sm_ds(const DevParams &);
 }  // namespace salsa
+
+namespace {
+// the kernels of one form of the step: [FP64, mixed] without diagnostics, with them, with
+// secondary ice
+struct Form {
+  cudaError_t (*warp)(const salsa::DevParams &, cudaStream_t, int);
+  int (*warp_bps)(const salsa::DevParams &);
+  cudaError_t (*lane)(const salsa::DevParams &, cudaStream_t, int);
+  int (*lane_bps)(const salsa::DevParams &);
+};
+const Form FORMS[3][2] = {
+    {{salsa::launch_d0, salsa::blocks_per_sm_d0, salsa::launch_lane_d0, salsa::lane_blocks_per_sm_d0},
+     {salsa::launch_f0, salsa::blocks_per_sm_f0, nullptr, nullptr}},
+    {{salsa::launch_d1, salsa::blocks_per_sm_d1, salsa::launch_lane_d1, salsa::lane_blocks_per_sm_d1},
+     {salsa::launch_f1, salsa::blocks_per_sm_f1, nullptr, nullptr}},
+    {{salsa::launch_ds, salsa::blocks_per_sm_ds, salsa::launch_lane_ds, salsa::lane_blocks_per_sm_ds},
+     {salsa::launch_fs, salsa::blocks_per_sm_fs, nullptr, nullptr}}};
+const Form &form_of(bool sip, bool diag, int precision) { return FORMS[sip ? 2 : (diag ? 1 : 0)][precision]; }
+}  // namespace
+
+// FP64 calls of at least this many cells take the lane form (one cell per lane); smaller ones
+// take the warp form, whose latency per cell is lower: a tile of 32 cells takes the lane form
+// 4 (warm cells) to 12 ms (cloudy ones), and that is what a call takes while every sub-core
+// holds at most one tile.  Both forms took the same time at about 24,000 cells of
+// grid16x16x40, grid256x256x128 and grid384x384x160 (5.8 / 6.3, 11.2 / 12.4 and
+// 12.6 / 12.2 ms, lane / warp form).  With secondary ice the warp form holds one block per SM
+// and runs the schemes on one lane: 13.3 / 47 ms at 13,824 cells, even at about 4,000.
+// The mixed form stays with the warp form, whose float partner sums round by its lanes.
+#define SALSA_LANE_MINCELLS 24576
+#define SALSA_LANE_MINCELLS_SIP 4096
 
 using salsa::DevParams;
 using salsa::Row;
@@ -150,6 +187,8 @@ struct salsa_handle {
   size_t kcache_bytes = 0;
   cudaStream_t s_in = nullptr, s_out = nullptr;     // copy streams of the host-buffer pipeline
   cudaEvent_t pev[3 * SALSA_PIPE_SLOTS + 2] = {};   // its slot and start/end events
+  double *lane_ws = nullptr;    // workspaces of the lane form, one per resident warp
+  size_t lane_ws_bytes = 0;
   int *d_order = nullptr;       // cell order list (salsa_order_kernel)
   long long order_cap = 0;
   int *na_order = nullptr;      // module scratch of salsa_gb300_run_noalloc on this handle's device
@@ -594,9 +633,7 @@ int salsa_gb300_init(const salsa_config_t *cfg, salsa_handle_t **out) {
     void *po = nullptr, *ps = nullptr;
     cudaFuncAttributes fa;
     const bool sip = g.lssecice.sw && g.level == 5;
-    const int bps = sip ? (g.precision == 0 ? salsa::blocks_per_sm_ds(B) : salsa::blocks_per_sm_fs(B))
-                        : (g.precision == 0 ? (g.diagnostics ? salsa::blocks_per_sm_d1(B) : salsa::blocks_per_sm_d0(B))
-                                            : (g.diagnostics ? salsa::blocks_per_sm_f1(B) : salsa::blocks_per_sm_f0(B)));
+    const int bps = form_of(sip, g.diagnostics, g.precision).warp_bps(B);
     if (bps <= 0 || cudaFuncGetAttributes(&fa, salsa_order_kernel) != cudaSuccess ||
         cudaGetSymbolAddress(&po, g_na_order) != cudaSuccess || cudaGetSymbolAddress(&ps, g_na_status) != cudaSuccess) {
       salsa_gb300_finalize(h);
@@ -617,6 +654,7 @@ void salsa_gb300_finalize(salsa_handle_t *h) {
   if (h->d_rows) cudaFree(h->d_rows);
   if (h->d_pairs) cudaFree(h->d_pairs);
   if (h->d_order) cudaFree(h->d_order);
+  if (h->lane_ws) cudaFree(h->lane_ws);
   for (int i = 0; i < 4; i++)
     if (h->scratch[i]) cudaFree(h->scratch[i]);
   if (h->d_status) cudaFree(h->d_status);
@@ -822,17 +860,36 @@ int run_impl(salsa_handle_t *h, int nzp, int nxp, int nyp, int ns, double tstep,
   // order pre-pass and step kernel over the cells of Q, on stream s
   auto launch = [&](DevParams &Q, int *order) -> int {
     const bool sip = Q.st_secice != 0;
-    int bps = sip ? (prec == 0 ? salsa::blocks_per_sm_ds(Q) : salsa::blocks_per_sm_fs(Q))
-                  : prec == 0 ? (dg ? salsa::blocks_per_sm_d1(Q) : salsa::blocks_per_sm_d0(Q))
-                              : (dg ? salsa::blocks_per_sm_f1(Q) : salsa::blocks_per_sm_f0(Q));
+    const Form &form = form_of(sip, dg, prec);
+    const int bps = form.warp_bps(Q);
     if (bps <= 0) return SALSA_E_CUDA;
     long long grid = (long long)bps * h->nsm * 8;
     if (grid > Q.ngroups) grid = Q.ngroups;
+    // the lane form, when the call is large enough and its workspaces are to be had
+    int lane_grid = 0;
+    if (!noalloc && order && form.lane && Q.ncells >= (sip ? SALSA_LANE_MINCELLS_SIP : SALSA_LANE_MINCELLS)) {
+      const int lbps = form.lane_bps(Q);
+      const long long need = ((Q.ncells + 31) / 32 + SALSA_LANE_WARPS - 1) / SALSA_LANE_WARPS;
+      lane_grid = (int)std::min((long long)lbps * h->nsm, need);
+      const size_t bytes = (size_t)lane_grid * SALSA_LANE_WARPS * 32 * (size_t)Q.ws_doubles * sizeof(double);
+      if (lane_grid > 0 && bytes > h->lane_ws_bytes) {
+        if (h->lane_ws) cudaFree(h->lane_ws);
+        h->lane_ws = nullptr;
+        h->lane_ws_bytes = 0;
+        if (cudaMalloc(&h->lane_ws, bytes) == cudaSuccess) {
+          h->lane_ws_bytes = bytes;
+        } else {
+          cudaGetLastError();   // no memory: the warp form needs none
+          lane_grid = 0;
+        }
+      }
+      Q.lane_ws = h->lane_ws;
+    }
     Q.order = order;
     if (order) {
-      // the order list's fill counters start at zero for every launch (a call may launch
+      // the order list's fill counters and the lane form's tile counter start at zero for every launch (a call may launch
       // several, one per slab)
-      if (cudaMemsetAsync(Q.status + salsa::ST_ORDER_CLEAR, 0, 2 * sizeof(unsigned long long), s) != cudaSuccess)
+      if (cudaMemsetAsync(Q.status + salsa::ST_ORDER_CLEAR, 0, 3 * sizeof(unsigned long long), s) != cudaSuccess)
         return SALSA_E_CUDA;
       long long og = (Q.ncells + 255) / 256;
       if (og > (long long)h->nsm * 16) og = (long long)h->nsm * 16;
@@ -840,9 +897,7 @@ int run_impl(salsa_handle_t *h, int nzp, int nxp, int nyp, int ns, double tstep,
       if (cudaGetLastError() != cudaSuccess) return SALSA_E_CUDA;
       launches++;
     }
-    cudaError_t e = sip ? (prec == 0 ? salsa::launch_ds(Q, s, (int)grid) : salsa::launch_fs(Q, s, (int)grid))
-                    : prec == 0 ? (dg ? salsa::launch_d1(Q, s, (int)grid) : salsa::launch_d0(Q, s, (int)grid))
-                                : (dg ? salsa::launch_f1(Q, s, (int)grid) : salsa::launch_f0(Q, s, (int)grid));
+    const cudaError_t e = lane_grid > 0 ? form.lane(Q, s, lane_grid) : form.warp(Q, s, (int)grid);
     if (e != cudaSuccess) return SALSA_E_CUDA;
     launches++;
     return SALSA_OK;

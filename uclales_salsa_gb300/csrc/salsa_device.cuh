@@ -10,6 +10,8 @@
 
 #define SALSA_CPG 4                 // cells (= warps) per block
 #define SALSA_THREADS (32 * SALSA_CPG)
+#define SALSA_LANE_WARPS 4          // warps per block of the lane form (32 cells each)
+#define SALSA_LANE_MINBLOCKS 4      // its resident blocks per SM
 #define SALSA_NSV 7                 // volume slots per bin (dry species + water + rime)
 #define SALSA_MAXNB 96
 
@@ -76,6 +78,7 @@ enum {
 // status counters
 enum { ST_CELLS = 0, ST_EQUIL, ST_DISTR, ST_NEGFRAC, ST_COND, ST_NEG, ST_NONFINITE,
        ST_ORDER_CLEAR, ST_ORDER_CLOUDY,   // fill counters of the cell order list
+       ST_TILE,                           // the lane form's next tile of 32 cells
        ST_N };
 
 struct Row {
@@ -138,6 +141,7 @@ struct DevParams {
   // offset of the tally region inside each warp's workspace (doubles)
   int st_secice, st_siprs, st_sipdf, st_sipib;
   int sip_rs_mode, sip_df_mode, sip_ib_mode, sip_splbin, sip_off;
+  double *lane_ws;   // workspaces of the lane form, one of 32 * ws_doubles per resident warp
   int raw_sip;   // first of the 3 x nice tracer rows (sipdrfr, siprmspl, sipiibr), or -1
 };
 

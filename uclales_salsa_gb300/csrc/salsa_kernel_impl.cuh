@@ -32,17 +32,47 @@ namespace {   // internal linkage: every instantiation unit carries its own copy
 // ----------------------------------------------------------------------------------------
 // per-warp workspace
 // ----------------------------------------------------------------------------------------
-template <typename KT>
+// LS lanes advance one cell:
+//   LS = 32 (warp form)  one warp per cell, the workspace in shared memory, rows contiguous;
+//   LS = 1  (lane form)  one lane per cell, the workspaces of a warp's 32 cells interleaved in
+//                        global memory: row r of lane l at r * 32 + l, so that a warp's access
+//                        to a row is one 256-byte (128 for float) segment.
+template <typename T>
+struct Col {
+  T *p;
+  __device__ __forceinline__ T &operator[](int i) const { return p[i * 32]; }
+  __device__ __forceinline__ Col operator+(int k) const { return {p + k * 32}; }
+  template <typename U> __device__ __forceinline__ operator Col<U>() const { return {p}; }   // T -> const T
+};
+template <typename T, int LS> using Ptr = typename std::conditional<LS == 1, Col<T>, T *>::type;
+// the same memory as rows of another type
+template <typename U, typename T> __device__ __forceinline__ U *row_cast(T *p) { return reinterpret_cast<U *>(p); }
+template <typename U, typename T> __device__ __forceinline__ Col<U> row_cast(Col<T> c) {
+  const int l = threadIdx.x & 31;
+  return {reinterpret_cast<U *>(c.p - l) + l};
+}
+
+template <typename KT, int LS>
 struct WS {
-  double *raw, *numc, *volc, *dwet, *ddry, *dins, *dnsp, *rhomean, *indef, *ctime, *scr, *misc;
-  KT *K;
-  int *pbuf;
+  using D = Ptr<double, LS>;
+  D raw, numc, volc, dwet, ddry, dins, dnsp, rhomean, indef, ctime, scr, misc;
+  Ptr<KT, LS> K;
+  int *pbuf;   // warp form
   int NB;
+  bool live;   // the lane form's last warp: lanes past the last cell repeat it and write nothing
+  // lane form: bins that reach their number limit in some cell of the warp before coagulation
+  // (bins 0-63, 64-95); pairs with the others have K = 0 and their terms are skipped
+  unsigned long long am0;
+  unsigned am1;
+  __device__ __forceinline__ bool on(int b) const {
+    if constexpr (LS == 1) return b < 64 ? (am0 >> b) & 1ull : (am1 >> (b - 64)) & 1u;
+    else return true;
+  }
   // float copies of numc and volc that the mixed form's coagulation update sums from
   // (in the scratch rows, valid from shadow_all to the end of the update)
-  float *nf, *vf;
+  Ptr<float, LS> nf, vf;
   __device__ __forceinline__ double &v(int s, int b) const { return volc[s * NB + b]; }
-  __device__ __forceinline__ double *sc(int k) const { return scr + k * NB; }
+  __device__ __forceinline__ D sc(int k) const { return scr + k * NB; }
   // partner values in the kernel type: the state itself (FP64 form) or its float copy
   __device__ __forceinline__ KT nk(int b) const {
     if constexpr (sizeof(KT) == 4) return nf[b];
@@ -53,6 +83,11 @@ struct WS {
     else return volc[s * NB + b];
   }
 };
+
+// reductions and barriers of the lanes of one cell
+template <int LS> __device__ __forceinline__ double wsum(double v) { return LS == 1 ? v : warp_sum(v); }
+template <int LS> __device__ __forceinline__ bool wany(bool b) { return LS == 1 ? b : (bool)warp_any(b); }
+template <int LS> __device__ __forceinline__ void wsync() { if constexpr (LS != 1) __syncwarp(); }
 
 // misc slots (doubles)
 enum {
@@ -78,8 +113,9 @@ __device__ __forceinline__ double dlim_of(int ph) {
 __device__ __forceinline__ int tri(int i, int j, int NB) {  // i <= j
   return i * NB - (i * (i - 1)) / 2 + (j - i);
 }
-template <typename KT>
-__device__ __forceinline__ KT kget(const WS<KT> &w, int i, int j) {
+template <typename KT, int LS>
+__device__ __forceinline__ KT kget(const WS<KT, LS> &w, int i, int j) {
+  if (!(w.on(i) && w.on(j))) return (KT)0;
   return i <= j ? w.K[tri(i, j, w.NB)] : w.K[tri(j, i, w.NB)];
 }
 
@@ -88,16 +124,16 @@ __device__ __forceinline__ KT kget(const WS<KT> &w, int i, int j) {
 // With limit set, dnsp = MIN(dwet, dlim) overwrites the non-spherical diameter (:149-150),
 // so getDiameter's value never survives a type="all" update and is not evaluated here.
 // ----------------------------------------------------------------------------------------
-__device__ void updateDiameterAll(const DevParams &P, const WS<double> *, double *numc, double *volc, double *dwet,
-                                  double *ddry, double *dins, double *dnsp, const double *dmid, int NB, int b) {
+template <typename KT, int LS>
+__device__ __forceinline__ void updateDiameterAll(const DevParams &P, const WS<KT, LS> &w, const double *dmid, int b) {
   int ph = phase_of(P, b);
-  double n = numc[b];
+  double n = w.numc[b];
   double dw, dd, di;
   if (n > nlim_of(ph)) {
     double vs = 0., vd = 0., vi = 0.;
-    for (int s = 0; s < P.nused; s++) vs += volc[s * NB + b];
-    for (int s = 0; s < P.ndry; s++) vd += volc[s * NB + b];
-    for (int k = 0; k < P.ninsoluble; k++) vi += volc[P.ind_insoluble[k] * NB + b];
+    for (int s = 0; s < P.nused; s++) vs += w.v(s, b);
+    for (int s = 0; s < P.ndry; s++) vd += w.v(s, b);
+    for (int k = 0; k < P.ninsoluble; k++) vi += w.v(P.ind_insoluble[k], b);
     // (v / numc / pi6)^(1/3) with one division for the three diameters
     const double q = drcp(n * K_PI6);
     dw = dcbrt(vs * q);
@@ -108,10 +144,10 @@ __device__ void updateDiameterAll(const DevParams &P, const WS<double> *, double
   }
   double dl = dlim_of(ph);
   dw = fmin(dw, dl);
-  dwet[b] = dw;
-  dnsp[b] = dw;
-  ddry[b] = fmin(dd, dl);
-  dins[b] = fmin(di, dl);
+  w.dwet[b] = dw;
+  w.dnsp[b] = dw;
+  w.ddry[b] = fmin(dd, dl);
+  w.dins[b] = fmin(di, dl);
 }
 
 __device__ __forceinline__ double rhomean_of(const DevParams &P, int ph, double n, double vw, double vr) {
@@ -352,8 +388,8 @@ __device__ T coag_pair(const CoagCell<T> &cc, const BinProps<T> &a, const BinPro
   return zbrown + zbrconv + t_sqrt(sq(zgrav) + sq(ztshear) + sq(zturb));
 }
 
-template <typename KT>
-__device__ __forceinline__ void load_props(const KT *S, int NB, int b, BinProps<KT> &o) {
+template <typename KT, typename PT>
+__device__ __forceinline__ void load_props(const PT &S, int NB, int b, BinProps<KT> &o) {
   KT *po = &o.diam;
 #pragma unroll
   for (int k = 0; k < 9; k++) po[k] = S[k * NB + b];
@@ -361,14 +397,14 @@ __device__ __forceinline__ void load_props(const KT *S, int NB, int b, BinProps<
 
 // Per-bin properties are evaluated in the kernel type: FP64 in the FP64 form, float in
 // the mixed form (its pair kernels are float too) except for ice bins.
-template <typename KT>
-__device__ __forceinline__ void store_props(KT *S, int NB, int b, const BinProps<double> &o) {
+template <typename KT, typename PT>
+__device__ __forceinline__ void store_props(const PT &S, int NB, int b, const BinProps<double> &o) {
   const double *po = &o.diam;
 #pragma unroll
   for (int k = 0; k < 9; k++) S[k * NB + b] = (KT)po[k];
 }
-template <typename KT>
-__device__ __forceinline__ void store_props_kt(KT *S, int NB, int b, const BinProps<KT> &o) {
+template <typename KT, typename PT>
+__device__ __forceinline__ void store_props_kt(const PT &S, int NB, int b, const BinProps<KT> &o) {
   const KT *po = &o.diam;
 #pragma unroll
   for (int k = 0; k < 9; k++) S[k * NB + b] = po[k];
@@ -382,13 +418,48 @@ __device__ __forceinline__ void to_kt(const BinProps<double> &d, BinProps<KT> &o
 }
 // FP64 shape coefficients of bin b: they share the memory of S rows 9-12 in the FP64
 // form and sit behind the float rows in the mixed form.
-template <typename KT>
-__device__ __forceinline__ double *shape_rows(const WS<KT> &w) {
+template <typename KT, int LS>
+__device__ __forceinline__ Ptr<double, LS> shape_rows(const WS<KT, LS> &w) {
   return sizeof(KT) == 8 ? w.scr + 9 * w.NB : w.scr + 7 * w.NB;
 }
 
+// Properties of the first particle of a pair of equal-size bins (i, j), the self-coagulation
+// offset (:273-276): 1.1 times the diameter and 1.33 times the mass of particle 2.  S and SH
+// are the property and shape rows.  For liquid bins they depend on bin j alone: the fall
+// speed takes the same branch for every liquid phase, every liquid density is that of water
+// and the sphere-equivalent diameter enters only for ice.
+template <typename KT, int LS>
+__device__ __forceinline__ void offset_props(const DevParams &P, const WS<KT, LS> &w, const CoagCell<KT> &cc,
+                                             const CoagCell<double> &cd, const Shape<double> &sh, int i, int j,
+                                             BinProps<KT> &a) {
+  if constexpr (sizeof(KT) == 4) {
+    if (phase_of(P, i) < 4) {
+      const float dj = (float)w.dwet[j], mj = (float)w.rhomean[j] * (float)K_PI6 * cube(dj);
+      Shape<float> shf;
+      shf.alpha = (float)sh.alpha; shf.beta = (float)sh.beta; shf.gamma = (float)sh.gamma; shf.sigma = (float)sh.sigma;
+      bin_props<float>(cc, phase_of(P, i), 1.1f * dj, (float)w.dwet[i], 1.33f * mj, (float)w.rhomean[i], shf, a);
+      return;
+    }
+  }
+  const double dj = w.dwet[j], mj = w.rhomean[j] * K_PI6 * cube(dj);
+  BinProps<double> ad;
+  bin_props<double>(cd, phase_of(P, i), 1.1 * dj, w.dwet[i], 1.33 * mj, w.rhomean[i], sh, ad);
+  to_kt<KT>(ad, a);
+}
+
+// charging enhancement (:411-416)
+template <typename KT, int LS>
+__device__ __forceinline__ KT charged(const DevParams &P, const WS<KT, LS> &w, KT k, int i, int j) {
+  if (P.lcharge) {
+    double kd = (double)k;
+    kd = kd + ddiv(kd * P.chargeCollEnh * 0.5 * (w.ctime[i] + w.ctime[j]), P.chargeTimeMax);
+    k = (KT)kd;
+  }
+  return k;
+}
+
 template <typename KT, bool OFFSET>
-__device__ void eval_pairs(const DevParams &P, const WS<KT> &w, const CoagCell<KT> &cc, const CoagCell<double> &cd,
+__device__ void eval_pairs(const DevParams &P, const WS<KT, 32> &w, const CoagCell<KT> &cc, const CoagCell<double> &cd,
                            const KT *S, const int *list, int n, int lane) {
   const int NB = w.NB;
   if (lane < n) {
@@ -397,38 +468,47 @@ __device__ void eval_pairs(const DevParams &P, const WS<KT> &w, const CoagCell<K
     BinProps<KT> a, b;
     load_props<KT>(S, NB, j, b);
     if (OFFSET) {
-      // self-coagulation offset (:273-276): particle 1 takes 1.1x the diameter and 1.33x the mass of particle 2
       const double *SH = shape_rows(w);
       Shape<double> sh;
       sh.alpha = SH[0 * NB + i]; sh.beta = SH[1 * NB + i]; sh.gamma = SH[2 * NB + i]; sh.sigma = SH[3 * NB + i];
-      bool done = false;
-      if constexpr (sizeof(KT) == 4) {
-        if (phase_of(P, i) < 4) {
-          const float dj = (float)w.dwet[j], mj = (float)w.rhomean[j] * (float)K_PI6 * cube(dj);
-          Shape<float> shf;
-          shf.alpha = (float)sh.alpha; shf.beta = (float)sh.beta; shf.gamma = (float)sh.gamma; shf.sigma = (float)sh.sigma;
-          bin_props<float>(cc, phase_of(P, i), 1.1f * dj, (float)w.dwet[i], 1.33f * mj, (float)w.rhomean[i], shf, a);
-          done = true;
-        }
-      }
-      if (!done) {
-        const double dj = w.dwet[j], mj = w.rhomean[j] * K_PI6 * cube(w.dwet[j]);
-        BinProps<double> ad;
-        bin_props<double>(cd, phase_of(P, i), 1.1 * dj, w.dwet[i], 1.33 * mj, w.rhomean[i], sh, ad);
-        to_kt<KT>(ad, a);
-      }
+      offset_props(P, w, cc, cd, sh, i, j, a);
     } else {
       load_props<KT>(S, NB, i, a);
     }
-    KT k = coag_pair<KT>(cc, a, b);
-    if (P.lcharge) {
-      // charging enhancement (:411-416)
-      double kd = (double)k;
-      kd = kd + ddiv(kd * P.chargeCollEnh * 0.5 * (w.ctime[i] + w.ctime[j]), P.chargeTimeMax);
-      k = (KT)kd;
-    }
-    w.K[tri(i, j, NB)] = k;
+    w.K[tri(i, j, NB)] = charged(P, w, coag_pair<KT>(cc, a, b), i, j);
   }
+}
+
+// shape coefficients and collision properties of bin b, in the kernel type
+template <typename KT, int LS>
+__device__ __forceinline__ void props_of_bin(const DevParams &P, const WS<KT, LS> &w, const CoagCell<KT> &cc,
+                                             const CoagCell<double> &cd, int b, Shape<double> &sh, BinProps<KT> &o) {
+  const int ph = phase_of(P, b);
+  if (ph == 4) {
+    double mp = 0.;
+    for (int s = 0; s < P.nused - 1; s++) mp += w.v(s, b) * K_RHOIC;
+    shape_coeffs<double>(P, sh, mp, w.v(P.nused - 1, b) * K_RHORI, w.numc[b]);
+  } else {
+    sh.alpha = sh.beta = sh.gamma = sh.sigma = 0.;
+  }
+  const double diam = w.dwet[b];   // dnsp == dwet after a limited "all" update
+  if constexpr (sizeof(KT) == 4) {
+    if (ph < 4) {
+      // the mixed form evaluates the per-bin properties of the liquid bins in float as
+      // well; ice keeps FP64 (the Khvorostyanov-Curry fall speed carries float rounding
+      // of its exponents into ice-drop speed differences, which cancel)
+      const float df = (float)diam;
+      const float mass = (float)w.rhomean[b] * (float)K_PI6 * cube(df);
+      Shape<float> shf;
+      shf.alpha = (float)sh.alpha; shf.beta = (float)sh.beta; shf.gamma = (float)sh.gamma; shf.sigma = (float)sh.sigma;
+      bin_props<float>(cc, ph, df, df, mass, (float)w.rhomean[b], shf, o);
+      return;
+    }
+  }
+  const double mass = w.rhomean[b] * K_PI6 * cube(diam);
+  BinProps<double> od;
+  bin_props<double>(cd, ph, diam, diam, mass, w.rhomean[b], sh, od);
+  to_kt<KT>(od, o);
 }
 
 // ----------------------------------------------------------------------------------------
@@ -437,11 +517,10 @@ __device__ void eval_pairs(const DevParams &P, const WS<KT> &w, const CoagCell<K
 // Scratch: the nine BinProps rows (diam fre cschm dfpart mtvel2 omega termv reyn ire), then
 // the FP64 shape coefficients (shape_rows).
 // ----------------------------------------------------------------------------------------
+// per-cell constants of the collision kernel
 template <typename KT>
-__device__ void build_kernels(const DevParams &P, const WS<KT> &w, const double *tb, double T, double pres,
-                              int lane) {
-  const int NB = w.NB;
-  CoagCell<double> cd;
+__device__ __forceinline__ void coag_cells(const DevParams &P, double T, double pres, CoagCell<double> &cd,
+                                           CoagCell<KT> &cc) {
   {
     double visc = ddiv(7.44523e-3 * dsqrt(cube(T)), 5093. * (T + 110.4));
     double mfp = ddiv((1.656e-10 * T + 1.828e-8) * K_PSTAND, pres);
@@ -451,9 +530,16 @@ __device__ void build_kernels(const DevParams &P, const WS<KT> &w, const double 
     cd.shearA = dsqrt(ddiv(8. * K_PI * P.eddy_dis, 15. * vkin));
     cd.turbB = ddiv(K_PI * dpow(P.eddy_dis, 0.75), K_GRAV * dsqrt(dsqrt(vkin)));
   }
-  CoagCell<KT> cc;
   cc.T_ = (KT)cd.T_; cc.visc = (KT)cd.visc; cc.mfp = (KT)cd.mfp; cc.zrhoa = (KT)cd.zrhoa; cc.vkin = (KT)cd.vkin;
   cc.shearA = (KT)cd.shearA; cc.turbB = (KT)cd.turbB;
+}
+
+template <typename KT>
+__device__ __forceinline__ void build_kernels(const DevParams &P, const WS<KT, 32> &w, double T, double pres, int lane) {
+  const int NB = w.NB;
+  CoagCell<double> cd;
+  CoagCell<KT> cc;
+  coag_cells<KT>(P, T, pres, cd, cc);
   KT *S = reinterpret_cast<KT *>(w.scr);   // KT-typed scratch, 9 * NB entries
   double *SH = shape_rows(w);
   // per-bin properties of the populated bins only (a pair with an empty bin has K = 0)
@@ -469,38 +555,10 @@ __device__ void build_kernels(const DevParams &P, const WS<KT> &w, const double 
   __syncwarp();
   for (int e = lane; e < nact; e += 32) {
     const int b = w.pbuf[e];
-    int ph = phase_of(P, b);
     Shape<double> sh;
-    if (ph == 4) {
-      double mp = 0.;
-      for (int s = 0; s < P.nused - 1; s++) mp += w.v(s, b) * K_RHOIC;
-      shape_coeffs<double>(P, sh, mp, w.v(P.nused - 1, b) * K_RHORI, w.numc[b]);
-    } else {
-      sh.alpha = sh.beta = sh.gamma = sh.sigma = 0.;
-    }
-    double diam = w.dwet[b];   // dnsp == dwet after a limited "all" update
-    bool done = false;
-    if constexpr (sizeof(KT) == 4) {
-      if (ph < 4) {
-        // the mixed form evaluates the per-bin properties of the liquid bins in float as
-        // well; ice keeps FP64 (the Khvorostyanov-Curry fall speed carries float rounding
-        // of its exponents into ice-drop speed differences, which cancel)
-        const float df = (float)diam;
-        const float mass = (float)w.rhomean[b] * (float)K_PI6 * cube(df);
-        Shape<float> shf;
-        shf.alpha = (float)sh.alpha; shf.beta = (float)sh.beta; shf.gamma = (float)sh.gamma; shf.sigma = (float)sh.sigma;
-        BinProps<float> o;
-        bin_props<float>(cc, ph, df, df, mass, (float)w.rhomean[b], shf, o);
-        store_props_kt<KT>(S, NB, b, o);
-        done = true;
-      }
-    }
-    if (!done) {
-      double mass = w.rhomean[b] * K_PI6 * cube(w.dwet[b]);
-      BinProps<double> o;
-      bin_props<double>(cd, ph, diam, w.dwet[b], mass, w.rhomean[b], sh, o);
-      store_props<KT>(S, NB, b, o);
-    }
+    BinProps<KT> o;
+    props_of_bin(P, w, cc, cd, b, sh, o);
+    store_props_kt<KT>(S, NB, b, o);
     SH[0 * NB + b] = sh.alpha; SH[1 * NB + b] = sh.beta; SH[2 * NB + b] = sh.gamma; SH[3 * NB + b] = sh.sigma;
   }
   __syncwarp();
@@ -536,6 +594,65 @@ __device__ void build_kernels(const DevParams &P, const WS<KT> &w, const double 
       else eval_pairs<KT, true>(P, w, cc, cd, S, w.pbuf, nbuf, lane);
     }
     __syncwarp();
+  }
+}
+
+
+// The lane form: the pair table in order (its entries are sorted by the first bin, whose
+// properties stay in registers), every cell of the warp at the same pair.  The kernel of an
+// equal-size pair of liquid bins is that of the larger bin with itself, evaluated once per
+// bin with the properties.
+template <typename KT>
+__device__ __forceinline__ void build_kernels(const DevParams &P, const WS<KT, 1> &w, double T, double pres, int) {
+  const int NB = w.NB;
+  CoagCell<double> cd;
+  CoagCell<KT> cc;
+  coag_cells<KT>(P, T, pres, cd, cc);
+  const Col<KT> S = row_cast<KT>(w.scr);
+  const Col<double> SH = shape_rows(w);
+  const bool eq = P.npairs > P.npairs_plain;
+  for (int b = 0; b < P.ntotal; b++) {
+    if (!w.on(b) || !(w.numc[b] >= nlim_of(phase_of(P, b)))) continue;
+    Shape<double> sh;
+    BinProps<KT> o;
+    props_of_bin(P, w, cc, cd, b, sh, o);
+    store_props_kt<KT>(S, NB, b, o);
+    SH[0 * NB + b] = sh.alpha; SH[1 * NB + b] = sh.beta; SH[2 * NB + b] = sh.gamma; SH[3 * NB + b] = sh.sigma;
+    if (eq) {
+      BinProps<KT> a;
+      offset_props(P, w, cc, cd, sh, b, b, a);
+      w.K[tri(b, b, NB)] = coag_pair<KT>(cc, a, o);
+    }
+  }
+  BinProps<KT> a;
+  int ia = -1;
+  for (int t = 0; t < P.npairs; t++) {
+    const int pk = __ldg(P.pairs + t), i = pk & 0xff, j = (pk >> 8) & 0xff, ij = tri(i, j, NB);
+    if (!w.on(i) || !w.on(j)) {
+      if (P.kc_mode == 1) w.K[ij] = (KT)0;   // the stored triangle; no sum reads it here
+      continue;
+    }
+    KT k = (KT)0;
+    if (w.numc[i] >= nlim_of(phase_of(P, i)) && w.numc[j] >= nlim_of(phase_of(P, j))) {
+      if (t < P.npairs_plain) {
+        BinProps<KT> b;
+        load_props<KT>(S, NB, j, b);
+        if (i != ia) load_props<KT>(S, NB, i, a);
+        k = coag_pair<KT>(cc, a, b);
+      } else if (i == j || phase_of(P, j) < 4) {
+        k = w.K[tri(j, j, NB)];   // pairs (i, j) come before (j, j), which is charged last
+      } else {
+        // a drop and a crystal bin of the same size
+        Shape<double> sh;
+        sh.alpha = SH[0 * NB + i]; sh.beta = SH[1 * NB + i]; sh.gamma = SH[2 * NB + i]; sh.sigma = SH[3 * NB + i];
+        BinProps<KT> c, b;
+        load_props<KT>(S, NB, j, b);
+        offset_props(P, w, cc, cd, sh, i, j, c);
+        k = coag_pair<KT>(cc, c, b);
+      }
+      k = charged(P, w, k, i, j);
+    }
+    w.K[ij] = k;
   }
 }
 
@@ -644,7 +761,7 @@ __device__ __forceinline__ void warp_sum8_comp(float (&hi)[8], float (&lo)[8], i
 
 // Partner sums of one target bin: FP64 in the FP64 form; compensated float sums in the
 // mixed form, from float kernels and float copies of the partner state.
-template <typename KT>
+template <typename KT, int LS>
 struct TAccT {
   using A = typename std::conditional<sizeof(KT) == 4, KahanF, double>::type;
   A sink, self;
@@ -665,7 +782,16 @@ struct TAccT {
     for (int d = 0; d < 7; d++) dg[d] = (KT)0;
   }
   __device__ __forceinline__ void reduce(bool diag, int lane) {
-    if constexpr (sizeof(KT) == 4) {
+    if constexpr (LS == 1) {
+      if constexpr (sizeof(KT) == 4) {   // the compensated sums, rounded once to float
+        sink = sink.s - sink.c;
+        self = self.s - self.c;
+#pragma unroll
+        for (int s = 0; s < SALSA_NSV; s++) src[s] = src[s].s - src[s].c;
+#pragma unroll
+        for (int d = 0; d < 7; d++) dg[d] = dg[d].s - dg[d].c;
+      }
+    } else if constexpr (sizeof(KT) == 4) {
       float h[8], l[8];
 #pragma unroll
       for (int s = 0; s < 7; s++) { h[s] = src[s].s; l[s] = -src[s].c; }
@@ -712,21 +838,23 @@ struct TAccT {
 
 // float copies of the partner state for the mixed form's coagulation update: every bin
 // before the sweep, then each bin again whenever the sweep changes it
-template <typename KT>
-__device__ __forceinline__ void shadow_all(const DevParams &P, const WS<KT> &w, int lane) {
+template <typename KT, int LS>
+__device__ __forceinline__ void shadow_all(const DevParams &P, const WS<KT, LS> &w, int lane) {
   if constexpr (sizeof(KT) == 4) {
     const int NB = w.NB, n = P.ntotal;
-    for (int b = lane; b < n; b += 32) w.nf[b] = (float)w.numc[b];
-    for (int e = lane; e < P.nused * NB; e += 32) w.vf[e] = (float)w.volc[e];
-    __syncwarp();
+    for (int b = lane; b < n; b += LS) w.nf[b] = (float)w.numc[b];
+    for (int e = lane; e < P.nused * NB; e += LS) w.vf[e] = (float)w.volc[e];
+    wsync<LS>();
   }
 }
-template <typename KT>
-__device__ __forceinline__ void shadow_bin(const DevParams &P, const WS<KT> &w, int b, int lane) {
+template <typename KT, int LS>
+__device__ __forceinline__ void shadow_bin(const DevParams &P, const WS<KT, LS> &w, int b, int lane) {
   if constexpr (sizeof(KT) == 4) {
-    if (lane < P.nused) w.vf[lane * w.NB + b] = (float)w.v(lane, b);
-    else if (lane == P.nused) w.nf[b] = (float)w.numc[b];
-    __syncwarp();
+    for (int s = lane; s <= P.nused; s += LS) {
+      if (s < P.nused) w.vf[s * w.NB + b] = (float)w.v(s, b);
+      else w.nf[b] = (float)w.numc[b];
+    }
+    wsync<LS>();
   }
 }
 
@@ -747,26 +875,28 @@ __device__ __forceinline__ void shadow_bin(const DevParams &P, const WS<KT> &w, 
 #define SIP_DLLIQ_DF 100.e-6   // mo_salsa_SIP_DF.f90:18: smallest drop that fractures on freezing
 #define SALSA_DIAG_SIPDRFR_SLOT 17   // diagnostic slot of s_n_sipdrfr (then s_n_siprmspl, s_n_sipiibr)
 
+template <typename D>
 struct SipT {
-  double *nrs, *mrs, *ndf, *mdf, *nii, *mii, *scr, *tr, *rate, *melt;
+  D nrs, mrs, ndf, mdf, nii, mii, scr, tr, rate, melt;
 };
-__device__ __forceinline__ SipT sip_tallies(const DevParams &P, double *wsbase) {
+template <typename D>
+__device__ __forceinline__ SipT<D> sip_tallies(const DevParams &P, D wsbase) {
   const int n = P.nice, pn = P.nprc * n, nn = n * n;
-  double *t = wsbase + P.sip_off;
-  double *scr = t + 4 * pn + 2 * nn, *tr = scr + 7 * n + 3 * n * SALSA_NSV;
-  return {t, t + pn, t + 2 * pn, t + 3 * pn, t + 4 * pn, t + 4 * pn + nn, scr, tr, tr + 3 * n, tr + 3 * n + 4};
+  const D t = wsbase + P.sip_off;
+  const D scr = t + (4 * pn + 2 * nn), tr = scr + (7 * n + 3 * n * SALSA_NSV);
+  return {t, t + pn, t + 2 * pn, t + 3 * pn, t + 4 * pn, t + (4 * pn + nn), scr, tr, tr + 3 * n, tr + (3 * n + 4)};
 }
 
 // zero tallies and rates; the tracers from their rows, per m3 of air (mo_salsa_driver.f90:258-262)
-template <typename KT>
-__device__ void sip_clear(const DevParams &P, const WS<KT> &w, double dn, int lane) {
-  double *t = w.raw + P.sip_off;
+template <typename KT, int LS>
+__device__ void sip_clear(const DevParams &P, const WS<KT, LS> &w, double dn, int lane) {
+  const auto t = w.raw + P.sip_off;
   const int n = 4 * P.nprc * P.nice + 2 * P.nice * P.nice;
-  for (int e = lane; e < n; e += 32) t[e] = 0.;
-  const SipT s = sip_tallies(P, w.raw);
-  for (int e = lane; e < 3 * P.nice; e += 32) s.tr[e] = w.raw[P.raw_sip + e] * dn;
-  if (lane < 4) s.rate[lane] = 0.;
-  __syncwarp();
+  for (int e = lane; e < n; e += LS) t[e] = 0.;
+  const auto s = sip_tallies(P, w.raw);
+  for (int e = lane; e < 3 * P.nice; e += LS) s.tr[e] = w.raw[P.raw_sip + e] * dn;
+  for (int e = lane; e < 4; e += LS) s.rate[e] = 0.;
+  wsync<LS>();
 }
 
 // accumulateSink's secondary-ice block (coagulation_processes.f90:863-944) for the liquid
@@ -774,10 +904,10 @@ __device__ void sip_clear(const DevParams &P, const WS<KT> &w, double dn, int la
 // numbers of drop fracturing (drops larger than the crystal) and rime splintering
 // (drops not larger), in row `row` (the precipitation bin, or 0 for every cloud bin).
 // tnlim is the target's number limit.  Lane 0.
-template <typename KT>
-__device__ void sip_drop_numbers(const DevParams &P, const WS<KT> &w, int tg, int row, double tnlim) {
+template <typename KT, int LS>
+__device__ void sip_drop_numbers(const DevParams &P, const WS<KT, LS> &w, int tg, int row, double tnlim) {
   const int I0 = P.nliquid, nice = P.nice;
-  const SipT s = sip_tallies(P, w.raw);
+  const auto s = sip_tallies(P, w.raw);
   double sum = 0.;
   for (int l = 0; l < nice; l++) sum += (double)kget(w, tg, I0 + l) * w.numc[I0 + l];
   const double fix = fmax(1. - sum, 0.1);
@@ -796,10 +926,10 @@ __device__ void sip_drop_numbers(const DevParams &P, const WS<KT> &w, int tg, in
 
 // accumulateSink's ice-ice breakup block (:881-896) for ice target kk: collisions with the
 // larger crystals kk+1..nice-1, with the aggregation efficiency of the pair.  Lane 0.
-template <typename KT>
-__device__ void sip_iibr_numbers(const DevParams &P, const WS<KT> &w, int kk, double rf_t) {
+template <typename KT, int LS>
+__device__ void sip_iibr_numbers(const DevParams &P, const WS<KT, LS> &w, int kk, double rf_t) {
   const int I0 = P.nliquid, nice = P.nice, tg = I0 + kk;
-  const SipT s = sip_tallies(P, w.raw);
+  const auto s = sip_tallies(P, w.raw);
   double sum = 0.;
   for (int l = 0; l < nice; l++) sum += (double)kget(w, tg, I0 + l) * w.numc[I0 + l];
   const double fix = fmax(1. - sum, 0.1);
@@ -818,15 +948,15 @@ __device__ void sip_iibr_numbers(const DevParams &P, const WS<KT> &w, int kk, do
 // the ice target's diameters are updated (:1291-1308), then the frozen-drop masses are
 // tallied; drops from cloud bins use the kernel of cloud bin 1 (ix = 1), as the
 // reference writes it.  Lane 0.
-template <typename KT>
-__device__ void sip_drop_masses(const DevParams &P, const WS<KT> &w, const double *dmid, int kk, int c0, int nb,
+template <typename KT, int LS>
+__device__ void sip_drop_masses(const DevParams &P, const WS<KT, LS> &w, const double *dmid, int kk, int c0, int nb,
                                 int istr, int iend, bool precip) {
   const int nice = P.nice, iwa = P.iwa, tg = P.nliquid + kk;
-  const SipT s = sip_tallies(P, w.raw);
+  const auto s = sip_tallies(P, w.raw);
   double sum = 0.;
   for (int l = 0; l < nb; l++) sum += (double)kget(w, c0 + l, tg) * w.numc[c0 + l];
   const double fix = fmax(1. - sum, 0.1);
-  updateDiameterAll(P, nullptr, w.numc, w.volc, w.dwet, w.ddry, w.dins, w.dnsp, dmid, w.NB, tg);
+  updateDiameterAll(P, w, dmid, tg);
   const double Dt = w.dnsp[tg], Nt = w.numc[tg];
   const double lnlim = precip ? K_PRLIM : K_NLIM;
   for (int ll = istr; ll <= iend; ll++) {
@@ -843,11 +973,11 @@ __device__ void sip_drop_masses(const DevParams &P, const WS<KT> &w, const doubl
 
 // accumulateSourceIce's ice-ice breakup block (:1429-1447) for ice target kk: the ice and
 // rime mass collected from the smaller crystals 0..kk-1.  Lane 0.
-template <typename KT>
-__device__ void sip_iibr_masses(const DevParams &P, const WS<KT> &w, const double *dmid, int kk, double rf_t) {
+template <typename KT, int LS>
+__device__ void sip_iibr_masses(const DevParams &P, const WS<KT, LS> &w, const double *dmid, int kk, double rf_t) {
   const int I0 = P.nliquid, nice = P.nice, tg = I0 + kk;
-  const SipT s = sip_tallies(P, w.raw);
-  updateDiameterAll(P, nullptr, w.numc, w.volc, w.dwet, w.ddry, w.dins, w.dnsp, dmid, w.NB, tg);
+  const auto s = sip_tallies(P, w.raw);
+  updateDiameterAll(P, w, dmid, tg);
   for (int ll = 0; ll < kk; ll++) {
     const int g = I0 + ll;
     if (w.dnsp[tg] > w.dnsp[g] && w.numc[tg] > K_PRLIM && w.numc[g] > K_PRLIM) {
@@ -862,8 +992,9 @@ __device__ void sip_iibr_masses(const DevParams &P, const WS<KT> &w, const doubl
 // The schemes' common end (mo_salsa_SIP_RS.f90:152-201, _DF.f90:183-237,
 // _IIBR.f90:195-250): per source bin, the sink is capped at the bin's content and scaled
 // to 99 % of its volume; then fragments are added and sinks removed.
-__device__ void sip_cap_sink(const DevParams &P, const double *numc, const double *volc, int NB, int g, double &sinkn,
-                             double *sinkv) {
+template <typename D>
+__device__ void sip_cap_sink(const DevParams &P, const D &numc, const D &volc, int NB, int g, double &sinkn,
+                             const D &sinkv) {
   const int nspec = P.nused;
   if (numc[g] < sinkn) {
     sinkn = numc[g];
@@ -878,8 +1009,9 @@ __device__ void sip_cap_sink(const DevParams &P, const double *numc, const doubl
     sinkn = fmin(sinkn, 0.99 * numc[g]);
   }
 }
-__device__ void sip_apply(const DevParams &P, double *numc, double *volc, int NB, const double *fragn,
-                          const double *fragv, const double *sinkn, const double *sinkv) {
+template <typename D>
+__device__ void sip_apply(const DevParams &P, const D &numc, const D &volc, int NB, const D &fragn, const D &fragv,
+                          const D &sinkn, const D &sinkv) {
   const int I0 = P.nliquid, nspec = P.nused;
   for (int bb = 0; bb < P.nice; bb++) {
     const int g = I0 + bb;
@@ -895,13 +1027,15 @@ __device__ void sip_apply(const DevParams &P, double *numc, double *volc, int NB
 }
 
 // Scratch of the schemes (inside the tally region).
+template <typename D>
 struct SipScr {
-  double *fragn, *sinkn, *fragn_loc, *dNb, *dVb, *diams, *bw, *fragv, *sinkv, *fragv_loc;
+  D fragn, sinkn, fragn_loc, dNb, dVb, diams, bw, fragv, sinkv, fragv_loc;
 };
-__device__ __forceinline__ SipScr sip_scratch(const DevParams &P, const SipT &t) {
+template <typename D>
+__device__ __forceinline__ SipScr<D> sip_scratch(const DevParams &P, const SipT<D> &t) {
   const int n = P.nice, V = SALSA_NSV;
-  double *p = t.scr;
-  SipScr q;
+  const D p = t.scr;
+  SipScr<D> q;
   q.fragn = p; q.sinkn = p + n; q.fragn_loc = p + 2 * n; q.dNb = p + 3 * n; q.dVb = p + 4 * n;
   q.diams = p + 5 * n; q.bw = p + 6 * n;
   q.fragv = p + 7 * n; q.sinkv = q.fragv + n * V; q.fragv_loc = q.sinkv + n * V;
@@ -909,7 +1043,8 @@ __device__ __forceinline__ SipScr sip_scratch(const DevParams &P, const SipT &t)
   return q;
 }
 // ice bin centres and widths in diameter (DF :82-88, IIBR :75-81)
-__device__ void sip_bin_geometry(const DevParams &P, const double *tb, SipScr &q) {
+template <typename D>
+__device__ void sip_bin_geometry(const DevParams &P, const double *tb, SipScr<D> &q) {
   const int I0 = P.nliquid;
   for (int bb = 0; bb < P.nice; bb++) {
     q.diams[bb] = tb[TAB_DMID * P.nb_pad + I0 + bb];
@@ -919,7 +1054,8 @@ __device__ void sip_bin_geometry(const DevParams &P, const double *tb, SipScr &q
 // Fragments dN spread over the ice bins 0..npmax-1 as d^-3 in number (DF :131-146, IIBR
 // :141-156): adds the fragment numbers and volumes (the source bin's composition);
 // returns the fragments' total volume sdv, and sv, the source bin g's.
-__device__ double sip_spread(const DevParams &P, const double *volc, int NB, int g, double dN, int npmax, SipScr &q,
+template <typename D>
+__device__ double sip_spread(const DevParams &P, const D &volc, int NB, int g, double dN, int npmax, SipScr<D> &q,
                              double &sv) {
   const int nspec = P.nused;
   for (int k = 0; k < P.nice; k++) q.dNb[k] = q.dVb[k] = 0.;
@@ -941,7 +1077,8 @@ __device__ double sip_spread(const DevParams &P, const double *volc, int NB, int
 }
 // the per-source-bin fragments join the totals before the sink safeguard (DF :175-176,
 // IIBR :187-188)
-__device__ void sip_fold_local(const DevParams &P, SipScr &q) {
+template <typename D>
+__device__ void sip_fold_local(const DevParams &P, SipScr<D> &q) {
   for (int k = 0; k < P.nice; k++) {
     q.fragn[k] = q.fragn[k] + q.fragn_loc[k];
     for (int s = 0; s < SALSA_NSV; s++) q.fragv[k * SALSA_NSV + s] = q.fragv[k * SALSA_NSV + s] + q.fragv_loc[k * SALSA_NSV + s];
@@ -952,11 +1089,11 @@ __device__ void sip_fold_local(const DevParams &P, SipScr &q) {
 
 // mo_salsa_SIP_RS.f90:28-215 rimesplintering (Hallett-Mossop per kg of rime, mode 1;
 // Mossop per frozen drop, mode 2; dltemp_rs = 5: no temperature shape).  Lane 0.
-template <typename KT>
-__device__ void sip_rimesplintering(const DevParams &P, const WS<KT> &w, double T, double dt) {
+template <typename KT, int LS>
+__device__ void sip_rimesplintering(const DevParams &P, const WS<KT, LS> &w, double T, double dt) {
   const int nprc = P.nprc, nice = P.nice, nspec = P.nused, I0 = P.nliquid, NB = w.NB;
-  const SipT t = sip_tallies(P, w.raw);
-  SipScr q = sip_scratch(P, t);
+  const auto t = sip_tallies(P, w.raw);
+  auto q = sip_scratch(P, t);
   const double v_i = 3.405365461487051e-16;   // a 10 um hexagonal column of bulk ice
   const int splbin = P.sip_splbin;
   for (int e = 0; e < nprc * nice; e++) {
@@ -967,7 +1104,7 @@ __device__ void sip_rimesplintering(const DevParams &P, const WS<KT> &w, double 
     const int g = I0 + bb;
     double vall = 0.;
     for (int s = 0; s < nspec; s++) vall += w.v(s, g);
-    double *sinkv = q.sinkv + bb * SALSA_NSV;
+    const auto sinkv = q.sinkv + bb * SALSA_NSV;
     for (int cc = 0; cc < nprc; cc++) {
       const double nf = t.nrs[cc * nice + bb], mf = t.mrs[cc * nice + bb];
       if (T < 238.15 || T > 273.15 || nf < 1.e-12 || vall < 1.e-15 || w.numc[g] < K_PRLIM || bb + 1 < splbin + 2)
@@ -1058,8 +1195,8 @@ __device__ double sip_df_phillips_mode2(const DevParams &P, double p, double T, 
   return 3. * fmin(4. * fT, 1.) * (1. - fT) * fmax(DE - 0.2, 0.);
 }
 // :313-372 the regime by the masses of drop and crystal (ice bin g)
-template <typename KT>
-__device__ double sip_df_phillips_full(const DevParams &P, const WS<KT> &w, double p, double T, double d, int g,
+template <typename KT, int LS>
+__device__ double sip_df_phillips_full(const DevParams &P, const WS<KT, LS> &w, double p, double T, double d, int g,
                                        double nf) {
   double sv = 0.;
   for (int s = 0; s < P.nused - 1; s++) sv += w.v(s, g);
@@ -1074,12 +1211,12 @@ __device__ double sip_df_phillips_full(const DevParams &P, const WS<KT> &w, doub
   return fmin(sip_df_phillips_mode2(P, p, T, d, w.dwet[g], w.dnsp[g], mrim, mpri, ncice, rhoip), 100.) * nf;
 }
 
-template <typename KT>
-__device__ void sip_dropfracturing(const DevParams &P, const WS<KT> &w, const double *tb, double T, double pres,
+template <typename KT, int LS>
+__device__ void sip_dropfracturing(const DevParams &P, const WS<KT, LS> &w, const double *tb, double T, double pres,
                                    double dt) {
   const int nprc = P.nprc, nice = P.nice, nspec = P.nused, I0 = P.nliquid, NB = w.NB;
-  const SipT t = sip_tallies(P, w.raw);
-  SipScr q = sip_scratch(P, t);
+  const auto t = sip_tallies(P, w.raw);
+  auto q = sip_scratch(P, t);
   sip_bin_geometry(P, tb, q);
   for (int e = 0; e < nprc * nice; e++) {
     t.mdf[e] = t.mdf[e] * dt;
@@ -1089,7 +1226,7 @@ __device__ void sip_dropfracturing(const DevParams &P, const WS<KT> &w, const do
     const int g = I0 + bb;
     double vall = 0.;
     for (int s = 0; s < nspec; s++) vall += w.v(s, g);
-    double *sinkv = q.sinkv + bb * SALSA_NSV;
+    const auto sinkv = q.sinkv + bb * SALSA_NSV;
     for (int cc = 0; cc < nprc; cc++) {
       const double nf = t.ndf[cc * nice + bb], mf = t.mdf[cc * nice + bb];
       if (T < 248.15 || T > 271.15 || nf < 1.e-12 || vall < 1.e-15 || w.numc[g] < K_PRLIM) continue;
@@ -1135,15 +1272,15 @@ __device__ double sip_iibr_imf(int mode, double T, double dmin) {
 // the smaller crystal; the source bin's diameters are updated first.  Lane 0.
 // mo_salsa_SIP_IIBR.f90:588-607 mip and :552-585 getvelocity: mean crystal mass of ice
 // bin g, and its fall speed with the bin's shape coefficients and rime-weighted density
-template <typename KT>
-__device__ __forceinline__ void sip_iibr_masses(const DevParams &P, const WS<KT> &w, int g, double &mrim, double &mpri) {
+template <typename KT, int LS>
+__device__ __forceinline__ void sip_iibr_masses(const DevParams &P, const WS<KT, LS> &w, int g, double &mrim, double &mpri) {
   double v = 0.;
   for (int k = 0; k <= P.iwa; k++) v += w.v(k, g);
   mrim = w.v(P.irim, g) * K_RHORI;
   mpri = v * K_RHOIC;
 }
-template <typename KT>
-__device__ double sip_iibr_velocity(const DevParams &P, const WS<KT> &w, int g, double visc, double rhoa, double mfp) {
+template <typename KT, int LS>
+__device__ double sip_iibr_velocity(const DevParams &P, const WS<KT, LS> &w, int g, double visc, double rhoa, double mfp) {
   const double knud = ddiv(2. * mfp, w.dnsp[g]);
   const double beta = 1. + knud * (1.142 + 0.558 * dexp(-ddiv(0.999, knud)));
   double mrim, mpri;
@@ -1157,8 +1294,8 @@ __device__ double sip_iibr_velocity(const DevParams &P, const WS<KT> &w, int g, 
 // Sotiropoulou et al. (2020); asperity parameters by the rime fraction of bin `small`, the
 // supersaturation over ice ssi and the distance from -15 C; the collision's kinetic energy
 // from both bins' fall speeds (:505-548)
-template <typename KT>
-__device__ double sip_imf_phillips(const DevParams &P, const WS<KT> &w, double p, double T, int large, int small,
+template <typename KT, int LS>
+__device__ double sip_imf_phillips(const DevParams &P, const WS<KT, LS> &w, double p, double T, int large, int small,
                                    double disphmin, double ssi) {
   const double T0 = 258.15;
   double mrim, mpri;
@@ -1191,13 +1328,13 @@ __device__ double sip_imf_phillips(const DevParams &P, const WS<KT> &w, double p
   return fmin(alpha * Am * (1 - dexp(-dpow(ddiv(ddiv(C * K0, alpha), Am), gg))), Nmax);
 }
 
-template <typename KT>
-__device__ void sip_iceicecollbreak(const DevParams &P, const WS<KT> &w, const double *tb, double T, double pres,
+template <typename KT, int LS>
+__device__ void sip_iceicecollbreak(const DevParams &P, const WS<KT, LS> &w, const double *tb, double T, double pres,
                                     double rv, double rsi, double dt) {
   const int nice = P.nice, nspec = P.nused, I0 = P.nliquid, NB = w.NB;
   const double *dmid = tb + TAB_DMID * P.nb_pad;
-  const SipT t = sip_tallies(P, w.raw);
-  SipScr q = sip_scratch(P, t);
+  const auto t = sip_tallies(P, w.raw);
+  auto q = sip_scratch(P, t);
   sip_bin_geometry(P, tb, q);
   for (int e = 0; e < nice * nice; e++) {
     t.mii[e] = t.mii[e] * dt;
@@ -1205,7 +1342,7 @@ __device__ void sip_iceicecollbreak(const DevParams &P, const WS<KT> &w, const d
   }
   for (int bb = 0; bb < nice; bb++) {
     const int g = I0 + bb;
-    double *sinkv = q.sinkv + bb * SALSA_NSV;
+    const auto sinkv = q.sinkv + bb * SALSA_NSV;
     for (int cc = bb; cc < nice; cc++) {
       const int h = I0 + cc;
       const double nii = t.nii[cc * nice + bb], mii = t.mii[cc * nice + bb];
@@ -1214,7 +1351,7 @@ __device__ void sip_iceicecollbreak(const DevParams &P, const WS<KT> &w, const d
       if (T < 248.15 || T > 270.15 || nii < 1.e-12 || mii < 1.e-15 || vb < 1.e-15 || w.numc[g] < K_PRLIM ||
           vc < 1.e-15 || w.numc[h] < K_PRLIM)
         continue;
-      updateDiameterAll(P, nullptr, w.numc, w.volc, w.dwet, w.ddry, w.dins, w.dnsp, dmid, NB, g);
+      updateDiameterAll(P, w, dmid, g);
       const double v_i = ddiv(ddiv(mii, nii), w.rhomean[g]);
       const double dinsphmin = dpow(divc(v_i, K_PI6), 1. / 3.);
       int npmax = 0;
@@ -1250,23 +1387,24 @@ __device__ void sip_iceicecollbreak(const DevParams &P, const WS<KT> &w, const d
 }
 
 // secondary_ice (mo_salsa_secondary_ice.f90:6-40), after coagulation (mo_salsa.f90:98-99)
-template <typename KT>
-__device__ void secondary_ice(const DevParams &P, const WS<KT> &w, const double *tb, double T, double pres, double rv,
+template <typename KT, int LS>
+__device__ void secondary_ice(const DevParams &P, const WS<KT, LS> &w, const double *tb, double T, double pres, double rv,
                               double rsi, double dt, int lane) {
-  __syncwarp();
+  wsync<LS>();
   if (lane == 0) {
     if (P.st_siprs) sip_rimesplintering<KT>(P, w, T, dt);
     if (P.st_sipdf) sip_dropfracturing<KT>(P, w, tb, T, pres, dt);
     if (P.st_sipib) sip_iceicecollbreak<KT>(P, w, tb, T, pres, rv, rsi, dt);
   }
-  __syncwarp();
+  wsync<LS>();
 }
 
-template <typename KT>
-__device__ __forceinline__ void source_range(const WS<KT> &w, int t, int g0, int istr, int iend, int nspec,
-                                             TAccT<KT> &a, int lane) {
-  for (int ll = istr + lane; ll <= iend; ll += 32) {
+template <typename KT, int LS>
+__device__ __forceinline__ void source_range(const WS<KT, LS> &w, int t, int g0, int istr, int iend, int nspec,
+                                             TAccT<KT, LS> &a, int lane) {
+  for (int ll = istr + lane; ll <= iend; ll += LS) {
     int g = g0 + ll;
+    if (!w.on(g)) continue;
     const KT k = kget(w, g, t);
 #pragma unroll
     for (int s = 0; s < SALSA_NSV; s++)
@@ -1281,21 +1419,23 @@ __device__ __forceinline__ const int16_t *partner_lists(const DevParams &P, cons
   return reinterpret_cast<const int16_t *>(tb + P.list_off);
 }
 
-template <typename KT>
-__device__ __forceinline__ void list_sinks(const WS<KT> &w, const int16_t *L, int t, TAccT<KT> &a, int lane) {
+template <typename KT, int LS>
+__device__ __forceinline__ void list_sinks(const WS<KT, LS> &w, const int16_t *L, int t, TAccT<KT, LS> &a, int lane) {
   const int off = L[4 * t], n = L[4 * t + 1];
-  for (int e = lane; e < n; e += 32) {
+  for (int e = lane; e < n; e += LS) {
     const int g = L[off + e];
+    if (!w.on(g)) continue;
     a.sink += kget(w, t, g) * w.nk(g);
   }
 }
 
-template <typename KT>
-__device__ __forceinline__ void list_sources(const WS<KT> &w, const int16_t *L, int t, int nspec, TAccT<KT> &a,
+template <typename KT, int LS>
+__device__ __forceinline__ void list_sources(const WS<KT, LS> &w, const int16_t *L, int t, int nspec, TAccT<KT, LS> &a,
                                              int lane) {
   const int off = L[4 * t + 2], n = L[4 * t + 3];
-  for (int e = lane; e < n; e += 32) {
+  for (int e = lane; e < n; e += LS) {
     const int g = L[off + e];
+    if (!w.on(g)) continue;
     const KT k = kget(w, g, t);
 #pragma unroll
     for (int s = 0; s < SALSA_NSV; s++)
@@ -1305,9 +1445,19 @@ __device__ __forceinline__ void list_sources(const WS<KT> &w, const int16_t *L, 
 
 // applyCoag (:539-559): lanes 0..nspec-1 update the volumes and lane nspec the number,
 // all in one division.
-template <typename KT>
-__device__ __forceinline__ void apply_coag(const DevParams &P, const WS<KT> &w, int t, int nspec, double dt,
-                                           const TAccT<KT> &a, int lane) {
+template <typename KT, int LS>
+__device__ __forceinline__ void apply_coag(const DevParams &P, const WS<KT, LS> &w, int t, int nspec, double dt,
+                                           const TAccT<KT, LS> &a, int lane) {
+  if constexpr (LS == 1) {
+    const double n = w.numc[t], sink = a.sink, self = a.self;
+    const double den = 1. + dt * sink, r = drcp(den);
+#pragma unroll
+    for (int s = 0; s < SALSA_NSV; s++)
+      if (s < nspec) w.v(s, t) = ddiv_r(w.v(s, t) + dt * (double)a.src[s] * n, den, r);
+    w.numc[t] = ddiv(n, 1. + dt * (sink + self));
+    shadow_bin<KT>(P, w, t, lane);
+    return;
+  }
   double my = 0.;
 #pragma unroll
   for (int s = 0; s < SALSA_NSV; s++)
@@ -1318,20 +1468,20 @@ __device__ __forceinline__ void apply_coag(const DevParams &P, const WS<KT> &w, 
   const double num = vol ? w.v(lane, t) + dt * my * n : n;
   const double den = vol ? 1. + dt * sink : 1. + dt * (sink + self);
   const double q = ddiv(num, den);
-  __syncwarp();
+  wsync<LS>();
   if (vol) w.v(lane, t) = q;
   else if (lane == nspec) w.numc[t] = q;
-  __syncwarp();
+  wsync<LS>();
   shadow_bin<KT>(P, w, t, lane);
 }
 
-template <typename KT>
-__device__ void coag_aero(const DevParams &P, const WS<KT> &w, const double *tb, double dt, int lane) {
+template <typename KT, int LS>
+__device__ void coag_aero(const DevParams &P, const WS<KT, LS> &w, const double *tb, double dt, int lane) {
   const int nspec = P.nwet;
   const int16_t *L = partner_lists(P, tb);
   for (int kk = P.in1a; kk <= P.fn2b; kk++) {
     if (w.numc[kk] < K_NLIM) continue;
-    TAccT<KT> a;
+    TAccT<KT, LS> a;
     a.zero();
     if (P.lscgaa && lane == 0) a.self = (KT)0.5 * kget(w, kk, kk) * w.nk(kk);
     list_sinks(w, L, kk, a, lane);
@@ -1344,15 +1494,58 @@ __device__ void coag_aero(const DevParams &P, const WS<KT> &w, const double *tb,
 // accumulatePrecipFormation (:1457-1584) for the partners istr..iend (cloud-local) of
 // target t (cloud-local).  Per-partner contributions are staged in partner slots and
 // summed per precipitation bin in partner order, which keeps the result deterministic.
-template <typename KT>
-__device__ void precip_formation(const DevParams &P, const WS<KT> &w, const double *tb, int t, int istr, int iend,
-                                 double fix, bool selfcoll, TAccT<KT> &a, bool diag, int lane) {
+template <typename KT, int LS>
+__device__ void precip_formation(const DevParams &P, const WS<KT, LS> &w, const double *tb, int t, int istr, int iend,
+                                 double fix, bool selfcoll, TAccT<KT, LS> &a, bool diag, int lane) {
   const int C0 = P.nbins, nspec = P.nwet, nprc = P.nprc, iwa = P.iwa;
   const double *pbins = tb + TAB_PRECPBINS * P.nb_pad;
-  double *pf = w.misc + M_PF;                // [0..6] volsink, then vol_prc[nprc][7], num_prc[nprc], INFnum[nprc]
-  double *vol_prc = pf + 7, *num_prc = pf + 7 + 7 * nprc, *inf_prc = num_prc + nprc;
-  double *slot = w.misc + M_PFSLOT;          // 8 slots x 10: tp, dvol[7], dnum, x*dnum
+  const auto pf = w.misc + M_PF;                // [0..6] volsink, then vol_prc[nprc][7], num_prc[nprc], INFnum[nprc]
+  const auto vol_prc = pf + 7, num_prc = pf + (7 + 7 * nprc), inf_prc = num_prc + nprc;
+  const auto slot = w.misc + M_PFSLOT;          // 8 slots x 10: tp, dvol[7], dnum, x*dnum
   const int tg = C0 + t;
+  if constexpr (LS == 1) {
+    for (int ll = istr; ll <= iend; ll++) {
+      const int lg = C0 + ll;
+      if (!w.on(lg)) continue;
+      const double D_new = dcbrt(cube(w.dwet[tg]) + cube(w.dwet[lg]));
+      int cnt = 0;
+      for (int i = 0; i < nprc; i++) cnt += (D_new > pbins[i]);
+      const double klt = (double)kget(w, lg, tg), nt = w.numc[tg], nl = w.numc[lg];
+      if (cnt > 0) {
+        const int tp = cnt - 1;
+        double dvw = 0., dnum, xin;
+        for (int s = 0; s < nspec; s++) {
+          const double dv = selfcoll ? w.v(s, lg) * nt * klt * fix : (w.v(s, lg) * nt + w.v(s, tg) * nl) * klt * fix;
+          vol_prc[tp * 7 + s] += dv;
+          if (selfcoll) pf[s] += dv;   // volsink_slf
+          if (s == iwa) dvw = dv;
+        }
+        if (selfcoll) {
+          dnum = (0.5 * klt * nl * nt) * fix;
+          xin = w.indef[lg] * dnum;
+          a.self += (KT)(0.5 * klt * nt);
+        } else {
+          dnum = (klt * nl * nt) * fix;
+          xin = 0.5 * (w.indef[lg] + w.indef[tg]) * dnum;
+          a.sink += (KT)(klt * nl);
+        }
+        num_prc[tp] += dnum;
+        inf_prc[tp] += xin;
+        if (diag) {
+          a.dg[0] += (KT)dvw;
+          if (D_new > 50.e-6) a.dg[2] += (KT)dvw;
+          if (D_new > 80.e-6) a.dg[1] += (KT)dvw;
+        }
+      } else if (selfcoll) {
+        a.self += (KT)(0.5 * klt * nl);
+      } else {
+#pragma unroll
+        for (int s = 0; s < SALSA_NSV; s++)
+          if (s < nspec) a.src[s] += (KT)(klt * w.v(s, lg));
+      }
+    }
+    return;
+  }
   for (int c0 = istr; c0 <= iend; c0 += 8) {
     int np = min(8, iend - c0 + 1);
     if (lane < np) {
@@ -1363,7 +1556,7 @@ __device__ void precip_formation(const DevParams &P, const WS<KT> &w, const doub
       for (int i = 0; i < nprc; i++) cnt += (D_new > pbins[i]);
       double klt = (double)kget(w, lg, tg);
       double nt = w.numc[tg], nl = w.numc[lg];
-      double *sl = slot + lane * 10;
+      const auto sl = slot + lane * 10;
       sl[0] = (double)(cnt - 1);
       double dnum = 0.;
       if (D_new > pbins[0]) {
@@ -1396,14 +1589,14 @@ __device__ void precip_formation(const DevParams &P, const WS<KT> &w, const doub
       }
       sl[8] = dnum;
     }
-    __syncwarp();
+    wsync<LS>();
     // sum the staged contributions per precipitation bin (partner order)
-    for (int e = lane; e < nprc * (nspec + 2); e += 32) {
+    for (int e = lane; e < nprc * (nspec + 2); e += LS) {
       int tp = e / (nspec + 2), q = e % (nspec + 2);
       double acc = 0.;
       bool any = false;
       for (int j = 0; j < np; j++) {
-        const double *sl = slot + j * 10;
+        const auto sl = slot + j * 10;
         if ((int)sl[0] == tp) { acc += (q < nspec) ? sl[1 + q] : (q == nspec ? sl[8] : sl[9]); any = true; }
       }
       if (any) {
@@ -1414,19 +1607,19 @@ __device__ void precip_formation(const DevParams &P, const WS<KT> &w, const doub
     }
     if (selfcoll && lane < nspec) {
       // volsink_slf: the single self partner's contribution (same expression as dvol)
-      const double *sl = slot;
+      const auto sl = slot;
       if ((int)sl[0] >= 0) pf[lane] += sl[1 + lane];
     }
-    __syncwarp();
+    wsync<LS>();
   }
 }
 
-template <typename KT, bool SIP>
-__device__ void coag_cloud(const DevParams &P, const WS<KT> &w, const double *tb, double dt, bool diag, int lane) {
+template <typename KT, bool SIP, int LS>
+__device__ void coag_cloud(const DevParams &P, const WS<KT, LS> &w, const double *tb, double dt, bool diag, int lane) {
   const int nspec = P.nwet, C0 = P.nbins, P0 = P.nbins + P.ncld, nprc = P.nprc;
   const bool autoc1 = P.st_auto && P.auto_mode == 1;
   const int16_t *L = partner_lists(P, tb);
-  double *pf = w.misc + M_PF;
+  const auto pf = w.misc + M_PF;
   for (int reg = 0; reg < 2; reg++) {
     int kfirst = reg == 0 ? P.ica_cur : P.icb_cur;
     int klast = reg == 0 ? P.fca_cur : P.fcb_cur;
@@ -1435,18 +1628,18 @@ __device__ void coag_cloud(const DevParams &P, const WS<KT> &w, const double *tb
     for (int kk = kfirst; kk <= klast; kk++) {
       int tg = C0 + kk;
       if (w.numc[tg] < K_NLIM) continue;
-      TAccT<KT> a;
+      TAccT<KT, LS> a;
       a.zero();
       if (autoc1) {
-        for (int e = lane; e < 7 + nprc * 9; e += 32) pf[e] = 0.;
-        __syncwarp();
+        for (int e = lane; e < 7 + nprc * 9; e += LS) pf[e] = 0.;
+        wsync<LS>();
       }
       int other = o_first + (kk - kfirst);
       int rel = kk - kfirst;
       list_sinks(w, L, tg, a, lane);
       if constexpr (SIP) {
         if (P.st_secice && P.lscgic && lane == 0) sip_drop_numbers<KT>(P, w, tg, 0, K_NLIM);
-        __syncwarp();
+        wsync<LS>();
       }
       if (P.lscgcc) {
         if (autoc1) {
@@ -1460,7 +1653,8 @@ __device__ void coag_cloud(const DevParams &P, const WS<KT> &w, const double *tb
       if (P.lscgca) {
         int iaa = P.ica_par + rel, iab = P.icb_par + rel;
         KT cm = 0;
-        for (int ll = P.in1a + lane; ll <= iaa; ll += 32) {
+        for (int ll = P.in1a + lane; ll <= iaa; ll += LS) {
+          if (!w.on(ll)) continue;
           const KT k = kget(w, ll, tg);
           {
 #pragma unroll
@@ -1469,7 +1663,8 @@ __device__ void coag_cloud(const DevParams &P, const WS<KT> &w, const double *tb
           }
           if (diag) for (int s = 0; s < P.ndry; s++) cm += k * w.vk(s, ll) * (KT)P.rholiq[s];
         }
-        for (int ll = P.in2b + lane; ll <= iab; ll += 32) {
+        for (int ll = P.in2b + lane; ll <= iab; ll += LS) {
+          if (!w.on(ll)) continue;
           const KT k = kget(w, ll, tg);
           {
 #pragma unroll
@@ -1483,13 +1678,13 @@ __device__ void coag_cloud(const DevParams &P, const WS<KT> &w, const double *tb
       if (P.lscgcc && kk > kfirst) {
         if (autoc1) {
           double s1 = 0.;
-          for (int i = kfirst + lane; i <= klast; i += 32) s1 += (double)kget(w, tg, C0 + i) * w.numc[C0 + i];
-          s1 = warp_sum(s1);
+          for (int i = kfirst + lane; i <= klast; i += LS) s1 += (double)kget(w, tg, C0 + i) * w.numc[C0 + i];
+          s1 = wsum<LS>(s1);
           double fix = fmax(1. - dt * s1, 0.1);
           precip_formation(P, w, tb, kk, kfirst, kk - 1, fix, false, a, diag, lane);
           double s2 = 0.;
-          for (int i = o_first + lane; i <= o_last; i += 32) s2 += (double)kget(w, tg, C0 + i) * w.numc[C0 + i];
-          s2 = warp_sum(s2);
+          for (int i = o_first + lane; i <= o_last; i += LS) s2 += (double)kget(w, tg, C0 + i) * w.numc[C0 + i];
+          s2 = wsum<LS>(s2);
           fix = fmax(1. - dt * s2, 0.1);
           precip_formation(P, w, tb, kk, o_first, other, fix, false, a, diag, lane);
         } else {
@@ -1508,14 +1703,14 @@ __device__ void coag_cloud(const DevParams &P, const WS<KT> &w, const double *tb
       apply_coag(P, w, tg, nspec, dt, a, lane);
       if (autoc1) {
         // applyCoagPrecipFormation (:654-702)
-        const double *vol_prc = pf + 7, *num_prc = pf + 7 + 7 * nprc, *inf_num = num_prc + nprc;
-        if (lane < nspec) w.v(lane, tg) = w.v(lane, tg) - dt * pf[lane];
-        for (int e = lane; e < nprc * nspec; e += 32) {
+        const auto vol_prc = pf + 7, num_prc = pf + (7 + 7 * nprc), inf_num = num_prc + nprc;
+        for (int s = lane; s < nspec; s += LS) w.v(s, tg) = w.v(s, tg) - dt * pf[s];
+        for (int e = lane; e < nprc * nspec; e += LS) {
           int cc = e / nspec, s = e % nspec;
           w.v(s, P0 + cc) = w.v(s, P0 + cc) + dt * vol_prc[cc * 7 + s];
         }
-        __syncwarp();
-        for (int cc = lane; cc < nprc; cc += 32) {
+        wsync<LS>();
+        for (int cc = lane; cc < nprc; cc += LS) {
           int g = P0 + cc;
           double nrate = num_prc[cc];
           double inf = nrate > 0. ? ddiv(inf_num[cc], nrate) : 0.;
@@ -1523,7 +1718,7 @@ __device__ void coag_cloud(const DevParams &P, const WS<KT> &w, const double *tb
           w.numc[g] = n;
           if (n > K_PRLIM) w.indef[g] = ddiv(w.indef[g] * (n - dt * nrate) + inf * dt * nrate, n);
         }
-        __syncwarp();
+        wsync<LS>();
         shadow_bin<KT>(P, w, tg, lane);
         for (int cc = 0; cc < nprc; cc++) shadow_bin<KT>(P, w, P0 + cc, lane);
       }
@@ -1531,27 +1726,28 @@ __device__ void coag_cloud(const DevParams &P, const WS<KT> &w, const double *tb
   }
 }
 
-template <typename KT, bool SIP>
-__device__ void coag_precp(const DevParams &P, const WS<KT> &w, const double *tb, double dt, bool diag, int lane) {
+template <typename KT, bool SIP, int LS>
+__device__ void coag_precp(const DevParams &P, const WS<KT, LS> &w, const double *tb, double dt, bool diag, int lane) {
   const int nspec = P.nwet, C0 = P.nbins, P0 = P.nbins + P.ncld, nprc = P.nprc, iwa = P.iwa;
   const double *pbins = tb + TAB_PRECPBINS * P.nb_pad;
   const int16_t *L = partner_lists(P, tb);
   for (int kk = 0; kk < nprc; kk++) {
     int tg = P0 + kk;
     if (w.numc[tg] < K_PRLIM) continue;
-    TAccT<KT> a;
+    TAccT<KT, LS> a;
     a.zero();
     double num_slf = 0.;
     list_sinks(w, L, tg, a, lane);
     if constexpr (SIP) {
       if (P.st_secice && P.lscgip && lane == 0) sip_drop_numbers<KT>(P, w, tg, kk, K_PRLIM);
-      __syncwarp();
+      wsync<LS>();
     }
     if (P.lscgpp && kk == nprc - 1 && lane == 0) a.self += (KT)0.5 * kget(w, tg, tg) * w.nk(tg);
     const double D = w.dwet[tg];
     if (P.lscgpa) {
       KT cm = 0;
-      for (int ll = P.in1a + lane; ll <= P.fn2b; ll += 32) {
+      for (int ll = P.in1a + lane; ll <= P.fn2b; ll += LS) {
+        if (!w.on(ll)) continue;
         const KT k = kget(w, ll, tg);
         {
 #pragma unroll
@@ -1564,8 +1760,9 @@ __device__ void coag_precp(const DevParams &P, const WS<KT> &w, const double *tb
     }
     if (P.lscgpc) {
       // source from cloud; accretion and autoconversion diagnostics (:1086-1215, coll phase 2)
-      for (int ll = lane; ll < P.ncld; ll += 32) {
+      for (int ll = lane; ll < P.ncld; ll += LS) {
         int g = C0 + ll;
+        if (!w.on(g)) continue;
         const KT k = kget(w, g, tg);
         {
 #pragma unroll
@@ -1585,8 +1782,9 @@ __device__ void coag_precp(const DevParams &P, const WS<KT> &w, const double *tb
     }
     if (P.lscgpp && kk > 0) {
       int ex80 = min(kk - 1, P.cnt80 - 1), ex50 = min(kk - 1, P.cnt50 - 1);
-      for (int ll = lane; ll <= kk - 1; ll += 32) {
+      for (int ll = lane; ll <= kk - 1; ll += LS) {
         int g = P0 + ll;
+        if (!w.on(g)) continue;
         const KT k = kget(w, g, tg);
         {
 #pragma unroll
@@ -1616,41 +1814,55 @@ __device__ void coag_precp(const DevParams &P, const WS<KT> &w, const double *tb
     // precipSelfCoag (:1588-1611) with the pre-update state
     double kself = (P.lscgpp && kk < nprc - 1) ? (double)kget(w, tg, tg) : 0.;
     double nold = w.numc[tg];
-    double vs_my = (lane < nspec) ? w.v(lane, tg) * nold * kself : 0.;
+    double vs_my[LS == 1 ? SALSA_NSV : 1];
+    if constexpr (LS == 1) {
+#pragma unroll
+      for (int s = 0; s < SALSA_NSV; s++) vs_my[s] = s < nspec ? w.v(s, tg) * nold * kself : 0.;
+    } else {
+      vs_my[0] = (lane < nspec) ? w.v(lane, tg) * nold * kself : 0.;
+    }
     num_slf = 0.5 * kself * nold * nold;
     apply_coag(P, w, tg, nspec, dt, a, lane);
     if (P.lscgpp && kk < nprc - 1) {
       // applyCoagPrecp (:584-599): self-coagulation products go to the next bin
-      if (lane < nspec) {
-        w.v(lane, tg + 1) = w.v(lane, tg + 1) + dt * vs_my;
-        w.v(lane, tg) = w.v(lane, tg) - dt * vs_my;
+      if constexpr (LS == 1) {
+#pragma unroll
+        for (int s = 0; s < SALSA_NSV; s++)
+          if (s < nspec) {
+            w.v(s, tg + 1) = w.v(s, tg + 1) + dt * vs_my[s];
+            w.v(s, tg) = w.v(s, tg) - dt * vs_my[s];
+          }
+      } else if (lane < nspec) {
+        w.v(lane, tg + 1) = w.v(lane, tg + 1) + dt * vs_my[0];
+        w.v(lane, tg) = w.v(lane, tg) - dt * vs_my[0];
       }
       if (lane == 0) {
         w.numc[tg + 1] = w.numc[tg + 1] + dt * num_slf;
         w.numc[tg] = w.numc[tg] - dt * num_slf;
       }
-      __syncwarp();
+      wsync<LS>();
       shadow_bin<KT>(P, w, tg, lane);
       shadow_bin<KT>(P, w, tg + 1, lane);
     }
   }
 }
 
-template <typename KT, bool SIP>
-__device__ void coag_ice(const DevParams &P, const WS<KT> &w, const double *tb, double dt, int lane) {
+template <typename KT, bool SIP, int LS>
+__device__ void coag_ice(const DevParams &P, const WS<KT, LS> &w, const double *tb, double dt, int lane) {
   const int nspec = P.nused, C0 = P.nbins, P0 = P.nbins + P.ncld, I0 = P.nliquid, nice = P.nice;
   const int iwa = P.iwa, irim = P.irim, ndry = P.ndry;
   (void)C0; (void)P0; (void)tb;
   for (int kk = 0; kk < nice; kk++) {
     int tg = I0 + kk;
     if (w.numc[tg] < K_PRLIM) continue;
-    TAccT<KT> a;
+    TAccT<KT, LS> a;
     a.zero();
     double rf_t = rimefrac(P, w.numc[tg], w.v(iwa, tg), w.v(irim, tg), 4);
     if (P.lscgii) {
       // Eagg from the larger rime fraction of the pair (:758-769)
-      for (int ll = kk + 1 + lane; ll <= nice - 1; ll += 32) {
+      for (int ll = kk + 1 + lane; ll <= nice - 1; ll += LS) {
         int g = I0 + ll;
+        if (!w.on(g)) continue;
         double rf = fmax(rimefrac(P, w.numc[g], w.v(iwa, g), w.v(irim, g), 4), rf_t);
         double E = P.Eiagg_max - rf * (P.Eiagg_max - P.Eiagg_min);
         a.sink += (KT)E * (KT)1.0 * kget(w, tg, g) * w.nk(g);
@@ -1671,11 +1883,12 @@ __device__ void coag_ice(const DevParams &P, const WS<KT> &w, const double *tb, 
         if (P.lscgip) sip_drop_masses<KT>(P, w, dmid, kk, P0, P.nprc, 0, P.nprc - 1, true);
         if (P.lscgii && kk > 0 && P.st_sipib) sip_iibr_masses<KT>(P, w, dmid, kk, rf_t);
       }
-      __syncwarp();
+      wsync<LS>();
     }
     // accumulateSourcePhaseChange (:1244-1280)
     if (P.lscgia)
-      for (int ll = P.in1a + lane; ll <= P.fn2b; ll += 32) {
+      for (int ll = P.in1a + lane; ll <= P.fn2b; ll += LS) {
+        if (!w.on(ll)) continue;
         const KT k = kget(w, ll, tg);
         {
 #pragma unroll
@@ -1685,8 +1898,9 @@ __device__ void coag_ice(const DevParams &P, const WS<KT> &w, const double *tb, 
         a.add_at(iwa, divc(k * w.vk(iwa, ll) * (KT)K_RHOWA, (KT)K_RHOIC));
       }
     if (P.lscgic)
-      for (int ll = lane; ll < P.ncld; ll += 32) {
+      for (int ll = lane; ll < P.ncld; ll += LS) {
         int g = C0 + ll;
+        if (!w.on(g)) continue;
         const KT k = kget(w, g, tg);
         {
 #pragma unroll
@@ -1696,8 +1910,9 @@ __device__ void coag_ice(const DevParams &P, const WS<KT> &w, const double *tb, 
         a.add_at(irim, divc(k * w.vk(iwa, g) * (KT)K_RHOWA, (KT)K_RHORI));
       }
     if (P.lscgip)
-      for (int ll = lane; ll < P.nprc; ll += 32) {
+      for (int ll = lane; ll < P.nprc; ll += LS) {
         int g = P0 + ll;
+        if (!w.on(g)) continue;
         const KT k = kget(w, g, tg);
         {
 #pragma unroll
@@ -1708,7 +1923,7 @@ __device__ void coag_ice(const DevParams &P, const WS<KT> &w, const double *tb, 
       }
     // accumulateSourceIce (:1385-1427)
     if (P.lscgii && kk > 0)
-      for (int ll = lane; ll <= kk - 1; ll += 32) {
+      for (int ll = lane; ll <= kk - 1; ll += LS) {
         int g = I0 + ll;
         double rf = fmax(rimefrac(P, w.numc[g], w.v(iwa, g), w.v(irim, g), 4), rf_t);
         double E = P.Eiagg_max - rf * (P.Eiagg_max - P.Eiagg_min);
@@ -1723,17 +1938,34 @@ __device__ void coag_ice(const DevParams &P, const WS<KT> &w, const double *tb, 
     // applyCoagIce (:605-651): every species slot with the same semi-implicit form
     apply_coag(P, w, tg, nspec, dt, a, lane);
     if (lane == 0) w.rhomean[tg] = rhomean_of(P, 4, w.numc[tg], w.v(iwa, tg), w.v(irim, tg));
-    __syncwarp();
+    wsync<LS>();
   }
 }
 
-template <typename KT, bool SIP>
-__device__ __forceinline__ void coagulation(const DevParams &P, const WS<KT> &w, const double *tb, double dt, double T, double pres,
+// the bins that reach their limit in some cell of the warp (all of them when the kernels come
+// from the storage, whose pairs were populated at another step); all 32 lanes arrive together
+template <typename KT>
+__device__ __forceinline__ void mark_populated(const DevParams &P, WS<KT, 1> &w) {
+  unsigned m[3] = {0u, 0u, 0u};
+#pragma unroll
+  for (int k = 0; k < 3; k++)
+    for (int b = 32 * k; b < min(P.ntotal, 32 * k + 32); b++)
+      if (P.kc_mode == 2 || w.numc[b] >= nlim_of(phase_of(P, b))) m[k] |= 1u << (b - 32 * k);
+  __syncwarp();
+#pragma unroll
+  for (int k = 0; k < 3; k++) m[k] = __reduce_or_sync(0xffffffffu, m[k]);
+  w.am0 = (unsigned long long)m[0] | ((unsigned long long)m[1] << 32);
+  w.am1 = m[2];
+}
+
+template <typename KT, bool SIP, int LS>
+__device__ __forceinline__ void coagulation(const DevParams &P, WS<KT, LS> &w, const double *tb, double dt, double T, double pres,
                             bool diag, long long cell, int lane) {
   const double *dmid = tb + TAB_DMID * P.nb_pad;
+  if constexpr (LS == 1) mark_populated(P, w);
   // updateDiameter("all") on every bin (:146-152) and rhomean of the kernel categories
-  for (int b = lane; b < P.ntotal; b += 32) {
-    updateDiameterAll(P, nullptr, w.numc, w.volc, w.dwet, w.ddry, w.dins, w.dnsp, dmid, w.NB, b);
+  for (int b = lane; b < P.ntotal; b += LS) {
+    updateDiameterAll(P, w, dmid, b);
     int ph = phase_of(P, b);
     bool inker = (ph == 1 && (P.lscgaa || P.lscgca || P.lscgpa || P.lscgia)) ||
                  (ph == 2 && (P.lscgcc || P.lscgca || P.lscgpc || P.lscgic)) ||
@@ -1741,7 +1973,7 @@ __device__ __forceinline__ void coagulation(const DevParams &P, const WS<KT> &w,
                  (ph == 4 && (P.lscgii || P.lscgia || P.lscgic || P.lscgip));
     if (inker) w.rhomean[b] = rhomean_of(P, ph, w.numc[b], w.v(P.iwa, b), w.v(P.irim, b));
   }
-  __syncwarp();
+  wsync<LS>();
 #ifdef SALSA_STAGE_TIMERS
   long long t_k0 = clock64();
 #endif
@@ -1749,17 +1981,17 @@ __device__ __forceinline__ void coagulation(const DevParams &P, const WS<KT> &w,
     // fetch_coag (mo_salsa_driver.f90:297-298, 676-697): the kernels stored at the last
     // update step of the low-frequency kernel mode
     const KT *src = static_cast<const KT *>(P.kcache) + (P.kc_base + cell) * (long long)P.kc_stride;
-    for (int e = lane; e < P.kc_stride; e += 32) w.K[e] = src[e];
-    __syncwarp();
+    for (int e = lane; e < P.kc_stride; e += LS) w.K[e] = src[e];
+    wsync<LS>();
   } else {
-    build_kernels<KT>(P, w, tb, T, pres, lane);
+    build_kernels<KT>(P, w, T, pres, lane);
     if (P.kc_mode == 1) {   // store_coag (:421-423, 655-674); the kernels do not change later in the step
       KT *dst = static_cast<KT *>(P.kcache) + (P.kc_base + cell) * (long long)P.kc_stride;
-      for (int e = lane; e < P.kc_stride; e += 32) dst[e] = w.K[e];
+      for (int e = lane; e < P.kc_stride; e += LS) dst[e] = w.K[e];
     }
   }
 #ifdef SALSA_STAGE_TIMERS
-  if (lane == 0 && P.stage_clocks) atomicAdd(P.stage_clocks + 8, (unsigned long long)(clock64() - t_k0));
+  if ((threadIdx.x & 31) == 0 && P.stage_clocks) atomicAdd(P.stage_clocks + 8, (unsigned long long)(clock64() - t_k0));
 #endif
   bool any_aero = P.lscgaa || P.lscgca || P.lscgpa || P.lscgia;
   bool any_cloud = P.lscgcc || P.lscgca || P.lscgpc || P.lscgic;
@@ -1771,13 +2003,13 @@ __device__ __forceinline__ void coagulation(const DevParams &P, const WS<KT> &w,
   if (any_aero) coag_aero<KT>(P, w, tb, dt, lane);
   if (any_cloud) coag_cloud<KT, SIP>(P, w, tb, dt, diag, lane);
   bool neg = false;
-  for (int b = lane; b < P.ntotal; b += 32) {
+  for (int b = lane; b < P.ntotal; b += LS) {
     if (w.numc[b] < -1.e-6) neg = true;
     w.numc[b] = fmax(0., w.numc[b]);
     for (int s = 0; s < P.nused; s++) w.v(s, b) = fmax(0., w.v(s, b));
   }
-  if (warp_any(neg) && lane == 0) w.misc[M_FLAGS + F_NEG] = 1.;
-  __syncwarp();
+  if (wany<LS>(neg) && lane == 0) w.misc[M_FLAGS + F_NEG] = 1.;
+  wsync<LS>();
 }
 
 
@@ -1787,15 +2019,15 @@ __device__ __forceinline__ void coagulation(const DevParams &P, const WS<KT> &w,
 // the bin loop), so its bins are visited in order; regime 2 (init) restarts zke per
 // bin and runs lane-parallel.
 // ----------------------------------------------------------------------------------------
-template <typename KT>
-__device__ __forceinline__ double zvolc_of(const DevParams &P, const WS<KT> &w, int which, int b) {
+template <typename KT, int LS>
+__device__ __forceinline__ double zvolc_of(const DevParams &P, const WS<KT, LS> &w, int which, int b) {
   const int ix[7] = {P.ix_so4, P.ix_oc, P.ix_bc, P.ix_du, P.ix_ss, P.ix_no, P.ix_nh};
   int d = ix[which];
   return (d >= 0 && which < 5) ? w.v(d, b) : 0.;   // only the first five are copied (:148)
 }
 
-template <typename KT>
-__device__ double equil_iterate(const DevParams &P, const WS<KT> &w, int b, double zrh, double T, double &zke,
+template <typename KT, int LS>
+__device__ double equil_iterate(const DevParams &P, const WS<KT, LS> &w, int b, double zrh, double T, double &zke,
                                 double tol, bool regime2, double &zdwet_out, double &zcore_out, int &nonconv) {
   double numc = w.numc[b];
   double zv0 = zvolc_of(P, w, 0, b), zv1 = zvolc_of(P, w, 1, b), zv4 = zvolc_of(P, w, 4, b);
@@ -1840,8 +2072,8 @@ struct EqJob {
   double q0, q1, q4, p56, pc, rinv;   // per-bin invariants of the iteration, computed once
 };
 
-template <typename KT>
-__device__ __forceinline__ void eq_load(const DevParams &P, const WS<KT> &w, int b, EqJob &j) {
+template <typename KT, int LS>
+__device__ __forceinline__ void eq_load(const DevParams &P, const WS<KT, LS> &w, int b, EqJob &j) {
   j.kk = b;
   j.count = 0;
   j.numc = w.numc[b];
@@ -1919,8 +2151,8 @@ struct EqJobF {
   float q0, q1, q4, p56, pc, rinv;
 };
 
-template <typename KT>
-__device__ __forceinline__ void eq_load_f(const DevParams &P, const WS<KT> &w, int b, EqJobF &j) {
+template <typename KT, int LS>
+__device__ __forceinline__ void eq_load_f(const DevParams &P, const WS<KT, LS> &w, int b, EqJobF &j) {
   j.kk = b;
   j.count = 0;
   const float numc = (float)w.numc[b], in = ddiv(1.f, numc);
@@ -1956,8 +2188,8 @@ __device__ __forceinline__ void eq_step_f(EqJobF &j, float ckt) {
 }
 
 // next regime-1a bin after b with numc > nlim; empty bins take dmid when initialising
-template <typename KT>
-__device__ __forceinline__ int eq_next_1a(const DevParams &P, const WS<KT> &w, const double *dmid, int b, bool init) {
+template <typename KT, int LS>
+__device__ __forceinline__ int eq_next_1a(const DevParams &P, const WS<KT, LS> &w, const double *dmid, int b, bool init) {
   for (int k = b + 1; k <= P.fn1a; k++) {
     if (w.numc[k] > K_NLIM) return k;
     if (init) w.dwet[k] = dmid[k];
@@ -1965,14 +2197,74 @@ __device__ __forceinline__ int eq_next_1a(const DevParams &P, const WS<KT> &w, c
   return -1;
 }
 
-template <typename KT>
-__device__ void equilibration(const DevParams &P, const WS<KT> &w, const double *tb, double prh, double T, bool init,
+template <typename KT, int LS>
+__device__ void equilibration(const DevParams &P, const WS<KT, LS> &w, const double *tb, double prh, double T, bool init,
                               int lane) {
   const double *dmid = tb + TAB_DMID * P.nb_pad;
   int nonconv = 0;
   const int n2 = init ? P.fn2b - P.in2a + 1 : 0;
   const double ckt = ddiv(2. * K_SURFW0 * K_MVWA, K_BOLTZ * T);
-  if (n2 <= 31 && sizeof(KT) == 4) {
+  if constexpr (LS == 1) {
+    // the regime-1a bins in order (1/zke carries from bin to bin), then the regime-2 bins
+    const double zrh1 = fmin(fmax(prh, 0.05), 0.98), zrh2 = fmin(fmax(prh, 0.37), 0.98);
+    if constexpr (sizeof(KT) == 4) {
+      const float cktf = (float)ckt;
+      EqJobF j;
+      j.em = (float)(1. - 1. / 1.001);
+      for (int k = eq_next_1a(P, w, dmid, P.in1a - 1, init); k >= 0; k = eq_next_1a(P, w, dmid, k, init)) {
+        j.r2 = false; j.tol = 1.e-2f; j.zrh = (float)zrh1; j.omrh = (float)(1. - zrh1);
+        eq_load_f(P, w, k, j);
+        while (fabsf(j.zdwet - j.zdold) > j.tol * j.zdold) {
+          eq_step_f(j, cktf);
+          if (j.count > 100) { nonconv = 1; break; }
+        }
+        w.v(P.iwa, k) = (double)j.zlwc * (1. / K_RHOWA);
+        if (init) w.dwet[k] = (double)j.zdwet;
+      }
+      for (int k = P.in2a; k < P.in2a + n2; k++) {
+        if (!(w.numc[k] > K_NLIM)) { w.dwet[k] = dmid[k]; continue; }
+        j.r2 = true; j.tol = 1.e-6f; j.zrh = (float)zrh2; j.omrh = (float)(1. - zrh2); j.em = (float)(1. - 1. / 1.02);
+        eq_load_f(P, w, k, j);
+        while (fabsf(j.zdwet - j.zdold) > j.tol * j.zdold) {
+          eq_step_f(j, cktf);
+          if (j.count > 100) { nonconv = 1; break; }
+        }
+        EqJob d;   // two FP64 passes from the float result
+        d.r2 = true; d.tol = 1.e-12; d.zrh = zrh2;
+        eq_load(P, w, k, d);
+        d.zdwet = (double)j.zdwet;
+        d.izke = dexp(-(ddiv(ckt, d.zdwet)));
+        eq_step(d, ckt);
+        eq_step(d, ckt);
+        w.v(P.iwa, k) = divc(d.zlwc, K_RHOWA);
+        w.dwet[k] = d.zdwet;
+      }
+    } else {
+      EqJob j;
+      j.izke = 1. / 1.001;
+      for (int k = eq_next_1a(P, w, dmid, P.in1a - 1, init); k >= 0; k = eq_next_1a(P, w, dmid, k, init)) {
+        j.r2 = false; j.tol = 1.e-2; j.zrh = zrh1;
+        eq_load(P, w, k, j);
+        while (fabs(j.zdwet - j.zdold) > j.tol * j.zdold) {
+          eq_step(j, ckt);
+          if (j.count > 100) { nonconv = 1; break; }
+        }
+        w.v(P.iwa, k) = divc(j.zlwc, K_RHOWA);
+        if (init) w.dwet[k] = j.zdwet;
+      }
+      for (int k = P.in2a; k < P.in2a + n2; k++) {
+        if (!(w.numc[k] > K_NLIM)) { w.dwet[k] = dmid[k]; continue; }
+        j.r2 = true; j.tol = 1.e-12; j.zrh = zrh2; j.izke = 1. / 1.02;
+        eq_load(P, w, k, j);
+        while (fabs(j.zdwet - j.zdold) > j.tol * j.zdold) {
+          eq_step(j, ckt);
+          if (j.count > 100) { nonconv = 1; break; }
+        }
+        w.v(P.iwa, k) = divc(j.zlwc, K_RHOWA);
+        w.dwet[k] = j.zdwet;
+      }
+    }
+  } else if (n2 <= 31 && sizeof(KT) == 4) {
     // the mixed form: lane 31 runs the regime-1a chain, lanes 0..n2-1 the regime-2 bins,
     // all in float; then the regime-2 lanes take two FP64 passes from the float result
     EqJobF j;
@@ -2028,7 +2320,7 @@ __device__ void equilibration(const DevParams &P, const WS<KT> &w, const double 
         w.dwet[r2k] = d.zdwet;
       }
     }
-    __syncwarp();
+    wsync<LS>();
   } else if (n2 <= 31) {
     // lane 31: the regime-1a chain in bin order; lanes 0..n2-1: regime-2 bins
     EqJob j;
@@ -2062,7 +2354,7 @@ __device__ void equilibration(const DevParams &P, const WS<KT> &w, const double 
         }
       }
     }
-    __syncwarp();
+    wsync<LS>();
   } else {
     // regime 1a, in bin order (all lanes run it; lane 0 writes)
     double zke = 1.001;
@@ -2071,7 +2363,7 @@ __device__ void equilibration(const DevParams &P, const WS<KT> &w, const double 
         double zrh = fmin(fmax(prh, 0.05), 0.98);
         double zd, zc;
         double zlwc = equil_iterate<KT>(P, w, kk, zrh, T, zke, 1.e-2, false, zd, zc, nonconv);
-        __syncwarp();
+        wsync<LS>();
         if (lane == 0) {
           w.v(P.iwa, kk) = divc(zlwc, K_RHOWA);
           if (init) w.dwet[kk] = zd;
@@ -2079,9 +2371,9 @@ __device__ void equilibration(const DevParams &P, const WS<KT> &w, const double 
       } else if (init && lane == 0) {
         w.dwet[kk] = dmid[kk];
       }
-      __syncwarp();
+      wsync<LS>();
     }
-    for (int kk = P.in2a + lane; kk <= P.fn2b; kk += 32) {
+    for (int kk = P.in2a + lane; kk <= P.fn2b; kk += LS) {
       if (w.numc[kk] > K_NLIM) {
         double zke = 1.02;
         double zrh = fmin(fmax(prh, 0.37), 0.98);
@@ -2094,8 +2386,8 @@ __device__ void equilibration(const DevParams &P, const WS<KT> &w, const double 
       }
     }
   }
-  if (warp_any(nonconv) && lane == 0) w.misc[M_FLAGS + F_EQUIL] = 1.;
-  __syncwarp();
+  if (wany<LS>(nonconv) && lane == 0) w.misc[M_FLAGS + F_EQUIL] = 1.;
+  wsync<LS>();
 }
 
 // ----------------------------------------------------------------------------------------
@@ -2103,8 +2395,8 @@ __device__ void equilibration(const DevParams &P, const WS<KT> &w, const double 
 // Scratch (per global bin): 0 kelvin 1 cwsurf 2 mt 3 wsat 4 cw (current) 5 zns (solute
 // moles in acth2o) 6 orgic 7 orgri
 // ----------------------------------------------------------------------------------------
-template <typename KT>
-__device__ __forceinline__ double solute_moles(const DevParams &P, const WS<KT> &w, int b, double kappa) {
+template <typename KT, int LS>
+__device__ __forceinline__ double solute_moles(const DevParams &P, const WS<KT, LS> &w, int b, double kappa) {
   double zns = 0.;
   if (P.has_kappa) {
     double vs = 0.;
@@ -2128,20 +2420,20 @@ __device__ __forceinline__ double acth2o_w(double znw, double zns) { return fmax
 // the 3 nm clusters from nucleation, only multiplies that zero.  Collision rates go to
 // scratch row 0, the non-volatile organic increments of the aerosol bins to row 1.
 // ----------------------------------------------------------------------------------------
-template <typename KT>
-__device__ __forceinline__ void condgas(const DevParams &P, const WS<KT> &w, const double *tb, double T, double pres,
-                                        double dt, double *gas, double zxsa, int lane) {
+template <typename KT, int LS>
+__device__ __forceinline__ void condgas(const DevParams &P, const WS<KT, LS> &w, const double *tb, double T, double pres,
+                                        double dt, const Ptr<double, LS> &gas, double zxsa, int lane) {
   double zg[5];
   for (int i = 0; i < 5; i++) zg[i] = gas[i];
   const double *dmid = tb + TAB_DMID * P.nb_pad;
   const int ntot = P.ntotal, in1a = P.in1a, in2a = P.in2a, fn2b = P.fn2b;
   const int C0 = P.nbins, P0 = P.nbins + P.ncld, I0 = P.nliquid;
   const int ioc = P.ix_oc, iso4 = P.ix_so4;
-  double *cr = w.scr, *dvoc = w.scr + w.NB;
+  const auto cr = w.scr, dvoc = w.scr + w.NB;
   const double zvisc = ddiv(7.44523e-3 * dsqrt(cube(T)), 5093. * (T + 110.4));
   const double zdfvap = ddiv(5.1111e-10 * dpow(T, 1.75) * K_PSTAND, pres);
   const double zmfp = 3. * zdfvap * dsqrt(ddiv(K_PI * K_MSU, 8. * K_RG * T));
-  for (int b = lane; b < ntot; b += 32) {
+  for (int b = lane; b < ntot; b += LS) {
     // updateDiameter(limit=.TRUE., type="wet") (:446-448)
     const int ph = phase_of(P, b);
     const double n = w.numc[b];
@@ -2174,7 +2466,7 @@ __device__ __forceinline__ void condgas(const DevParams &P, const WS<KT> &w, con
     }
     cr[b] = r;
   }
-  __syncwarp();
+  wsync<LS>();
   // condensation sinks, summed in bin order as Fortran's SUM (:545, :603-606)
   double sa = 0., sca = 0., spa = 0., sia = 0., sa2 = 0.;
   for (int k = in1a; k <= fn2b; k++) sa += cr[k];
@@ -2190,7 +2482,7 @@ __device__ __forceinline__ void condgas(const DevParams &P, const WS<KT> &w, con
     const double cnew = ddiv(zg[3], 1. + dt * zcs);
     const double dv = zg[3] - cnew;
     zg[3] = cnew;
-    for (int b = lane; b < ntot; b += 32) {
+    for (int b = lane; b < ntot; b += LS) {
       const double inc = ddiv(cr[b], zcs) * K_MVOC * dv;
       if (b <= fn2b) dvoc[b] = inc;
       w.v(ioc, b) = w.v(ioc, b) + inc;
@@ -2203,7 +2495,7 @@ __device__ __forceinline__ void condgas(const DevParams &P, const WS<KT> &w, con
     const double cnew = ddiv(zg[4], 1. + dt * zcs_ocsv);
     const double dv = zg[4] - cnew;
     zg[4] = cnew;
-    for (int b = lane; b < ntot; b += 32) {
+    for (int b = lane; b < ntot; b += LS) {
       if (b <= fn2b) {
         double d = dvoc[b];
         if (b >= in2a) d = d + ddiv(cr[b], zcs_ocsv) * K_MVOC * dv;
@@ -2219,28 +2511,81 @@ __device__ __forceinline__ void condgas(const DevParams &P, const WS<KT> &w, con
     const double cnew = ddiv(zg[0], 1. + dt * zcs);
     const double dv = zg[0] - cnew;
     zg[0] = cnew;
-    for (int b = lane; b < ntot; b += 32) {
+    for (int b = lane; b < ntot; b += LS) {
       const double inc = ddiv(cr[b], zcs) * K_MVSU * dv;
       w.v(iso4, b) = w.v(iso4, b) + inc;
       if (b == in1a && zxsa > 0.) w.numc[b] = w.numc[b] + ddiv(divc(zn_vs_c * inc, K_MVSU), K_N3 * zxsa);
     }
   }
-  __syncwarp();
-  if (lane < 5) gas[lane] = zg[lane];
-  __syncwarp();
+  wsync<LS>();
+  for (int i = 0; i < 5; i++)
+    if (LS == 1 || lane == i) gas[i] = zg[i];
+  wsync<LS>();
 }
 
-template <typename KT>
-__device__ void gpparth2o(const DevParams &P, const WS<KT> &w, const double *tb, double T, double pres, double prs,
+// Two sums over the bins 0..n-1 in the order of the warp form's lane partial sums and
+// butterfly (bins l, l + 32, .. of leaf l; leaves paired over 16, 8, 4, 2, 1 apart).  The
+// explicit substeps take the vapour as a difference of such sums and magnify their rounding
+// in the Aitken bins' water by orders of magnitude, so both forms round alike.  f(b, first,
+// x, y) sets (first) or adds to the leaf's two partial sums.
+template <typename F>
+__device__ __forceinline__ void tree_sum2(int n, F f, double &X, double &Y) {
+  double x0 = 0., y0 = 0., x1 = 0., y1 = 0., x2 = 0., y2 = 0.;
+#pragma unroll 1
+  for (int o = 0; o < 8; o++) {   // bits 0, 1, 2 of the leaf from the outside in
+    const int l3 = (o >> 2) | (o & 2) | ((o & 1) << 2);
+    double x3 = 0., y3 = 0.;
+#pragma unroll
+    for (int i3 = 0; i3 < 2; i3++) {
+      double x4 = 0., y4 = 0.;
+#pragma unroll
+      for (int i4 = 0; i4 < 2; i4++) {
+        double x = 0., y = 0.;
+        bool first = true;
+        for (int b = l3 + 8 * i3 + 16 * i4; b < n; b += 32) {
+          f(b, first, x, y);
+          first = false;
+        }
+        x4 = i4 ? x4 + x : x;
+        y4 = i4 ? y4 + y : y;
+      }
+      x3 = i3 ? x3 + x4 : x4;
+      y3 = i3 ? y3 + y4 : y4;
+    }
+    if (o & 1) { x2 += x3; y2 += y3; } else { x2 = x3; y2 = y3; }
+    if (o & 1) {
+      if (o & 2) { x1 += x2; y1 += y2; } else { x1 = x2; y1 = y2; }
+      if (o & 2) {
+        if (o & 4) { x0 += x1; y0 += y1; } else { x0 = x1; y0 = y1; }
+      }
+    }
+  }
+  X = x0;
+  Y = y0;
+}
+// one sum in that order; f(b) is bin b's term
+template <int LS, typename F>
+__device__ __forceinline__ double bins_sum(int n, int lane, F f) {
+  double X, Y;
+  if constexpr (LS == 1) {
+    tree_sum2(n, [&](int b, bool first, double &x, double &) { x = first ? f(b) : x + f(b); }, X, Y);
+  } else {
+    X = 0.;
+    for (int b = lane; b < n; b += LS) X += f(b);
+    X = warp_sum(X);
+  }
+  return X;
+}
+
+template <typename KT, int LS>
+__device__ void gpparth2o(const DevParams &P, const WS<KT, LS> &w, const double *tb, double T, double pres, double prs,
                           double prsi, double &prv, double dt, double kappa, bool diag, int lane) {
   const int nbins = P.nbins, ncld = P.ncld, nprc = P.nprc, nice = P.nice, ntot = P.ntotal;
   const int iwa = P.iwa, irim = P.irim, C0 = nbins, P0 = nbins + ncld, I0 = P.nliquid;
   const double *dmid = tb + TAB_DMID * P.nb_pad;
   const double zrh = ddiv(prv, prs);
   // aerosol water before/after the equilibrium update
-  double l1 = 0.;
-  for (int b = lane; b <= P.fn2b; b += 32) l1 += w.v(iwa, b);
-  double zaelwc1 = warp_sum(l1) * K_RHOWA;
+  double zaelwc1 = bins_sum<LS>(P.fn2b + 1, lane, [&](int b) { return w.v(iwa, b); }) * K_RHOWA;
   // The init-form call repeats the 1a update with identical inputs (dwet untouched by
   // the first call, zke restarted at 1.001), so running it alone gives the same state.
 #ifdef SALSA_STAGE_TIMERS
@@ -2249,15 +2594,13 @@ __device__ void gpparth2o(const DevParams &P, const WS<KT> &w, const double *tb,
   if (zrh < 0.98 || !P.lscndh2oae) equilibration<KT>(P, w, tb, zrh, T, true, lane);
   else equilibration<KT>(P, w, tb, zrh, T, false, lane);
 #ifdef SALSA_STAGE_TIMERS
-  if (lane == 0 && P.stage_clocks) atomicAdd(P.stage_clocks + 10, (unsigned long long)(clock64() - t_eq0));
+  if ((threadIdx.x & 31) == 0 && P.stage_clocks) atomicAdd(P.stage_clocks + 10, (unsigned long long)(clock64() - t_eq0));
 #endif
-  double l2 = 0.;
-  for (int b = lane; b <= P.fn2b; b += 32) l2 += w.v(iwa, b);
-  double zaelwc2 = warp_sum(l2) * K_RHOWA;
+  double zaelwc2 = bins_sum<LS>(P.fn2b + 1, lane, [&](int b) { return w.v(iwa, b); }) * K_RHOWA;
   prv = prv - ddiv(zaelwc2 - zaelwc1, ddiv(pres * K_MAIR, K_RG * T));
 
   bool anycl = false, anypr = false, anyic = false, anyae = false;
-  for (int b = lane; b < ntot; b += 32) {
+  for (int b = lane; b < ntot; b += LS) {
     int ph = phase_of(P, b);
     double n = w.numc[b];
     if (ph == 1) anyae |= n > K_NLIM;
@@ -2265,7 +2608,7 @@ __device__ void gpparth2o(const DevParams &P, const WS<KT> &w, const double *tb,
     else if (ph == 3) anypr |= n > K_PRLIM;
     else anyic |= n > K_PRLIM;
   }
-  anyae = warp_any(anyae); anycl = warp_any(anycl); anypr = warp_any(anypr); anyic = warp_any(anyic);
+  anyae = wany<LS>(anyae); anycl = wany<LS>(anycl); anypr = wany<LS>(anypr); anyic = wany<LS>(anyic);
   if (!((anycl || (anypr && P.lscndh2ocl)) || (anyic && P.lscndh2oic) || (anyae && zrh > 0.98 && P.lscndh2oae)))
     return;
 
@@ -2276,12 +2619,12 @@ __device__ void gpparth2o(const DevParams &P, const WS<KT> &w, const double *tb,
   const double zmfph2o = 3. * zdfh2o * dsqrt(ddiv(K_PI * K_MWA, 8. * K_RG * T));
   const double zthcond = 0.023807 + 7.1128e-5 * (T - 273.16);
   const int NB = w.NB;
-  double *kel = w.sc(0), *surf = w.sc(1), *mt = w.sc(2), *wsat = w.sc(3), *cw = w.sc(4), *zns = w.sc(5),
-         *orgic = w.sc(6), *orgri = w.sc(7);
+  const auto kel = w.sc(0), surf = w.sc(1), mt = w.sc(2), wsat = w.sc(3), cw = w.sc(4), zns = w.sc(5),
+             orgic = w.sc(6), orgri = w.sc(7);
   (void)NB;
   // diameters and densities (:819-822), then per-bin coefficients (:826-955)
-  for (int b = lane; b < ntot; b += 32) {
-    updateDiameterAll(P, nullptr, w.numc, w.volc, w.dwet, w.ddry, w.dins, w.dnsp, dmid, w.NB, b);
+  for (int b = lane; b < ntot; b += LS) {
+    updateDiameterAll(P, w, dmid, b);
     int ph = phase_of(P, b);
     w.rhomean[b] = rhomean_of(P, ph, w.numc[b], w.v(iwa, b), w.v(irim, b));
     double n = w.numc[b];
@@ -2331,26 +2674,22 @@ __device__ void gpparth2o(const DevParams &P, const WS<KT> &w, const double *tb,
       orgri[b] = divc(w.v(irim, b) * K_RHORI, K_MWA);
     }
   }
-  __syncwarp();
+  wsync<LS>();
   // categories updated inside the substep loop (:1002-1031)
   bool upd_ae = false, upd_cl = false, upd_pr = false, upd_ic = false;
   {
     bool a = false, c = false, p = false, i = false;
-    for (int b = lane; b < ntot; b += 32) {
+    for (int b = lane; b < ntot; b += LS) {
       int ph = phase_of(P, b);
       double n = w.numc[b];
       if (ph == 1) a |= n > K_NLIM; else if (ph == 2) c |= n > K_NLIM; else if (ph == 3) p |= n > K_PRLIM; else i |= n > K_PRLIM;
     }
-    upd_ae = warp_any(a) && zrh > 0.98; upd_cl = warp_any(c); upd_pr = warp_any(p); upd_ic = warp_any(i);
+    upd_ae = wany<LS>(a) && zrh > 0.98; upd_cl = wany<LS>(c); upd_pr = wany<LS>(p); upd_ic = wany<LS>(i);
   }
   double zcwc = divc(prv * rhoair, K_MWA);
-  double tsum = 0., msum = 0.;
-  for (int b = lane; b < ntot; b += 32) {
-    tsum += cw[b];
-    if (b >= P.in2a) msum += mt[b];   // the substep sums skip regime 1a (nstr = in2a)
-  }
-  const double zcwtot = zcwc + warp_sum(tsum);
-  const double mtot = warp_sum(msum);
+  const double zcwtot = zcwc + bins_sum<LS>(ntot, lane, [&](int b) { return cw[b]; });
+  // the substep sums skip regime 1a (nstr = in2a)
+  const double mtot = bins_sum<LS>(ntot, lane, [&](int b) { return b >= P.in2a ? mt[b] : 0.; });
   double ttot = 0., zcwint = 0.;
   int counter = 0;
 #ifdef SALSA_STAGE_TIMERS
@@ -2362,9 +2701,15 @@ __device__ void gpparth2o(const DevParams &P, const WS<KT> &w, const double *tb,
   // so the totals are those of two separate butterflies over those partial sums.
   const double adt = 2.e-2;
   double spsum;
-  {
+  if constexpr (LS == 1) {
+    double unused;
+    tree_sum2(ntot, [&](int b, bool first, double &x, double &) {
+      const double p = b >= P.in2a ? mt[b] * wsat[b] : 0.;
+      x = first ? p * surf[b] : fma(p, surf[b], x);
+    }, spsum, unused);
+  } else {
     double sp = 0.;
-    for (int b = lane; b < ntot; b += 32)
+    for (int b = lane; b < ntot; b += LS)
       if (b >= P.in2a) sp += mt[b] * wsat[b] * surf[b];
     spsum = warp_sum(sp);
   }
@@ -2372,8 +2717,7 @@ __device__ void gpparth2o(const DevParams &P, const WS<KT> &w, const double *tb,
     double zhlp1 = zcwc + adt * spsum;
     double zhlp2 = 1. + adt * mtot;
     zcwint = fmin(ddiv(zhlp1, zhlp2), zcwtot);
-    double cs = 0., sp = 0.;
-    for (int b = lane; b < ntot; b += 32) {
+    auto substep_bin = [&](int b) {   // bin b through the substep; its water
       int ph = phase_of(P, b);
       double c = cw[b];
       bool upd = (ph == 1) ? (upd_ae && b >= P.in2a) : (ph == 2 ? upd_cl : (ph == 3 ? upd_pr : upd_ic));
@@ -2383,10 +2727,24 @@ __device__ void gpparth2o(const DevParams &P, const WS<KT> &w, const double *tb,
         c = fmax(ci, 0.);
       }
       cw[b] = c;
-      cs += c;
-      if (b >= P.in2a) sp += mt[b] * wsat[b] * surf[b];
-    }
-    {
+      return c;
+    };
+    if constexpr (LS == 1) {
+      double cs, sp;
+      tree_sum2(ntot, [&](int b, bool first, double &x, double &y) {
+        const double c = substep_bin(b);
+        x = first ? c : x + c;
+        const double p = b >= P.in2a ? mt[b] * wsat[b] : 0.;
+        y = first ? p * surf[b] : fma(p, surf[b], y);
+      }, cs, sp);
+      zcwint = zcwtot - cs;
+      spsum = sp;
+    } else {
+      double cs = 0., sp = 0.;
+      for (int b = lane; b < ntot; b += LS) {
+        cs += substep_bin(b);
+        if (b >= P.in2a) sp += mt[b] * wsat[b] * surf[b];
+      }
       // lanes 0-15 reduce cs, lanes 16-31 reduce sp
       const bool hi = lane & 16;
       double v = (hi ? sp : cs) + __shfl_xor_sync(0xffffffffu, hi ? cs : sp, 16);
@@ -2404,7 +2762,7 @@ __device__ void gpparth2o(const DevParams &P, const WS<KT> &w, const double *tb,
   }
   if (counter > 100 && lane == 0) w.misc[M_FLAGS + F_COND] = 1.;
 #ifdef SALSA_STAGE_TIMERS
-  if (lane == 0 && P.stage_clocks) atomicAdd(P.stage_clocks + 9, (unsigned long long)(clock64() - t_sub0));
+  if ((threadIdx.x & 31) == 0 && P.stage_clocks) atomicAdd(P.stage_clocks + 9, (unsigned long long)(clock64() - t_sub0));
 #endif
   prv = ddiv(zcwint * K_MWA, rhoair);
   // Cond_i diagnostic (:1086-1112): vrate(irim) is only assigned on sublimation and keeps
@@ -2424,10 +2782,10 @@ __device__ void gpparth2o(const DevParams &P, const WS<KT> &w, const double *tb,
       }
     }
   }
-  __syncwarp();
+  wsync<LS>();
   // write back and diagnostics (:1061-1117)
   double dca = 0., dcc = 0., dcp = 0.;
-  for (int b = lane; b < ntot; b += 32) {
+  for (int b = lane; b < ntot; b += LS) {
     int ph = phase_of(P, b);
     if (ph <= 3) {
       double nv = fmax(0., divc(cw[b] * K_MWA, K_RHOWA));
@@ -2449,7 +2807,7 @@ __device__ void gpparth2o(const DevParams &P, const WS<KT> &w, const double *tb,
     if (w.numc[b] > nlim_of(ph)) w.rhomean[b] = rhomean_of(P, ph, w.numc[b], w.v(iwa, b), w.v(irim, b));
   }
   if (diag) {
-    dca = warp_sum(dca); dcc = warp_sum(dcc); dcp = warp_sum(dcp);
+    dca = wsum<LS>(dca); dcc = wsum<LS>(dcc); dcp = wsum<LS>(dcp);
     if (lane == 0) {
       w.misc[M_DIAG + DG_CONDA] += dca;
       w.misc[M_DIAG + DG_CONDC] += dcc;
@@ -2457,7 +2815,7 @@ __device__ void gpparth2o(const DevParams &P, const WS<KT> &w, const double *tb,
       w.misc[M_DIAG + DG_CONDI] += dci;
     }
   }
-  __syncwarp();
+  wsync<LS>();
 }
 
 // ----------------------------------------------------------------------------------------
@@ -2480,17 +2838,17 @@ __device__ __forceinline__ double intgV(double k, double c, double lo, double hi
 // activated-droplet outputs (raw rows, per kg of air).  One lane per aerosol bin, then
 // one lane per cloud bin; sums run in bin order on every lane.
 // ----------------------------------------------------------------------------------------
-template <typename KT>
-__device__ __forceinline__ void act_cloudbase(const DevParams &P, const WS<KT> &w, const double *tb, double pres,
-                                              double T, double wvel, double dn, double *raw, int lane) {
+template <typename KT, int LS>
+__device__ __forceinline__ void act_cloudbase(const DevParams &P, const WS<KT, LS> &w, const double *tb, double pres,
+                                              double T, double wvel, double dn, const Ptr<double, LS> &raw, int lane) {
   const int in1a = P.in1a, fn2a = P.fn2a, in2b = P.in2b, fn2b = P.fn2b, ndry = P.ndry, nwet = P.nwet;
   const int iwa = P.iwa, ncld = P.ncld;
   const double *dmid = tb + TAB_DMID * P.nb_pad, *vlo = tb + TAB_VLO * P.nb_pad, *vhi = tb + TAB_VHI * P.nb_pad;
   const double *vrlo = tb + TAB_VRLO * P.nb_pad, *vrhi = tb + TAB_VRHI * P.nb_pad;
-  double *ns = w.sc(0), *zdcrit = w.sc(1), *zdcrlo = w.sc(2), *zdcrhi = w.sc(3), *frac = w.sc(4), *term = w.sc(5);
+  const auto ns = w.sc(0), zdcrit = w.sc(1), zdcrlo = w.sc(2), zdcrhi = w.sc(3), frac = w.sc(4), term = w.sc(5);
   const double bb = 6. * K_MWA / (K_PI * K_RHOWA);   // Raoult term per mole of solute [m3]
   // getSolute (:116-157): moles of dissolved solute per particle
-  for (int k = lane; k <= fn2b; k += 32) {
+  for (int k = lane; k <= fn2b; k += LS) {
     double n_ = 0.;
     if (w.numc[k] > K_NLIM) {
       for (int nn = 0; nn < ndry; nn++) n_ = n_ + ddiv(P.diss[nn] * w.v(nn, k) * P.rholiq[nn], P.MM[nn]);
@@ -2499,17 +2857,17 @@ __device__ __forceinline__ void act_cloudbase(const DevParams &P, const WS<KT> &
     ns[k] = n_;
     frac[k] = zdcrit[k] = zdcrlo[k] = zdcrhi[k] = 0.;
   }
-  __syncwarp();
+  wsync<LS>();
   int bcrita = fn2a;
   double zdcstar = 0.;
   if (wvel > 0.) {
     const double aa = ddiv(4. * K_MWA * K_SURFW0, K_RG * K_RHOWA * T);   // Kelvin term [m]
     const double x = divc(4. * cube(aa), 27. * bb);
-    for (int k = in1a + lane; k <= fn2b; k += 32) {
+    for (int k = in1a + lane; k <= fn2b; k += LS) {
       const double scrit = dexp(dsqrt(ddiv(x, fmax(K_EPS, ns[k])))) - 1.;
       term[k] = ddiv(w.numc[k], dpow(scrit, 2. / 3.));
     }
-    __syncwarp();
+    wsync<LS>();
     double ntot = 0., sum1 = 0.;   // part 3, eq. (8)
     for (int k = in1a; k <= fn2b; k++) ntot += w.numc[k];
     for (int k = in1a; k <= fn2b; k++) sum1 += term[k];
@@ -2530,7 +2888,7 @@ __device__ __forceinline__ void act_cloudbase(const DevParams &P, const WS<KT> &
       const double khi = (2. / 3.) * aa * dsqrt(ddiv(alpha * V, Gc));
       const double s_max = ddiv(s_eff, dsqrt(0.5 * dsqrt(cube(ddiv(khi, theta))) + dpow(ddiv(sq(s_eff), theta + 3. * khi), 0.75)));
       zdcstar = ddiv(2. * aa, 3. * s_max);
-      for (int kk = in1a + lane; kk <= fn2b; kk += 32) {
+      for (int kk = in1a + lane; kk <= fn2b; kk += LS) {
         if (w.numc[kk] < K_NLIM) continue;
         const double nshi = ns[kk] * vrhi[kk];
         const double sil = dexp(dsqrt(ddiv(x, nshi))) - 1.;
@@ -2542,15 +2900,15 @@ __device__ __forceinline__ void act_cloudbase(const DevParams &P, const WS<KT> &
         zdcrhi[kk] = 2. * dsqrt(ddiv(3. * nshi * bb, aa));
         zdcrit[kk] = 2. * dsqrt(ddiv(3. * ns[kk] * bb, aa));
       }
-      __syncwarp();
+      wsync<LS>();
       for (int kk = in1a; kk <= fn2a; kk++)   // the critical bin of regime a
         if (frac[kk] < 1. && frac[kk] > 0.) { bcrita = kk; break; }
     }
   }
   // activate3: nothing activates when no bin has a critical diameter
   bool big = false;
-  for (int k = lane; k <= fn2b; k += 32) big |= !(zdcrit[k] < K_EPS);
-  if (!warp_any(big)) return;
+  for (int k = lane; k <= fn2b; k += LS) big |= !(zdcrit[k] < K_EPS);
+  if (!wany<LS>(big)) return;
   double Vmid, Vlo, Vhi;
   if (w.numc[bcrita] < K_NLIM) {
     Vmid = K_PI6 * cube(dmid[bcrita]);
@@ -2572,7 +2930,7 @@ __device__ __forceinline__ void act_cloudbase(const DevParams &P, const WS<KT> &
   }
   zvcstar = fmax(zvcstar, vlo[bcrita]);
   zvcstar = fmin(zvcstar, vhi[bcrita]);
-  for (int cb = lane; cb < ncld; cb += 32) {
+  for (int cb = lane; cb < ncld; cb += LS) {
     const int ab = (cb <= P.fca_cur) ? P.ica_par + (cb - P.ica_cur) : P.icb_par + (cb - P.icb_cur);
     if (w.numc[ab] < K_NLIM) continue;
     const double Nmid = fmax(w.numc[ab], K_NLIM);
@@ -2638,8 +2996,8 @@ __device__ __forceinline__ void act_cloudbase(const DevParams &P, const WS<KT> &
   }
 }
 
-template <typename KT>
-__device__ void act_interst(const DevParams &P, const WS<KT> &w, const double *tb, double prv, double prs, double T,
+template <typename KT, int LS>
+__device__ void act_interst(const DevParams &P, const WS<KT, LS> &w, const double *tb, double prv, double prs, double T,
                             bool diag, int lane) {
   if (ddiv(prv, prs) <= 1.000) return;
   const int ndry = P.ndry, nwet = P.nwet, iwa = P.iwa, C0 = P.nbins;
@@ -2648,10 +3006,10 @@ __device__ void act_interst(const DevParams &P, const WS<KT> &w, const double *t
   double zkelvin = ddiv(4. * K_MWA * K_SURFW0, K_RG * K_RHOWA * T);
   double zdcstar = ddiv(2. * zkelvin, 3. * ((ddiv(prv, prs)) - 1.));
   double zvcstar = K_PI6 * cube(zdcstar);
-  double *actn = w.sc(8);        // per cloud bin
-  double *actv = w.sc(0);        // [s * NB + cb] (reuses condensation scratch 0..nwet-1)
+  const auto actn = w.sc(8);        // per cloud bin
+  const auto actv = w.sc(0);        // [s * NB + cb] (reuses condensation scratch 0..nwet-1)
   double nsum = 0.;
-  for (int cb = lane; cb < P.ncld; cb += 32) {
+  for (int cb = lane; cb < P.ncld; cb += LS) {
     int ab = (cb <= P.fca_cur) ? P.ica_par + (cb - P.ica_cur) : P.icb_par + (cb - P.icb_cur);
     double an = 0.;
     double av[SALSA_NSV];
@@ -2733,12 +3091,12 @@ __device__ void act_interst(const DevParams &P, const WS<KT> &w, const double *t
     for (int s = 0; s < nwet; s++) actv[s * w.NB + cb] = av[s];
     nsum += an;
   }
-  __syncwarp();
+  wsync<LS>();
   if (diag) {
-    nsum = warp_sum(nsum);
+    nsum = wsum<LS>(nsum);
     if (lane == 0) w.misc[M_DIAG + DG_ACTIV] += nsum;
   }
-  for (int cb = lane; cb < P.ncld; cb += 32) {
+  for (int cb = lane; cb < P.ncld; cb += LS) {
     int ab = P.ica_par + cb, cg = C0 + cb;
     double an = actn[cb];
     if (an > 0.) w.ctime[cg] = ddiv(an * P.chargeTimeMax + w.numc[cg] * w.ctime[cg], an + w.numc[cg]);
@@ -2752,12 +3110,12 @@ __device__ void act_interst(const DevParams &P, const WS<KT> &w, const double *t
     }
     if (nc > 0.) w.indef[cg] = ddiv(w.indef[cg] * (nc - an) + w.indef[ab] * an, nc);
   }
-  __syncwarp();
+  wsync<LS>();
 }
 
 // mo_salsa_cloud.f90:1401-1477 autoconv2 (cloud bins from the largest; all move to precip bin 1)
-template <typename KT>
-__device__ void autoconv2(const DevParams &P, const WS<KT> &w, double dt, int lane) {
+template <typename KT, int LS>
+__device__ void autoconv2(const DevParams &P, const WS<KT, LS> &w, double dt, int lane) {
   if (lane == 0) {
     const double zd0 = 50.e-6, sigmag = 1.2, max_rate_autoc = 1.0e10;
     const int C0 = P.nbins, P0 = P.nbins + P.ncld;
@@ -2788,7 +3146,7 @@ __device__ void autoconv2(const DevParams &P, const WS<KT> &w, double dt, int la
       }
     }
   }
-  __syncwarp();
+  wsync<LS>();
 }
 
 
@@ -2897,8 +3255,8 @@ __device__ double J_hf(double Tk, double Sw) {   // :335-371
 }
 
 // calcSweq (mo_particle_external_properties.f90:402-447)
-template <typename KT>
-__device__ double calc_sweq(const DevParams &P, const WS<KT> &w, int b, double T, double kappa) {
+template <typename KT, int LS>
+__device__ double calc_sweq(const DevParams &P, const WS<KT, LS> &w, int b, double T, double kappa) {
   double n = w.numc[b];
   if (n < nlim_of(phase_of(P, b))) return 0.;
   double vs = 0.;
@@ -2932,22 +3290,39 @@ __device__ __forceinline__ int precip_bin_of(const DevParams &P, const double *v
 }
 
 // staged ice contribution of one liquid bin: [0] target ice bin (-1 none), [1..nused] volumes, [8] number
-template <typename KT>
-__device__ void ice_apply_staged(const DevParams &P, const WS<KT> &w, const double *stage, int nsrc, int lane) {
+template <typename KT, int LS>
+__device__ void ice_apply_staged(const DevParams &P, const WS<KT, LS> &w, const Ptr<double, LS> &stage, int nsrc, int lane) {
+  if constexpr (LS == 1) {
+    // sources in order; each goes to one ice bin
+    for (int k = 0; k < nsrc; k++) {
+      const auto st = stage + k * 10;
+      const int ib = (int)st[0];
+      if (ib < 0) continue;
+      const int g = P.nliquid + ib;
+      const bool all = st[9] != 0.;
+      for (int q = 0; q <= P.nused; q++) {
+        const double add = (q < P.nused) ? st[1 + q] : st[8];
+        if (add == 0. && !all) continue;
+        if (q < P.nused) w.v(q, g) = fmax(0., w.v(q, g) + add);
+        else w.numc[g] = fmax(0., w.numc[g] + add);
+      }
+    }
+    return;
+  }
   // one lane per ice bin and component, sources in order
   const int ncomp = P.nused + 1;
-  for (int e = lane; e < P.nice * ncomp; e += 32) {
+  for (int e = lane; e < P.nice * ncomp; e += LS) {
     int ib = e / ncomp, q = e % ncomp, g = P.nliquid + ib;
     double val = (q < P.nused) ? w.v(q, g) : w.numc[g];
     for (int k = 0; k < nsrc; k++) {
-      const double *st = stage + k * 10;
+      const auto st = stage + k * 10;
       if ((int)st[0] != ib) continue;
       double add = (q < P.nused) ? st[1 + q] : st[8];
       if (add != 0. || st[9] != 0.) val = fmax(0., val + add);
     }
     if (q < P.nused) w.v(q, g) = val; else w.numc[g] = val;
   }
-  __syncwarp();
+  wsync<LS>();
 }
 
 // SE ice nucleation (mo_salsa_SecondaryIce / iceNucleation, :394-538).  Pass A (lanes
@@ -2955,26 +3330,26 @@ __device__ void ice_apply_staged(const DevParams &P, const WS<KT> &w, const doub
 // Gauss-Legendre integral over contact angles; pass B evaluates the integrands with one
 // lane per (bin, node), three bins per warp pass, and sums each bin's ten terms in node
 // order; pass C (lanes over bins) applies the frozen fractions.
-template <typename KT>
-__device__ void ice_nucl_SE(const DevParams &P, const WS<KT> &w, const double *tb, double T, double prv, double prs,
+template <typename KT, int LS>
+__device__ void ice_nucl_SE(const DevParams &P, const WS<KT, LS> &w, const double *tb, double T, double prv, double prs,
                             double prsi, double dt, double kappa, bool diag, int lane) {
   if (P.ninsoluble <= 0) return;
   const double *dmid = tb + TAB_DMID * P.nb_pad, *vlo = tb + TAB_VLO * P.nb_pad;
   const double dmin = 1.e-10, tmax_homog = 237.9, minVin = K_PI6 * cube(1.e-8);
   const int nl = P.nliquid, ndry = P.ndry, iwa = P.iwa, irim = P.irim, idu = P.ix_du;
   const unsigned F = 0xffffffffu;
-  double *stage = w.scr;   // nl * 10 doubles
+  const auto stage = w.scr;   // nl * 10 doubles
   // per-bin records in the (now unused) collision-kernel area: 8 doubles per bin
-  double *rec = reinterpret_cast<double *>(w.K);
+  const auto rec = row_cast<double>(w.K);
   enum { R_MODE = 0, R_THMIN, R_DIN, R_AE, R_SIG, R_DG, R_FHOM, R_FINT };
   const double Si = ddiv(prv, prsi);
   // pass A
-  for (int kk = lane; kk < nl; kk += 32) {
-    double *st = stage + kk * 10;
+  for (int kk = lane; kk < nl; kk += LS) {
+    const auto st = stage + kk * 10;
     for (int q = 0; q < 10; q++) st[q] = 0.;
     st[0] = -1.;
-    double *r = rec + kk * 8;
-    updateDiameterAll(P, nullptr, w.numc, w.volc, w.dwet, w.ddry, w.dins, w.dnsp, dmid, w.NB, kk);
+    const auto r = rec + kk * 8;
+    updateDiameterAll(P, w, dmid, kk);
     const double dwet = w.dwet[kk], dins_ = w.ddry[kk];
     const double n = w.numc[kk];
     const int ph = phase_of(P, kk);
@@ -3008,61 +3383,71 @@ __device__ void ice_nucl_SE(const DevParams &P, const WS<KT> &w, const double *t
     }
     r[R_FINT] = 0.;
   }
-  __syncwarp();
+  wsync<LS>();
   // pass B: gauss_legendre (:131-206) for the bins that need it
-  {
+  const GaussC g_imm = gauss_c(P.sigma_theta_imm, P.mean_theta_imm);
+  const GaussC g_dep = gauss_c(P.sigma_theta_dep, P.mean_theta_dep);
+  const double kth = divc(K_BOLTZ * T, K_PLANCK);
+  auto node_term = [&](const Ptr<double, LS> &r, int node) {
+    const double thmin = r[R_THMIN], thmax = 180.;
+    const double th1 = mrn(0.5 * (thmax - thmin), c_gl_x[node]) + 0.5 * (thmax + thmin);
+    double J, ft;
+    if (r[R_MODE] == 1.) {
+      JimmPre q;
+      q.act_energy = r[R_AE]; q.sigma_is = r[R_SIG]; q.d_g = r[R_DG]; q.ok = r[R_DG] >= 0.;
+      J = J_imm(q, th1, T, r[R_DIN], kth);
+      ft = th1 > thmin ? f_gauss(th1, g_imm) : 0.;
+    } else {
+      J = J_dep(th1, T, r[R_DIN], Si);
+      ft = th1 > thmin ? f_gauss(th1, g_dep) : 0.;
+    }
+    return ft * c_gl_w[node] * (1. - dexp(-J * dt));
+  };
+  if constexpr (LS == 1) {
+    for (int kk = 0; kk < nl; kk++) {
+      const auto r = rec + kk * 8;
+      if (r[R_MODE] == 0.) continue;
+      double acc = 0.;
+      for (int node = 0; node < 10; node++) acc = acc + node_term(r, node);
+      r[R_FINT] = 0.5 * (180. - r[R_THMIN]) * acc;
+    }
+  } else {
     const unsigned lt = (1u << lane) - 1u;
     int nlist = 0;
     int *list = w.pbuf;
-    for (int base = 0; base < nl; base += 32) {
+    for (int base = 0; base < nl; base += LS) {
       int kk = base + lane;
       bool need = kk < nl && rec[kk * 8 + R_MODE] != 0.;
       unsigned bal = __ballot_sync(F, need);
       if (need) list[nlist + __popc(bal & lt)] = kk;
       nlist += __popc(bal);
     }
-    __syncwarp();
+    wsync<LS>();
     const int grp = lane / 10, node = lane - grp * 10;
-    const GaussC g_imm = gauss_c(P.sigma_theta_imm, P.mean_theta_imm);
-    const GaussC g_dep = gauss_c(P.sigma_theta_dep, P.mean_theta_dep);
-    const double kth = divc(K_BOLTZ * T, K_PLANCK);
     for (int b0 = 0; b0 < nlist; b0 += 3) {
       const int slot = b0 + grp;
       const bool on = grp < 3 && slot < nlist;
       const int kk = on ? list[slot] : 0;
       double term = 0.;
       if (on) {
-        const double *r = rec + kk * 8;
-        const double thmin = r[R_THMIN], thmax = 180.;
-        const double th1 = mrn(0.5 * (thmax - thmin), c_gl_x[node]) + 0.5 * (thmax + thmin);
-        double J, ft;
-        if (r[R_MODE] == 1.) {
-          JimmPre q;
-          q.act_energy = r[R_AE]; q.sigma_is = r[R_SIG]; q.d_g = r[R_DG]; q.ok = r[R_DG] >= 0.;
-          J = J_imm(q, th1, T, r[R_DIN], kth);
-          ft = th1 > thmin ? f_gauss(th1, g_imm) : 0.;
-        } else {
-          J = J_dep(th1, T, r[R_DIN], Si);
-          ft = th1 > thmin ? f_gauss(th1, g_dep) : 0.;
-        }
-        term = ft * c_gl_w[node] * (1. - dexp(-J * dt));
+        term = node_term(rec + kk * 8, node);
       }
       double acc = 0.;
       const int g10 = (grp < 3 ? grp : 0) * 10;
 #pragma unroll
       for (int i = 0; i < 10; i++) acc = acc + __shfl_sync(F, term, g10 + i);
       if (on && node == 0) {
-        double *r = rec + kk * 8;
+        const auto r = rec + kk * 8;
         r[R_FINT] = 0.5 * (180. - r[R_THMIN]) * acc;
       }
     }
-    __syncwarp();
+    wsync<LS>();
   }
   // pass C: iceNucleation (:421-538)
   double dh = 0., dd = 0., di = 0.;
-  for (int kk = lane; kk < nl; kk += 32) {
-    double *st = stage + kk * 10;
-    const double *r = rec + kk * 8;
+  for (int kk = lane; kk < nl; kk += LS) {
+    const auto st = stage + kk * 10;
+    const auto r = rec + kk * 8;
     const double dwet = w.dwet[kk];
     const double n = w.numc[kk];
     const int ph = phase_of(P, kk);
@@ -3109,9 +3494,9 @@ __device__ void ice_nucl_SE(const DevParams &P, const WS<KT> &w, const double *t
     w.numc[kk] = fmax(0., n * (1. - frac2));
     if (!mk) st[9] = 0.;
   }
-  __syncwarp();
+  wsync<LS>();
   if (diag) {
-    dh = warp_sum(dh); dd = warp_sum(dd); di = warp_sum(di);
+    dh = wsum<LS>(dh); dd = wsum<LS>(dd); di = wsum<LS>(di);
     if (lane == 0) {
       w.misc[M_DIAG + DG_ICEHOM] += dh;
       w.misc[M_DIAG + DG_ICEDEP] += dd;
@@ -3166,21 +3551,21 @@ __device__ double calc_Jhf(double temp, double Sw) {
          dexp(ddiv(-crit - act, K_BOLTZ * temp));
 }
 
-template <typename KT>
-__device__ void ice_nucl_classic(const DevParams &P, const WS<KT> &w, const double *tb, double T, double prv,
+template <typename KT, int LS>
+__device__ void ice_nucl_classic(const DevParams &P, const WS<KT, LS> &w, const double *tb, double T, double prv,
                                  double prs, double prsi, double dt, double kappa, bool diag, int lane) {
   const double *dmid = tb + TAB_DMID * P.nb_pad, *vlo = tb + TAB_VLO * P.nb_pad;
   const double tmax_homog = 237.9, dmin = 1.e-10;
   const int nl = P.nliquid, ndry = P.ndry, iwa = P.iwa, irim = P.irim;
-  double *stage = w.scr;
+  const auto stage = w.scr;
   double dh = 0., dd = 0., di = 0.;
-  for (int kk = lane; kk < nl; kk += 32) {
-    double *st = stage + kk * 10;
+  for (int kk = lane; kk < nl; kk += LS) {
+    const auto st = stage + kk * 10;
     for (int q = 0; q < 10; q++) st[q] = 0.;
     st[0] = -1.;
     int ph = phase_of(P, kk);
     if (T > 273.15 || w.numc[kk] < nlim_of(ph)) continue;
-    updateDiameterAll(P, nullptr, w.numc, w.volc, w.dwet, w.ddry, w.dins, w.dnsp, dmid, w.NB, kk);
+    updateDiameterAll(P, w, dmid, kk);
     double dins_ = w.dins[kk], dwet = w.dwet[kk];
     double Sw = calc_sweq(P, w, kk, T, kappa);
     double pf_imm = 0., pf_dep = 0., pf_hom = 0.;
@@ -3207,9 +3592,9 @@ __device__ void ice_nucl_classic(const DevParams &P, const WS<KT> &w, const doub
     // iceDiagnostics is called after iceNucleation (:130-132): the reduced number
     dh += nn * pf_hom; dd += nn * pf_dep; di += nn * pf_imm;
   }
-  __syncwarp();
+  wsync<LS>();
   if (diag) {
-    dh = warp_sum(dh); dd = warp_sum(dd); di = warp_sum(di);
+    dh = wsum<LS>(dh); dd = wsum<LS>(dd); di = wsum<LS>(di);
     if (lane == 0) {
       w.misc[M_DIAG + DG_ICEHOM] += dh;
       w.misc[M_DIAG + DG_ICEDEP] += dd;
@@ -3217,22 +3602,22 @@ __device__ void ice_nucl_classic(const DevParams &P, const WS<KT> &w, const doub
     }
   }
   ice_apply_staged(P, w, stage, nl, lane);
-  for (int b = P.nliquid + lane; b < P.ntotal; b += 32)
+  for (int b = P.nliquid + lane; b < P.ntotal; b += LS)
     w.rhomean[b] = rhomean_of(P, 4, w.numc[b], w.v(iwa, b), w.v(irim, b));
-  __syncwarp();
+  wsync<LS>();
 }
 
 // ice_melt (mo_salsa_cloud_ice.f90:393-462): ice bins staged per lane, precip bins add in ice order
-template <typename KT>
-__device__ void ice_melt(const DevParams &P, const WS<KT> &w, const double *tb, double T, int lane) {
+template <typename KT, int LS>
+__device__ void ice_melt(const DevParams &P, const WS<KT, LS> &w, const double *tb, double T, int lane) {
   if (T < 273.15) return;
   const double *dmid = tb + TAB_DMID * P.nb_pad, *vlo = tb + TAB_VLO * P.nb_pad;
   const double maxfrac = 0.999;
   const int ndry = P.ndry, iwa = P.iwa, irim = P.irim, I0 = P.nliquid, P0 = P.nbins + P.ncld;
-  double *stage = w.scr;   // nice * 10
-  for (int k = lane; k < P.nice; k += 32) {
+  const auto stage = w.scr;   // nice * 10
+  for (int k = lane; k < P.nice; k += LS) {
     int g = I0 + k;
-    double *st = stage + k * 10;
+    const auto st = stage + k * 10;
     for (int q = 0; q < 10; q++) st[q] = 0.;
     st[0] = -1.;
     if (w.numc[g] < K_PRLIM) continue;
@@ -3263,19 +3648,19 @@ __device__ void ice_melt(const DevParams &P, const WS<KT> &w, const double *tb, 
     w.v(iwa, g) = (1. - maxfrac) * w.v(iwa, g);
     w.v(irim, g) = (1. - maxfrac) * w.v(irim, g);
   }
-  __syncwarp();
+  wsync<LS>();
   // precip bin gets dry species, number, water in ice-bin order
-  for (int e = lane; e < P.nprc * (P.nwet + 1); e += 32) {
+  for (int e = lane; e < P.nprc * (P.nwet + 1); e += LS) {
     int pb = e / (P.nwet + 1), q = e % (P.nwet + 1), g = P0 + pb;
     double val = (q < P.nwet) ? w.v(q, g) : w.numc[g];
     for (int k = 0; k < P.nice; k++) {
-      const double *st = stage + k * 10;
+      const auto st = stage + k * 10;
       if ((int)st[0] != pb) continue;
       val = val + ((q < P.nwet) ? st[1 + q] : st[8]);
     }
     if (q < P.nwet) w.v(q, g) = val; else w.numc[g] = val;
   }
-  __syncwarp();
+  wsync<LS>();
 }
 
 // ----------------------------------------------------------------------------------------
@@ -3403,8 +3788,8 @@ __device__ __forceinline__ void distr_bin(const DevParams &P, const double *tb, 
 }
 
 // Sequential part of a sweep (one thread): bins kk = from .. lo in descending order.
-template <int CAT, typename KT>
-__device__ void distr_serial(const DevParams &P, const WS<KT> &w, const double *tb, int base, int from, int lo,
+template <int CAT, typename KT, int LS>
+__device__ void distr_serial(const DevParams &P, const WS<KT, LS> &w, const double *tb, int base, int from, int lo,
                              bool &has_check, bool &within, bool &neg) {
   const int nmove = (CAT == DC_ICE) ? P.nused : P.nwet;
   for (int kk = from; kk >= lo; kk--) {
@@ -3428,13 +3813,13 @@ __device__ void distr_serial(const DevParams &P, const WS<KT> &w, const double *
 
 // One sweep over bins lo..hi of a category (global index base + kk); hi_recv > hi when
 // the bin above the sweep range can receive particles.  Returns the bin-limit flag.
-template <int CAT, typename KT>
-__device__ bool distr_sweep(const DevParams &P, const WS<KT> &w, const double *tb, int lane, int base, int lo,
+template <int CAT, typename KT, int LS>
+__device__ bool distr_sweep(const DevParams &P, const WS<KT, LS> &w, const double *tb, int lane, int base, int lo,
                             int hi, int hi_recv, bool &neg_flag) {
   const unsigned F = 0xffffffffu;
   const int nmove = (CAT == DC_ICE) ? P.nused : P.nwet;
   bool has_check = false, within = true, neg = false;
-  if (hi_recv >= 32) {
+  if (LS == 1 || hi_recv >= 32) {
     if (lane == 0) distr_serial<CAT>(P, w, tb, base, hi, lo, has_check, within, neg);
   } else {
     const int kk = lane, g = base + lane;
@@ -3478,21 +3863,24 @@ __device__ bool distr_sweep(const DevParams &P, const WS<KT> &w, const double *t
     const unsigned cm = __ballot_sync(F, par && o.check);
     if (cm) within = __shfl_sync(F, o.within, __ffs(cm) - 1);
     neg = __any_sync(F, par && o.neg);
-    __syncwarp();
+    wsync<LS>();
     if (lane == 0 && D > lo) {
       bool hc = false, wi = true;
       distr_serial<CAT>(P, w, tb, base, D - 1, lo, hc, wi, neg);
       if (hc) within = wi;
     }
   }
-  __syncwarp();
-  within = __shfl_sync(F, within, 0);
-  neg_flag = neg_flag || __shfl_sync(F, neg, 0);
+  wsync<LS>();
+  if constexpr (LS != 1) {
+    within = __shfl_sync(F, within, 0);
+    neg = __shfl_sync(F, neg, 0);
+  }
+  neg_flag = neg_flag || neg;
   return within;
 }
 
-template <typename KT>
-__device__ void distr_update(const DevParams &P, const WS<KT> &w, const double *tb, int lane) {
+template <typename KT, int LS>
+__device__ void distr_update(const DevParams &P, const WS<KT, LS> &w, const double *tb, int lane) {
   bool f_distr = false, f_neg = false;
 #pragma unroll 1
   for (int c = 0; c < 4; c++) {
@@ -3513,7 +3901,7 @@ __device__ void distr_update(const DevParams &P, const WS<KT> &w, const double *
     if (f_distr) w.misc[M_FLAGS + F_DISTR] = 1.;
     if (f_neg) w.misc[M_FLAGS + F_NEGFRAC] = 1.;
   }
-  __syncwarp();
+  wsync<LS>();
 }
 
 
@@ -3529,21 +3917,27 @@ __device__ void distr_update(const DevParams &P, const WS<KT> &w, const double *
 #define STAGE_MARK(k)                                                              \
   do {                                                                             \
     long long t_ = clock64();                                                      \
-    if (lane == 0 && P.stage_clocks) atomicAdd(P.stage_clocks + (k), (unsigned long long)(t_ - t_stage)); \
+    if ((threadIdx.x & 31) == 0 && P.stage_clocks) atomicAdd(P.stage_clocks + (k), (unsigned long long)(t_ - t_stage)); \
     t_stage = t_;                                                                  \
   } while (0)
 #else
 #define STAGE_MARK(k) do { } while (0)
 #endif
 
-template <typename KT, bool DIAG, bool SIP>
-__device__ __forceinline__ void cell_step(const DevParams &P, const WS<KT> &w, const double *tb, long long cell,
+// The lane form's warps of a block meet between the stages: a stage's code then stays in the
+// instruction cache while they run it (without the meetings a 1.1 M-cell block of
+// grid384x384x160 took 127 ms instead of 105, with each warp on a tile of its own 179 ms).
+template <int LS> __device__ __forceinline__ void stage_sync() {
+  if constexpr (LS == 1) { __syncwarp(); __syncthreads(); }
+}
+template <typename KT, bool DIAG, bool SIP, int LS>
+__device__ __forceinline__ void cell_step(const DevParams &P, WS<KT, LS> &w, const double *tb, long long cell,
                                           int lane) {
 #ifdef SALSA_STAGE_TIMERS
   long long t_stage = clock64();
 #endif
   const double *dmid = tb + TAB_DMID * P.nb_pad;
-  double *raw = w.raw;
+  const auto raw = w.raw;
   const double T = raw[RW_T], pres = raw[RW_P], rs = raw[RW_RS], rsi = raw[RW_RSI], dn = raw[RW_DN];
   const double kappa = raw[RW_KAPPA];
   const double dt = P.dt;
@@ -3552,7 +3946,7 @@ __device__ __forceinline__ void cell_step(const DevParams &P, const WS<KT> &w, c
   const int nwet = P.nwet, irim = P.irim;
   const int bstart[4] = {0, P.nbins, P.nbins + P.ncld, P.nliquid};
   const int bnum[4] = {P.nbins, P.ncld, P.nprc, P.nice};
-  for (int b = lane; b < P.ntotal; b += 32) {
+  for (int b = lane; b < P.ntotal; b += LS) {
     int icat = phase_of(P, b) - 1;
     w.dwet[b] = dmid[b];
     w.ddry[b] = w.dins[b] = w.dnsp[b] = 0.;
@@ -3562,12 +3956,12 @@ __device__ __forceinline__ void cell_step(const DevParams &P, const WS<KT> &w, c
     w.indef[b] = (!absent && icat < 3 && P.raw_indef >= 0) ? raw[P.raw_indef + b] : 0.;
     w.ctime[b] = (!absent && icat < 3 && P.raw_charge >= 0) ? raw[P.raw_charge + b] : 0.;
   }
-  __syncwarp();
+  wsync<LS>();
   // mass rows of all categories, one lane per (category, species, bin) row
   const int ncat = P.level == 5 ? 4 : 3;
   const int m0 = P.raw_mbase[0];
   const int nmrow = (ncat == 4 ? P.raw_mbase[3] + (nwet + 1) * P.nice : P.raw_mbase[2] + nwet * P.nprc) - m0;
-  for (int e = lane; e < nmrow; e += 32) {
+  for (int e = lane; e < nmrow; e += LS) {
     const int r = m0 + e;
     const int icat = (ncat == 4 && r >= P.raw_mbase[3]) ? 3 : (r >= P.raw_mbase[2] ? 2 : (r >= P.raw_mbase[1] ? 1 : 0));
     const int loc = r - P.raw_mbase[icat], nbc = bnum[icat];
@@ -3575,19 +3969,21 @@ __device__ __forceinline__ void cell_step(const DevParams &P, const WS<KT> &w, c
     const double irho = icat < 3 ? P.irholiq[sp] : (sp < nwet ? P.irhoice[sp] : 1. / K_RHORI);
     w.v(sp, b) = raw[r] * dn * irho;
   }
-  __syncwarp();
-  for (int b = lane; b < P.ntotal; b += 32) {
+  wsync<LS>();
+  for (int b = lane; b < P.ntotal; b += LS) {
     int icat = phase_of(P, b) - 1;
     w.rhomean[b] = (icat == 3 && P.level < 5) ? 0. : rhomean_of(P, icat + 1, w.numc[b], w.v(P.iwa, b), w.v(irim, b));
   }
-  for (int i = lane; i < M_PF; i += 32) w.misc[i] = 0.;
-  __syncwarp();
+  for (int i = lane; i < M_PF; i += LS) w.misc[i] = 0.;
+  wsync<LS>();
   if constexpr (SIP) {
     if (P.st_secice) sip_clear<KT>(P, w, dn, lane);
   }
   if (P.initialize) equilibration<KT>(P, w, tb, 0.3, T, true, lane);
   // gases in #/m3 (mo_salsa_driver.f90:285-290)
-  if (P.raw_gas >= 0 && lane < 5) w.misc[M_GAS + lane] = raw[P.raw_gas + lane] * dn;
+  if (P.raw_gas >= 0)
+    for (int i = lane; i < 5; i += LS) w.misc[M_GAS + i] = raw[P.raw_gas + i] * dn;
+  stage_sync<LS>();
   STAGE_MARK(0);
 
   // ---- salsa() ----
@@ -3595,6 +3991,7 @@ __device__ __forceinline__ void cell_step(const DevParams &P, const WS<KT> &w, c
   if constexpr (SIP) {
     if (P.st_secice) secondary_ice<KT>(P, w, tb, T, pres, rv, rsi, dt, lane);
   }
+  stage_sync<LS>();
   STAGE_MARK(1);
   if (P.st_cnd) {
     // condensation (mo_salsa_dynamics.f90:276-342): nucleation returns only the 3 nm
@@ -3604,10 +4001,12 @@ __device__ __forceinline__ void cell_step(const DevParams &P, const WS<KT> &w, c
     if (P.lscndgas) condgas<KT>(P, w, tb, T, pres, dt, w.misc + M_GAS, P.nsnucl > 0 ? 1. : 0., lane);
     if (P.lscndh2ocl || P.lscndh2oae || P.lscndh2oic) gpparth2o<KT>(P, w, tb, T, pres, rs, rsi, rv, dt, kappa, DIAG, lane);
   }
+  stage_sync<LS>();
   STAGE_MARK(2);
   if (P.st_auto && P.auto_mode == 2) autoconv2<KT>(P, w, dt, lane);
   if (P.st_activ && P.activ_mode == 1) act_interst<KT>(P, w, tb, rv, rs, T, DIAG, lane);
   if (P.st_activ && P.activ_mode == 2) act_cloudbase<KT>(P, w, tb, pres, T, raw[RW_W], dn, raw, lane);
+  stage_sync<LS>();
   STAGE_MARK(3);
   if ((P.st_icenucl || P.icenucl_mode == 2) && (P.lsicehom || P.lsiceimm || P.lsicedep)) {
     if (P.ice_theta_dist) ice_nucl_SE<KT>(P, w, tb, T, rv, rs, rsi, dt, kappa, DIAG, lane);
@@ -3616,22 +4015,24 @@ __device__ __forceinline__ void cell_step(const DevParams &P, const WS<KT> &w, c
   if constexpr (SIP) {
     // ice_melt's bins (numbers not below prlim) before it runs: their tracers melt with them
     if (P.st_secice && P.st_icemelt) {
-      const SipT s = sip_tallies(P, w.raw);
-      for (int k = lane; k < P.nice; k += 32) s.melt[k] = w.numc[P.nliquid + k] < K_PRLIM ? 0. : 1.;
-      __syncwarp();
+      const auto s = sip_tallies(P, w.raw);
+      for (int k = lane; k < P.nice; k += LS) s.melt[k] = w.numc[P.nliquid + k] < K_PRLIM ? 0. : 1.;
+      wsync<LS>();
     }
   }
   if (P.st_icemelt) ice_melt<KT>(P, w, tb, T, lane);
   if constexpr (SIP) {
     if (P.st_secice && P.st_icemelt && T >= 273.15) {   // mo_salsa_cloud_ice.f90:453-456
-      const SipT s = sip_tallies(P, w.raw);
-      for (int e = lane; e < 3 * P.nice; e += 32)
+      const auto s = sip_tallies(P, w.raw);
+      for (int e = lane; e < 3 * P.nice; e += LS)
         if (s.melt[e % P.nice] != 0.) s.tr[e] = (1. - 0.999) * s.tr[e];
-      __syncwarp();
+      wsync<LS>();
     }
   }
+  stage_sync<LS>();
   STAGE_MARK(4);
   if (P.lsdistupdate) distr_update<KT>(P, w, tb, lane);
+  stage_sync<LS>();
   STAGE_MARK(5);
 
   // ---- tendencies and outputs (mo_salsa_driver.f90:310-419) into the raw slots ----
@@ -3639,7 +4040,7 @@ __device__ __forceinline__ void cell_step(const DevParams &P, const WS<KT> &w, c
   // product when dt is a power of two (then it is the same number)
   bool bad = false;
   const double idn = drcp(dn);
-  for (int e = lane; e < nmrow; e += 32) {
+  for (int e = lane; e < nmrow; e += LS) {
     const int r = m0 + e;
     const int icat = (ncat == 4 && r >= P.raw_mbase[3]) ? 3 : (r >= P.raw_mbase[2] ? 2 : (r >= P.raw_mbase[1] ? 1 : 0));
     const int loc = r - P.raw_mbase[icat], nbc = bnum[icat];
@@ -3648,35 +4049,37 @@ __device__ __forceinline__ void cell_step(const DevParams &P, const WS<KT> &w, c
     const double d = (w.v(sp, b) * rho * idn) - raw[r];
     raw[r] = P.inv_dt != 0. ? d * P.inv_dt : ddiv(d, dt);
   }
-  for (int b = lane; b < P.ntotal; b += 32) {
+  for (int b = lane; b < P.ntotal; b += LS) {
     int icat = phase_of(P, b) - 1;
     if (icat == 3 && P.level < 5) continue;
     if (icat < 3) {
       if (P.raw_indef >= 0) raw[P.raw_indef + b] = w.indef[b];
       if (P.raw_charge >= 0) raw[P.raw_charge + b] = w.ctime[b];
     }
-    double *on = raw + P.raw_num + b;
-    const double d = (w.numc[b] * idn) - *on;
-    *on = P.inv_dt != 0. ? d * P.inv_dt : ddiv(d, dt);
+    double &on = raw[P.raw_num + b];
+    const double d = (w.numc[b] * idn) - on;
+    on = P.inv_dt != 0. ? d * P.inv_dt : ddiv(d, dt);
     bad |= !isfinite(w.numc[b]);
   }
   // interstitial activation leaves the activated-droplet outputs at zero (:879, local pactd);
   // cloud-base activation has written them
   if (!(P.st_activ && P.activ_mode == 2))
-    for (int i = lane; i < P.ncld * (1 + nwet); i += 32) raw[P.raw_nact + i] = 0.;
+    for (int i = lane; i < P.ncld * (1 + nwet); i += LS) raw[P.raw_nact + i] = 0.;
   if (lane == 0) raw[RW_RV] = ddiv(rv - rv_old, dt);
   if constexpr (SIP) {
     if (P.st_secice) {   // :345-349 and :412-416
-      const SipT s = sip_tallies(P, w.raw);
-      for (int e = lane; e < 3 * P.nice; e += 32) raw[P.raw_sip + e] = ddiv(s.tr[e], dn);
-      if (P.raw_diag >= 0 && lane < 3) raw[P.raw_diag + SALSA_DIAG_SIPDRFR_SLOT + lane] = ddiv(s.rate[lane], dn);
+      const auto s = sip_tallies(P, w.raw);
+      for (int e = lane; e < 3 * P.nice; e += LS) raw[P.raw_sip + e] = ddiv(s.tr[e], dn);
+      if (P.raw_diag >= 0)
+        for (int e = lane; e < 3; e += LS) raw[P.raw_diag + SALSA_DIAG_SIPDRFR_SLOT + e] = ddiv(s.rate[e], dn);
     }
   }
-  if (P.raw_gas >= 0 && lane < 5)   // :369-384
-    raw[P.raw_gas + lane] = ddiv((ddiv(w.misc[M_GAS + lane], dn)) - raw[P.raw_gas + lane], dt);
+  if (P.raw_gas >= 0)   // :369-384
+    for (int i = lane; i < 5; i += LS)
+      raw[P.raw_gas + i] = ddiv((ddiv(w.misc[M_GAS + i], dn)) - raw[P.raw_gas + i], dt);
   if (DIAG && P.raw_diag >= 0 && lane == 0) {
-    const double *d = w.misc + M_DIAG;
-    double *o = raw + P.raw_diag;
+    const auto d = w.misc + M_DIAG;
+    const auto o = raw + P.raw_diag;
     o[DG_AUTOC] = ddiv(d[DG_AUTOC] * K_RHOWA, dn);
     o[DG_AUTOC80] = ddiv(d[DG_AUTOC80] * K_RHOWA, dn);
     o[DG_AUTOC50] = ddiv(d[DG_AUTOC50] * K_RHOWA, dn);
@@ -3697,10 +4100,11 @@ __device__ __forceinline__ void cell_step(const DevParams &P, const WS<KT> &w, c
       o[DG_CONDI] = ddiv(d[DG_CONDI], dn);
     }
   }
-  bad = warp_any(bad);
+  bad = wany<LS>(bad);
+  stage_sync<LS>();
   STAGE_MARK(6);
-  if (lane == 0 && P.status) {
-    const double *f = w.misc + M_FLAGS;
+  if (lane == 0 && P.status && w.live) {
+    const auto f = w.misc + M_FLAGS;
     if (f[F_EQUIL] != 0.) atomicAdd(P.status + ST_EQUIL, 1ull);
     if (f[F_DISTR] != 0.) atomicAdd(P.status + ST_DISTR, 1ull);
     if (f[F_NEGFRAC] != 0.) atomicAdd(P.status + ST_NEGFRAC, 1ull);
@@ -3708,31 +4112,35 @@ __device__ __forceinline__ void cell_step(const DevParams &P, const WS<KT> &w, c
     if (f[F_NEG] != 0.) atomicAdd(P.status + ST_NEG, 1ull);
     if (bad) atomicAdd(P.status + ST_NONFINITE, 1ull);
   }
-  __syncwarp();
+  wsync<LS>();
 }
 
-template <typename KT>
-__device__ __forceinline__ WS<KT> make_ws(const DevParams &P, double *base) {
-  WS<KT> w;
+template <typename KT, int LS>
+__device__ __forceinline__ WS<KT, LS> make_ws(const DevParams &P, Ptr<double, LS> base) {
+  WS<KT, LS> w;
+  w.am0 = ~0ull;
+  w.am1 = ~0u;
+  w.live = true;
   const int NB = P.nb_pad;
   w.NB = NB;
-  double *p = base;
-  w.raw = p; p += (P.nraw + 1) & ~1;
-  w.numc = p; p += NB;
-  w.volc = p; p += SALSA_NSV * NB;
-  w.dwet = p; p += NB;
-  w.ddry = p; p += NB;
-  w.dins = p; p += NB;
-  w.dnsp = p; p += NB;
-  w.rhomean = p; p += NB;
-  w.indef = p; p += NB;
-  w.ctime = p; p += NB;
-  w.scr = p; p += SALSA_NSCR * NB;
-  w.nf = reinterpret_cast<float *>(w.scr);   // NB floats, then SALSA_NSV * NB floats (4 scratch rows)
+  Ptr<double, LS> p = base;
+  w.raw = p; p = p + ((P.nraw + 1) & ~1);
+  w.numc = p; p = p + NB;
+  w.volc = p; p = p + SALSA_NSV * NB;
+  w.dwet = p; p = p + NB;
+  w.ddry = p; p = p + NB;
+  w.dins = p; p = p + NB;
+  w.dnsp = p; p = p + NB;
+  w.rhomean = p; p = p + NB;
+  w.indef = p; p = p + NB;
+  w.ctime = p; p = p + NB;
+  w.scr = p; p = p + SALSA_NSCR * NB;
+  w.nf = row_cast<float>(w.scr);   // NB floats, then SALSA_NSV * NB floats (4 scratch rows)
   w.vf = w.nf + NB;
-  w.misc = p; p += SALSA_MISC_DOUBLES;
-  w.pbuf = reinterpret_cast<int *>(p); p += 64;   // 128 ints: bin lists (<= 96) and pair batches (<= 63)
-  w.K = reinterpret_cast<KT *>(p);
+  w.misc = p; p = p + SALSA_MISC_DOUBLES;
+  if constexpr (LS != 1) w.pbuf = reinterpret_cast<int *>(p);
+  p = p + 64;   // 128 ints: bin lists (<= 96) and pair batches (<= 63)
+  w.K = row_cast<KT>(p);
   return w;
 }
 
@@ -3744,7 +4152,7 @@ __global__ void __launch_bounds__(SALSA_THREADS, 2) salsa_step_kernel(const DevP
   double *tb = smem;
   for (int i = tid; i < P.tab_doubles; i += SALSA_THREADS) tb[i] = P.tables[i];
   double *wsbase = smem + P.tab_doubles;
-  WS<KT> w = make_ws<KT>(P, wsbase + (size_t)warp * P.ws_doubles);
+  WS<KT, 32> w = make_ws<KT, 32>(P, wsbase + (size_t)warp * P.ws_doubles);
   __syncthreads();
   for (long long g = blockIdx.x; g < P.ngroups; g += gridDim.x) {
     // stage the group's input rows: consecutive threads read the group's cells of one row
@@ -3783,6 +4191,65 @@ __global__ void __launch_bounds__(SALSA_THREADS, 2) salsa_step_kernel(const DevP
   }
 }
 
+// The lane form: one cell per lane, a warp's 32 cells side by side from the order list.  Every
+// FP64 instruction then serves 32 cells, where the warp form leaves half of the lanes idle,
+// adds up partial sums across them and repeats per-cell scalars on all of them; the FP64 pipe
+// takes as long for one active lane as for 32.  The workspaces (about 25 KB a cell) live in
+// global memory, a slot per resident warp, interleaved by lane: HBM and L2 have bandwidth to
+// spare (they are 5-15 % busy).  Blocks take four tiles of 32 cells from a counter, the cloudy
+// end of the list first (its cells take several times as long as clear ones).
+// FP64 instructions per cell of grid384x384x160: 6,190 in the warp form, 1,300 here; a 1.1 M
+// cell block took 299 ms in the warp form, 105 ms here.  Four blocks of 128 threads per SM
+// (128 registers) measured better than two or three (clear cells 61.7, 69.4 and 66 ns a
+// cell): the FP64 pipe waits for memory less (67-78 % busy).
+template <typename KT, bool DIAG, bool SIP>
+__global__ void __launch_bounds__(32 * SALSA_LANE_WARPS, SALSA_LANE_MINBLOCKS) salsa_lane_kernel(const DevParams P) {
+  extern __shared__ double smem[];
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  double *tb = smem;
+  for (int i = tid; i < P.tab_doubles; i += 32 * SALSA_LANE_WARPS) tb[i] = P.tables[i];
+  __syncthreads();
+  WS<KT, 1> w = make_ws<KT, 1>(
+      P, Col<double>{P.lane_ws + ((size_t)blockIdx.x * SALSA_LANE_WARPS + warp) * (size_t)P.ws_doubles * 32 + lane});
+  const long long ntiles = (P.ncells + 31) / 32;
+  __shared__ unsigned long long next;
+  for (;;) {
+    // the block's warps take neighbouring tiles together
+    if (tid == 0) next = atomicAdd(P.status + ST_TILE, (unsigned long long)SALSA_LANE_WARPS);
+    __syncthreads();
+    const long long k0 = (long long)next, k = k0 + warp;
+    __syncthreads();
+    if (k0 >= ntiles) break;
+    // warps past the last tile repeat it
+    const long long q = (ntiles - 1 - min(k, ntiles - 1)) * 32 + lane;
+    w.live = k < ntiles && q < P.ncells;
+    const long long cell = cell_at(P, min(q, P.ncells - 1)), off = cell_offset(P, cell);
+    for (int r = 0; r < P.nrows; r++) {
+      const Row row = P.rows[r];
+      double v = 0.;
+      if (row.fin >= 0) {
+        const double *f = P.fin[row.fin];
+        if (f) v = __ldg(f + off + P.plane * row.idx);
+      }
+      w.raw[r] = v;
+    }
+    cell_step<KT, DIAG, SIP>(P, w, tb, cell, 0);
+    __syncwarp();
+    if (w.live)
+      for (int r = 0; r < P.nrows; r++) {
+        const Row row = P.rows[r];
+        if (row.fout < 0) continue;
+        double *f = P.fout[row.fout];
+        if (!f) continue;
+        double *a = f + off + P.plane * row.idx;
+        if (row.mode == ROW_TEND) *a = *a + w.raw[r];
+        else *a = w.raw[r];
+      }
+    const unsigned nlive = __popc(__ballot_sync(0xffffffffu, w.live));
+    if (lane == 0) atomicAdd(P.status + ST_CELLS, (unsigned long long)nlive);
+  }
+}
+
 // Host-side launch helpers, instantiated per form in salsa_k_*.cu.
 inline size_t smem_bytes(const DevParams &P) {
   return sizeof(double) * ((size_t)P.tab_doubles + (size_t)SALSA_CPG * P.ws_doubles);
@@ -3796,6 +4263,20 @@ cudaError_t launch_t(const DevParams &P, cudaStream_t st, int grid) {
   if (e != cudaSuccess) return e;
   salsa_step_kernel<KT, DIAG, SIP><<<grid, SALSA_THREADS, sm, st>>>(P);
   return cudaGetLastError();
+}
+
+template <typename KT, bool DIAG, bool SIP = false>
+cudaError_t launch_lane_t(const DevParams &P, cudaStream_t st, int grid) {
+  salsa_lane_kernel<KT, DIAG, SIP><<<grid, 32 * SALSA_LANE_WARPS, sizeof(double) * (size_t)P.tab_doubles, st>>>(P);
+  return cudaGetLastError();
+}
+template <typename KT, bool DIAG, bool SIP = false>
+int lane_blocks_per_sm_t(const DevParams &P) {
+  int nb = 0;
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, salsa_lane_kernel<KT, DIAG, SIP>, 32 * SALSA_LANE_WARPS,
+                                                    sizeof(double) * (size_t)P.tab_doubles) != cudaSuccess)
+    return 0;
+  return nb;
 }
 
 template <typename KT, bool DIAG, bool SIP = false>

@@ -1,0 +1,9 @@
+// salsa_l_d0.cu -- instantiation of the step's lane form for KT=double, without diagnostics.
+#include "salsa_kernel_impl.cuh"
+
+namespace salsa {
+cudaError_t launch_lane_d0(const DevParams &P, cudaStream_t st, int grid) {
+  return launch_lane_t<double, false>(P, st, grid);
+}
+int lane_blocks_per_sm_d0(const DevParams &P) { return lane_blocks_per_sm_t<double, false>(P); }
+}  // namespace salsa

@@ -96,6 +96,12 @@ __device__ __forceinline__ double drcp(double d) {
   return fma(fma(-d, r, 1.), r, r);
 }
 
+// n/d with r = drcp(d) at hand (several quotients by one denominator)
+__device__ __forceinline__ double ddiv_r(double n, double d, double r) {
+  const double q = n * r;
+  return fma(fma(-d, q, n), r, q);
+}
+
 // n/d.  Exponents within +-500; n = 0 too.
 __device__ __forceinline__ double ddiv(double n, double d) {
   const unsigned hi = (unsigned)__double2hiint(d), hn = (unsigned)__double2hiint(n);
