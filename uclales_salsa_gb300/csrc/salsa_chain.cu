@@ -464,8 +464,8 @@ __device__ __forceinline__ R chain_zvolc(const DevParams &P, const CW<R> &w, int
   return (d >= 0 && which < 5) ? w.V(d, b) : R(0.);
 }
 
-// one iteration of the regime-1a water uptake (equil_iterate, :196-245) in the form of
-// the step kernel's eq_step, operation for operation: izke = 1/zke -> (zlwc, zdwet, izke')
+// one iteration of the regime-1a water uptake (equil_iterate, :196-245), carrying 1/zke as
+// the step kernel's eq_step does: izke = 1/zke -> (zlwc, zdwet, izke')
 template <typename R>
 __device__ __forceinline__ void eq1a_iter(R zrh, R &izke, R zv0, R zv1, R numc, R zvp56, R zcore, double T, R &zlwc,
                                           R &zdwet) {

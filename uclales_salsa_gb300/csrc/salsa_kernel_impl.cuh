@@ -59,7 +59,8 @@ struct WS {
   Ptr<KT, LS> K;
   int *pbuf;   // warp form
   int NB;
-  bool live;   // the lane form's last warp: lanes past the last cell repeat it and write nothing
+  bool live;   // lane form, last warp: lanes past the last cell repeat it and write nothing
+  long long off;   // lane form: the cell's offset inside a field plane
   // lane form: bins that reach their number limit in some cell of the warp before coagulation
   // (bins 0-63, 64-95); pairs with the others have K = 0 and their terms are skipped
   unsigned long long am0;
@@ -110,6 +111,32 @@ __device__ __forceinline__ double nlim_of(int ph) { return ph <= 2 ? K_NLIM : K_
 __device__ __forceinline__ double dlim_of(int ph) {
   return ph == 1 ? 30.e-6 : (ph == 2 ? 100.e-6 : (ph == 3 ? 5.e-3 : 10.e-3));
 }
+// Comparisons of a number with a positive constant, and minima and maxima of non-negative
+// ones, on the bit patterns: an FP64 comparison occupies the FP64 pipe as long as a sum
+// does.  The results equal the FP64 ones for every x that arithmetic produces (NaNs are
+// positive quiet ones here).
+#define FM_INF 0x7ff0000000000000ll
+__device__ __forceinline__ bool num_ge(double x, double c) {
+  const long long b = __double_as_longlong(x);
+  return b >= __double_as_longlong(c) && b <= FM_INF;
+}
+__device__ __forceinline__ bool num_gt(double x, double c) {
+  const long long b = __double_as_longlong(x);
+  return b > __double_as_longlong(c) && b <= FM_INF;
+}
+__device__ __forceinline__ bool num_lt(double x, double c) { return __double_as_longlong(x) < __double_as_longlong(c); }
+__device__ __forceinline__ double min_pos(double a, double b) { return __double_as_longlong(a) < __double_as_longlong(b) ? a : b; }
+// fmax(0., x)
+__device__ __forceinline__ double pos_part(double x) {
+  return (unsigned long long)__double_as_longlong(x) > (unsigned long long)FM_INF ? 0. : x;
+}
+// fmax(c, x) of x >= 0 (or NaN: c)
+__device__ __forceinline__ double max_pos(double c, double x) { return num_gt(x, c) ? x : c; }
+// fmin(fmax(x, -t), t) of t >= 0
+__device__ __forceinline__ double limit_pos(double x, double t) {
+  const long long b = __double_as_longlong(x), m = b & 0x7fffffffffffffffll, bt = __double_as_longlong(t);
+  return m > bt ? __longlong_as_double(bt | (b ^ m)) : x;
+}
 __device__ __forceinline__ int tri(int i, int j, int NB) {  // i <= j
   return i * NB - (i * (i - 1)) / 2 + (j - i);
 }
@@ -129,7 +156,7 @@ __device__ __forceinline__ void updateDiameterAll(const DevParams &P, const WS<K
   int ph = phase_of(P, b);
   double n = w.numc[b];
   double dw, dd, di;
-  if (n > nlim_of(ph)) {
+  if (num_gt(n, nlim_of(ph))) {
     double vs = 0., vd = 0., vi = 0.;
     for (int s = 0; s < P.nused; s++) vs += w.v(s, b);
     for (int s = 0; s < P.ndry; s++) vd += w.v(s, b);
@@ -143,18 +170,18 @@ __device__ __forceinline__ void updateDiameterAll(const DevParams &P, const WS<K
     dw = dd = di = dmid[b];
   }
   double dl = dlim_of(ph);
-  dw = fmin(dw, dl);
+  dw = min_pos(dw, dl);
   w.dwet[b] = dw;
   w.dnsp[b] = dw;
-  w.ddry[b] = fmin(dd, dl);
-  w.dins[b] = fmin(di, dl);
+  w.ddry[b] = min_pos(dd, dl);
+  w.dins[b] = min_pos(di, dl);
 }
 
 __device__ __forceinline__ double rhomean_of(const DevParams &P, int ph, double n, double vw, double vr) {
   if (ph > 3) {
-    if (n > nlim_of(ph)) {
+    if (num_gt(n, nlim_of(ph))) {
       double mp = K_RHOIC * vw, mr = K_RHORI * vr, mt = mp + mr;
-      double r = ddiv(mp * K_RHOIC + mr * K_RHORI, fmax(mt, 7.e-25));
+      double r = ddiv(mp * K_RHOIC + mr * K_RHORI, max_pos(7.e-25, mt));
       return fmin(r, K_RHOIC);
     }
     return K_RHOIC;
@@ -165,7 +192,7 @@ __device__ __forceinline__ double rhomean_of(const DevParams &P, int ph, double 
 // classSection.f90:202-224 getRimeFraction
 __device__ __forceinline__ double rimefrac(const DevParams &P, double n, double vw, double vr, int ph) {
   double r = 0.;
-  if (ph == 4 && vw > 1.e-23 && vr > 1.e-23 && n > nlim_of(ph)) r = ddiv(vr * K_RHORI, vw * K_RHOIC + vr * K_RHORI);
+  if (ph == 4 && num_gt(vw, 1.e-23) && num_gt(vr, 1.e-23) && num_gt(n, nlim_of(ph))) r = ddiv(vr * K_RHORI, vw * K_RHOIC + vr * K_RHORI);
   return r;
 }
 
@@ -388,63 +415,203 @@ __device__ T coag_pair(const CoagCell<T> &cc, const BinProps<T> &a, const BinPro
   return zbrown + zbrconv + t_sqrt(sq(zgrav) + sq(ztshear) + sq(zturb));
 }
 
-template <typename KT, typename PT>
-__device__ __forceinline__ void load_props(const PT &S, int NB, int b, BinProps<KT> &o) {
-  KT *po = &o.diam;
-#pragma unroll
-  for (int k = 0; k < 9; k++) po[k] = S[k * NB + b];
+// ---- the FP64 step's form of the pair kernel ----
+// The same kernel as coag_pair in fewer FP64 operations (64 instead of 92 a pair, 48 instead
+// of 75 a bin): what depends on one particle is taken once per bin, per-cell factors once per
+// cell, and common factors leave the sums.  With m the mean diameter, w the mean free path of
+// a particle (omega), D4 four times its diffusion coefficient, v2 its squared thermal speed:
+//   flux matching   ((m+w)^3 - (m^2+w^2)^(3/2)) / (3 m w) - m, by the reciprocals of m and 3 w
+//                     (the differences as coag_pair rounds them: they cancel to 1e-14 for a
+//                     drop and an Aitken particle, and condensation magnifies that)
+//   Brownian        pi X Y / (X + Y),  X = m^2 sqrt(v2_a + v2_b),  Y = (D4_a + D4_b) (m + f)
+//   gravity, shear, turbulence  m^2 sqrt((pi E dv)^2 + (A m)^2 + (B dv)^2)
+// On grid384x384x160 the collision kernels were 42 % of the lane form's time.
+struct PairProps {
+  double h, D4, v2, om, i3om, tv;   // half diameter, D4, v2, omega, 1/(3 omega), fall speed
+  double fre, cs, rre, G;   // Re^(1/3 or 1/2); 0.45 pi Sc^(1/3); pi Re/(60 + Re); 2/(d g)
+};
+// per-cell factors
+struct PairCell {
+  CoagCell<double> c;
+  double mfp2, kx, kD4, kv2, k18, ivkin, vkin4;   // 2 mfp, 0.999/(2 mfp), 4kT/(3 pi mu), 8kT/pi, g/(18 mu), 1/nu, 4 nu
+};
+
+__device__ __forceinline__ bool bits_ge(double a, double b) {   // a >= b of non-negative numbers
+  return __double_as_longlong(a) >= __double_as_longlong(b);
 }
 
-// Per-bin properties are evaluated in the kernel type: FP64 in the FP64 form, float in
-// the mixed form (its pair kernels are float too) except for ice bins.
+// rd = 1/diam, im = 1/mass
+__device__ __forceinline__ void pair_props(const PairCell &k, int ph, double diam, double rd, double im, double dsph,
+                                           double rho, const Shape<double> &sh, PairProps &o) {
+  const double beta = fma(k.mfp2 * rd, fma(0.558, dexp(-(k.kx * diam)), 1.142), 1.);
+  o.h = 0.5 * diam;
+  o.D4 = beta * rd * k.kD4;
+  o.v2 = k.kv2 * im;
+  const double v = dsqrt(o.v2);
+  o.om = ddiv((2. / K_PI) * o.D4, v);
+  o.i3om = drcp(3. * o.om);
+  if (ph < 4 && bits_ge(19E-6, diam)) o.tv = diam * diam * (rho - k.c.zrhoa) * beta * k.k18;
+  else if (ph < 4) o.tv = terminal_vel<double>(diam, rho, k.c.zrhoa, k.c.visc, beta, ph, sh, 0.);
+  else o.tv = terminal_vel<double>(dsph, rho, k.c.zrhoa, k.c.visc, beta, ph, sh, diam);
+  const double re = diam * o.tv * k.ivkin;
+  o.fre = re <= 1. ? dcbrt(re) : dsqrt(re);
+  o.cs = (0.45 * K_PI) * dcbrt(ddiv(k.vkin4, o.D4));
+  o.rre = ddiv(K_PI * re, 60. + re);
+  o.G = (2. / K_GRAV) * rd;
+}
+
+__device__ __forceinline__ double pair_kernel(const PairCell &k, const PairProps &a, const PairProps &b) {
+  const double m = a.h + b.h, m2 = m * m, im = drcp(m);
+  const double oa = fma(a.om, a.om, m2), ob = fma(b.om, b.om, m2), sa = m + a.om, sb = m + b.om;
+  const double ta = fma(fma(sa * sa, sa, -(oa * dsqrt(oa))) * im, a.i3om, -m);
+  const double tb = fma(fma(sb * sb, sb, -(ob * dsqrt(ob))) * im, b.i3om, -m);
+  const double X = m2 * dsqrt(a.v2 + b.v2), Y = (a.D4 + b.D4) * (m + dsqrt(fma(tb, tb, ta * ta)));
+  const double zb = ddiv(X * Y, X + Y);
+  const bool al = bits_ge(a.h, b.h);
+  const double Lrre = al ? a.rre : b.rre;
+  const double dv = fabs(a.tv - b.tv);
+  const double stok = (al ? b.tv : a.tv) * dv * (al ? a.G : b.G);
+  const double q = ddiv(stok, stok + 0.5);
+  double e = q * q * Lrre;   // pi times the collision efficiency
+  if (stok > 1.214) {
+    double z = ddiv(0.75 * dlog(2. * stok), stok - 1.214);
+    z = drcp(sq(1. + z));
+    e = fma(z, K_PI - Lrre, e);   // 60/(60 + Re) = 1 - Re/(60 + Re)
+  }
+  const double g = e * dv, t1 = k.c.shearA * m, t2 = k.c.turbB * dv;
+  return fma(zb, fma(al ? a.fre : b.fre, al ? b.cs : a.cs, K_PI), m2 * dsqrt(fma(g, g, fma(t1, t1, t2 * t2))));
+}
+
+// What the two kernel types use: properties of a bin, rows that hold them, cell constants
+template <typename KT> struct KForm;
+template <> struct KForm<float> {
+  typedef BinProps<float> Props;
+  struct Cell { CoagCell<double> cd; CoagCell<float> cc; };
+  static constexpr int NROW = 9;
+};
+template <> struct KForm<double> {
+  typedef PairProps Props;
+  typedef PairCell Cell;
+  static constexpr int NROW = 10;
+};
+template <typename KT> using KProps = typename KForm<KT>::Props;
+template <typename KT> using KCell = typename KForm<KT>::Cell;
+
 template <typename KT, typename PT>
-__device__ __forceinline__ void store_props(const PT &S, int NB, int b, const BinProps<double> &o) {
-  const double *po = &o.diam;
+__device__ __forceinline__ void load_props(const PT &S, int NB, int b, KProps<KT> &o) {
+  KT *po = reinterpret_cast<KT *>(&o);
 #pragma unroll
-  for (int k = 0; k < 9; k++) S[k * NB + b] = (KT)po[k];
+  for (int k = 0; k < KForm<KT>::NROW; k++) po[k] = S[k * NB + b];
 }
 template <typename KT, typename PT>
-__device__ __forceinline__ void store_props_kt(const PT &S, int NB, int b, const BinProps<KT> &o) {
-  const KT *po = &o.diam;
+__device__ __forceinline__ void store_props(const PT &S, int NB, int b, const KProps<KT> &o) {
+  const KT *po = reinterpret_cast<const KT *>(&o);
 #pragma unroll
-  for (int k = 0; k < 9; k++) S[k * NB + b] = po[k];
+  for (int k = 0; k < KForm<KT>::NROW; k++) S[k * NB + b] = po[k];
 }
-template <typename KT>
-__device__ __forceinline__ void to_kt(const BinProps<double> &d, BinProps<KT> &o) {
+__device__ __forceinline__ void to_float(const BinProps<double> &d, BinProps<float> &o) {
   const double *pd = &d.diam;
-  KT *po = &o.diam;
+  float *po = &o.diam;
 #pragma unroll
-  for (int k = 0; k < 9; k++) po[k] = (KT)pd[k];
-}
-// FP64 shape coefficients of bin b: they share the memory of S rows 9-12 in the FP64
-// form and sit behind the float rows in the mixed form.
-template <typename KT, int LS>
-__device__ __forceinline__ Ptr<double, LS> shape_rows(const WS<KT, LS> &w) {
-  return sizeof(KT) == 8 ? w.scr + 9 * w.NB : w.scr + 7 * w.NB;
+  for (int k = 0; k < 9; k++) po[k] = (float)pd[k];
 }
 
-// Properties of the first particle of a pair of equal-size bins (i, j), the self-coagulation
-// offset (:273-276): 1.1 times the diameter and 1.33 times the mass of particle 2.  S and SH
-// are the property and shape rows.  For liquid bins they depend on bin j alone: the fall
-// speed takes the same branch for every liquid phase, every liquid density is that of water
-// and the sphere-equivalent diameter enters only for ice.
+// per-cell constants of the collision kernel
+__device__ __forceinline__ void coag_cell(const DevParams &P, double T, double pres, CoagCell<double> &cd) {
+  double visc = ddiv(7.44523e-3 * dsqrt(cube(T)), 5093. * (T + 110.4));
+  double mfp = ddiv((1.656e-10 * T + 1.828e-8) * K_PSTAND, pres);
+  double zrhoa = ddiv(pres, K_RD * T);
+  double vkin = ddiv(visc, zrhoa);
+  cd.T_ = T; cd.visc = visc; cd.mfp = mfp; cd.zrhoa = zrhoa; cd.vkin = vkin;
+  cd.shearA = dsqrt(ddiv(8. * K_PI * P.eddy_dis, 15. * vkin));
+  cd.turbB = ddiv(K_PI * dpow(P.eddy_dis, 0.75), K_GRAV * dsqrt(dsqrt(vkin)));
+}
+__device__ __forceinline__ void kcell(const DevParams &P, double T, double pres, KCell<float> &k) {
+  coag_cell(P, T, pres, k.cd);
+  const CoagCell<double> &cd = k.cd;
+  CoagCell<float> &cc = k.cc;
+  cc.T_ = (float)cd.T_; cc.visc = (float)cd.visc; cc.mfp = (float)cd.mfp; cc.zrhoa = (float)cd.zrhoa;
+  cc.vkin = (float)cd.vkin; cc.shearA = (float)cd.shearA; cc.turbB = (float)cd.turbB;
+}
+__device__ __forceinline__ void kcell(const DevParams &P, double T, double pres, KCell<double> &k) {
+  coag_cell(P, T, pres, k.c);
+  const double imu = drcp(k.c.visc);
+  k.mfp2 = 2. * k.c.mfp;
+  k.kx = ddiv(0.999, k.mfp2);
+  k.kD4 = (4. * K_BOLTZ / (3. * K_PI)) * T * imu;
+  k.kv2 = (8. * K_BOLTZ / K_PI) * T;
+  k.k18 = (K_GRAV / 18.) * imu;
+  k.ivkin = drcp(k.c.vkin);
+  k.vkin4 = 4. * k.c.vkin;
+}
+
 template <typename KT, int LS>
-__device__ __forceinline__ void offset_props(const DevParams &P, const WS<KT, LS> &w, const CoagCell<KT> &cc,
-                                             const CoagCell<double> &cd, const Shape<double> &sh, int i, int j,
-                                             BinProps<KT> &a) {
-  if constexpr (sizeof(KT) == 4) {
-    if (phase_of(P, i) < 4) {
-      const float dj = (float)w.dwet[j], mj = (float)w.rhomean[j] * (float)K_PI6 * cube(dj);
-      Shape<float> shf;
-      shf.alpha = (float)sh.alpha; shf.beta = (float)sh.beta; shf.gamma = (float)sh.gamma; shf.sigma = (float)sh.sigma;
-      bin_props<float>(cc, phase_of(P, i), 1.1f * dj, (float)w.dwet[i], 1.33f * mj, (float)w.rhomean[i], shf, a);
-      return;
-    }
+__device__ __forceinline__ void shape_of_bin(const DevParams &P, const WS<KT, LS> &w, int b, Shape<double> &sh) {
+  if (phase_of(P, b) == 4) {
+    double mp = 0.;
+    for (int s = 0; s < P.nused - 1; s++) mp += w.v(s, b) * K_RHOIC;
+    shape_coeffs<double>(P, sh, mp, w.v(P.nused - 1, b) * K_RHORI, w.numc[b]);
+  } else {
+    sh.alpha = sh.beta = sh.gamma = sh.sigma = 0.;
+  }
+}
+
+// Collision properties of bin b (diam == dwet: dnsp equals it after a limited "all" update)
+template <int LS>
+__device__ __forceinline__ void props_of_bin(const DevParams &P, const WS<float, LS> &w, const KCell<float> &k, int b,
+                                             const Shape<double> &sh, BinProps<float> &o) {
+  const int ph = phase_of(P, b);
+  const double diam = w.dwet[b];
+  if (ph < 4) {
+    // the mixed form evaluates the per-bin properties of the liquid bins in float as
+    // well; ice keeps FP64 (the Khvorostyanov-Curry fall speed carries float rounding
+    // of its exponents into ice-drop speed differences, which cancel)
+    const float df = (float)diam;
+    const float mass = (float)w.rhomean[b] * (float)K_PI6 * cube(df);
+    const Shape<float> shf = {0.f, 0.f, 0.f, 0.f};
+    bin_props<float>(k.cc, ph, df, df, mass, (float)w.rhomean[b], shf, o);
+    return;
+  }
+  BinProps<double> od;
+  bin_props<double>(k.cd, ph, diam, diam, w.rhomean[b] * K_PI6 * cube(diam), w.rhomean[b], sh, od);
+  to_float(od, o);
+}
+template <int LS>
+__device__ __forceinline__ void props_of_bin(const DevParams &P, const WS<double, LS> &w, const KCell<double> &k, int b,
+                                             const Shape<double> &sh, PairProps &o) {
+  const double d = w.dwet[b], rho = w.rhomean[b], rd = drcp(d);
+  const double im = rd * rd * rd * (phase_of(P, b) < 4 ? 1. / (K_RHOWA * K_PI6) : drcp(rho * K_PI6));
+  pair_props(k, phase_of(P, b), d, rd, im, d, rho, sh, o);
+}
+// Properties of the first particle of a pair of equal-size bins (i, j), the self-coagulation
+// offset (:273-276): 1.1 times the diameter and 1.33 times the mass of particle 2; sh is bin
+// i's shape.  For liquid bins they depend on bin j alone: the fall speed takes the same
+// branch for every liquid phase, every liquid density is that of water and the
+// sphere-equivalent diameter enters only for ice.
+template <int LS>
+__device__ __forceinline__ void offset_props(const DevParams &P, const WS<float, LS> &w, const KCell<float> &k,
+                                             const Shape<double> &sh, int i, int j, BinProps<float> &a) {
+  if (phase_of(P, i) < 4) {
+    const float dj = (float)w.dwet[j], mj = (float)w.rhomean[j] * (float)K_PI6 * cube(dj);
+    const Shape<float> shf = {0.f, 0.f, 0.f, 0.f};
+    bin_props<float>(k.cc, phase_of(P, i), 1.1f * dj, (float)w.dwet[i], 1.33f * mj, (float)w.rhomean[i], shf, a);
+    return;
   }
   const double dj = w.dwet[j], mj = w.rhomean[j] * K_PI6 * cube(dj);
   BinProps<double> ad;
-  bin_props<double>(cd, phase_of(P, i), 1.1 * dj, w.dwet[i], 1.33 * mj, w.rhomean[i], sh, ad);
-  to_kt<KT>(ad, a);
+  bin_props<double>(k.cd, phase_of(P, i), 1.1 * dj, w.dwet[i], 1.33 * mj, w.rhomean[i], sh, ad);
+  to_float(ad, a);
+}
+template <int LS>
+__device__ __forceinline__ void offset_props(const DevParams &P, const WS<double, LS> &w, const KCell<double> &k,
+                                             const Shape<double> &sh, int i, int j, PairProps &a) {
+  const double dj = w.dwet[j], rdj = drcp(dj);
+  const double im = rdj * rdj * rdj *
+                    (phase_of(P, j) < 4 ? 1. / (1.33 * K_RHOWA * K_PI6) : drcp(1.33 * K_PI6 * w.rhomean[j]));
+  pair_props(k, phase_of(P, i), 1.1 * dj, (1. / 1.1) * rdj, im, w.dwet[i], w.rhomean[i], sh, a);
+}
+__device__ __forceinline__ float pair_kernel(const KCell<float> &k, const BinProps<float> &a, const BinProps<float> &b) {
+  return coag_pair<float>(k.cc, a, b);
 }
 
 // charging enhancement (:411-416)
@@ -459,95 +626,42 @@ __device__ __forceinline__ KT charged(const DevParams &P, const WS<KT, LS> &w, K
 }
 
 template <typename KT, bool OFFSET>
-__device__ void eval_pairs(const DevParams &P, const WS<KT, 32> &w, const CoagCell<KT> &cc, const CoagCell<double> &cd,
-                           const KT *S, const int *list, int n, int lane) {
+__device__ void eval_pairs(const DevParams &P, const WS<KT, 32> &w, const KCell<KT> &kc, const KT *S, const int *list,
+                           int n, int lane) {
   const int NB = w.NB;
   if (lane < n) {
     int q = list[lane];
     int i = q & 0xff, j = (q >> 8) & 0xff;
-    BinProps<KT> a, b;
+    KProps<KT> a, b;
     load_props<KT>(S, NB, j, b);
     if (OFFSET) {
-      const double *SH = shape_rows(w);
       Shape<double> sh;
-      sh.alpha = SH[0 * NB + i]; sh.beta = SH[1 * NB + i]; sh.gamma = SH[2 * NB + i]; sh.sigma = SH[3 * NB + i];
-      offset_props(P, w, cc, cd, sh, i, j, a);
+      shape_of_bin(P, w, i, sh);
+      offset_props(P, w, kc, sh, i, j, a);
     } else {
       load_props<KT>(S, NB, i, a);
     }
-    w.K[tri(i, j, NB)] = charged(P, w, coag_pair<KT>(cc, a, b), i, j);
+    w.K[tri(i, j, NB)] = charged(P, w, pair_kernel(kc, a, b), i, j);
   }
-}
-
-// shape coefficients and collision properties of bin b, in the kernel type
-template <typename KT, int LS>
-__device__ __forceinline__ void props_of_bin(const DevParams &P, const WS<KT, LS> &w, const CoagCell<KT> &cc,
-                                             const CoagCell<double> &cd, int b, Shape<double> &sh, BinProps<KT> &o) {
-  const int ph = phase_of(P, b);
-  if (ph == 4) {
-    double mp = 0.;
-    for (int s = 0; s < P.nused - 1; s++) mp += w.v(s, b) * K_RHOIC;
-    shape_coeffs<double>(P, sh, mp, w.v(P.nused - 1, b) * K_RHORI, w.numc[b]);
-  } else {
-    sh.alpha = sh.beta = sh.gamma = sh.sigma = 0.;
-  }
-  const double diam = w.dwet[b];   // dnsp == dwet after a limited "all" update
-  if constexpr (sizeof(KT) == 4) {
-    if (ph < 4) {
-      // the mixed form evaluates the per-bin properties of the liquid bins in float as
-      // well; ice keeps FP64 (the Khvorostyanov-Curry fall speed carries float rounding
-      // of its exponents into ice-drop speed differences, which cancel)
-      const float df = (float)diam;
-      const float mass = (float)w.rhomean[b] * (float)K_PI6 * cube(df);
-      Shape<float> shf;
-      shf.alpha = (float)sh.alpha; shf.beta = (float)sh.beta; shf.gamma = (float)sh.gamma; shf.sigma = (float)sh.sigma;
-      bin_props<float>(cc, ph, df, df, mass, (float)w.rhomean[b], shf, o);
-      return;
-    }
-  }
-  const double mass = w.rhomean[b] * K_PI6 * cube(diam);
-  BinProps<double> od;
-  bin_props<double>(cd, ph, diam, diam, mass, w.rhomean[b], sh, od);
-  to_kt<KT>(od, o);
 }
 
 // ----------------------------------------------------------------------------------------
 // Collision kernels for all enabled bin pairs: mo_salsa_coagulation_kernels.f90:24-180
 // (buildKernelSelf/buildKernel: pairs whose partner has numc < nlim are zero).
-// Scratch: the nine BinProps rows (diam fre cschm dfpart mtvel2 omega termv reyn ire), then
-// the FP64 shape coefficients (shape_rows).
+// Scratch: the rows of the bins' properties (KForm<KT>::NROW of them).
 // ----------------------------------------------------------------------------------------
-// per-cell constants of the collision kernel
-template <typename KT>
-__device__ __forceinline__ void coag_cells(const DevParams &P, double T, double pres, CoagCell<double> &cd,
-                                           CoagCell<KT> &cc) {
-  {
-    double visc = ddiv(7.44523e-3 * dsqrt(cube(T)), 5093. * (T + 110.4));
-    double mfp = ddiv((1.656e-10 * T + 1.828e-8) * K_PSTAND, pres);
-    double zrhoa = ddiv(pres, K_RD * T);
-    double vkin = ddiv(visc, zrhoa);
-    cd.T_ = T; cd.visc = visc; cd.mfp = mfp; cd.zrhoa = zrhoa; cd.vkin = vkin;
-    cd.shearA = dsqrt(ddiv(8. * K_PI * P.eddy_dis, 15. * vkin));
-    cd.turbB = ddiv(K_PI * dpow(P.eddy_dis, 0.75), K_GRAV * dsqrt(dsqrt(vkin)));
-  }
-  cc.T_ = (KT)cd.T_; cc.visc = (KT)cd.visc; cc.mfp = (KT)cd.mfp; cc.zrhoa = (KT)cd.zrhoa; cc.vkin = (KT)cd.vkin;
-  cc.shearA = (KT)cd.shearA; cc.turbB = (KT)cd.turbB;
-}
-
 template <typename KT>
 __device__ __forceinline__ void build_kernels(const DevParams &P, const WS<KT, 32> &w, double T, double pres, int lane) {
   const int NB = w.NB;
-  CoagCell<double> cd;
-  CoagCell<KT> cc;
-  coag_cells<KT>(P, T, pres, cd, cc);
-  KT *S = reinterpret_cast<KT *>(w.scr);   // KT-typed scratch, 9 * NB entries
-  double *SH = shape_rows(w);
+  KCell<KT> kc;
+  kcell(P, T, pres, kc);
+  KT *S = reinterpret_cast<KT *>(w.scr);   // KT-typed scratch, NROW * NB entries
   // per-bin properties of the populated bins only (a pair with an empty bin has K = 0)
   const unsigned lt = (1u << lane) - 1u;
   int nact = 0;
   for (int base = 0; base < P.ntotal; base += 32) {
     int b = base + lane;
-    bool act = b < P.ntotal && w.numc[b] >= nlim_of(phase_of(P, b));
+    bool act = b < P.ntotal && num_ge(w.numc[b], nlim_of(phase_of(P, b)));
     unsigned bal = __ballot_sync(0xffffffffu, act);
     if (act) w.pbuf[nact + __popc(bal & lt)] = b;
     nact += __popc(bal);
@@ -556,10 +670,10 @@ __device__ __forceinline__ void build_kernels(const DevParams &P, const WS<KT, 3
   for (int e = lane; e < nact; e += 32) {
     const int b = w.pbuf[e];
     Shape<double> sh;
-    BinProps<KT> o;
-    props_of_bin(P, w, cc, cd, b, sh, o);
-    store_props_kt<KT>(S, NB, b, o);
-    SH[0 * NB + b] = sh.alpha; SH[1 * NB + b] = sh.beta; SH[2 * NB + b] = sh.gamma; SH[3 * NB + b] = sh.sigma;
+    KProps<KT> o;
+    shape_of_bin(P, w, b, sh);
+    props_of_bin(P, w, kc, b, sh, o);
+    store_props<KT>(S, NB, b, o);
   }
   __syncwarp();
   // Scan the pair table, compact the active pairs into pbuf and evaluate them 32 at a
@@ -575,7 +689,7 @@ __device__ __forceinline__ void build_kernels(const DevParams &P, const WS<KT, 3
       if (t < p1) {
         pk = __ldg(P.pairs + t);
         int i = pk & 0xff, j = (pk >> 8) & 0xff;
-        act = w.numc[i] >= nlim_of(phase_of(P, i)) && w.numc[j] >= nlim_of(phase_of(P, j));
+        act = num_ge(w.numc[i], nlim_of(phase_of(P, i))) && num_ge(w.numc[j], nlim_of(phase_of(P, j)));
         if (!act) w.K[tri(i, j, NB)] = (KT)0;
       }
       unsigned bal = __ballot_sync(0xffffffffu, act);
@@ -583,15 +697,15 @@ __device__ __forceinline__ void build_kernels(const DevParams &P, const WS<KT, 3
       nbuf += __popc(bal);
       __syncwarp();
       if (nbuf >= 32) {
-        if (sec == 0) eval_pairs<KT, false>(P, w, cc, cd, S, w.pbuf + nbuf - 32, 32, lane);
-        else eval_pairs<KT, true>(P, w, cc, cd, S, w.pbuf + nbuf - 32, 32, lane);
+        if (sec == 0) eval_pairs<KT, false>(P, w, kc, S, w.pbuf + nbuf - 32, 32, lane);
+        else eval_pairs<KT, true>(P, w, kc, S, w.pbuf + nbuf - 32, 32, lane);
         nbuf -= 32;
         __syncwarp();
       }
     }
     if (nbuf > 0) {
-      if (sec == 0) eval_pairs<KT, false>(P, w, cc, cd, S, w.pbuf, nbuf, lane);
-      else eval_pairs<KT, true>(P, w, cc, cd, S, w.pbuf, nbuf, lane);
+      if (sec == 0) eval_pairs<KT, false>(P, w, kc, S, w.pbuf, nbuf, lane);
+      else eval_pairs<KT, true>(P, w, kc, S, w.pbuf, nbuf, lane);
     }
     __syncwarp();
   }
@@ -605,26 +719,24 @@ __device__ __forceinline__ void build_kernels(const DevParams &P, const WS<KT, 3
 template <typename KT>
 __device__ __forceinline__ void build_kernels(const DevParams &P, const WS<KT, 1> &w, double T, double pres, int) {
   const int NB = w.NB;
-  CoagCell<double> cd;
-  CoagCell<KT> cc;
-  coag_cells<KT>(P, T, pres, cd, cc);
+  KCell<KT> kc;
+  kcell(P, T, pres, kc);
   const Col<KT> S = row_cast<KT>(w.scr);
-  const Col<double> SH = shape_rows(w);
   const bool eq = P.npairs > P.npairs_plain;
   for (int b = 0; b < P.ntotal; b++) {
-    if (!w.on(b) || !(w.numc[b] >= nlim_of(phase_of(P, b)))) continue;
+    if (!w.on(b) || !(num_ge(w.numc[b], nlim_of(phase_of(P, b))))) continue;
     Shape<double> sh;
-    BinProps<KT> o;
-    props_of_bin(P, w, cc, cd, b, sh, o);
-    store_props_kt<KT>(S, NB, b, o);
-    SH[0 * NB + b] = sh.alpha; SH[1 * NB + b] = sh.beta; SH[2 * NB + b] = sh.gamma; SH[3 * NB + b] = sh.sigma;
+    KProps<KT> o;
+    shape_of_bin(P, w, b, sh);
+    props_of_bin(P, w, kc, b, sh, o);
+    store_props<KT>(S, NB, b, o);
     if (eq) {
-      BinProps<KT> a;
-      offset_props(P, w, cc, cd, sh, b, b, a);
-      w.K[tri(b, b, NB)] = coag_pair<KT>(cc, a, o);
+      KProps<KT> a;
+      offset_props(P, w, kc, sh, b, b, a);
+      w.K[tri(b, b, NB)] = pair_kernel(kc, a, o);
     }
   }
-  BinProps<KT> a;
+  KProps<KT> a;
   int ia = -1;
   for (int t = 0; t < P.npairs; t++) {
     const int pk = __ldg(P.pairs + t), i = pk & 0xff, j = (pk >> 8) & 0xff, ij = tri(i, j, NB);
@@ -632,23 +744,26 @@ __device__ __forceinline__ void build_kernels(const DevParams &P, const WS<KT, 1
       if (P.kc_mode == 1) w.K[ij] = (KT)0;   // the stored triangle; no sum reads it here
       continue;
     }
+    if (t < P.npairs_plain && i != ia) {
+      load_props<KT>(S, NB, i, a);   // every lane, whether its bin i is populated or not
+      ia = i;
+    }
     KT k = (KT)0;
-    if (w.numc[i] >= nlim_of(phase_of(P, i)) && w.numc[j] >= nlim_of(phase_of(P, j))) {
+    if (num_ge(w.numc[i], nlim_of(phase_of(P, i))) && num_ge(w.numc[j], nlim_of(phase_of(P, j)))) {
       if (t < P.npairs_plain) {
-        BinProps<KT> b;
+        KProps<KT> b;
         load_props<KT>(S, NB, j, b);
-        if (i != ia) load_props<KT>(S, NB, i, a);
-        k = coag_pair<KT>(cc, a, b);
+        k = pair_kernel(kc, a, b);
       } else if (i == j || phase_of(P, j) < 4) {
         k = w.K[tri(j, j, NB)];   // pairs (i, j) come before (j, j), which is charged last
       } else {
         // a drop and a crystal bin of the same size
         Shape<double> sh;
-        sh.alpha = SH[0 * NB + i]; sh.beta = SH[1 * NB + i]; sh.gamma = SH[2 * NB + i]; sh.sigma = SH[3 * NB + i];
-        BinProps<KT> c, b;
+        shape_of_bin(P, w, i, sh);
+        KProps<KT> c, b;
         load_props<KT>(S, NB, j, b);
-        offset_props(P, w, cc, cd, sh, i, j, c);
-        k = coag_pair<KT>(cc, c, b);
+        offset_props(P, w, kc, sh, i, j, c);
+        k = pair_kernel(kc, c, b);
       }
       k = charged(P, w, k, i, j);
     }
@@ -1480,7 +1595,7 @@ __device__ void coag_aero(const DevParams &P, const WS<KT, LS> &w, const double 
   const int nspec = P.nwet;
   const int16_t *L = partner_lists(P, tb);
   for (int kk = P.in1a; kk <= P.fn2b; kk++) {
-    if (w.numc[kk] < K_NLIM) continue;
+    if (num_lt(w.numc[kk], K_NLIM)) continue;
     TAccT<KT, LS> a;
     a.zero();
     if (P.lscgaa && lane == 0) a.self = (KT)0.5 * kget(w, kk, kk) * w.nk(kk);
@@ -1627,7 +1742,7 @@ __device__ void coag_cloud(const DevParams &P, const WS<KT, LS> &w, const double
     int o_last = reg == 0 ? P.fcb_cur : P.fca_cur;
     for (int kk = kfirst; kk <= klast; kk++) {
       int tg = C0 + kk;
-      if (w.numc[tg] < K_NLIM) continue;
+      if (num_lt(w.numc[tg], K_NLIM)) continue;
       TAccT<KT, LS> a;
       a.zero();
       if (autoc1) {
@@ -1733,7 +1848,7 @@ __device__ void coag_precp(const DevParams &P, const WS<KT, LS> &w, const double
   const int16_t *L = partner_lists(P, tb);
   for (int kk = 0; kk < nprc; kk++) {
     int tg = P0 + kk;
-    if (w.numc[tg] < K_PRLIM) continue;
+    if (num_lt(w.numc[tg], K_PRLIM)) continue;
     TAccT<KT, LS> a;
     a.zero();
     double num_slf = 0.;
@@ -1854,7 +1969,7 @@ __device__ void coag_ice(const DevParams &P, const WS<KT, LS> &w, const double *
   (void)C0; (void)P0; (void)tb;
   for (int kk = 0; kk < nice; kk++) {
     int tg = I0 + kk;
-    if (w.numc[tg] < K_PRLIM) continue;
+    if (num_lt(w.numc[tg], K_PRLIM)) continue;
     TAccT<KT, LS> a;
     a.zero();
     double rf_t = rimefrac(P, w.numc[tg], w.v(iwa, tg), w.v(irim, tg), 4);
@@ -1950,7 +2065,7 @@ __device__ __forceinline__ void mark_populated(const DevParams &P, WS<KT, 1> &w)
 #pragma unroll
   for (int k = 0; k < 3; k++)
     for (int b = 32 * k; b < min(P.ntotal, 32 * k + 32); b++)
-      if (P.kc_mode == 2 || w.numc[b] >= nlim_of(phase_of(P, b))) m[k] |= 1u << (b - 32 * k);
+      if (P.kc_mode == 2 || num_ge(w.numc[b], nlim_of(phase_of(P, b)))) m[k] |= 1u << (b - 32 * k);
   __syncwarp();
 #pragma unroll
   for (int k = 0; k < 3; k++) m[k] = __reduce_or_sync(0xffffffffu, m[k]);
@@ -2004,9 +2119,10 @@ __device__ __forceinline__ void coagulation(const DevParams &P, WS<KT, LS> &w, c
   if (any_cloud) coag_cloud<KT, SIP>(P, w, tb, dt, diag, lane);
   bool neg = false;
   for (int b = lane; b < P.ntotal; b += LS) {
-    if (w.numc[b] < -1.e-6) neg = true;
-    w.numc[b] = fmax(0., w.numc[b]);
-    for (int s = 0; s < P.nused; s++) w.v(s, b) = fmax(0., w.v(s, b));
+    const double n = w.numc[b];
+    if (num_gt(-n, 1.e-6)) neg = true;
+    w.numc[b] = pos_part(n);
+    for (int s = 0; s < P.nused; s++) w.v(s, b) = pos_part(w.v(s, b));
   }
   if (wany<LS>(neg) && lane == 0) w.misc[M_FLAGS + F_NEG] = 1.;
   wsync<LS>();
@@ -2069,7 +2185,7 @@ struct EqJob {
   int kk, count;
   bool r2;
   double tol, zrh, izke, numc, zv0, zv1, zv4, zvp56, zcore, zdwet, zdold, zlwc;
-  double q0, q1, q4, p56, pc, rinv;   // per-bin invariants of the iteration, computed once
+  double q0, q1, q4, ppc, rinv;   // per-bin invariants of the iteration, computed once
 };
 
 template <typename KT, int LS>
@@ -2085,10 +2201,9 @@ __device__ __forceinline__ void eq_load(const DevParams &P, const WS<KT, LS> &w,
   {
     const double rhosu_msu = 1830. / 98.08e-3, rhooc_moc = 1400. / 150.e-3, rhoss_mss = 2165. / 58.44e-3;
     j.q0 = j.zv0 * rhosu_msu;
-    j.q1 = K_EPSOC * j.zv1 * rhooc_moc;
+    j.q1 = K_EPSOC * j.zv1 * rhooc_moc * K_MWA;
     j.q4 = j.zv4 * rhoss_mss;
-    j.p56 = divc(j.zvp56, K_PI6);
-    j.pc = divc(j.zcore, K_PI6);
+    j.ppc = divc(j.zvp56, K_PI6) + divc(j.zcore, K_PI6);
     j.rinv = drcp(j.numc * (K_RHOWA * K_PI6));   // zlwc / numc / rhowa / pi6 as one product
   }
   j.zdwet = w.dwet[b];
@@ -2096,26 +2211,30 @@ __device__ __forceinline__ void eq_load(const DevParams &P, const WS<KT, LS> &w,
   j.zlwc = 0.;
 }
 
-// one pass of the equil_iterate loop body (mo_salsa_properties.f90:196-230, :305-340).
-// FP64 divisions are the scarce resource here, so the pass takes three instead of ten:
-// the molality quotients share one denominator, the per-bin factor 1/(numc rhowa pi6)
-// and c = 2 sigma v_w / kT are computed once, and 1/zke = exp(-c/dwet) is carried.
-// The values move by an ulp or so against the reference's operation order.
+// one pass of the equil_iterate loop body (mo_salsa_properties.f90:196-230, :305-340) in 32
+// FP64 operations: one division for the water content and one for the Kelvin exponent.  The
+// molality quotients share one denominator, with 1/bm2 = aw M/(1 - aw) for
+// bm2 = 1/(aw M) - 1/M; the factor 1/(numc rhowa pi6) and c = 2 sigma v_w / kT are computed
+// once, and 1/zke = exp(-c/dwet) is carried.  The values move by an ulp or so against the
+// reference's operation order.  UNI: the lanes are all in one regime (lane form); the warp
+// form runs regime 1a as regime 2 with bm5 = 1 and no sea salt, on the same code.
+template <bool UNI>
 __device__ __forceinline__ void eq_step(EqJob &j, double ckt) {
-  j.zdold = fmax(j.zdwet, 1.e-20);
-  double zaw = j.zrh * j.izke;
-  double a2 = zaw * zaw, a3 = a2 * zaw, a4 = a2 * a2;
-  double bm1 = +1.1065495e+2 - 3.6759197e+2 * zaw + 5.0462934e+2 * a2 - 3.1543839e+2 * a3 + 6.770824e+1 * a4;
-  double bm2 = drcp(zaw * K_MWA) - 1. / K_MWA;
-  // regime 1a is the same sum with bm5 = 1 and no sea salt term (one code path for the
-  // 1a lane and the regime-2 lanes; explicit fmas so the gradient harness's copy of the
-  // 1a iteration rounds the same)
-  double bm5 = +5.875248e+1 - 1.8781997e+2 * zaw + 2.7211377e+2 * a2 - 1.8458287e+2 * a3 + 4.153689e+1 * a4;
-  bm5 = j.r2 ? bm5 : 1.;
-  const double q4 = j.r2 ? j.q4 : 0.;
-  const double zlwc = ddiv(fma(q4, bm1 * bm2, fma(j.q1, bm1 * bm5, j.q0 * (bm2 * bm5))), bm1 * bm2 * bm5);
-  j.zlwc = zlwc;
-  j.zdwet = dcbrt(fma(zlwc, j.rinv, j.p56) + j.pc);
+  j.zdold = max_pos(1.e-20, j.zdwet);
+  const double zaw = j.zrh * j.izke;
+  const double bm1 = fma(fma(fma(fma(6.770824e+1, zaw, -3.1543839e+2), zaw, 5.0462934e+2), zaw, -3.6759197e+2), zaw,
+                         1.1065495e+2);
+  const double b2 = 1. - zaw;
+  if (UNI && !j.r2) {
+    j.zlwc = ddiv(fma(j.q1 * zaw, bm1, j.q0 * b2), bm1 * b2);
+  } else {
+    double bm5 = fma(fma(fma(fma(4.153689e+1, zaw, -1.8458287e+2), zaw, 2.7211377e+2), zaw, -1.8781997e+2), zaw,
+                     5.875248e+1);
+    if (!UNI) bm5 = j.r2 ? bm5 : 1.;
+    const double q4 = (UNI || j.r2) ? j.q4 : 0., b12 = bm1 * b2;
+    j.zlwc = ddiv(fma(q4, b12, fma(j.q1 * zaw, bm1 * bm5, j.q0 * (b2 * bm5))), b12 * bm5);
+  }
+  j.zdwet = dcbrt(fma(j.zlwc, j.rinv, j.ppc));
   j.izke = dexp(-(ddiv(ckt, j.zdwet)));
   j.count++;
 }
@@ -2191,7 +2310,7 @@ __device__ __forceinline__ void eq_step_f(EqJobF &j, float ckt) {
 template <typename KT, int LS>
 __device__ __forceinline__ int eq_next_1a(const DevParams &P, const WS<KT, LS> &w, const double *dmid, int b, bool init) {
   for (int k = b + 1; k <= P.fn1a; k++) {
-    if (w.numc[k] > K_NLIM) return k;
+    if (num_gt(w.numc[k], K_NLIM)) return k;
     if (init) w.dwet[k] = dmid[k];
   }
   return -1;
@@ -2222,7 +2341,7 @@ __device__ void equilibration(const DevParams &P, const WS<KT, LS> &w, const dou
         if (init) w.dwet[k] = (double)j.zdwet;
       }
       for (int k = P.in2a; k < P.in2a + n2; k++) {
-        if (!(w.numc[k] > K_NLIM)) { w.dwet[k] = dmid[k]; continue; }
+        if (!num_gt(w.numc[k], K_NLIM)) { w.dwet[k] = dmid[k]; continue; }
         j.r2 = true; j.tol = 1.e-6f; j.zrh = (float)zrh2; j.omrh = (float)(1. - zrh2); j.em = (float)(1. - 1. / 1.02);
         eq_load_f(P, w, k, j);
         while (fabsf(j.zdwet - j.zdold) > j.tol * j.zdold) {
@@ -2234,8 +2353,8 @@ __device__ void equilibration(const DevParams &P, const WS<KT, LS> &w, const dou
         eq_load(P, w, k, d);
         d.zdwet = (double)j.zdwet;
         d.izke = dexp(-(ddiv(ckt, d.zdwet)));
-        eq_step(d, ckt);
-        eq_step(d, ckt);
+        eq_step<true>(d, ckt);
+        eq_step<true>(d, ckt);
         w.v(P.iwa, k) = divc(d.zlwc, K_RHOWA);
         w.dwet[k] = d.zdwet;
       }
@@ -2246,18 +2365,18 @@ __device__ void equilibration(const DevParams &P, const WS<KT, LS> &w, const dou
         j.r2 = false; j.tol = 1.e-2; j.zrh = zrh1;
         eq_load(P, w, k, j);
         while (fabs(j.zdwet - j.zdold) > j.tol * j.zdold) {
-          eq_step(j, ckt);
+          eq_step<true>(j, ckt);
           if (j.count > 100) { nonconv = 1; break; }
         }
         w.v(P.iwa, k) = divc(j.zlwc, K_RHOWA);
         if (init) w.dwet[k] = j.zdwet;
       }
       for (int k = P.in2a; k < P.in2a + n2; k++) {
-        if (!(w.numc[k] > K_NLIM)) { w.dwet[k] = dmid[k]; continue; }
+        if (!num_gt(w.numc[k], K_NLIM)) { w.dwet[k] = dmid[k]; continue; }
         j.r2 = true; j.tol = 1.e-12; j.zrh = zrh2; j.izke = 1. / 1.02;
         eq_load(P, w, k, j);
         while (fabs(j.zdwet - j.zdold) > j.tol * j.zdold) {
-          eq_step(j, ckt);
+          eq_step<true>(j, ckt);
           if (j.count > 100) { nonconv = 1; break; }
         }
         w.v(P.iwa, k) = divc(j.zlwc, K_RHOWA);
@@ -2314,8 +2433,8 @@ __device__ void equilibration(const DevParams &P, const WS<KT, LS> &w, const dou
         eq_load(P, w, r2k, d);
         d.zdwet = (double)j.zdwet;
         d.izke = dexp(-(ddiv(ckt, d.zdwet)));
-        eq_step(d, ckt);
-        eq_step(d, ckt);
+        eq_step<false>(d, ckt);
+        eq_step<false>(d, ckt);
         w.v(P.iwa, r2k) = divc(d.zlwc, K_RHOWA);
         w.dwet[r2k] = d.zdwet;
       }
@@ -2342,7 +2461,7 @@ __device__ void equilibration(const DevParams &P, const WS<KT, LS> &w, const dou
       if (j.kk >= 0) {
         bool go = fabs(j.zdwet - j.zdold) > j.tol * j.zdold;   // |zdwet/zdold - 1| > tol, zdold > 0
         if (go) {
-          eq_step(j, ckt);
+          eq_step<false>(j, ckt);
           if (j.count > 100) { nonconv = 1; go = false; }
         }
         if (!go) {
@@ -2407,7 +2526,9 @@ __device__ __forceinline__ double solute_moles(const DevParams &P, const WS<KT, 
   }
   return zns;
 }
-__device__ __forceinline__ double acth2o_w(double znw, double zns) { return fmax(0.1, ddiv(znw, fmax(K_EPS, (znw + zns)))); }
+__device__ __forceinline__ double acth2o_w(double znw, double zns) {
+  return max_pos(0.1, ddiv(znw, max_pos(K_EPS, znw + zns)));
+}
 
 // ----------------------------------------------------------------------------------------
 // Gas condensation: mo_salsa_dynamics.f90:348-685 (condgas).  H2SO4 and the non- and
@@ -2603,10 +2724,11 @@ __device__ void gpparth2o(const DevParams &P, const WS<KT, LS> &w, const double 
   for (int b = lane; b < ntot; b += LS) {
     int ph = phase_of(P, b);
     double n = w.numc[b];
-    if (ph == 1) anyae |= n > K_NLIM;
-    else if (ph == 2) anycl |= n > K_NLIM;
-    else if (ph == 3) anypr |= n > K_PRLIM;
-    else anyic |= n > K_PRLIM;
+    const bool on = num_gt(n, nlim_of(ph));
+    if (ph == 1) anyae |= on;
+    else if (ph == 2) anycl |= on;
+    else if (ph == 3) anypr |= on;
+    else anyic |= on;
   }
   anyae = wany<LS>(anyae); anycl = wany<LS>(anycl); anypr = wany<LS>(anypr); anyic = wany<LS>(anyic);
   if (!((anycl || (anypr && P.lscndh2ocl)) || (anyic && P.lscndh2oic) || (anyae && zrh > 0.98 && P.lscndh2oae)))
@@ -2619,29 +2741,31 @@ __device__ void gpparth2o(const DevParams &P, const WS<KT, LS> &w, const double 
   const double zmfph2o = 3. * zdfh2o * dsqrt(ddiv(K_PI * K_MWA, 8. * K_RG * T));
   const double zthcond = 0.023807 + 7.1128e-5 * (T - 273.16);
   const int NB = w.NB;
-  const auto kel = w.sc(0), surf = w.sc(1), mt = w.sc(2), wsat = w.sc(3), cw = w.sc(4), zns = w.sc(5),
+  const auto kel = w.sc(0), amt = w.sc(1), mt = w.sc(2), wsat = w.sc(3), cw = w.sc(4), zns = w.sc(5),
              orgic = w.sc(6), orgri = w.sc(7);
   (void)NB;
+  const double sfl = divc(prs * rhoair, K_MWA), sfi = divc(prsi * rhoair, K_MWA);   // saturation, liquid and ice
+  const double adt = 2.e-2;                                                         // substep [s]
   // diameters and densities (:819-822), then per-bin coefficients (:826-955)
   for (int b = lane; b < ntot; b += LS) {
     updateDiameterAll(P, w, dmid, b);
     int ph = phase_of(P, b);
     w.rhomean[b] = rhomean_of(P, ph, w.numc[b], w.v(iwa, b), w.v(irim, b));
     double n = w.numc[b];
-    double k_ = 1., sf = 0., m = 0., ws = 0.;
+    double k_ = 1., m = 0., ws = 0.;
     double ns_ = (ph <= 3) ? solute_moles(P, w, b, kappa) : 0.;
     bool act;
-    if (ph == 1) act = n > K_NLIM && zrh > 0.98 && P.lscndh2oae;
-    else if (ph == 2) act = n > K_NLIM && P.lscndh2ocl;
-    else if (ph == 3) act = n > K_PRLIM && P.lscndh2ocl;
-    else act = n > K_PRLIM && P.lscndh2oic && T < 273.15;
+    if (ph == 1) act = zrh > 0.98 && P.lscndh2oae;
+    else if (ph <= 3) act = P.lscndh2ocl;
+    else act = P.lscndh2oic && T < 273.15;
+    act = act && num_gt(n, nlim_of(ph));
     if (act) {
       if (ph <= 3) {
         double dwet = w.dwet[b];
         double znw = ddiv(w.v(iwa, b) * P.rholiq[iwa], P.MM[iwa]);
         double zact = acth2o_w(znw, ns_);
         k_ = dexp(ddiv(4. * K_SURFW0 * K_MWA, K_RG * T * K_RHOWA * dwet));
-        sf = divc(prs * rhoair, K_MWA);
+        const double sf = sfl;
         ws = zact * k_;
         KT zknud = ddiv((KT)2. * (KT)zmfph2o, (KT)dwet);
         KT zbeta = ddiv(zknud + (KT)1., (KT)0.377 * zknud + (KT)1. + (KT)4. / ((KT)3. * (KT)1.) * (zknud + zknud * zknud));
@@ -2653,7 +2777,7 @@ __device__ void gpparth2o(const DevParams &P, const WS<KT, LS> &w, const double 
         double dwet = w.dnsp[b];
         double cap = 0.5 * dwet;
         k_ = dexp(ddiv(4. * K_SURFI0 * K_MWA, K_RG * T * K_RHOWA * dwet));
-        sf = divc(prsi * rhoair, K_MWA);
+        const double sf = sfi;
         ws = 1.0 * k_;
         KT zknud = ddiv((KT)2. * (KT)zmfph2o, (KT)dwet);
         KT zbeta = ddiv(zknud + (KT)1., (KT)0.377 * zknud + (KT)1. + (KT)4. / (KT)3. * (zknud + zknud * zknud));
@@ -2663,7 +2787,7 @@ __device__ void gpparth2o(const DevParams &P, const WS<KT, LS> &w, const double 
         m = (double)(ddiv(h1, h2 * h3 + (KT)1.));
       }
     }
-    kel[b] = k_; surf[b] = sf; mt[b] = m; wsat[b] = ws; zns[b] = ns_;
+    kel[b] = k_; amt[b] = adt * m; mt[b] = m; wsat[b] = ws; zns[b] = ns_;
     if (ph <= 3) {
       cw[b] = divc(w.v(iwa, b) * K_RHOWA, K_MWA);
       orgic[b] = orgri[b] = 0.;
@@ -2682,7 +2806,8 @@ __device__ void gpparth2o(const DevParams &P, const WS<KT, LS> &w, const double 
     for (int b = lane; b < ntot; b += LS) {
       int ph = phase_of(P, b);
       double n = w.numc[b];
-      if (ph == 1) a |= n > K_NLIM; else if (ph == 2) c |= n > K_NLIM; else if (ph == 3) p |= n > K_PRLIM; else i |= n > K_PRLIM;
+      const bool on = num_gt(n, nlim_of(ph));
+      if (ph == 1) a |= on; else if (ph == 2) c |= on; else if (ph == 3) p |= on; else i |= on;
     }
     upd_ae = wany<LS>(a) && zrh > 0.98; upd_cl = wany<LS>(c); upd_pr = wany<LS>(p); upd_ic = wany<LS>(i);
   }
@@ -2699,51 +2824,78 @@ __device__ void gpparth2o(const DevParams &P, const WS<KT, LS> &w, const double 
   // one and reduced together with its vapour sum: one paired butterfly of 5 adds
   // instead of two of 5.  Lane l holds bins l, l+32 (the same partial sums for both),
   // so the totals are those of two separate butterflies over those partial sums.
-  const double adt = 2.e-2;
   double spsum;
   if constexpr (LS == 1) {
     double unused;
     tree_sum2(ntot, [&](int b, bool first, double &x, double &) {
-      const double p = b >= P.in2a ? mt[b] * wsat[b] : 0.;
-      x = first ? p * surf[b] : fma(p, surf[b], x);
+      const double p = b >= P.in2a ? mt[b] * wsat[b] : 0., sf = b < I0 ? sfl : sfi;
+      x = first ? p * sf : fma(p, sf, x);
     }, spsum, unused);
   } else {
     double sp = 0.;
     for (int b = lane; b < ntot; b += LS)
-      if (b >= P.in2a) sp += mt[b] * wsat[b] * surf[b];
+      if (b >= P.in2a) sp += mt[b] * wsat[b] * (b < I0 ? sfl : sfi);
     spsum = warp_sum(sp);
   }
   while (ttot < dt) {
     double zhlp1 = zcwc + adt * spsum;
     double zhlp2 = 1. + adt * mtot;
     zcwint = fmin(ddiv(zhlp1, zhlp2), zcwtot);
-    auto substep_bin = [&](int b) {   // bin b through the substep; its water
-      int ph = phase_of(P, b);
-      double c = cw[b];
-      bool upd = (ph == 1) ? (upd_ae && b >= P.in2a) : (ph == 2 ? upd_cl : (ph == 3 ? upd_pr : upd_ic));
+    struct SubBin { double c, am, ws, zn, ke, m; };
+    auto load = [&](int b) -> SubBin { return {cw[b], amt[b], wsat[b], zns[b], kel[b], mt[b]}; };
+    auto substep_bin = [&](int b, SubBin &q) {   // bin b through the substep: water q.c and activity q.ws
+      const int ph = phase_of(P, b);
+      const bool upd = (ph == 1) ? (upd_ae && b >= P.in2a) : (ph == 2 ? upd_cl : (ph == 3 ? upd_pr : upd_ic));
       if (upd) {
-        double ci = c + fmin(fmax(adt * mt[b] * (zcwint - wsat[b] * surf[b]), -1.e-1 * c), 1.e-1 * c);
-        wsat[b] = (ph <= 3) ? acth2o_w(ci, zns[b]) * kel[b] : kel[b];
-        c = fmax(ci, 0.);
+        const double x = q.am * (zcwint - q.ws * (ph <= 3 ? sfl : sfi));
+        const double t = 1.e-1 * q.c;
+        const double ci = q.c + (__double2hiint(t) >= 0 ? limit_pos(x, t) : fmin(fmax(x, -t), t));
+        q.ws = (ph <= 3) ? acth2o_w(ci, q.zn) * q.ke : q.ke;
+        wsat[b] = q.ws;
+        q.c = pos_part(ci);
+        cw[b] = q.c;
       }
-      cw[b] = c;
-      return c;
     };
     if constexpr (LS == 1) {
-      double cs, sp;
-      tree_sum2(ntot, [&](int b, bool first, double &x, double &y) {
-        const double c = substep_bin(b);
-        x = first ? c : x + c;
-        const double p = b >= P.in2a ? mt[b] * wsat[b] : 0.;
-        y = first ? p * surf[b] : fma(p, surf[b], y);
-      }, cs, sp);
+      // tree_sum2's order, the next bin's values loaded ahead of the current bin's stores
+      double cs = 0., sp = 0., x4 = 0., y4 = 0., x3 = 0., y3 = 0., x2 = 0., y2 = 0., x1 = 0., y1 = 0., x0 = 0., y0 = 0.;
+      SubBin nx = load(0);
+      int have = 0;   // the bin in nx
+#pragma unroll 1
+      for (int k = 0; k < 32; k++) {
+        double x = 0., y = 0.;
+        const int l = (int)(__brev((unsigned)k) >> 27), ln = (int)(__brev((unsigned)k + 1u) >> 27);
+#pragma unroll 1
+        for (int b = l; b < ntot; b += 32) {
+          SubBin q = nx;
+          if (have != b) q = load(b);   // layouts of fewer than 32 bins leave some leaves empty
+          have = b + 32 < ntot ? b + 32 : ln;
+          if (have < ntot) nx = load(have);
+          substep_bin(b, q);
+          const double p = b >= P.in2a ? q.m * q.ws : 0., sf = b < I0 ? sfl : sfi;
+          x = b == l ? q.c : x + q.c;
+          y = b == l ? p * sf : fma(p, sf, y);
+        }
+        if (!(k & 1)) { x4 = x; y4 = y; continue; }
+        x = x4 + x; y = y4 + y;
+        if (!(k & 2)) { x3 = x; y3 = y; continue; }
+        x = x3 + x; y = y3 + y;
+        if (!(k & 4)) { x2 = x; y2 = y; continue; }
+        x = x2 + x; y = y2 + y;
+        if (!(k & 8)) { x1 = x; y1 = y; continue; }
+        x = x1 + x; y = y1 + y;
+        if (!(k & 16)) { x0 = x; y0 = y; continue; }
+        cs = x0 + x; sp = y0 + y;
+      }
       zcwint = zcwtot - cs;
       spsum = sp;
     } else {
       double cs = 0., sp = 0.;
       for (int b = lane; b < ntot; b += LS) {
-        cs += substep_bin(b);
-        if (b >= P.in2a) sp += mt[b] * wsat[b] * surf[b];
+        SubBin q = load(b);
+        substep_bin(b, q);
+        cs += q.c;
+        if (b >= P.in2a) sp += q.m * q.ws * (b < I0 ? sfl : sfi);
       }
       // lanes 0-15 reduce cs, lanes 16-31 reduce sp
       const bool hi = lane & 16;
@@ -2788,7 +2940,7 @@ __device__ void gpparth2o(const DevParams &P, const WS<KT, LS> &w, const double 
   for (int b = lane; b < ntot; b += LS) {
     int ph = phase_of(P, b);
     if (ph <= 3) {
-      double nv = fmax(0., divc(cw[b] * K_MWA, K_RHOWA));
+      double nv = pos_part(divc(cw[b] * K_MWA, K_RHOWA));
       double d = nv - w.v(iwa, b);
       if (ph == 1) dca += d; else if (ph == 2) dcc += d; else dcp += d;
       w.v(iwa, b) = nv;
@@ -2804,7 +2956,7 @@ __device__ void gpparth2o(const DevParams &P, const WS<KT, LS> &w, const double 
         w.v(irim, b) = w.v(irim, b) + divc(dvrime * K_MWA, K_RHORI);
       }
     }
-    if (w.numc[b] > nlim_of(ph)) w.rhomean[b] = rhomean_of(P, ph, w.numc[b], w.v(iwa, b), w.v(irim, b));
+    if (num_gt(w.numc[b], nlim_of(ph))) w.rhomean[b] = rhomean_of(P, ph, w.numc[b], w.v(iwa, b), w.v(irim, b));
   }
   if (diag) {
     dca = wsum<LS>(dca); dcc = wsum<LS>(dcc); dcp = wsum<LS>(dcp);
@@ -2889,7 +3041,7 @@ __device__ __forceinline__ void act_cloudbase(const DevParams &P, const WS<KT, L
       const double s_max = ddiv(s_eff, dsqrt(0.5 * dsqrt(cube(ddiv(khi, theta))) + dpow(ddiv(sq(s_eff), theta + 3. * khi), 0.75)));
       zdcstar = ddiv(2. * aa, 3. * s_max);
       for (int kk = in1a + lane; kk <= fn2b; kk += LS) {
-        if (w.numc[kk] < K_NLIM) continue;
+        if (num_lt(w.numc[kk], K_NLIM)) continue;
         const double nshi = ns[kk] * vrhi[kk];
         const double sil = dexp(dsqrt(ddiv(x, nshi))) - 1.;
         if (s_max < sil) continue;
@@ -3258,7 +3410,7 @@ __device__ double J_hf(double Tk, double Sw) {   // :335-371
 template <typename KT, int LS>
 __device__ double calc_sweq(const DevParams &P, const WS<KT, LS> &w, int b, double T, double kappa) {
   double n = w.numc[b];
-  if (n < nlim_of(phase_of(P, b))) return 0.;
+  if (num_lt(n, nlim_of(phase_of(P, b)))) return 0.;
   double vs = 0.;
   for (int s = 0; s < P.nused; s++) vs += w.v(s, b);
   double dwet = dcbrt(divc(ddiv(vs, n), K_PI6));
@@ -3346,14 +3498,24 @@ __device__ void ice_nucl_SE(const DevParams &P, const WS<KT, LS> &w, const doubl
   // pass A
   for (int kk = lane; kk < nl; kk += LS) {
     const auto st = stage + kk * 10;
-    for (int q = 0; q < 10; q++) st[q] = 0.;
     st[0] = -1.;
     const auto r = rec + kk * 8;
+    if constexpr (LS == 1) {
+      // no scheme can freeze this bin (dry aerosol with immersion freezing alone, empty bins)
+      const int ph = phase_of(P, kk);
+      const bool cnt = !(T > 273.15) && !num_lt(w.numc[kk], nlim_of(ph));
+      if (!((P.lsicehom && T < tmax_homog) || (cnt && ph > 1 && P.lsiceimm) || (cnt && ph == 1 && P.lsicedep))) {
+        r[R_FHOM] = 0.;
+        r[R_MODE] = 0.;
+        continue;
+      }
+    }
+    for (int q = 1; q < 10; q++) st[q] = 0.;
     updateDiameterAll(P, w, dmid, kk);
     const double dwet = w.dwet[kk], dins_ = w.ddry[kk];
     const double n = w.numc[kk];
     const int ph = phase_of(P, kk);
-    const bool countable = !(T > 273.15) && !(n < nlim_of(ph));
+    const bool countable = !(T > 273.15) && !num_lt(n, nlim_of(ph));
     const bool hom = dwet - dins_ > dmin && T < tmax_homog && P.lsicehom;
     const bool imm = P.lsiceimm && (ph == 2 || ph == 3) && (w.dins[kk] > dmin) && countable;
     const bool dep = P.lsicedep && (ph == 1 && ddiv(prv, prs) < 1.0) && (w.dwet[kk] - w.dins[kk] < dmin) &&
@@ -3445,18 +3607,34 @@ __device__ void ice_nucl_SE(const DevParams &P, const WS<KT, LS> &w, const doubl
   }
   // pass C: iceNucleation (:421-538)
   double dh = 0., dd = 0., di = 0.;
+  bool any0 = false;
   for (int kk = lane; kk < nl; kk += LS) {
     const auto st = stage + kk * 10;
     const auto r = rec + kk * 8;
     const double dwet = w.dwet[kk];
     const double n = w.numc[kk];
     const int ph = phase_of(P, kk);
+    if constexpr (LS == 1) {
+      if ((__double_as_longlong(r[R_MODE]) | __double_as_longlong(r[R_FHOM])) == 0) {
+        // nothing freezes: what is left of the update below are its limits, and an IN deficit
+        // of 0/0 -> 0 without dust
+        if (num_lt(n, nlim_of(ph))) continue;
+        double vins = 0.;
+        for (int k = 0; k < P.ninsoluble; k++) vins += w.v(P.ind_insoluble[k], kk);
+        if (num_lt(vins, minVin)) continue;
+        any0 = true;
+        w.indef[kk] = __double_as_longlong(w.v(idu, kk)) << 1 == 0 ? 0. : min_pos(pos_part(w.indef[kk]), 1.);
+        for (int s = 0; s < P.nwet; s++) w.v(s, kk) = pos_part(w.v(s, kk));
+        w.numc[kk] = pos_part(n);
+        continue;
+      }
+    }
     const double f_hom = r[R_FHOM];
     const double f_imm = r[R_MODE] == 1. ? r[R_FINT] : 0.;
     const double f_dep = r[R_MODE] == 2. ? r[R_FINT] : 0.;
     dh += mrn(n, f_hom); dd += mrn(n, f_dep); di += mrn(n, f_imm);
     double frac = fmax(0., fmin(0.99, f_imm + f_hom + f_dep - mrn((f_imm + f_dep), f_hom)));
-    if (n < nlim_of(ph)) continue;
+    if (num_lt(n, nlim_of(ph))) continue;
     double vins = 0.;
     for (int k = 0; k < P.ninsoluble; k++) vins += w.v(P.ind_insoluble[k], kk);
     if (vins < minVin) continue;
@@ -3503,7 +3681,14 @@ __device__ void ice_nucl_SE(const DevParams &P, const WS<KT, LS> &w, const doubl
       w.misc[M_DIAG + DG_ICEIMM] += di;
     }
   }
-  if (P.st_icenucl) ice_apply_staged(P, w, stage, nl, lane);
+  if (P.st_icenucl) {
+    ice_apply_staged(P, w, stage, nl, lane);
+    if (any0)
+      for (int g = P.nliquid; g < P.ntotal; g++) {
+        for (int s = 0; s < P.nused; s++) w.v(s, g) = pos_part(w.v(s, g));
+        w.numc[g] = pos_part(w.numc[g]);
+      }
+  }
 }
 
 // classic ice nucleation (mo_salsa_cloud_ice.f90:26-140 with calc_Jhet/Jdep/Jhf :146-291)
@@ -3700,7 +3885,7 @@ __device__ __forceinline__ void distr_bin(const DevParams &P, const double *tb, 
 #pragma unroll
   for (int s = 0; s < SALSA_NSV; s++) if (s < nsum) sd += v[s];
   if (CAT == DC_AERO) {
-    if (!(n > K_NLIM) || g == P.fn2a) return;
+    if (!num_gt(n, K_NLIM) || g == P.fn2a) return;
     const double zvpart = ddiv(sd, n);
     if (vlo[g] > zvpart) {
       if (g == P.in1a) return;
@@ -3735,7 +3920,7 @@ __device__ __forceinline__ void distr_bin(const DevParams &P, const double *tb, 
     return;
   }
   const double lim = (CAT == DC_CLOUD) ? K_NLIM : K_PRLIM;
-  if (!(n > lim) || (CAT == DC_CLOUD && !(sd > 1.e-30))) return;
+  if (!num_gt(n, lim) || (CAT == DC_CLOUD && !num_gt(sd, 1.e-30))) return;
   const double zvpart = ddiv(sd, n);
   const double zVrat = ddiv(vhi[g], vlo[g]);
   const double zVilo = ddiv(2. * zvpart, 1. + zVrat);
@@ -3930,6 +4115,102 @@ __device__ void distr_update(const DevParams &P, const WS<KT, LS> &w, const doub
 template <int LS> __device__ __forceinline__ void stage_sync() {
   if constexpr (LS == 1) { __syncwarp(); __syncthreads(); }
 }
+// ---- the lane form's unit conversion, straight between the fields and the workspace ----
+// x a and x a b, without FP64 products for the zeros of unpopulated bins (rounded as in the
+// warp form: the substeps magnify last-bit differences of the water)
+__device__ __forceinline__ double scaled(double x, double a) { return __double_as_longlong(x) == 0 ? 0. : x * a; }
+__device__ __forceinline__ double scaled(double x, double a, double b) {
+  return __double_as_longlong(x) == 0 ? 0. : x * a * b;
+}
+
+// (mo_salsa_driver.f90:196-283) the cell's bins in particles and volume per m3 of air
+template <typename KT>
+__device__ __forceinline__ void lane_unpack(const DevParams &P, const WS<KT, 1> &w, const double *dmid, double dn) {
+  int b0 = 0;
+#pragma unroll 1
+  for (int c = 0; c < 4; c++) {
+    const int nb = c == 0 ? P.nbins : (c == 1 ? P.ncld : (c == 2 ? P.nprc : P.nice));
+    const bool absent = c == 3 && P.level < 5;
+    const double *fn = absent ? nullptr : P.fin[FI_NAERO + c] + w.off;
+    const double *fi = c < 3 && P.raw_indef >= 0 ? P.fin[FI_INDEF] + w.off : nullptr;
+    const double *fc = c < 3 && P.fin[FI_CHARGE] ? P.fin[FI_CHARGE] + w.off : nullptr;
+#pragma unroll 4
+    for (int b = 0; b < nb; b++) {
+      const int g = b0 + b;
+      const double n = fn ? __ldg(fn + P.plane * b) : 0.;
+      const double d = fi ? __ldg(fi + P.plane * g) : 0.;
+      const double t = fc ? __ldg(fc + P.plane * g) : 0.;
+      w.dwet[g] = dmid[g];
+      w.ddry[g] = 0.;
+      w.dins[g] = 0.;
+      w.dnsp[g] = 0.;
+      w.numc[g] = scaled(n, dn);
+      w.indef[g] = d;
+      w.ctime[g] = t;
+    }
+    const int ns = absent ? 0 : (c == 3 ? P.nwet + 1 : P.nwet);
+    const double *fm = absent ? nullptr : P.fin[FI_MAERO + c] + w.off;
+#pragma unroll 1
+    for (int s = 0; s < P.nused; s++) {
+      const double irho = c < 3 ? P.irholiq[s] : (s < P.nwet ? P.irhoice[s] : 1. / K_RHORI);
+      const double *f = s < ns ? fm + P.plane * ((long long)s * nb) : nullptr;
+#pragma unroll 8
+      for (int b = 0; b < nb; b++) w.v(s, b0 + b) = f ? scaled(__ldg(f + P.plane * b), dn, irho) : 0.;
+    }
+    for (int b = 0; b < nb; b++) {
+      const int g = b0 + b;
+      w.rhomean[g] = absent ? 0. : rhomean_of(P, c + 1, w.numc[g], w.v(P.iwa, g), w.v(P.irim, g));
+    }
+    b0 += nb;
+  }
+}
+
+// (mo_salsa_driver.f90:310-349) tendencies (new - old) / dt into the fields, the IN deficit
+// and the charge times in place; returns whether a number is not finite
+template <typename KT>
+__device__ __forceinline__ bool lane_output(const DevParams &P, const WS<KT, 1> &w, double idn) {
+  const double dt = P.dt, idt = P.inv_dt != 0. ? P.inv_dt : drcp(dt);
+  auto add = [&](double *f, double x, double v, double rho) {   // f += (v rho / dn - x) / dt
+    if ((__double_as_longlong(v) | __double_as_longlong(x)) == 0 || !w.live) return;
+    const double d = (v * rho * idn) - x;
+    *f = *f + (P.inv_dt != 0. ? d * idt : ddiv_r(d, dt, idt));
+  };
+  bool bad = false;
+  int b0 = 0;
+#pragma unroll 1
+  for (int c = 0; c < 4; c++) {
+    const int nb = c == 0 ? P.nbins : (c == 1 ? P.ncld : (c == 2 ? P.nprc : P.nice));
+    if (c == 3 && P.level < 5) break;
+    const double *fn = P.fin[FI_NAERO + c] + w.off;
+    double *tn = P.fout[FO_NAEROT + c] + w.off;
+#pragma unroll 4
+    for (int b = 0; b < nb; b++) {
+      const double n = w.numc[b0 + b];
+      bad |= (__double_as_longlong(n) & FM_INF) == FM_INF;
+      add(tn + P.plane * b, __ldg(fn + P.plane * b), n, 1.);
+    }
+    const int ns = c == 3 ? P.nwet + 1 : P.nwet;
+    const double *fm = P.fin[FI_MAERO + c] + w.off;
+    double *tm = P.fout[FO_MAEROT + c] + w.off;
+#pragma unroll 1
+    for (int s = 0; s < ns; s++) {
+      const double rho = c < 3 ? P.rholiq[s] : (s < P.nwet ? P.rhoice[s] : K_RHORI);
+      const long long r = P.plane * ((long long)s * nb);
+#pragma unroll 4
+      for (int b = 0; b < nb; b++) add(tm + r + P.plane * b, __ldg(fm + r + P.plane * b), w.v(s, b0 + b), rho);
+    }
+    if (c < 3 && w.live) {
+      double *oi = P.raw_indef >= 0 ? P.fout[FO_INDEF] : nullptr, *oc = P.fout[FO_CHARGE];
+      for (int b = b0; b < b0 + nb; b++) {
+        if (oi) oi[w.off + P.plane * b] = w.indef[b];
+        if (oc) oc[w.off + P.plane * b] = w.ctime[b];
+      }
+    }
+    b0 += nb;
+  }
+  return bad;
+}
+
 template <typename KT, bool DIAG, bool SIP, int LS>
 __device__ __forceinline__ void cell_step(const DevParams &P, WS<KT, LS> &w, const double *tb, long long cell,
                                           int lane) {
@@ -3946,33 +4227,37 @@ __device__ __forceinline__ void cell_step(const DevParams &P, WS<KT, LS> &w, con
   const int nwet = P.nwet, irim = P.irim;
   const int bstart[4] = {0, P.nbins, P.nbins + P.ncld, P.nliquid};
   const int bnum[4] = {P.nbins, P.ncld, P.nprc, P.nice};
-  for (int b = lane; b < P.ntotal; b += LS) {
-    int icat = phase_of(P, b) - 1;
-    w.dwet[b] = dmid[b];
-    w.ddry[b] = w.dins[b] = w.dnsp[b] = 0.;
-    for (int s = 0; s < SALSA_NSV; s++) w.v(s, b) = 0.;
-    const bool absent = icat == 3 && P.level < 5;
-    w.numc[b] = absent ? 0. : raw[P.raw_num + b] * dn;
-    w.indef[b] = (!absent && icat < 3 && P.raw_indef >= 0) ? raw[P.raw_indef + b] : 0.;
-    w.ctime[b] = (!absent && icat < 3 && P.raw_charge >= 0) ? raw[P.raw_charge + b] : 0.;
-  }
-  wsync<LS>();
-  // mass rows of all categories, one lane per (category, species, bin) row
   const int ncat = P.level == 5 ? 4 : 3;
   const int m0 = P.raw_mbase[0];
   const int nmrow = (ncat == 4 ? P.raw_mbase[3] + (nwet + 1) * P.nice : P.raw_mbase[2] + nwet * P.nprc) - m0;
-  for (int e = lane; e < nmrow; e += LS) {
-    const int r = m0 + e;
-    const int icat = (ncat == 4 && r >= P.raw_mbase[3]) ? 3 : (r >= P.raw_mbase[2] ? 2 : (r >= P.raw_mbase[1] ? 1 : 0));
-    const int loc = r - P.raw_mbase[icat], nbc = bnum[icat];
-    const int sp = loc / nbc, b = bstart[icat] + (loc - sp * nbc);
-    const double irho = icat < 3 ? P.irholiq[sp] : (sp < nwet ? P.irhoice[sp] : 1. / K_RHORI);
-    w.v(sp, b) = raw[r] * dn * irho;
-  }
-  wsync<LS>();
-  for (int b = lane; b < P.ntotal; b += LS) {
-    int icat = phase_of(P, b) - 1;
-    w.rhomean[b] = (icat == 3 && P.level < 5) ? 0. : rhomean_of(P, icat + 1, w.numc[b], w.v(P.iwa, b), w.v(irim, b));
+  if constexpr (LS == 1) {
+    lane_unpack(P, w, dmid, dn);
+  } else {
+    for (int b = lane; b < P.ntotal; b += LS) {
+      int icat = phase_of(P, b) - 1;
+      w.dwet[b] = dmid[b];
+      w.ddry[b] = w.dins[b] = w.dnsp[b] = 0.;
+      for (int s = 0; s < SALSA_NSV; s++) w.v(s, b) = 0.;
+      const bool absent = icat == 3 && P.level < 5;
+      w.numc[b] = absent ? 0. : raw[P.raw_num + b] * dn;
+      w.indef[b] = (!absent && icat < 3 && P.raw_indef >= 0) ? raw[P.raw_indef + b] : 0.;
+      w.ctime[b] = (!absent && icat < 3 && P.raw_charge >= 0) ? raw[P.raw_charge + b] : 0.;
+    }
+    wsync<LS>();
+    // mass rows of all categories, one lane per (category, species, bin) row
+    for (int e = lane; e < nmrow; e += LS) {
+      const int r = m0 + e;
+      const int icat = (ncat == 4 && r >= P.raw_mbase[3]) ? 3 : (r >= P.raw_mbase[2] ? 2 : (r >= P.raw_mbase[1] ? 1 : 0));
+      const int loc = r - P.raw_mbase[icat], nbc = bnum[icat];
+      const int sp = loc / nbc, b = bstart[icat] + (loc - sp * nbc);
+      const double irho = icat < 3 ? P.irholiq[sp] : (sp < nwet ? P.irhoice[sp] : 1. / K_RHORI);
+      w.v(sp, b) = raw[r] * dn * irho;
+    }
+    wsync<LS>();
+    for (int b = lane; b < P.ntotal; b += LS) {
+      int icat = phase_of(P, b) - 1;
+      w.rhomean[b] = (icat == 3 && P.level < 5) ? 0. : rhomean_of(P, icat + 1, w.numc[b], w.v(P.iwa, b), w.v(irim, b));
+    }
   }
   for (int i = lane; i < M_PF; i += LS) w.misc[i] = 0.;
   wsync<LS>();
@@ -4040,30 +4325,34 @@ __device__ __forceinline__ void cell_step(const DevParams &P, WS<KT, LS> &w, con
   // product when dt is a power of two (then it is the same number)
   bool bad = false;
   const double idn = drcp(dn);
-  for (int e = lane; e < nmrow; e += LS) {
-    const int r = m0 + e;
-    const int icat = (ncat == 4 && r >= P.raw_mbase[3]) ? 3 : (r >= P.raw_mbase[2] ? 2 : (r >= P.raw_mbase[1] ? 1 : 0));
-    const int loc = r - P.raw_mbase[icat], nbc = bnum[icat];
-    const int sp = loc / nbc, b = bstart[icat] + (loc - sp * nbc);
-    const double rho = icat < 3 ? P.rholiq[sp] : (sp < nwet ? P.rhoice[sp] : K_RHORI);
-    const double d = (w.v(sp, b) * rho * idn) - raw[r];
-    raw[r] = P.inv_dt != 0. ? d * P.inv_dt : ddiv(d, dt);
-  }
-  for (int b = lane; b < P.ntotal; b += LS) {
-    int icat = phase_of(P, b) - 1;
-    if (icat == 3 && P.level < 5) continue;
-    if (icat < 3) {
-      if (P.raw_indef >= 0) raw[P.raw_indef + b] = w.indef[b];
-      if (P.raw_charge >= 0) raw[P.raw_charge + b] = w.ctime[b];
+  if constexpr (LS == 1) {
+    bad = lane_output(P, w, idn);
+  } else {
+    for (int e = lane; e < nmrow; e += LS) {
+      const int r = m0 + e;
+      const int icat = (ncat == 4 && r >= P.raw_mbase[3]) ? 3 : (r >= P.raw_mbase[2] ? 2 : (r >= P.raw_mbase[1] ? 1 : 0));
+      const int loc = r - P.raw_mbase[icat], nbc = bnum[icat];
+      const int sp = loc / nbc, b = bstart[icat] + (loc - sp * nbc);
+      const double rho = icat < 3 ? P.rholiq[sp] : (sp < nwet ? P.rhoice[sp] : K_RHORI);
+      const double d = (w.v(sp, b) * rho * idn) - raw[r];
+      raw[r] = P.inv_dt != 0. ? d * P.inv_dt : ddiv(d, dt);
     }
-    double &on = raw[P.raw_num + b];
-    const double d = (w.numc[b] * idn) - on;
-    on = P.inv_dt != 0. ? d * P.inv_dt : ddiv(d, dt);
-    bad |= !isfinite(w.numc[b]);
+    for (int b = lane; b < P.ntotal; b += LS) {
+      int icat = phase_of(P, b) - 1;
+      if (icat == 3 && P.level < 5) continue;
+      if (icat < 3) {
+        if (P.raw_indef >= 0) raw[P.raw_indef + b] = w.indef[b];
+        if (P.raw_charge >= 0) raw[P.raw_charge + b] = w.ctime[b];
+      }
+      double &on = raw[P.raw_num + b];
+      const double d = (w.numc[b] * idn) - on;
+      on = P.inv_dt != 0. ? d * P.inv_dt : ddiv(d, dt);
+      bad |= !isfinite(w.numc[b]);
+    }
   }
   // interstitial activation leaves the activated-droplet outputs at zero (:879, local pactd);
   // cloud-base activation has written them
-  if (!(P.st_activ && P.activ_mode == 2))
+  if (LS != 1 && !(P.st_activ && P.activ_mode == 2))
     for (int i = lane; i < P.ncld * (1 + nwet); i += LS) raw[P.raw_nact + i] = 0.;
   if (lane == 0) raw[RW_RV] = ddiv(rv - rv_old, dt);
   if constexpr (SIP) {
@@ -4198,10 +4487,10 @@ __global__ void __launch_bounds__(SALSA_THREADS, 2) salsa_step_kernel(const DevP
 // global memory, a slot per resident warp, interleaved by lane: HBM and L2 have bandwidth to
 // spare (they are 5-15 % busy).  Blocks take four tiles of 32 cells from a counter, the cloudy
 // end of the list first (its cells take several times as long as clear ones).
-// FP64 instructions per cell of grid384x384x160: 6,190 in the warp form, 1,300 here; a 1.1 M
-// cell block took 299 ms in the warp form, 105 ms here.  Four blocks of 128 threads per SM
-// (128 registers) measured better than two or three (clear cells 61.7, 69.4 and 66 ns a
-// cell): the FP64 pipe waits for memory less (67-78 % busy).
+// FP64 instructions per cell of grid384x384x160: 6,190 in the warp form, about 1,000 here; a
+// 1.1 M cell block takes 78 ms, where the warp form took 299 ms.  Four blocks of 128 threads
+// per SM (128 registers) measured better than three (164 registers): clear cells 39.3
+// against 43.9 ns a cell, cloudy ones 397 against 455; the FP64 pipe is 71-80 % busy.
 template <typename KT, bool DIAG, bool SIP>
 __global__ void __launch_bounds__(32 * SALSA_LANE_WARPS, SALSA_LANE_MINBLOCKS) salsa_lane_kernel(const DevParams P) {
   extern __shared__ double smem[];
@@ -4223,28 +4512,32 @@ __global__ void __launch_bounds__(32 * SALSA_LANE_WARPS, SALSA_LANE_MINBLOCKS) s
     // warps past the last tile repeat it
     const long long q = (ntiles - 1 - min(k, ntiles - 1)) * 32 + lane;
     w.live = k < ntiles && q < P.ncells;
-    const long long cell = cell_at(P, min(q, P.ncells - 1)), off = cell_offset(P, cell);
-    for (int r = 0; r < P.nrows; r++) {
-      const Row row = P.rows[r];
-      double v = 0.;
-      if (row.fin >= 0) {
-        const double *f = P.fin[row.fin];
-        if (f) v = __ldg(f + off + P.plane * row.idx);
+    const long long cell = cell_at(P, min(q, P.ncells - 1));
+    w.off = cell_offset(P, cell);
+    // thermodynamics, gases and tracers through the workspace; the bins in lane_unpack
+    auto stage = [&](int r0, int r1) {
+#pragma unroll 4
+      for (int r = r0; r < r1; r++) {
+        const Row row = P.rows[r];
+        const double *f = row.fin >= 0 ? P.fin[row.fin] : nullptr;
+        w.raw[r] = f ? __ldg(f + w.off + P.plane * row.idx) : 0.;
       }
-      w.raw[r] = v;
-    }
+    };
+    const bool nact0 = !(P.st_activ && P.activ_mode == 2);   // no activated droplets to report
+    stage(0, P.raw_num);
+    stage(nact0 ? P.raw_diag : P.raw_nact, P.nrows);
     cell_step<KT, DIAG, SIP>(P, w, tb, cell, 0);
     __syncwarp();
-    if (w.live)
-      for (int r = 0; r < P.nrows; r++) {
+    if (w.live) {
+      for (int r = 0; r < P.nrows; r = r + 1 == P.raw_num ? P.raw_nact : r + 1) {
         const Row row = P.rows[r];
-        if (row.fout < 0) continue;
-        double *f = P.fout[row.fout];
+        double *f = row.fout >= 0 ? P.fout[row.fout] : nullptr;
         if (!f) continue;
-        double *a = f + off + P.plane * row.idx;
-        if (row.mode == ROW_TEND) *a = *a + w.raw[r];
-        else *a = w.raw[r];
+        double *o = f + w.off + P.plane * row.idx;
+        const double v = nact0 && r >= P.raw_nact && r < P.raw_diag ? 0. : w.raw[r];
+        *o = row.mode == ROW_TEND ? *o + v : v;
       }
+    }
     const unsigned nlive = __popc(__ballot_sync(0xffffffffu, w.live));
     if (lane == 0) atomicAdd(P.status + ST_CELLS, (unsigned long long)nlive);
   }

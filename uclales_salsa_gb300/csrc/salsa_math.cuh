@@ -49,6 +49,7 @@ __device__ __forceinline__ float fm_ex2_32(float x) { float r; asm("ex2.approx.f
 #ifdef SALSA_MATH_PLAIN
 __device__ __forceinline__ double drcp(double d) { return 1. / d; }
 __device__ __forceinline__ double ddiv(double n, double d) { return n / d; }
+__device__ __forceinline__ double ddiv_r(double n, double d, double) { return n / d; }
 __device__ __forceinline__ double divc(double x, double c) { return x / c; }
 __device__ __forceinline__ double dsqrt(double x) { return sqrt(x); }
 __device__ __forceinline__ double dcbrt(double x) { return cbrt(x); }
