@@ -111,29 +111,41 @@ __device__ __forceinline__ void clamp_tendency(long long bp, long long bt, long 
   if (lo > __longlong_as_double(bt)) *tp = __double_as_longlong(lo);
 }
 
+// Two elements (16 bytes) per load where both arrays are 16-byte aligned, as allocations are
+// (the last element of an odd count, and arrays that are not, go one by one); B pairs per
+// thread and pass, loaded before any store.  HBM-bound: a 1.15 M point block takes 1.11 ms,
+// 5.7 TB/s (1.17 ms with four 8-byte loads, 1.30 with one pair in flight, 1.11 with four).
 __global__ void __launch_bounds__(256) tend_constrain_kernel(const ClampArgs A) {
   const long long stride = (long long)gridDim.x * blockDim.x;
   const long long i0 = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  constexpr int B = 4;   // elements per thread and pass, loaded before any store
+  constexpr int B = 2;
   for (int a = 0; a < 9; a++) {
     const long long *__restrict__ p = reinterpret_cast<const long long *>(A.p[a]);
     long long *__restrict__ t = reinterpret_cast<long long *>(A.t[a]);
     if (!p || !t) continue;
     const long long n = A.n[a];
-    for (long long e0 = i0; e0 < n; e0 += B * stride) {
-      long long vp[B], vt[B];
+    const bool al = ((reinterpret_cast<unsigned long long>(p) | reinterpret_cast<unsigned long long>(t)) & 15ull) == 0;
+    const long long n2 = al ? n >> 1 : 0;
+    const longlong2 *__restrict__ p2 = reinterpret_cast<const longlong2 *>(p);
+    const longlong2 *__restrict__ t2 = reinterpret_cast<const longlong2 *>(t);
+    for (long long e0 = i0; e0 < n2; e0 += B * stride) {
+      longlong2 vp[B], vt[B];
 #pragma unroll
       for (int u = 0; u < B; u++) {
-        const long long e = e0 + u * stride;
-        vp[u] = e < n ? __ldg(p + e) : 0LL;
-        vt[u] = e < n ? t[e] : 0LL;
+        const long long e = min(e0 + u * stride, n2 - 1);
+        vp[u] = __ldcs(p2 + e);
+        vt[u] = __ldcs(t2 + e);
       }
 #pragma unroll
       for (int u = 0; u < B; u++) {
         const long long e = e0 + u * stride;
-        if (e < n) clamp_tendency(vp[u], vt[u], t + e, A);
+        if (e < n2) {
+          clamp_tendency(vp[u].x, vt[u].x, t + 2 * e, A);
+          clamp_tendency(vp[u].y, vt[u].y, t + 2 * e + 1, A);
+        }
       }
     }
+    for (long long e = 2 * n2 + i0; e < n; e += stride) clamp_tendency(__ldg(p + e), t[e], t + e, A);
   }
   // the IN deficit to [0, 1] (MIN(MAX(v, 0), 1)), decided on the bits: NaN and v < 0
   // become 0, v > 1 becomes 1; -0 and values inside stay as they are
@@ -204,23 +216,172 @@ __device__ __forceinline__ void to_aerosol(const PostArgs &A, double *nh, double
   }
 }
 
-// negative values of n planes of one point to zero; the loads of a batch are issued
-// before any store, so they are in flight together
-__device__ __forceinline__ void clamp_neg(double *a, long long p, long long pl, int n) {
-  constexpr int B = 8;
-  for (int e0 = 0; e0 < n; e0 += B) {
-    double v[B];
-#pragma unroll
-    for (int u = 0; u < B; u++) v[u] = e0 + u < n ? a[p + pl * (e0 + u)] : 0.;
-#pragma unroll
-    for (int u = 0; u < B; u++)
-      if (neg_bits(bits_of(v[u]))) a[p + pl * (e0 + u)] = 0.;
+// ---- SALSA_diagnostics (:52-370) ----
+#define AT(arr, nb, s, b) (arr)[p + pl * ((long long)(s) * (nb) + (b))]
+
+// The steps that few points need (evaporating droplets, drops and ice, vanishing aerosol
+// bins), from and to memory in the reference's order.
+__device__ __noinline__ void evaporate_point(const PostArgs &A, long long p) {
+  const long long pl = A.plane;
+  const salsa_post_fields_t &f = A.f;
+  double *na = f.naero, *nc = f.ncloud, *np = f.nprecp, *ni = f.nice;
+  double *ma = f.maero, *mc = f.mcloud, *mp = f.mprecp, *mi = f.mice;
+  const int nbins = A.nbins, ncld = A.ncld, nprc = A.nprc, nice = A.nice, nspec = A.nspec;
+  const int iwa = A.iwa, irim = A.irim;
+  const bool lvl5 = A.level == 5;
+  const double massTH = 1.e-25;
+  const long long BITS_NLIM = bits_of(K_NLIM), BITS_PRLIM = bits_of(K_PRLIM);
+  const long long BITS_1EM5 = bits_of(1.e-5), BITS_1EM6 = bits_of(1.e-6), BITS_1EM15 = bits_of(1.e-15);
+  const double T = f.temp[p];
+  const bool dry = f.rh[p] < 0.999;
+  const double zaa = 4. * K_MWA * K_SURFW0 / (K_RG * K_RHOWA * T);
+  // evaporating cloud droplets: back to the parallel aerosol bin
+  for (int bc = A.ica_cur; bc <= A.fcb_cur; bc++) {
+    const double n_ = nc[p + pl * bc];
+    if (dry && gt_bits(bits_of(n_), BITS_NLIM) && lt_bits(bits_of(AT(mc, ncld, iwa, bc)), BITS_1EM5)) {
+      double ns = 0., zvol = 0.;
+      for (int s = 0; s < nspec - 1; s++) ns += A.diss[s] * AT(mc, ncld, s, bc) / A.MM[s];
+      ns = ns / n_;
+      const double zbb = 6. * K_MWA * ns / (K_PI * K_RHOWA);
+      const double cdcld = sqrt(3. * zbb / zaa);
+      for (int s = 0; s < nspec; s++) zvol += AT(mc, ncld, s, bc) / A.rholiq[s];
+      zvol = zvol / n_;
+      const double zdh2o = pow(zvol / K_PI6, 1. / 3.);
+      if (zdh2o < fmin(0.7 * cdcld, 1.3e-5) || AT(mc, ncld, iwa, bc) < massTH * n_) {
+        const int ba = bc <= A.fca_cur ? A.ica_par + (bc - A.ica_cur) : A.icb_par + (bc - A.icb_cur);
+        to_aerosol(A, nc, mc, ncld, bc, ba, p);
+        if (A.lcharge) f.chargeTime[p + pl * (nbins + bc)] = 0.;
+      }
+    }
+  }
+  // evaporating drops: to the aerosol bin of the closest dry size and composition
+  for (int bc = 0; bc < nprc; bc++) {
+    const double n_ = np[p + pl * bc];
+    if (dry && gt_bits(bits_of(n_), BITS_PRLIM) && lt_bits(bits_of(AT(mp, nprc, iwa, bc)), BITS_1EM6)) {
+      double ns = 0., zvol = 0.;
+      for (int s = 0; s < nspec - 1; s++) ns += A.diss[s] * AT(mp, nprc, s, bc) / A.MM[s];
+      ns = ns / n_;
+      const double zbb = 6. * K_MWA * ns / (K_PI * K_RHOWA);
+      const double cdprc = sqrt(3. * zbb / zaa);
+      for (int s = 0; s < nspec; s++) zvol += AT(mp, nprc, s, bc) / A.rholiq[s];
+      zvol = zvol / n_;
+      const double zdh2o = pow(zvol / K_PI6, 1. / 3.);
+      if (zdh2o < fmin(0.2 * cdprc, 10.e-6) || AT(mp, nprc, iwa, bc) < massTH * n_) {
+        const int ba = find_dry4wet(A, np, mp, nprc, bc, p);
+        to_aerosol(A, np, mp, nprc, bc, ba, p);
+        if (A.lcharge) f.chargeTime[p + pl * (nbins + ncld + bc)] = 0.;
+      }
+    }
+  }
+  // evaporating ice (rime goes to the aerosol water)
+  if (lvl5 && f.rhi[p] < 0.999)
+    for (int bc = 0; bc < nice; bc++) {
+      const double n_ = ni[p + pl * bc];
+      if (!gt_bits(bits_of(n_), BITS_PRLIM)) continue;
+      const double w_ = AT(mi, nice, iwa, bc), r_ = AT(mi, nice, irim, bc);
+      if (!lt_bits(bits_of(w_), BITS_1EM15) || !lt_bits(bits_of(r_), BITS_1EM15)) continue;
+      if (w_ + r_ < 1.e-15) {
+        double vt = 0.;
+        for (int s = 0; s < nspec + 1; s++) vt += AT(mi, nice, s, bc) / A.rhoice[s];
+        double cdice = vt / n_;
+        cdice = pow(cdice / K_PI6, 1. / 3.);
+        double zdrms = 0., zwams = 0.;
+        for (int s = 0; s < A.ndry; s++) zdrms += AT(mi, nice, s, bc);
+        for (int s = 0; s < nspec + 1; s++) zwams += AT(mi, nice, s, bc);
+        if (zdrms / zwams > 0.5 || cdice < 2.e-6) {
+          const int ba = find_dry4wet(A, ni, mi, nice, bc, p);
+          to_aerosol(A, ni, mi, nice, bc, ba, p);
+          double *dst = ma + p + pl * ((long long)iwa * nbins + ba), *src = mi + p + pl * ((long long)irim * nice + bc);
+          *dst = *dst + *src;
+          *src = 0.;
+        }
+      }
+    }
+  // aerosol bins below 0.1 nm dry diameter vanish; volatile species to the gases
+  for (int ba = 0; ba < nbins; ba++) {
+    const double n_ = na[p + pl * ba];
+    if (gt_bits(bits_of(n_), BITS_NLIM)) {
+      // the dry volume per particle is at least m_s / 2650 for every dry species s
+      // (no density is larger): when the largest m_s is 2^88 times below n, the
+      // particle is above 0.1 nm (pi/6 1e-30 * 2650 < 2^-88) and the sum is not needed
+      long long mx = 0;
+      for (int s = 0; s < nspec - 1; s++) mx = max(mx, bits_of(AT(ma, nbins, s, ba)));
+      if (mx <= INF_BITS && bexp(mx) != 0 && bexp(mx) + 88 >= bexp(bits_of(n_))) continue;
+      double zvol = 0.;
+      for (int s = 0; s < nspec - 1; s++) zvol += AT(ma, nbins, s, ba) / A.rholiq[s];
+      zvol = zvol / n_;
+      if (zvol < K_PI6 * cube(1.e-10)) {
+        if (A.lscndgas) {
+          const int gi[4] = {0, 4, 1, 2};   // SO4 -> 1, OC -> 5, NO -> 2, NH -> 3
+          for (int q = 0; q < 4; q++) {
+            const int ix = A.gas_ix[q];
+            if (ix >= 0) {
+              double *gq = f.gaero + p + pl * gi[q];
+              *gq = *gq + AT(ma, nbins, ix, ba) / A.MM[ix] * K_AVOG;
+            }
+          }
+        }
+        for (int s = 0; s < nspec; s++) AT(ma, nbins, s, ba) = 0.;
+        na[p + pl * ba] = 0.;
+      }
+    }
   }
 }
 
-// ---- SALSA_diagnostics (:52-370) ----
-// at most 64 registers (8 blocks of 128 threads per SM): a point's passes over its bins
-// are dependent loads, so the kernel is bound by latency and gains from warps in flight
+constexpr int PB_NSP = SALSA_NSV;   // most masses of a bin (wet species and rime)
+
+// number and nsp masses of bin b as bit patterns, negative ones set to zero (also in memory).
+// No double is formed: a test on the bits of a double can be compiled into an FP64 compare,
+// which costs as much as any FP64 operation here.
+__device__ __forceinline__ void load_bin(double *num, double *mass, int nb, int nsp, int b, long long p, long long pl,
+                                         long long &n, long long (&v)[PB_NSP]) {
+  long long *pn = reinterpret_cast<long long *>(num) + p + pl * b, *pm = reinterpret_cast<long long *>(mass) + p + pl * b;
+  const long long ps = pl * nb;
+  n = *pn;
+#pragma unroll
+  for (int s = 0; s < PB_NSP; s++) v[s] = s < nsp ? pm[ps * s] : 0;
+  long long any = n;   // sign bit set: some value is negative (or a negative zero or NaN)
+#pragma unroll
+  for (int s = 0; s < PB_NSP; s++) any |= v[s];
+  if (any < 0) {
+    if (neg_bits(n)) { n = 0; *pn = 0; }
+#pragma unroll
+    for (int s = 0; s < PB_NSP; s++)
+      if (neg_bits(v[s])) { v[s] = 0; pm[ps * s] = 0; }
+  }
+}
+// the mass at a species index known at run time, the array staying in registers
+__device__ __forceinline__ long long mass_at(const long long (&v)[PB_NSP], int i) {
+  long long x = 0;
+#pragma unroll
+  for (int s = 0; s < PB_NSP; s++) if (s == i) x = v[s];
+  return x;
+}
+// zero a bin in memory and in registers
+__device__ __forceinline__ void clear_bin(double *num, double *mass, int nb, int nsp, int b, long long p, long long pl,
+                                          long long &n, long long (&v)[PB_NSP]) {
+  num[p + pl * b] = 0.;
+  n = 0;
+#pragma unroll
+  for (int s = 0; s < PB_NSP; s++) {
+    v[s] = 0;
+    if (s < nsp) mass[p + pl * ((long long)s * nb + b)] = 0.;
+  }
+}
+// x + the number of bits b; nothing to add for the zeros of empty bins
+__device__ __forceinline__ double plus_bits(double x, long long b) { return b == 0 ? x : x + __longlong_as_double(b); }
+
+// One thread per point.  Each bin's number and masses are read once, together: the negative
+// values, the particles without mass, the water sums and the test for the rare steps
+// (evaporate_point) all come from those registers; a point that takes a rare step sums its
+// water again from memory.  Before, every pass over the bins (negative values, empty bins,
+// evaporation, vanishing bins, sums) read them from memory again, eight loads or one in
+// flight, and formed FP64 compares: a 1.15 M point block took 1.31 ms, 32 % of the HBM
+// bandwidth; this kernel takes 0.48 ms, 6.4 TB/s or 95 % of the measured copy rate.  64
+// registers and eight blocks per SM (six: 0.56 ms, four: 0.68; two bins per pass 0.52): the
+// loads of a bin and the warps in flight cover the latency.
+// (the values are >= 0 or NaN after the clamp: a sum of them is <= 0 exactly when every term
+// is +-0, and x > 0 is a bit test)
 __global__ void __launch_bounds__(128, 8) diagnostics_kernel(const PostArgs A) {
   const long long pl = A.plane;
   const salsa_post_fields_t &f = A.f;
@@ -233,176 +394,108 @@ __global__ void __launch_bounds__(128, 8) diagnostics_kernel(const PostArgs A) {
   const long long BITS_MASSTH = bits_of(1.e-25), BITS_NLIM = bits_of(K_NLIM), BITS_PRLIM = bits_of(K_PRLIM);
   const long long BITS_1EM5 = bits_of(1.e-5), BITS_1EM6 = bits_of(1.e-6), BITS_1EM15 = bits_of(1.e-15);
   for (long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x; p < pl; p += (long long)gridDim.x * blockDim.x) {
-#define AT(arr, nb, s, b) (arr)[p + pl * ((long long)(s) * (nb) + (b))]
-    // negative values (whole arrays)
-    clamp_neg(na, p, pl, nbins);
-    clamp_neg(nc, p, pl, ncld);
-    clamp_neg(np, p, pl, nprc);
-    clamp_neg(ma, p, pl, nspec * nbins);
-    clamp_neg(mc, p, pl, nspec * ncld);
-    clamp_neg(mp, p, pl, nspec * nprc);
-    if (lvl5) {
-      clamp_neg(ni, p, pl, nice);
-      clamp_neg(mi, p, pl, (nspec + 1) * nice);
-    }
     const long long r = p / A.nzp;
     const int i = (int)(r % A.nxp), j = (int)(r / A.nxp);
-    if (!A.only_diag && i >= 2 && i <= A.nxp - 3 && j >= 2 && j <= A.nyp - 3) {
-      // particles with number but no mass
-      // (the values are >= 0 or NaN now: a sum of them is <= 0 exactly when every term
-      // is +-0, and x > 0 is a bit test)
-      for (int bc = 0; bc < nbins; bc++) {
+    const bool inner = !A.only_diag && i >= 2 && i <= A.nxp - 3 && j >= 2 && j <= A.nyp - 3;
+    bool dry = false, dryi = false, rare = false;
+    if (inner) {
+      dry = f.rh[p] < 0.999;
+      if (lvl5) dryi = f.rhi[p] < 0.999;
+    }
+    long long n, v[PB_NSP];
+    double rc = 0., rcc = 0., srp = 0., snrp = 0., ri = 0., riri = 0.;
+#pragma unroll 1
+    for (int bc = 0; bc < nbins; bc++) {
+      load_bin(na, ma, nbins, nspec, bc, p, pl, n, v);
+      if (inner) {
         bool empty = true;
-        for (int s = 0; s < nspec; s++) empty &= le0_bits(bits_of(AT(ma, nbins, s, bc)));
-        if (empty && gt_bits(bits_of(na[p + pl * bc]), 0)) {
-          na[p + pl * bc] = 0.;
-          for (int s = 0; s < nspec; s++) AT(ma, nbins, s, bc) = 0.;
+        long long mx = 0;   // largest dry mass
+#pragma unroll
+        for (int s = 0; s < PB_NSP; s++) {
+          empty &= le0_bits(v[s]);
+          if (s < nspec - 1) mx = max(mx, v[s]);
+        }
+        if (empty && gt_bits(n, 0)) {
+          clear_bin(na, ma, nbins, nspec, bc, p, pl, n, v);
           if (A.lcharge) f.chargeTime[p + pl * bc] = 0.;
         }
+        // may vanish: not settled by the exponents (see evaporate_point)
+        if (gt_bits(n, BITS_NLIM) && !(mx <= INF_BITS && bexp(mx) != 0 && bexp(mx) + 88 >= bexp(n)))
+          rare = true;
       }
-      for (int bc = 0; bc < ncld; bc++) {
+      rc = plus_bits(rc, mass_at(v, iwa));
+    }
+#pragma unroll 1
+    for (int bc = 0; bc < ncld; bc++) {
+      load_bin(nc, mc, ncld, nspec, bc, p, pl, n, v);
+      if (inner) {
         bool empty = true;
-        for (int s = 0; s < nspec; s++) empty &= le0_bits(bits_of(AT(mc, ncld, s, bc)));
-        if (empty && gt_bits(bits_of(nc[p + pl * bc]), 0)) {
-          nc[p + pl * bc] = 0.;
-          for (int s = 0; s < nspec; s++) AT(mc, ncld, s, bc) = 0.;
+#pragma unroll
+        for (int s = 0; s < PB_NSP; s++) empty &= le0_bits(v[s]);
+        if (empty && gt_bits(n, 0)) {
+          clear_bin(nc, mc, ncld, nspec, bc, p, pl, n, v);
           if (A.lcharge) f.chargeTime[p + pl * (nbins + bc)] = 0.;
         }
+        rare |= dry && gt_bits(n, BITS_NLIM) && lt_bits(mass_at(v, iwa), BITS_1EM5);
       }
-      for (int bc = 0; bc < nprc; bc++)
-        if (le0_bits(bits_of(AT(mp, nprc, iwa, bc))) && gt_bits(bits_of(np[p + pl * bc]), 0)) {
-          np[p + pl * bc] = 0.;
-          for (int s = 0; s < nspec; s++) AT(mp, nprc, s, bc) = 0.;
+      rcc = plus_bits(rcc, mass_at(v, iwa));
+    }
+#pragma unroll 1
+    for (int bc = 0; bc < nprc; bc++) {
+      load_bin(np, mp, nprc, nspec, bc, p, pl, n, v);
+      if (inner) {
+        if (le0_bits(mass_at(v, iwa)) && gt_bits(n, 0)) {
+          clear_bin(np, mp, nprc, nspec, bc, p, pl, n, v);
           if (A.lcharge) f.chargeTime[p + pl * (nbins + ncld + bc)] = 0.;
         }
-      if (lvl5)
-        for (int bc = 0; bc < nice; bc++) {
-          if (!gt_bits(bits_of(ni[p + pl * bc]), 0)) continue;
-          const double w_ = AT(mi, nice, iwa, bc), r_ = AT(mi, nice, irim, bc);
-          if (!lt_bits(bits_of(w_), BITS_MASSTH) || !lt_bits(bits_of(r_), BITS_MASSTH)) continue;
-          if (w_ + r_ < massTH) {
-            ni[p + pl * bc] = 0.;
-            for (int s = 0; s < nspec + 1; s++) AT(mi, nice, s, bc) = 0.;
-          }
-        }
-      const double T = f.temp[p];
-      const bool dry = f.rh[p] < 0.999;
-      const double zaa = 4. * K_MWA * K_SURFW0 / (K_RG * K_RHOWA * T);
-      // evaporating cloud droplets: back to the parallel aerosol bin
-      for (int bc = A.ica_cur; bc <= A.fcb_cur; bc++) {
-        const double n_ = nc[p + pl * bc];
-        if (dry && gt_bits(bits_of(n_), BITS_NLIM) && lt_bits(bits_of(AT(mc, ncld, iwa, bc)), BITS_1EM5)) {
-          double ns = 0., zvol = 0.;
-          for (int s = 0; s < nspec - 1; s++) ns += A.diss[s] * AT(mc, ncld, s, bc) / A.MM[s];
-          ns = ns / n_;
-          const double zbb = 6. * K_MWA * ns / (K_PI * K_RHOWA);
-          const double cdcld = sqrt(3. * zbb / zaa);
-          for (int s = 0; s < nspec; s++) zvol += AT(mc, ncld, s, bc) / A.rholiq[s];
-          zvol = zvol / n_;
-          const double zdh2o = pow(zvol / K_PI6, 1. / 3.);
-          if (zdh2o < fmin(0.7 * cdcld, 1.3e-5) || AT(mc, ncld, iwa, bc) < massTH * n_) {
-            const int ba = bc <= A.fca_cur ? A.ica_par + (bc - A.ica_cur) : A.icb_par + (bc - A.icb_cur);
-            to_aerosol(A, nc, mc, ncld, bc, ba, p);
-            if (A.lcharge) f.chargeTime[p + pl * (nbins + bc)] = 0.;
-          }
-        }
+        rare |= dry && gt_bits(n, BITS_PRLIM) && lt_bits(mass_at(v, iwa), BITS_1EM6);
       }
-      // evaporating drops: to the aerosol bin of the closest dry size and composition
-      for (int bc = 0; bc < nprc; bc++) {
-        const double n_ = np[p + pl * bc];
-        if (dry && gt_bits(bits_of(n_), BITS_PRLIM) && lt_bits(bits_of(AT(mp, nprc, iwa, bc)), BITS_1EM6)) {
-          double ns = 0., zvol = 0.;
-          for (int s = 0; s < nspec - 1; s++) ns += A.diss[s] * AT(mp, nprc, s, bc) / A.MM[s];
-          ns = ns / n_;
-          const double zbb = 6. * K_MWA * ns / (K_PI * K_RHOWA);
-          const double cdprc = sqrt(3. * zbb / zaa);
-          for (int s = 0; s < nspec; s++) zvol += AT(mp, nprc, s, bc) / A.rholiq[s];
-          zvol = zvol / n_;
-          const double zdh2o = pow(zvol / K_PI6, 1. / 3.);
-          if (zdh2o < fmin(0.2 * cdprc, 10.e-6) || AT(mp, nprc, iwa, bc) < massTH * n_) {
-            const int ba = find_dry4wet(A, np, mp, nprc, bc, p);
-            to_aerosol(A, np, mp, nprc, bc, ba, p);
-            if (A.lcharge) f.chargeTime[p + pl * (nbins + ncld + bc)] = 0.;
+      srp = plus_bits(srp, mass_at(v, iwa));
+      snrp = plus_bits(snrp, n);
+    }
+    if (lvl5)
+#pragma unroll 1
+      for (int bc = 0; bc < nice; bc++) {
+        load_bin(ni, mi, nice, nspec + 1, bc, p, pl, n, v);
+        long long w_ = mass_at(v, iwa), r_ = mass_at(v, irim);
+        if (inner && gt_bits(n, 0)) {
+          if (lt_bits(w_, BITS_MASSTH) && lt_bits(r_, BITS_MASSTH) &&
+              __longlong_as_double(w_) + __longlong_as_double(r_) < massTH) {
+            clear_bin(ni, mi, nice, nspec + 1, bc, p, pl, n, v);
+            w_ = r_ = 0;
           }
+          rare |= dryi && gt_bits(n, BITS_PRLIM) && lt_bits(w_, BITS_1EM15) && lt_bits(r_, BITS_1EM15);
         }
+        ri = plus_bits(ri, w_);
+        riri = plus_bits(riri, r_);
       }
-      // evaporating ice (rime goes to the aerosol water)
-      if (lvl5 && f.rhi[p] < 0.999)
-        for (int bc = 0; bc < nice; bc++) {
-          const double n_ = ni[p + pl * bc];
-          if (!gt_bits(bits_of(n_), BITS_PRLIM)) continue;
-          const double w_ = AT(mi, nice, iwa, bc), r_ = AT(mi, nice, irim, bc);
-          if (!lt_bits(bits_of(w_), BITS_1EM15) || !lt_bits(bits_of(r_), BITS_1EM15)) continue;
-          if (w_ + r_ < 1.e-15) {
-            double vt = 0.;
-            for (int s = 0; s < nspec + 1; s++) vt += AT(mi, nice, s, bc) / A.rhoice[s];
-            double cdice = vt / n_;
-            cdice = pow(cdice / K_PI6, 1. / 3.);
-            double zdrms = 0., zwams = 0.;
-            for (int s = 0; s < A.ndry; s++) zdrms += AT(mi, nice, s, bc);
-            for (int s = 0; s < nspec + 1; s++) zwams += AT(mi, nice, s, bc);
-            if (zdrms / zwams > 0.5 || cdice < 2.e-6) {
-              const int ba = find_dry4wet(A, ni, mi, nice, bc, p);
-              to_aerosol(A, ni, mi, nice, bc, ba, p);
-              double *dst = ma + p + pl * ((long long)iwa * nbins + ba), *src = mi + p + pl * ((long long)irim * nice + bc);
-              *dst = *dst + *src;
-              *src = 0.;
-            }
-          }
-        }
-      // aerosol bins below 0.1 nm dry diameter vanish; volatile species to the gases
-      for (int ba = 0; ba < nbins; ba++) {
-        const double n_ = na[p + pl * ba];
-        if (gt_bits(bits_of(n_), BITS_NLIM)) {
-          // the dry volume per particle is at least m_s / 2650 for every dry species s
-          // (no density is larger): when the largest m_s is 2^88 times below n, the
-          // particle is above 0.1 nm (pi/6 1e-30 * 2650 < 2^-88) and the sum is not needed
-          long long mx = 0;
-          for (int s = 0; s < nspec - 1; s++) mx = max(mx, bits_of(AT(ma, nbins, s, ba)));
-          if (mx <= INF_BITS && bexp(mx) != 0 && bexp(mx) + 88 >= bexp(bits_of(n_))) continue;
-          double zvol = 0.;
-          for (int s = 0; s < nspec - 1; s++) zvol += AT(ma, nbins, s, ba) / A.rholiq[s];
-          zvol = zvol / n_;
-          if (zvol < K_PI6 * cube(1.e-10)) {
-            if (A.lscndgas) {
-              const int gi[4] = {0, 4, 1, 2};   // SO4 -> 1, OC -> 5, NO -> 2, NH -> 3
-              for (int q = 0; q < 4; q++) {
-                const int ix = A.gas_ix[q];
-                if (ix >= 0) {
-                  double *gq = f.gaero + p + pl * gi[q];
-                  *gq = *gq + AT(ma, nbins, ix, ba) / A.MM[ix] * K_AVOG;
-                }
-              }
-            }
-            for (int s = 0; s < nspec; s++) AT(ma, nbins, s, ba) = 0.;
-            na[p + pl * ba] = 0.;
-          }
-        }
+    if (rare) {
+      evaporate_point(A, p);
+      rc = rcc = srp = snrp = ri = riri = 0.;
+      for (int b = A.in1a; b <= A.fn2b; b++) rc += AT(ma, nbins, iwa, b);
+      for (int b = A.ica_cur; b <= A.fcb_cur; b++) rcc += AT(mc, ncld, iwa, b);
+      for (int b = 0; b < nprc; b++) srp += AT(mp, nprc, iwa, b);
+      for (int b = 0; b < nprc; b++) snrp += np[p + pl * b];
+      if (lvl5) {
+        for (int b = 0; b < nice; b++) ri += AT(mi, nice, iwa, b);
+        for (int b = 0; b < nice; b++) riri += AT(mi, nice, irim, b);
       }
     }
     // water diagnostics
-    double rc = 0., rcc = 0., srp = 0., snrp = 0.;
-    for (int b = A.in1a; b <= A.fn2b; b++) rc += AT(ma, nbins, iwa, b);
-    for (int b = A.ica_cur; b <= A.fcb_cur; b++) rcc += AT(mc, ncld, iwa, b);
     rc = rc + rcc;
-    for (int b = 0; b < nprc; b++) srp += AT(mp, nprc, iwa, b);
-    for (int b = 0; b < nprc; b++) snrp += np[p + pl * b];
     f.rc[p] = rc;
     f.srp[p] = srp;
     f.snrp[p] = snrp;
     double rt = rc + srp + f.rp[p];
     if (lvl5) {
-      double ri = 0., riri = 0.;
-      for (int b = 0; b < nice; b++) ri += AT(mi, nice, iwa, b);
-      for (int b = 0; b < nice; b++) riri += AT(mi, nice, irim, b);
       f.ri[p] = ri;
       f.riri[p] = riri;
       rt = rt + ri + riri;
     }
     f.rtot[p] = rt;
-#undef AT
   }
 }
+#undef AT
 
 }  // namespace
 }  // namespace salsa
