@@ -21,55 +21,52 @@
 #include "salsa_internal.h"
 
 namespace salsa {
-cudaError_t launch_d0(const DevParams &, cudaStream_t, int);
 cudaError_t launch_d1(const DevParams &, cudaStream_t, int);
-cudaError_t launch_f0(const DevParams &, cudaStream_t, int);
 cudaError_t launch_f1(const DevParams &, cudaStream_t, int);
-int blocks_per_sm_d0(const DevParams &);
 int blocks_per_sm_d1(const DevParams &);
-int blocks_per_sm_f0(const DevParams &);
 int blocks_per_sm_f1(const DevParams &);
 cudaError_t launch_ds(const DevParams &, cudaStream_t, int);
 cudaError_t launch_fs(const DevParams &, cudaStream_t, int);
 int blocks_per_sm_ds(const DevParams &);
 int blocks_per_sm_fs(const DevParams &);
-// the lane form of the FP64 ones
-cudaError_t launch_lane_d0(const DevParams &, cudaStream_t, int);
+// the lane form of each
 cudaError_t launch_lane_d1(const DevParams &, cudaStream_t, int);
 cudaError_t launch_lane_ds(const DevParams &, cudaStream_t, int);
-int lane_blocks_per_sm_d0(const DevParams &);
+cudaError_t launch_lane_f1(const DevParams &, cudaStream_t, int);
+cudaError_t launch_lane_fs(const DevParams &, cudaStream_t, int);
 int lane_blocks_per_sm_d1(const DevParams &);
 int lane_blocks_per_sm_ds(const DevParams &);
+int lane_blocks_per_sm_f1(const DevParams &);
+int lane_blocks_per_sm_fs(const DevParams &);
 }  // namespace salsa
 
 namespace {
-// the kernels of one form of the step: [FP64, mixed] without diagnostics, with them, with
-// secondary ice
+// the kernels of one form of the step: FP64 and mixed, without and with secondary ice
 struct Form {
   cudaError_t (*warp)(const salsa::DevParams &, cudaStream_t, int);
   int (*warp_bps)(const salsa::DevParams &);
   cudaError_t (*lane)(const salsa::DevParams &, cudaStream_t, int);
   int (*lane_bps)(const salsa::DevParams &);
 };
-const Form FORMS[3][2] = {
-    {{salsa::launch_d0, salsa::blocks_per_sm_d0, salsa::launch_lane_d0, salsa::lane_blocks_per_sm_d0},
-     {salsa::launch_f0, salsa::blocks_per_sm_f0, nullptr, nullptr}},
+const Form FORMS[2][2] = {
     {{salsa::launch_d1, salsa::blocks_per_sm_d1, salsa::launch_lane_d1, salsa::lane_blocks_per_sm_d1},
-     {salsa::launch_f1, salsa::blocks_per_sm_f1, nullptr, nullptr}},
+     {salsa::launch_f1, salsa::blocks_per_sm_f1, salsa::launch_lane_f1, salsa::lane_blocks_per_sm_f1}},
     {{salsa::launch_ds, salsa::blocks_per_sm_ds, salsa::launch_lane_ds, salsa::lane_blocks_per_sm_ds},
-     {salsa::launch_fs, salsa::blocks_per_sm_fs, nullptr, nullptr}}};
-const Form &form_of(bool sip, bool diag, int precision) { return FORMS[sip ? 2 : (diag ? 1 : 0)][precision]; }
+     {salsa::launch_fs, salsa::blocks_per_sm_fs, salsa::launch_lane_fs, salsa::lane_blocks_per_sm_fs}}};
+const Form &form_of(bool sip, int precision) { return FORMS[sip ? 1 : 0][precision]; }
 }  // namespace
 
-// FP64 calls of at least this many cells take the lane form (one cell per lane); smaller ones
+// Calls of at least this many cells take the lane form (one cell per lane); smaller ones
 // take the warp form, whose latency per cell is lower: a tile of 32 cells takes the lane form
 // 4 (warm cells) to 12 ms (cloudy ones), and that is what a call takes while every sub-core
-// holds at most one tile.  Both forms took the same time at about 24,000 cells of
-// grid16x16x40, grid256x256x128 and grid384x384x160 (5.8 / 6.3, 11.2 / 12.4 and
-// 12.6 / 12.2 ms, lane / warp form).  With secondary ice the warp form holds one block per SM
-// and runs the schemes on one lane: 13.3 / 47 ms at 13,824 cells, even at about 4,000.
-// The mixed form stays with the warp form, whose float partner sums round by its lanes.
+// holds at most one tile.  At 24,576 cells of grid16x16x40, grid256x256x128 and
+// grid384x384x160 the FP64 forms take 5.4 / 5.6, 9.3 / 11.2 and 10.5 / 10.8 ms (lane / warp
+// form); the mixed ones, whose warp form is faster, 5.4 / 4.3, 9.8 / 9.1 and 10.8 / 9.2 ms, and
+// 7.2 / 8.6, 15.8 / 19.5 and 17.1 / 13.0 ms at 49,152.  With secondary ice the warp form holds
+// one block per SM and runs the schemes on one lane: 12.8 / 47 ms at 13,824 cells, even at
+// about 4,000.
 #define SALSA_LANE_MINCELLS 24576
+#define SALSA_LANE_MINCELLS_MIXED 40960
 #define SALSA_LANE_MINCELLS_SIP 4096
 
 using salsa::DevParams;
@@ -633,7 +630,7 @@ int salsa_gb300_init(const salsa_config_t *cfg, salsa_handle_t **out) {
     void *po = nullptr, *ps = nullptr;
     cudaFuncAttributes fa;
     const bool sip = g.lssecice.sw && g.level == 5;
-    const int bps = form_of(sip, g.diagnostics, g.precision).warp_bps(B);
+    const int bps = form_of(sip, g.precision).warp_bps(B);
     if (bps <= 0 || cudaFuncGetAttributes(&fa, salsa_order_kernel) != cudaSuccess ||
         cudaGetSymbolAddress(&po, g_na_order) != cudaSuccess || cudaGetSymbolAddress(&ps, g_na_status) != cudaSuccess) {
       salsa_gb300_finalize(h);
@@ -847,7 +844,7 @@ int run_impl(salsa_handle_t *h, int nzp, int nxp, int nyp, int ns, double tstep,
   if (noalloc && P.ncells > SALSA_NOALLOC_MAXCELLS) return SALSA_E_ARG;
   unsigned long long *d_status = noalloc ? h->na_status : h->d_status;
   P.status = d_status;
-  const int prec = g.precision, dg = g.diagnostics ? 1 : 0;
+  const int prec = g.precision;
   auto bind = [&](DevParams &Q, const F &x, double *dp) {
     if (x.fi >= 0) Q.fin[x.fi] = dp;
     if (x.fo >= 0) {
@@ -860,18 +857,19 @@ int run_impl(salsa_handle_t *h, int nzp, int nxp, int nyp, int ns, double tstep,
   // order pre-pass and step kernel over the cells of Q, on stream s
   auto launch = [&](DevParams &Q, int *order) -> int {
     const bool sip = Q.st_secice != 0;
-    const Form &form = form_of(sip, dg, prec);
+    const Form &form = form_of(sip, prec);
     const int bps = form.warp_bps(Q);
     if (bps <= 0) return SALSA_E_CUDA;
     long long grid = (long long)bps * h->nsm * 8;
     if (grid > Q.ngroups) grid = Q.ngroups;
     // the lane form, when the call is large enough and its workspaces are to be had
     int lane_grid = 0;
-    if (!noalloc && order && form.lane && Q.ncells >= (sip ? SALSA_LANE_MINCELLS_SIP : SALSA_LANE_MINCELLS)) {
+    if (!noalloc && order && Q.ncells >= (sip ? SALSA_LANE_MINCELLS_SIP : (prec == 0 ? SALSA_LANE_MINCELLS : SALSA_LANE_MINCELLS_MIXED))) {
       const int lbps = form.lane_bps(Q);
       const long long need = ((Q.ncells + 31) / 32 + SALSA_LANE_WARPS - 1) / SALSA_LANE_WARPS;
       lane_grid = (int)std::min((long long)lbps * h->nsm, need);
-      const size_t bytes = (size_t)lane_grid * SALSA_LANE_WARPS * 32 * (size_t)Q.ws_doubles * sizeof(double);
+      Q.lane_rows = Q.ws_doubles + (prec == 0 ? 0 : SALSA_LEAF_ROWS);
+      const size_t bytes = (size_t)lane_grid * SALSA_LANE_WARPS * 32 * (size_t)Q.lane_rows * sizeof(double);
       if (lane_grid > 0 && bytes > h->lane_ws_bytes) {
         if (h->lane_ws) cudaFree(h->lane_ws);
         h->lane_ws = nullptr;

@@ -12,6 +12,7 @@
 #define SALSA_THREADS (32 * SALSA_CPG)
 #define SALSA_LANE_WARPS 4          // warps per block of the lane form (32 cells each)
 #define SALSA_LANE_MINBLOCKS 4      // its resident blocks per SM
+#define SALSA_LEAF_ROWS (32 * 17)   // doubles of the lane form's float sums: 32 leaves of 17 pairs
 #define SALSA_NSV 7                 // volume slots per bin (dry species + water + rime)
 #define SALSA_MAXNB 96
 
@@ -141,7 +142,8 @@ struct DevParams {
   // offset of the tally region inside each warp's workspace (doubles)
   int st_secice, st_siprs, st_sipdf, st_sipib;
   int sip_rs_mode, sip_df_mode, sip_ib_mode, sip_splbin, sip_off;
-  double *lane_ws;   // workspaces of the lane form, one of 32 * ws_doubles per resident warp
+  double *lane_ws;   // workspaces of the lane form, one of 32 * lane_rows doubles per resident warp
+  int lane_rows;     // ws_doubles, and in the mixed form the leaves of its partner sums
   int raw_sip;   // first of the 3 x nice tracer rows (sipdrfr, siprmspl, sipiibr), or -1
 };
 

@@ -1,5 +1,5 @@
 // salsa_kernel_impl.cuh -- the fused SALSA microphysics step for sm_103a (templates;
-// instantiated by salsa_k_*.cu, one translation unit per precision/diagnostics form).
+// instantiated by salsa_k_*.cu and salsa_l_*.cu, one translation unit per form).
 //
 // One launch advances every interior grid cell by one SALSA call
 // (UCLALES-SALSA src/src_salsa/mo_salsa_driver.f90:180-427 -> mo_salsa.f90:45-153).
@@ -72,6 +72,7 @@ struct WS {
   // float copies of numc and volc that the mixed form's coagulation update sums from
   // (in the scratch rows, valid from shadow_all to the end of the update)
   Ptr<float, LS> nf, vf;
+  Ptr<float, LS> lf;   // lane form of the mixed form: the leaves of the partner sums
   __device__ __forceinline__ double &v(int s, int b) const { return volc[s * NB + b]; }
   __device__ __forceinline__ D sc(int k) const { return scr + k * NB; }
   // partner values in the kernel type: the state itself (FP64 form) or its float copy
@@ -882,14 +883,18 @@ struct TAccT {
   A sink, self;
   A src[SALSA_NSV];
   A dg[7];   // 0 autoc(abs) 1 autoc80 2 autoc50 3 accr 4 accr80 5 accr50 6 coll mass
-  // src[s0] += x for a species index known only at run time, with every index of src
-  // constant after unrolling, so that the accumulator stays in registers
-  __device__ __forceinline__ void add_at(int s0, KT x) {
-#pragma unroll
-    for (int s = 0; s < SALSA_NSV; s++)
-      if (s == s0) src[s] += x;
-  }
-  __device__ __forceinline__ void zero() {
+  KT cm;     // the lane's part of dg[6], added at the end
+  // additions of a partner's term; `leaf` is its lane in the warp form (see the lane form's
+  // float sums below)
+  __device__ __forceinline__ void add_sink(KT x, int) { sink += x; }
+  __device__ __forceinline__ void add_self(KT x, int) { self += x; }
+  __device__ __forceinline__ void add_src(int s, KT x, int) { src[s] += x; }
+  __device__ __forceinline__ void add_dg(int d, KT x, int) { dg[d] += x; }
+  __device__ __forceinline__ KT cm_get(int) const { return cm; }
+  __device__ __forceinline__ void cm_put(int, KT x) { cm = x; }
+  __device__ __forceinline__ void cm_add() { dg[6] += cm; }
+  template <typename W> __device__ __forceinline__ void zero(const W &) {
+    cm = (KT)0;
     sink = (KT)0; self = (KT)0;
 #pragma unroll
     for (int s = 0; s < SALSA_NSV; s++) src[s] = (KT)0;
@@ -898,14 +903,7 @@ struct TAccT {
   }
   __device__ __forceinline__ void reduce(bool diag, int lane) {
     if constexpr (LS == 1) {
-      if constexpr (sizeof(KT) == 4) {   // the compensated sums, rounded once to float
-        sink = sink.s - sink.c;
-        self = self.s - self.c;
-#pragma unroll
-        for (int s = 0; s < SALSA_NSV; s++) src[s] = src[s].s - src[s].c;
-#pragma unroll
-        for (int d = 0; d < 7; d++) dg[d] = dg[d].s - dg[d].c;
-      }
+      // one lane holds the totals
     } else if constexpr (sizeof(KT) == 4) {
       float h[8], l[8];
 #pragma unroll
@@ -950,6 +948,94 @@ struct TAccT {
     }
   }
 };
+
+// The mixed form's sums in the lane form.  Each of the warp form's 32 lanes adds its partners
+// in a compensated float pair and the pairs are added over the lanes in a fixed tree, with
+// one rounding to float at the end; the lane form keeps those pairs in its workspace
+// (`leaf`: the warp form's lane of a partner) and adds them in the same tree, so that both
+// forms round alike.
+struct LeafSums {
+  static constexpr int SINK = 7, SELF = 8, DG = 9, CM = 16, N = 17;   // slots; 0-6 are the species
+  Col<float> lf;
+  unsigned m[N];   // leaves that hold something
+  float src[SALSA_NSV], sink, self, dg[7];
+  __device__ __forceinline__ void acc(int i, float x, int leaf) {
+    const Col<float> q = lf + (leaf * N + i) * 2;
+    KahanF k;
+    k = 0.f;
+    if ((m[i] >> leaf) & 1u) { k.s = q[0]; k.c = q[1]; }
+    m[i] |= 1u << leaf;
+    k += x;
+    q[0] = k.s;
+    q[1] = k.c;
+  }
+  __device__ __forceinline__ void add_sink(float x, int leaf) { acc(SINK, x, leaf); }
+  __device__ __forceinline__ void add_self(float x, int leaf) { acc(SELF, x, leaf); }
+  __device__ __forceinline__ void add_src(int s, float x, int leaf) { acc(s, x, leaf); }
+  __device__ __forceinline__ void add_dg(int d, float x, int leaf) { acc(DG + d, x, leaf); }
+  __device__ __forceinline__ float cm_get(int leaf) const { return (m[CM] >> leaf) & 1u ? lf[(leaf * N + CM) * 2] : 0.f; }
+  __device__ __forceinline__ void cm_put(int leaf, float x) {
+    lf[(leaf * N + CM) * 2] = x;
+    m[CM] |= 1u << leaf;
+  }
+  __device__ __forceinline__ void cm_add() {
+    for (int l = 0; l < 32; l++)
+      if ((m[CM] >> l) & 1u) acc(DG + 6, lf[(l * N + CM) * 2], l);
+  }
+  template <typename W> __device__ __forceinline__ void zero(const W &w) {
+    lf = w.lf;
+#pragma unroll
+    for (int i = 0; i < N; i++) m[i] = 0u;
+  }
+  // the total of slot i over the leaves (warp_sum8_comp's tree)
+  __device__ __forceinline__ float total(int i) const {
+    if (m[i] == 0u) return 0.f;
+    float h4 = 0.f, l4 = 0.f, h3 = 0.f, l3 = 0.f, h2 = 0.f, l2 = 0.f, h1 = 0.f, l1 = 0.f, h0 = 0.f, l0 = 0.f;
+    float h = 0.f, l = 0.f;
+    auto merge = [&](float a, float b) {   // (a, b) + (h, l)
+      float t, e;
+      two_sum(a, h, t, e);
+      l = b + l + e;
+      h = t;
+    };
+#pragma unroll 1
+    for (int k = 0; k < 32; k++) {
+      const int leaf = (int)(__brev((unsigned)k) >> 27);
+      h = 0.f;
+      l = 0.f;
+      if ((m[i] >> leaf) & 1u) {
+        const Col<float> q = lf + (leaf * N + i) * 2;
+        h = q[0];
+        l = -q[1];
+      }
+      if (!(k & 1)) { h4 = h; l4 = l; continue; }
+      merge(h4, l4);
+      if (!(k & 2)) { h3 = h; l3 = l; continue; }
+      merge(h3, l3);
+      if (!(k & 4)) { h2 = h; l2 = l; continue; }
+      merge(h2, l2);
+      if (!(k & 8)) { h1 = h; l1 = l; continue; }
+      merge(h1, l1);
+      if (!(k & 16)) { h0 = h; l0 = l; continue; }
+      merge(h0, l0);
+    }
+    return h + l;
+  }
+  __device__ __forceinline__ void reduce(bool diag, int) {
+#pragma unroll
+    for (int s = 0; s < SALSA_NSV; s++) src[s] = total(s);
+    sink = total(SINK);
+    if (diag) {
+      self = total(SELF);
+#pragma unroll
+      for (int d = 0; d < 7; d++) dg[d] = total(DG + d);
+    } else {
+      self = m[SELF] & 1u ? lf[SELF * 2] - lf[SELF * 2 + 1] : 0.f;   // lane 0 alone
+    }
+  }
+};
+template <> struct TAccT<float, 1> : LeafSums {};
+static_assert(SALSA_LEAF_ROWS == 32 * LeafSums::N, "32 leaves of N float pairs");
 
 // float copies of the partner state for the mixed form's coagulation update: every bin
 // before the sweep, then each bin again whenever the sweep changes it
@@ -1519,11 +1605,12 @@ __device__ __forceinline__ void source_range(const WS<KT, LS> &w, int t, int g0,
                                              TAccT<KT, LS> &a, int lane) {
   for (int ll = istr + lane; ll <= iend; ll += LS) {
     int g = g0 + ll;
+    const int leaf = (ll - istr) & 31;
     if (!w.on(g)) continue;
     const KT k = kget(w, g, t);
 #pragma unroll
     for (int s = 0; s < SALSA_NSV; s++)
-      if (s < nspec) a.src[s] += k * w.vk(s, g);
+      if (s < nspec) a.add_src(s, k * w.vk(s, g), leaf);
   }
 }
 
@@ -1538,9 +1625,9 @@ template <typename KT, int LS>
 __device__ __forceinline__ void list_sinks(const WS<KT, LS> &w, const int16_t *L, int t, TAccT<KT, LS> &a, int lane) {
   const int off = L[4 * t], n = L[4 * t + 1];
   for (int e = lane; e < n; e += LS) {
-    const int g = L[off + e];
+    const int g = L[off + e], leaf = e & 31;
     if (!w.on(g)) continue;
-    a.sink += kget(w, t, g) * w.nk(g);
+    a.add_sink(kget(w, t, g) * w.nk(g), leaf);
   }
 }
 
@@ -1549,12 +1636,12 @@ __device__ __forceinline__ void list_sources(const WS<KT, LS> &w, const int16_t 
                                              int lane) {
   const int off = L[4 * t + 2], n = L[4 * t + 3];
   for (int e = lane; e < n; e += LS) {
-    const int g = L[off + e];
+    const int g = L[off + e], leaf = e & 31;
     if (!w.on(g)) continue;
     const KT k = kget(w, g, t);
 #pragma unroll
     for (int s = 0; s < SALSA_NSV; s++)
-      if (s < nspec) a.src[s] += k * w.vk(s, g);
+      if (s < nspec) a.add_src(s, k * w.vk(s, g), leaf);
   }
 }
 
@@ -1597,8 +1684,8 @@ __device__ void coag_aero(const DevParams &P, const WS<KT, LS> &w, const double 
   for (int kk = P.in1a; kk <= P.fn2b; kk++) {
     if (num_lt(w.numc[kk], K_NLIM)) continue;
     TAccT<KT, LS> a;
-    a.zero();
-    if (P.lscgaa && lane == 0) a.self = (KT)0.5 * kget(w, kk, kk) * w.nk(kk);
+    a.zero(w);
+    if (P.lscgaa && lane == 0) a.add_self((KT)0.5 * kget(w, kk, kk) * w.nk(kk), 0);
     list_sinks(w, L, kk, a, lane);
     list_sources(w, L, kk, nspec, a, lane);
     a.reduce(false, lane);
@@ -1619,12 +1706,13 @@ __device__ void precip_formation(const DevParams &P, const WS<KT, LS> &w, const 
   const auto slot = w.misc + M_PFSLOT;          // 8 slots x 10: tp, dvol[7], dnum, x*dnum
   const int tg = C0 + t;
   if constexpr (LS == 1) {
+    const double dt3 = cube(w.dwet[tg]);
     for (int ll = istr; ll <= iend; ll++) {
-      const int lg = C0 + ll;
+      const int lg = C0 + ll, leaf = (ll - istr) & 7;   // partners in chunks of eight lanes
       if (!w.on(lg)) continue;
-      const double D_new = dcbrt(cube(w.dwet[tg]) + cube(w.dwet[lg]));
+      const double D_new = dcbrt(dt3 + cube(w.dwet[lg]));
       int cnt = 0;
-      for (int i = 0; i < nprc; i++) cnt += (D_new > pbins[i]);
+      for (int i = 0; i < nprc; i++) cnt += num_gt(D_new, pbins[i]);
       const double klt = (double)kget(w, lg, tg), nt = w.numc[tg], nl = w.numc[lg];
       if (cnt > 0) {
         const int tp = cnt - 1;
@@ -1638,25 +1726,25 @@ __device__ void precip_formation(const DevParams &P, const WS<KT, LS> &w, const 
         if (selfcoll) {
           dnum = (0.5 * klt * nl * nt) * fix;
           xin = w.indef[lg] * dnum;
-          a.self += (KT)(0.5 * klt * nt);
+          a.add_self((KT)(0.5 * klt * nt), leaf);
         } else {
           dnum = (klt * nl * nt) * fix;
           xin = 0.5 * (w.indef[lg] + w.indef[tg]) * dnum;
-          a.sink += (KT)(klt * nl);
+          a.add_sink((KT)(klt * nl), leaf);
         }
         num_prc[tp] += dnum;
         inf_prc[tp] += xin;
         if (diag) {
-          a.dg[0] += (KT)dvw;
-          if (D_new > 50.e-6) a.dg[2] += (KT)dvw;
-          if (D_new > 80.e-6) a.dg[1] += (KT)dvw;
+          a.add_dg(0, (KT)dvw, leaf);
+          if (num_gt(D_new, 50.e-6)) a.add_dg(2, (KT)dvw, leaf);
+          if (num_gt(D_new, 80.e-6)) a.add_dg(1, (KT)dvw, leaf);
         }
       } else if (selfcoll) {
-        a.self += (KT)(0.5 * klt * nl);
+        a.add_self((KT)(0.5 * klt * nl), leaf);
       } else {
 #pragma unroll
         for (int s = 0; s < SALSA_NSV; s++)
-          if (s < nspec) a.src[s] += (KT)(klt * w.v(s, lg));
+          if (s < nspec) a.add_src(s, (KT)(klt * w.v(s, lg)), leaf);
       }
     }
     return;
@@ -1680,26 +1768,26 @@ __device__ void precip_formation(const DevParams &P, const WS<KT, LS> &w, const 
           for (int s = 0; s < nspec; s++) sl[1 + s] = w.v(s, lg) * nt * klt * fix;
           dnum = (0.5 * klt * nl * nt) * fix;
           sl[9] = w.indef[lg] * dnum;
-          a.self += (KT)(0.5 * klt * nt);
+          a.add_self((KT)(0.5 * klt * nt), lane);
         } else {
           for (int s = 0; s < nspec; s++) sl[1 + s] = (w.v(s, lg) * nt + w.v(s, tg) * nl) * klt * fix;
           dnum = (klt * nl * nt) * fix;
           sl[9] = 0.5 * (w.indef[lg] + w.indef[tg]) * dnum;
-          a.sink += (KT)((double)kget(w, tg, lg) * nl);
+          a.add_sink((KT)((double)kget(w, tg, lg) * nl), lane);
         }
         dvw = sl[1 + iwa];
         if (diag) {
-          a.dg[0] += (KT)dvw;
-          if (D_new > 50.e-6) a.dg[2] += (KT)dvw;
-          if (D_new > 80.e-6) a.dg[1] += (KT)dvw;
+          a.add_dg(0, (KT)dvw, lane);
+          if (D_new > 50.e-6) a.add_dg(2, (KT)dvw, lane);
+          if (D_new > 80.e-6) a.add_dg(1, (KT)dvw, lane);
         }
       } else {
         sl[0] = -1.;
-        if (selfcoll) a.self += (KT)(0.5 * (double)kget(w, tg, lg) * nl);
+        if (selfcoll) a.add_self((KT)(0.5 * (double)kget(w, tg, lg) * nl), lane);
         else {
 #pragma unroll
           for (int s = 0; s < SALSA_NSV; s++)
-            if (s < nspec) a.src[s] += (KT)(klt * w.v(s, lg));
+            if (s < nspec) a.add_src(s, (KT)(klt * w.v(s, lg)), lane);
         }
       }
       sl[8] = dnum;
@@ -1744,7 +1832,7 @@ __device__ void coag_cloud(const DevParams &P, const WS<KT, LS> &w, const double
       int tg = C0 + kk;
       if (num_lt(w.numc[tg], K_NLIM)) continue;
       TAccT<KT, LS> a;
-      a.zero();
+      a.zero(w);
       if (autoc1) {
         for (int e = lane; e < 7 + nprc * 9; e += LS) pf[e] = 0.;
         wsync<LS>();
@@ -1762,33 +1850,42 @@ __device__ void coag_cloud(const DevParams &P, const WS<KT, LS> &w, const double
           double fix = fmax(1. - dt * (ddiv(0.5 * (double)kget(w, tg, tg) * (n * n), n)), 0.1);
           precip_formation(P, w, tb, kk, kk, kk, fix, true, a, diag, lane);
         } else if (lane == 0) {
-          a.self += (KT)0.5 * kget(w, tg, tg) * w.nk(tg);
+          a.add_self((KT)0.5 * kget(w, tg, tg) * w.nk(tg), 0);
         }
       }
       if (P.lscgca) {
         int iaa = P.ica_par + rel, iab = P.icb_par + rel;
-        KT cm = 0;
         for (int ll = P.in1a + lane; ll <= iaa; ll += LS) {
+          const int leaf = (ll - P.in1a) & 31;
           if (!w.on(ll)) continue;
           const KT k = kget(w, ll, tg);
           {
 #pragma unroll
             for (int s = 0; s < SALSA_NSV; s++)
-              if (s < nspec) a.src[s] += k * w.vk(s, ll);
+              if (s < nspec) a.add_src(s, k * w.vk(s, ll), leaf);
           }
-          if (diag) for (int s = 0; s < P.ndry; s++) cm += k * w.vk(s, ll) * (KT)P.rholiq[s];
+          if (diag) {
+            KT cm = a.cm_get(leaf);
+            for (int s = 0; s < P.ndry; s++) cm += k * w.vk(s, ll) * (KT)P.rholiq[s];
+            a.cm_put(leaf, cm);
+          }
         }
         for (int ll = P.in2b + lane; ll <= iab; ll += LS) {
+          const int leaf = (ll - P.in2b) & 31;
           if (!w.on(ll)) continue;
           const KT k = kget(w, ll, tg);
           {
 #pragma unroll
             for (int s = 0; s < SALSA_NSV; s++)
-              if (s < nspec) a.src[s] += k * w.vk(s, ll);
+              if (s < nspec) a.add_src(s, k * w.vk(s, ll), leaf);
           }
-          if (diag) for (int s = 0; s < P.ndry; s++) cm += k * w.vk(s, ll) * (KT)P.rholiq[s];
+          if (diag) {
+            KT cm = a.cm_get(leaf);
+            for (int s = 0; s < P.ndry; s++) cm += k * w.vk(s, ll) * (KT)P.rholiq[s];
+            a.cm_put(leaf, cm);
+          }
         }
-        a.dg[6] += cm;
+        a.cm_add();
       }
       if (P.lscgcc && kk > kfirst) {
         if (autoc1) {
@@ -1850,48 +1947,55 @@ __device__ void coag_precp(const DevParams &P, const WS<KT, LS> &w, const double
     int tg = P0 + kk;
     if (num_lt(w.numc[tg], K_PRLIM)) continue;
     TAccT<KT, LS> a;
-    a.zero();
+    a.zero(w);
     double num_slf = 0.;
     list_sinks(w, L, tg, a, lane);
     if constexpr (SIP) {
       if (P.st_secice && P.lscgip && lane == 0) sip_drop_numbers<KT>(P, w, tg, kk, K_PRLIM);
       wsync<LS>();
     }
-    if (P.lscgpp && kk == nprc - 1 && lane == 0) a.self += (KT)0.5 * kget(w, tg, tg) * w.nk(tg);
-    const double D = w.dwet[tg];
+    if (P.lscgpp && kk == nprc - 1 && lane == 0) a.add_self((KT)0.5 * kget(w, tg, tg) * w.nk(tg), 0);
+    const double D = w.dwet[tg], D3 = cube(D);
+    const bool lt80 = num_gt(D, 0.) && num_lt(D, 80.e-6), lt50 = num_gt(D, 0.) && num_lt(D, 50.e-6);
+    const bool bin80 = num_gt(pbins[kk], 80.e-6), bin50 = num_gt(pbins[kk], 50.e-6);
     if (P.lscgpa) {
-      KT cm = 0;
       for (int ll = P.in1a + lane; ll <= P.fn2b; ll += LS) {
+        const int leaf = (ll - P.in1a) & 31;
         if (!w.on(ll)) continue;
         const KT k = kget(w, ll, tg);
         {
 #pragma unroll
           for (int s = 0; s < SALSA_NSV; s++)
-            if (s < nspec) a.src[s] += k * w.vk(s, ll);
+            if (s < nspec) a.add_src(s, k * w.vk(s, ll), leaf);
         }
-        if (diag) for (int s = 0; s < P.ndry; s++) cm += k * w.vk(s, ll) * (KT)P.rholiq[s];
+        if (diag) {
+          KT cm = a.cm_get(leaf);
+          for (int s = 0; s < P.ndry; s++) cm += k * w.vk(s, ll) * (KT)P.rholiq[s];
+          a.cm_put(leaf, cm);
+        }
       }
-      a.dg[6] += cm;
+      a.cm_add();
     }
     if (P.lscgpc) {
       // source from cloud; accretion and autoconversion diagnostics (:1086-1215, coll phase 2)
       for (int ll = lane; ll < P.ncld; ll += LS) {
         int g = C0 + ll;
+        const int leaf = ll & 31;
         if (!w.on(g)) continue;
         const KT k = kget(w, g, tg);
         {
 #pragma unroll
           for (int s = 0; s < SALSA_NSV; s++)
-            if (s < nspec) a.src[s] += k * w.vk(s, g);
+            if (s < nspec) a.add_src(s, k * w.vk(s, g), leaf);
         }
         if (diag) {
           const KT kw = k * w.vk(iwa, g);
-          a.dg[3] += kw;
-          double dd = cube(D) + cube(w.dwet[g]);
-          if (D > 0. && D < 80.e-6 && dd > cube(80.e-6)) a.dg[1] += kw;
-          if (D > 0. && D < 50.e-6 && dd > cube(50.e-6)) a.dg[2] += kw;
-          if (pbins[kk] > 80.e-6) a.dg[4] += kw;
-          if (pbins[kk] > 50.e-6) a.dg[5] += kw;
+          a.add_dg(3, kw, leaf);
+          double dd = D3 + cube(w.dwet[g]);
+          if (lt80 && num_gt(dd, cube(80.e-6))) a.add_dg(1, kw, leaf);
+          if (lt50 && num_gt(dd, cube(50.e-6))) a.add_dg(2, kw, leaf);
+          if (bin80) a.add_dg(4, kw, leaf);
+          if (bin50) a.add_dg(5, kw, leaf);
         }
       }
     }
@@ -1899,20 +2003,21 @@ __device__ void coag_precp(const DevParams &P, const WS<KT, LS> &w, const double
       int ex80 = min(kk - 1, P.cnt80 - 1), ex50 = min(kk - 1, P.cnt50 - 1);
       for (int ll = lane; ll <= kk - 1; ll += LS) {
         int g = P0 + ll;
+        const int leaf = ll & 31;
         if (!w.on(g)) continue;
         const KT k = kget(w, g, tg);
         {
 #pragma unroll
           for (int s = 0; s < SALSA_NSV; s++)
-            if (s < nspec) a.src[s] += k * w.vk(s, g);
+            if (s < nspec) a.add_src(s, k * w.vk(s, g), leaf);
         }
         if (diag) {
           const KT kw = k * w.vk(iwa, g);
-          double dd = cube(D) + cube(w.dwet[g]);
-          if (ll <= ex80 && D > 0. && D < 80.e-6 && dd > cube(80.e-6)) a.dg[1] += kw;
-          if (ll <= ex50 && D > 0. && D < 50.e-6 && dd > cube(50.e-6)) a.dg[2] += kw;
-          if (ll <= ex80 && pbins[kk] > 80.e-6) a.dg[4] += kw;
-          if (ll <= ex50 && pbins[kk] > 50.e-6) a.dg[5] += kw;
+          double dd = D3 + cube(w.dwet[g]);
+          if (ll <= ex80 && lt80 && num_gt(dd, cube(80.e-6))) a.add_dg(1, kw, leaf);
+          if (ll <= ex50 && lt50 && num_gt(dd, cube(50.e-6))) a.add_dg(2, kw, leaf);
+          if (ll <= ex80 && bin80) a.add_dg(4, kw, leaf);
+          if (ll <= ex50 && bin50) a.add_dg(5, kw, leaf);
         }
       }
     }
@@ -1971,20 +2076,21 @@ __device__ void coag_ice(const DevParams &P, const WS<KT, LS> &w, const double *
     int tg = I0 + kk;
     if (num_lt(w.numc[tg], K_PRLIM)) continue;
     TAccT<KT, LS> a;
-    a.zero();
+    a.zero(w);
     double rf_t = rimefrac(P, w.numc[tg], w.v(iwa, tg), w.v(irim, tg), 4);
     if (P.lscgii) {
       // Eagg from the larger rime fraction of the pair (:758-769)
       for (int ll = kk + 1 + lane; ll <= nice - 1; ll += LS) {
         int g = I0 + ll;
+        const int leaf = (ll - (kk + 1)) & 31;
         if (!w.on(g)) continue;
         double rf = fmax(rimefrac(P, w.numc[g], w.v(iwa, g), w.v(irim, g), 4), rf_t);
         double E = P.Eiagg_max - rf * (P.Eiagg_max - P.Eiagg_min);
-        a.sink += (KT)E * (KT)1.0 * kget(w, tg, g) * w.nk(g);
+        a.add_sink((KT)E * (KT)1.0 * kget(w, tg, g) * w.nk(g), leaf);
       }
       if (lane == 0) {
         double E = P.Eiagg_max - fmax(rf_t, rf_t) * (P.Eiagg_max - P.Eiagg_min);
-        a.self += (KT)E * (KT)0.5 * kget(w, tg, tg) * w.nk(tg);
+        a.add_self((KT)E * (KT)0.5 * kget(w, tg, tg) * w.nk(tg), 0);
       }
     }
     if constexpr (SIP) {
@@ -2003,50 +2109,64 @@ __device__ void coag_ice(const DevParams &P, const WS<KT, LS> &w, const double *
     // accumulateSourcePhaseChange (:1244-1280)
     if (P.lscgia)
       for (int ll = P.in1a + lane; ll <= P.fn2b; ll += LS) {
+        const int leaf = (ll - P.in1a) & 31;
         if (!w.on(ll)) continue;
         const KT k = kget(w, ll, tg);
         {
 #pragma unroll
           for (int s = 0; s < SALSA_NSV; s++)
-            if (s < ndry) a.src[s] += k * w.vk(s, ll);
+            if (s < ndry) a.add_src(s, k * w.vk(s, ll), leaf);
         }
-        a.add_at(iwa, divc(k * w.vk(iwa, ll) * (KT)K_RHOWA, (KT)K_RHOIC));
+        const KT xw = divc(k * w.vk(iwa, ll) * (KT)K_RHOWA, (KT)K_RHOIC);
+#pragma unroll
+        for (int s = 0; s < SALSA_NSV; s++)
+          if (s == iwa) a.add_src(s, xw, leaf);
       }
     if (P.lscgic)
       for (int ll = lane; ll < P.ncld; ll += LS) {
         int g = C0 + ll;
+        const int leaf = ll & 31;
         if (!w.on(g)) continue;
         const KT k = kget(w, g, tg);
         {
 #pragma unroll
           for (int s = 0; s < SALSA_NSV; s++)
-            if (s < ndry) a.src[s] += k * w.vk(s, g);
+            if (s < ndry) a.add_src(s, k * w.vk(s, g), leaf);
         }
-        a.add_at(irim, divc(k * w.vk(iwa, g) * (KT)K_RHOWA, (KT)K_RHORI));
+        const KT xw = divc(k * w.vk(iwa, g) * (KT)K_RHOWA, (KT)K_RHORI);
+#pragma unroll
+        for (int s = 0; s < SALSA_NSV; s++)
+          if (s == irim) a.add_src(s, xw, leaf);
       }
     if (P.lscgip)
       for (int ll = lane; ll < P.nprc; ll += LS) {
         int g = P0 + ll;
+        const int leaf = ll & 31;
         if (!w.on(g)) continue;
         const KT k = kget(w, g, tg);
         {
 #pragma unroll
           for (int s = 0; s < SALSA_NSV; s++)
-            if (s < ndry) a.src[s] += k * w.vk(s, g);
+            if (s < ndry) a.add_src(s, k * w.vk(s, g), leaf);
         }
-        a.add_at(irim, divc(k * w.vk(iwa, g) * (KT)K_RHOWA, (KT)K_RHORI));
+        const KT xw = divc(k * w.vk(iwa, g) * (KT)K_RHOWA, (KT)K_RHORI);
+#pragma unroll
+        for (int s = 0; s < SALSA_NSV; s++)
+          if (s == irim) a.add_src(s, xw, leaf);
       }
     // accumulateSourceIce (:1385-1427)
     if (P.lscgii && kk > 0)
       for (int ll = lane; ll <= kk - 1; ll += LS) {
         int g = I0 + ll;
+        const int leaf = ll & 31;
+        if (!w.on(g)) continue;
         double rf = fmax(rimefrac(P, w.numc[g], w.v(iwa, g), w.v(irim, g), 4), rf_t);
         double E = P.Eiagg_max - rf * (P.Eiagg_max - P.Eiagg_min);
         const KT k = kget(w, g, tg);
         {
 #pragma unroll
           for (int s = 0; s < SALSA_NSV; s++)
-            if (s < nspec) a.src[s] += (KT)E * k * w.vk(s, g);
+            if (s < nspec) a.add_src(s, (KT)E * k * w.vk(s, g), leaf);
         }
       }
     a.reduce(false, lane);
@@ -2871,10 +2991,18 @@ __device__ void gpparth2o(const DevParams &P, const WS<KT, LS> &w, const double 
           if (have != b) q = load(b);   // layouts of fewer than 32 bins leave some leaves empty
           have = b + 32 < ntot ? b + 32 : ln;
           if (have < ntot) nx = load(have);
-          substep_bin(b, q);
-          const double p = b >= P.in2a ? q.m * q.ws : 0., sf = b < I0 ? sfl : sfi;
+          // a bin without transfer coefficient keeps its water and adds nothing to the vapour sum
+          const bool still = __double_as_longlong(q.am) == 0 && __double_as_longlong(q.c) >= 0;
+          double ps = 0.;
+          if (!still) {
+            substep_bin(b, q);
+            const double p = b >= P.in2a ? q.m * q.ws : 0., sf = b < I0 ? sfl : sfi;
+            ps = b == l ? p * sf : fma(p, sf, y);
+          } else if (b != l) {
+            ps = y;
+          }
           x = b == l ? q.c : x + q.c;
-          y = b == l ? p * sf : fma(p, sf, y);
+          y = ps;
         }
         if (!(k & 1)) { x4 = x; y4 = y; continue; }
         x = x4 + x; y = y4 + y;
@@ -3370,11 +3498,11 @@ __device__ JimmPre jimm_pre(double Tk, double Seq) {
   if (r.d_g <= 1e-10) r.ok = false;
   return r;
 }
-// kth = K_BOLTZ * Tk / K_PLANCK, taken once per cell
-__device__ double J_imm(const JimmPre &q, double theta, double Tk, double Din, double kth) {
+// kth = K_BOLTZ * Tk / K_PLANCK, taken once per cell; x = Din / d_g, once per bin
+__device__ double J_imm(const JimmPre &q, double theta, double Tk, double Din, double x, double kth) {
   if (Din < 1e-10 || !q.ok) return 0.;
   double costh = cos(divc(theta * K_PI, 180.));
-  double sf = het_sf(ddiv(Din, q.d_g), costh);
+  double sf = het_sf(x, costh);
   double crit = mrn(mrn(mrn((K_PI / 3.), q.sigma_is), mrn(q.d_g, q.d_g)), sf) -
                 mrn(mrn(mrn((1. / 4.) * 0.0, (1. - costh)), Din), Din);
   return kth * 1.e19 * K_PI * (Din * Din) * dexp(-ddiv(q.act_energy + crit, K_BOLTZ * Tk));
@@ -3530,6 +3658,7 @@ __device__ void ice_nucl_SE(const DevParams &P, const WS<KT, LS> &w, const doubl
     r[R_FHOM] = f_hom;
     r[R_MODE] = imm ? 1. : (dep ? 2. : 0.);
     r[R_DIN] = w.ddry[kk];
+    double fint = 0.;
     if (imm) {
       // low_theta (:394-417)
       double th00 = P.mean_theta_imm + mrn(sqrt(2.) * P.sigma_theta_imm, erfm1(mrn(2., w.indef[kk]) - 1.));
@@ -3537,13 +3666,14 @@ __device__ void ice_nucl_SE(const DevParams &P, const WS<KT, LS> &w, const doubl
       if (!P.st_freeTheta) th00 = fmax(P.initMinTheta, th00);
       JimmPre q = jimm_pre(T, Seq);
       r[R_THMIN] = th00; r[R_AE] = q.act_energy; r[R_SIG] = q.sigma_is; r[R_DG] = q.ok ? q.d_g : -1.;
+      fint = q.ok ? ddiv(r[R_DIN], q.d_g) : 0.;   // the integrand's size ratio, until the integral takes its place
     } else if (dep) {
       double th00 = P.mean_theta_dep + mrn(sqrt(2.) * P.sigma_theta_dep, erfm1(mrn(2., w.indef[kk]) - 1.));
       th00 = fmin(fmax(th00, 0.), 180.);
       if (!P.st_freeTheta) th00 = fmax(P.initMinTheta, th00);
       r[R_THMIN] = th00;
     }
-    r[R_FINT] = 0.;
+    r[R_FINT] = fint;
   }
   wsync<LS>();
   // pass B: gauss_legendre (:131-206) for the bins that need it
@@ -3557,7 +3687,7 @@ __device__ void ice_nucl_SE(const DevParams &P, const WS<KT, LS> &w, const doubl
     if (r[R_MODE] == 1.) {
       JimmPre q;
       q.act_energy = r[R_AE]; q.sigma_is = r[R_SIG]; q.d_g = r[R_DG]; q.ok = r[R_DG] >= 0.;
-      J = J_imm(q, th1, T, r[R_DIN], kth);
+      J = J_imm(q, th1, T, r[R_DIN], r[R_FINT], kth);
       ft = th1 > thmin ? f_gauss(th1, g_imm) : 0.;
     } else {
       J = J_dep(th1, T, r[R_DIN], Si);
@@ -4211,7 +4341,7 @@ __device__ __forceinline__ bool lane_output(const DevParams &P, const WS<KT, 1> 
   return bad;
 }
 
-template <typename KT, bool DIAG, bool SIP, int LS>
+template <typename KT, bool SIP, int LS>
 __device__ __forceinline__ void cell_step(const DevParams &P, WS<KT, LS> &w, const double *tb, long long cell,
                                           int lane) {
 #ifdef SALSA_STAGE_TIMERS
@@ -4272,7 +4402,7 @@ __device__ __forceinline__ void cell_step(const DevParams &P, WS<KT, LS> &w, con
   STAGE_MARK(0);
 
   // ---- salsa() ----
-  if (P.st_coag) coagulation<KT, SIP>(P, w, tb, dt, T, pres, DIAG, cell, lane);
+  if (P.st_coag) coagulation<KT, SIP>(P, w, tb, dt, T, pres, true, cell, lane);
   if constexpr (SIP) {
     if (P.st_secice) secondary_ice<KT>(P, w, tb, T, pres, rv, rsi, dt, lane);
   }
@@ -4284,18 +4414,18 @@ __device__ __forceinline__ void cell_step(const DevParams &P, WS<KT, LS> &w, con
     // clusters: 1 for nsnucl = 1-3; for the mixed schemes it only multiplies condgas's
     // vanishing nucleation term, and 1 stands in
     if (P.lscndgas) condgas<KT>(P, w, tb, T, pres, dt, w.misc + M_GAS, P.nsnucl > 0 ? 1. : 0., lane);
-    if (P.lscndh2ocl || P.lscndh2oae || P.lscndh2oic) gpparth2o<KT>(P, w, tb, T, pres, rs, rsi, rv, dt, kappa, DIAG, lane);
+    if (P.lscndh2ocl || P.lscndh2oae || P.lscndh2oic) gpparth2o<KT>(P, w, tb, T, pres, rs, rsi, rv, dt, kappa, true, lane);
   }
   stage_sync<LS>();
   STAGE_MARK(2);
   if (P.st_auto && P.auto_mode == 2) autoconv2<KT>(P, w, dt, lane);
-  if (P.st_activ && P.activ_mode == 1) act_interst<KT>(P, w, tb, rv, rs, T, DIAG, lane);
+  if (P.st_activ && P.activ_mode == 1) act_interst<KT>(P, w, tb, rv, rs, T, true, lane);
   if (P.st_activ && P.activ_mode == 2) act_cloudbase<KT>(P, w, tb, pres, T, raw[RW_W], dn, raw, lane);
   stage_sync<LS>();
   STAGE_MARK(3);
   if ((P.st_icenucl || P.icenucl_mode == 2) && (P.lsicehom || P.lsiceimm || P.lsicedep)) {
-    if (P.ice_theta_dist) ice_nucl_SE<KT>(P, w, tb, T, rv, rs, rsi, dt, kappa, DIAG, lane);
-    else ice_nucl_classic<KT>(P, w, tb, T, rv, rs, rsi, dt, kappa, DIAG, lane);
+    if (P.ice_theta_dist) ice_nucl_SE<KT>(P, w, tb, T, rv, rs, rsi, dt, kappa, true, lane);
+    else ice_nucl_classic<KT>(P, w, tb, T, rv, rs, rsi, dt, kappa, true, lane);
   }
   if constexpr (SIP) {
     // ice_melt's bins (numbers not below prlim) before it runs: their tracers melt with them
@@ -4366,7 +4496,7 @@ __device__ __forceinline__ void cell_step(const DevParams &P, WS<KT, LS> &w, con
   if (P.raw_gas >= 0)   // :369-384
     for (int i = lane; i < 5; i += LS)
       raw[P.raw_gas + i] = ddiv((ddiv(w.misc[M_GAS + i], dn)) - raw[P.raw_gas + i], dt);
-  if (DIAG && P.raw_diag >= 0 && lane == 0) {
+  if (P.raw_diag >= 0 && lane == 0) {
     const auto d = w.misc + M_DIAG;
     const auto o = raw + P.raw_diag;
     o[DG_AUTOC] = ddiv(d[DG_AUTOC] * K_RHOWA, dn);
@@ -4430,11 +4560,12 @@ __device__ __forceinline__ WS<KT, LS> make_ws(const DevParams &P, Ptr<double, LS
   if constexpr (LS != 1) w.pbuf = reinterpret_cast<int *>(p);
   p = p + 64;   // 128 ints: bin lists (<= 96) and pair batches (<= 63)
   w.K = row_cast<KT>(p);
+  if constexpr (LS == 1 && sizeof(KT) == 4) w.lf = row_cast<float>(base + P.ws_doubles);
   return w;
 }
 
 
-template <typename KT, bool DIAG, bool SIP>
+template <typename KT, bool SIP>
 __global__ void __launch_bounds__(SALSA_THREADS, 2) salsa_step_kernel(const DevParams P) {
   extern __shared__ double smem[];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -4461,7 +4592,7 @@ __global__ void __launch_bounds__(SALSA_THREADS, 2) salsa_step_kernel(const DevP
       }
     __syncthreads();
     long long q = g * SALSA_CPG + warp;
-    if (q < P.ncells) cell_step<KT, DIAG, SIP>(P, w, tb, cell_at(P, q), lane);
+    if (q < P.ncells) cell_step<KT, SIP>(P, w, tb, cell_at(P, q), lane);
     __syncthreads();
     // write the group's output rows
     if (okc)
@@ -4491,7 +4622,7 @@ __global__ void __launch_bounds__(SALSA_THREADS, 2) salsa_step_kernel(const DevP
 // 1.1 M cell block takes 78 ms, where the warp form took 299 ms.  Four blocks of 128 threads
 // per SM (128 registers) measured better than three (164 registers): clear cells 39.3
 // against 43.9 ns a cell, cloudy ones 397 against 455; the FP64 pipe is 71-80 % busy.
-template <typename KT, bool DIAG, bool SIP>
+template <typename KT, bool SIP>
 __global__ void __launch_bounds__(32 * SALSA_LANE_WARPS, SALSA_LANE_MINBLOCKS) salsa_lane_kernel(const DevParams P) {
   extern __shared__ double smem[];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -4499,7 +4630,7 @@ __global__ void __launch_bounds__(32 * SALSA_LANE_WARPS, SALSA_LANE_MINBLOCKS) s
   for (int i = tid; i < P.tab_doubles; i += 32 * SALSA_LANE_WARPS) tb[i] = P.tables[i];
   __syncthreads();
   WS<KT, 1> w = make_ws<KT, 1>(
-      P, Col<double>{P.lane_ws + ((size_t)blockIdx.x * SALSA_LANE_WARPS + warp) * (size_t)P.ws_doubles * 32 + lane});
+      P, Col<double>{P.lane_ws + ((size_t)blockIdx.x * SALSA_LANE_WARPS + warp) * (size_t)P.lane_rows * 32 + lane});
   const long long ntiles = (P.ncells + 31) / 32;
   __shared__ unsigned long long next;
   for (;;) {
@@ -4526,7 +4657,7 @@ __global__ void __launch_bounds__(32 * SALSA_LANE_WARPS, SALSA_LANE_MINBLOCKS) s
     const bool nact0 = !(P.st_activ && P.activ_mode == 2);   // no activated droplets to report
     stage(0, P.raw_num);
     stage(nact0 ? P.raw_diag : P.raw_nact, P.nrows);
-    cell_step<KT, DIAG, SIP>(P, w, tb, cell, 0);
+    cell_step<KT, SIP>(P, w, tb, cell, 0);
     __syncwarp();
     if (w.live) {
       for (int r = 0; r < P.nrows; r = r + 1 == P.raw_num ? P.raw_nact : r + 1) {
@@ -4548,38 +4679,38 @@ inline size_t smem_bytes(const DevParams &P) {
   return sizeof(double) * ((size_t)P.tab_doubles + (size_t)SALSA_CPG * P.ws_doubles);
 }
 
-template <typename KT, bool DIAG, bool SIP = false>
+template <typename KT, bool SIP = false>
 cudaError_t launch_t(const DevParams &P, cudaStream_t st, int grid) {
   size_t sm = smem_bytes(P);
   cudaError_t e =
-      cudaFuncSetAttribute(salsa_step_kernel<KT, DIAG, SIP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+      cudaFuncSetAttribute(salsa_step_kernel<KT, SIP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
   if (e != cudaSuccess) return e;
-  salsa_step_kernel<KT, DIAG, SIP><<<grid, SALSA_THREADS, sm, st>>>(P);
+  salsa_step_kernel<KT, SIP><<<grid, SALSA_THREADS, sm, st>>>(P);
   return cudaGetLastError();
 }
 
-template <typename KT, bool DIAG, bool SIP = false>
+template <typename KT, bool SIP = false>
 cudaError_t launch_lane_t(const DevParams &P, cudaStream_t st, int grid) {
-  salsa_lane_kernel<KT, DIAG, SIP><<<grid, 32 * SALSA_LANE_WARPS, sizeof(double) * (size_t)P.tab_doubles, st>>>(P);
+  salsa_lane_kernel<KT, SIP><<<grid, 32 * SALSA_LANE_WARPS, sizeof(double) * (size_t)P.tab_doubles, st>>>(P);
   return cudaGetLastError();
 }
-template <typename KT, bool DIAG, bool SIP = false>
+template <typename KT, bool SIP = false>
 int lane_blocks_per_sm_t(const DevParams &P) {
   int nb = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, salsa_lane_kernel<KT, DIAG, SIP>, 32 * SALSA_LANE_WARPS,
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, salsa_lane_kernel<KT, SIP>, 32 * SALSA_LANE_WARPS,
                                                     sizeof(double) * (size_t)P.tab_doubles) != cudaSuccess)
     return 0;
   return nb;
 }
 
-template <typename KT, bool DIAG, bool SIP = false>
+template <typename KT, bool SIP = false>
 int blocks_per_sm_t(const DevParams &P) {
   size_t sm = smem_bytes(P);
-  if (cudaFuncSetAttribute(salsa_step_kernel<KT, DIAG, SIP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm) !=
+  if (cudaFuncSetAttribute(salsa_step_kernel<KT, SIP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm) !=
       cudaSuccess)
     return 0;
   int nb = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, salsa_step_kernel<KT, DIAG, SIP>, SALSA_THREADS, sm) !=
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, salsa_step_kernel<KT, SIP>, SALSA_THREADS, sm) !=
       cudaSuccess)
     return 0;
   return nb;
