@@ -78,7 +78,7 @@ enum {
 
 // status counters
 enum { ST_CELLS = 0, ST_EQUIL, ST_DISTR, ST_NEGFRAC, ST_COND, ST_NEG, ST_NONFINITE,
-       ST_ORDER_CLEAR, ST_ORDER_CLOUDY,   // fill counters of the cell order list
+       ST_ORDER_CLEAR, ST_ORDER_CLOUDY, ST_ORDER_MOIST,   // fill counters of the cell order lists
        ST_TILE,                           // the lane form's next tile of 32 cells
        ST_N };
 
@@ -135,7 +135,8 @@ struct DevParams {
   const double *tables;     // bin tables (see TAB_* offsets)
   const int *pairs;         // packed pair list (i | j << 8)
   unsigned long long *status;
-  const int *order;         // processing order of the cells (clear cells first), or null
+  const int *order;         // clear cells from the front, cloudy ones from the back, or null
+  const int *order_moist;   // clear cells near saturation, or null (then they are in `order`)
   unsigned long long *stage_clocks;   // per-stage clock sums (instrumented builds only)
   // secondary ice (mo_salsa_secondary_ice.f90): states of lssecice and the three schemes,
   // the schemes' modes, the first splinter bin (1-based, mo_salsa_SIP_RS.f90:72) and the
@@ -173,6 +174,12 @@ __device__ __forceinline__ long long cell_offset(const DevParams &P, long long q
   long long iq = r % P.nx_int, jq = r / P.nx_int;
   return (1 + kq) + (long long)P.nzp * ((2 + iq) + (long long)P.nxp * (2 + jq));
 }
-__device__ __forceinline__ long long cell_at(const DevParams &P, long long i) { return P.order ? P.order[i] : i; }
+// the i-th cell in processing order: dry clear cells, moist clear ones, cloudy ones
+__device__ __forceinline__ long long cell_at(const DevParams &P, long long i) {
+  if (!P.order) return i;
+  if (!P.order_moist) return P.order[i];
+  const long long nd = (long long)P.status[ST_ORDER_CLEAR], nm = (long long)P.status[ST_ORDER_MOIST];
+  return i < nd ? P.order[i] : (i < nd + nm ? P.order_moist[i - nd] : P.order[P.ncells - 1 - (i - nd - nm)]);
+}
 
 }  // namespace salsa
