@@ -26,14 +26,13 @@ namespace {
 //     and marks the levels it changes; pass B gathers, for every marked level, the
 //     contributions of the sources in the order the reference adds them (sources from
 //     the top down, a level's removal of its own parcel before its re-deposit).
-// The FP64 pipe bounds it: a column of 128 levels moves 0.6 ms worth of bytes per million
-// points and computes for 6.  So the surface level's dry deposition (two powers and six
+// The FP64 pipe bounds it: a full pass over a million points moves bytes for 1.2 ms.  So the surface level's dry deposition (two powers and six
 // quotients) is taken for 32 bins at a time, one per lane, before their loop, where one lane
 // of the first round did it for every bin; the flux divergence is two products per species
 // with the level's coefficients; the shares of a falling parcel are taken once per source;
 // the number limits are compared as integers; an ice crystal's shape and dimension share their
 // limits.  grid256x256x128, 96 x 96 columns, all four parts: 13.7 ms before the fast division
-// and roots, 10.8 with them, 7.9 now.
+// and roots, 10.8 with them, 7.9 with these, 7.7 with four blocks of 55 KB per SM instead of three of 66.
 // Levels and bins that the reference visits only to add a zero are skipped.  The sums
 // over bins (rrate, tlt, the surface rates) run in the reference's index order,
 // including the range (ns-1)*nb:ns*nb of its water sums, which starts at the last bin
@@ -52,7 +51,7 @@ constexpr double R_PI6 = 1. / K_PI6;
 constexpr int SED_KF = 0xffff, SED_BR = 1 << 16, SED_DEP = 1 << 17;   // pass-A code: kf | branch | deposited
 constexpr int SED_NS = SALSA_MAXSPEC + 2;   // species slots of a bin (wet species and rime)
 // per-warp shared arrays of nzp doubles
-enum { W_AD = 0, W_AVIS, W_LAM, W_ILAM, W_R18, W_Q, W_TLT, W_RR, W_IR, W_VC, W_P0, W_P1, W_P2, W_P3, W_N,
+enum { W_AD = 0, W_LAM, W_ILAM, W_R18, W_Q, W_RR, W_VC, W_P0, W_P1, W_P2, W_P3, W_N,
        W_G1 = W_Q };   // W_Q serves the slow part, W_G1 the fast one after it
 
 struct SedArgs {
@@ -99,7 +98,7 @@ __device__ double ice_form(const DevParams &P, double mpri, double mrim, double 
 // fall speed of one bin at one level (:999-1011, :1148-1173): wet diameter
 // (calcDiamLES), particle density, slip correction GG and terminal_vel
 __device__ __forceinline__ double sed_vel(const SedArgs &A, int flag, int ns, double n, const double (&m)[SED_NS],
-                                          double ad, double avis, double lam, double ilam, double r18v, double &dwet,
+                                          double ad, double lam, double ilam, double r18v, double &dwet,
                                           double &GG) {
   double v = 0., sm = 0.;
 #pragma unroll
@@ -126,7 +125,7 @@ __device__ __forceinline__ double sed_vel(const SedArgs &A, int flag, int ns, do
   const double Kn = 2. * lam * rd;                            // 2 lambda / dwet
   GG = 1. + Kn * (SED_A + SED_B * dexp(-SED_C * 0.5 * dwet * ilam));
   if (flag <= 3 && dwet <= 19E-6) return sq(dwet) * (zdn - ad) * K_GRAV * GG * r18v;   // Stokes, eq. 3.21
-  return terminal_vel<double>(dwet, zdn, ad, avis, GG, flag, sh, dnsp);
+  return terminal_vel<double>(dwet, zdn, ad, drcp(18. * r18v), GG, flag, sh, dnsp);
 }
 
 __device__ __forceinline__ bool act_bit(const unsigned *w, int k) { return (w[k >> 5] >> (k & 31)) & 1u; }
@@ -163,9 +162,9 @@ __device__ void sed_slow(const SedArgs &A, double *sm, const double *blk, long l
                          int flag, const double *numc, const double *mass, double *tn, double *tm, int lane) {
   const int nzp = A.nzp, ns = A.nspec, R = (nzp + 31) >> 5;
   const long long pl = A.plane, ps = pl * nb;
-  const double *ad_s = sm + W_AD * nzp, *avis_s = sm + W_AVIS * nzp, *lam_s = sm + W_LAM * nzp,
+  const double *ad_s = sm + W_AD * nzp, *lam_s = sm + W_LAM * nzp,
                *ilam_s = sm + W_ILAM * nzp, *r18_s = sm + W_R18 * nzp, *q_s = sm + W_Q * nzp;
-  double *tlt_s = sm + W_TLT * nzp, *rr_s = sm + W_RR * nzp, *vc_s = sm + W_VC * nzp;
+  double *rr_s = sm + W_RR * nzp, *vc_s = sm + W_VC * nzp;
   double *rs_s = sm + W_P0 * nzp, *ts_s = sm + W_P1 * nzp, *wr_s = sm + W_P2 * nzp, *wd_s = sm + W_P3 * nzp;
   int *la = (int *)(sm + A.off_int), *lf = la + nzp;
   unsigned *actw = (unsigned *)(lf + nzp);
@@ -185,10 +184,10 @@ __device__ void sed_slow(const SedArgs &A, double *sm, const double *blk, long l
 #pragma unroll
         for (int s = 0; s < SED_NS; s++) m[s] = s < ns ? mass[col + 1 + pl * bl + ps * s] : 0.;
         double dwet, GG;
-        const double vc = fmin(sed_vel(A, flag, ns, n, m, ad_s[1], avis_s[1], lam_s[1], ilam_s[1], r18_s[1], dwet, GG),
+        const double vc = fmin(sed_vel(A, flag, ns, n, m, ad_s[1], lam_s[1], ilam_s[1], r18_s[1], dwet, GG),
                                vmax_b[1]);
         // dry deposition to the surface (:1020-1028)
-        const double T = A.f.tk[col + 1], us = A.f.ustar[c2], avis = avis_s[1];
+        const double T = A.f.tk[col + 1], us = A.f.ustar[c2], avis = drcp(18. * r18_s[1]);
         const double kvis = ddiv(avis, ad_s[1]);
         const double mdiff = ddiv(LES_KB * T * GG, 3.0 * LES_PI * avis * dwet);
         const double Sc = ddiv(kvis, mdiff);
@@ -211,7 +210,7 @@ __device__ void sed_slow(const SedArgs &A, double *sm, const double *blk, long l
 #pragma unroll
       for (int s = 0; s < SED_NS; s++) m[s] = s < ns ? mcol[k + ps * s] : 0.;
       double dwet, GG;
-      const double vc = sed_vel(A, flag, ns, n, m, ad_s[k], avis_s[k], lam_s[k], ilam_s[k], r18_s[k], dwet, GG);
+      const double vc = sed_vel(A, flag, ns, n, m, ad_s[k], lam_s[k], ilam_s[k], r18_s[k], dwet, GG);
       vc_s[k] = k == 1 ? v1b : fmin(vc, vmax_b[k]);
     }
     // the levels with a non-zero divergence: own or upper level populated
@@ -259,7 +258,7 @@ __device__ void sed_slow(const SedArgs &A, double *sm, const double *blk, long l
       if (kc == 1) sr_s[0] = sr_s[0] - rsum * ad_s[kc] * LES_ALVL;
     }
     const double tsum = ts_s[kc] + wd_s[kc];
-    tlt_s[kc] = tlt_s[kc] + ddiv(tsum * (LES_ALVL / LES_CP) * A.f.th[col + kc], A.f.tk[col + kc]);
+    A.f.tlt[col + kc] += ddiv(tsum * (LES_ALVL / LES_CP) * A.f.th[col + kc], A.f.tk[col + kc]);
   }
   __syncwarp();
 }
@@ -273,9 +272,9 @@ __device__ void sed_fast(const SedArgs &A, double *sm, const double *blk, long l
   const long long pl = A.plane, ps = pl * nb;
   const double alv = flag == 4 ? LES_ALVI : LES_ALVL;
   const int iw = flag == 4 ? ns - 2 : ns - 1;   // water; for ice the rime follows it
-  const double *ad_s = sm + W_AD * nzp, *avis_s = sm + W_AVIS * nzp, *lam_s = sm + W_LAM * nzp,
+  const double *ad_s = sm + W_AD * nzp, *lam_s = sm + W_LAM * nzp,
                *ilam_s = sm + W_ILAM * nzp, *r18_s = sm + W_R18 * nzp;
-  double *tlt_s = sm + W_TLT * nzp, *vc_s = sm + W_VC * nzp, *f1_s = sm + W_P0 * nzp, *ws_s = sm + W_P2 * nzp,
+  double *vc_s = sm + W_VC * nzp, *f1_s = sm + W_P0 * nzp, *ws_s = sm + W_P2 * nzp,
          *wq_s = sm + W_P3 * nzp, *g1_s = sm + W_G1 * nzp;
   int *kf_s = (int *)(sm + W_P1 * nzp), *tg_s = kf_s + nzp;
   int *la = (int *)(sm + A.off_int), *lt = la + nzp;
@@ -302,7 +301,7 @@ __device__ void sed_fast(const SedArgs &A, double *sm, const double *blk, long l
       for (int s = 0; s < SED_NS; s++) m[s] = s < ns ? mcol[kc + ps * s] : 0.;
       const double ad = ad_s[kc];
       double dwet, GG;
-      const double vc = sed_vel(A, flag, ns, n, m, ad, avis_s[kc], lam_s[kc], ilam_s[kc], r18_s[kc], dwet, GG);
+      const double vc = sed_vel(A, flag, ns, n, m, ad, lam_s[kc], ilam_s[kc], r18_s[kc], dwet, GG);
       vt[kc] = vc;
       const double fdmax = A.dtlt * vc;
       double fd = 0.;
@@ -406,7 +405,7 @@ __device__ void sed_fast(const SedArgs &A, double *sm, const double *blk, long l
     const int L = r * 32 + lane;
     if (L > nzp - 2) continue;
     const double S = flag == 4 ? ws_s[L] + wq_s[L] : ws_s[L];
-    tlt_s[L] = tlt_s[L] - ddiv((S * A.rdtlt) * divc(alv, LES_CP) * A.f.th[col + L], A.f.tk[col + L]);
+    A.f.tlt[col + L] -= ddiv((S * A.rdtlt) * divc(alv, LES_CP) * A.f.th[col + L], A.f.tk[col + L]);
   }
   __syncwarp();
 }
@@ -442,9 +441,9 @@ __global__ void __launch_bounds__(128) sedimentation_kernel(const SedArgs A) {
     return;
   }
   double *sm = sed_smem + 3 * nzp + (size_t)wib * A.warp_doubles;
-  double *ad_s = sm + W_AD * nzp, *avis_s = sm + W_AVIS * nzp, *lam_s = sm + W_LAM * nzp, *ilam_s = sm + W_ILAM * nzp,
+  double *ad_s = sm + W_AD * nzp, *lam_s = sm + W_LAM * nzp, *ilam_s = sm + W_ILAM * nzp,
          *r18_s = sm + W_R18 * nzp, *q_s = sm + W_Q * nzp;
-  double *tlt_s = sm + W_TLT * nzp, *rr_s = sm + W_RR * nzp, *ir_s = sm + W_IR * nzp, *sr_s = sm + A.off_sr;
+  double *rr_s = sm + W_RR * nzp, *sr_s = sm + A.off_sr;
   // air properties per level, atm modelling eq. 4.54 (:986-989)
   for (int k = lane; k < nzp; k += 32) {
     const long long p = col + k;
@@ -460,14 +459,11 @@ __global__ void __launch_bounds__(128) sedimentation_kernel(const SedArgs A) {
       r18 = drcp(18. * avis);
       q = A.f.dzt[k] / ad;
     }
-    avis_s[k] = avis;
     lam_s[k] = lam;
     ilam_s[k] = ilam;
     r18_s[k] = r18;
     q_s[k] = q;
-    tlt_s[k] = A.f.tlt[p];
     rr_s[k] = 0.;
-    ir_s[k] = 0.;
   }
   if (lane == 0) sr_s[0] = sr_s[1] = 0.;
   __syncwarp();
@@ -476,14 +472,16 @@ __global__ void __launch_bounds__(128) sedimentation_kernel(const SedArgs A) {
   if (fprc)
     sed_fast(A, sm, blk, col, A.P.nprc, A.nspec, 3, A.f.nprecp, A.f.mprecp, A.f.nprecpt, A.f.mprecpt, A.f.VtPrc,
              rr_s, sr_s, lane);
-  if (fice)
-    sed_fast(A, sm, blk, col, A.P.nice, A.nspec + 1, 4, A.f.nice, A.f.mice, A.f.nicet, A.f.micet, A.f.VtIce, ir_s,
-             sr_s + 1, lane);
   for (int k = lane; k < nzp; k += 32) {
-    A.f.tlt[col + k] = tlt_s[k];
     A.f.rrate[col + k] = rr_s[k];
-    if (A.lvl5) A.f.irate[col + k] = ir_s[k];
+    rr_s[k] = 0.;   // the same array takes the ice rate
   }
+  __syncwarp();
+  if (fice)
+    sed_fast(A, sm, blk, col, A.P.nice, A.nspec + 1, 4, A.f.nice, A.f.mice, A.f.nicet, A.f.micet, A.f.VtIce, rr_s,
+             sr_s + 1, lane);
+  if (A.lvl5)
+    for (int k = lane; k < nzp; k += 32) A.f.irate[col + k] = rr_s[k];
   if (lane == 0) {
     A.f.sfcrrate[c2] = sr_s[0];
     if (A.lvl5) A.f.sfcirate[c2] = sr_s[1];
@@ -543,7 +541,7 @@ int salsa_gb300_sedimentation(salsa_handle_t *h, int nzp, int nxp, int nyp, doub
   int warps = 4;
   while (warps > 1 && bbytes + warps * wbytes > 100u * 1024u) warps >>= 1;
   const size_t smem = bbytes + warps * wbytes;
-  if (smem > 200u * 1024u) return SALSA_E_UNSUPPORTED;
+  if (smem + warps * (size_t)3 * nzp * sizeof(double) > 200u * 1024u) return SALSA_E_UNSUPPORTED;   // about 1,400 levels
   if (cudaSetDevice(dev) != cudaSuccess) return SALSA_E_NODEV;
   if (smem > 48u * 1024u &&
       cudaFuncSetAttribute(salsa::sedimentation_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
