@@ -18,7 +18,8 @@ ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 FLAGS = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC", "-Xptxas", "-v"]
 UNITS = ["salsa_k_d1.cu", "salsa_k_f1.cu", "salsa_k_ds.cu", "salsa_k_fs.cu",
          "salsa_l_d1.cu", "salsa_l_f1.cu", "salsa_l_ds.cu", "salsa_l_fs.cu",
-         "salsa_chain.cu", "salsa_post.cu", "salsa_sedim.cu", "salsa_capi.cu"]
+         "salsa_chain.cu", "salsa_chain_taped.cu", "salsa_chain_rev.cu",
+         "salsa_post.cu", "salsa_sedim.cu", "salsa_capi.cu"]
 # Units compiled without multiply-add contraction, so that their arithmetic rounds
 # like the reference's x86-64 SSE2 build: the post-step constraints, which match the
 # oracle bit for bit.  The step kernels (both forms), the gradient harness (whose

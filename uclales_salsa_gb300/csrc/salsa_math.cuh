@@ -28,7 +28,7 @@
 //
 // Arguments outside the fast range (zero, subnormal, infinite, NaN, extreme exponents) take
 // the plain operation, out of line.  A unit that defines SALSA_MATH_PLAIN gets the plain
-// operations throughout.
+// operations throughout, one that defines SALSA_MATH_PLAIN_FUNCTIONS CUDA's cbrt, exp, log and pow.
 #pragma once
 #include <cstdint>
 #include "salsa_math_tables.h"
@@ -52,18 +52,10 @@ __device__ __forceinline__ double ddiv(double n, double d) { return n / d; }
 __device__ __forceinline__ double ddiv_r(double n, double d, double) { return n / d; }
 __device__ __forceinline__ double divc(double x, double c) { return x / c; }
 __device__ __forceinline__ double dsqrt(double x) { return sqrt(x); }
-__device__ __forceinline__ double dcbrt(double x) { return cbrt(x); }
-__device__ __forceinline__ double dexp(double x) { return exp(x); }
-__device__ __forceinline__ double dlog(double x) { return log(x); }
-__device__ __forceinline__ double dpow(double x, double y) { return pow(x, y); }
 #else
 // the plain operations, out of line: arguments outside the fast ranges
 __device__ __noinline__ double fm_div_slow(double n, double d) { return n / d; }
 __device__ __noinline__ double fm_sqrt_slow(double x) { return sqrt(x); }
-__device__ __noinline__ double fm_cbrt_slow(double x) { return cbrt(x); }
-__device__ __noinline__ double fm_exp_slow(double x) { return exp(x); }
-__device__ __noinline__ double fm_log_slow(double x) { return log(x); }
-__device__ __noinline__ double fm_pow_slow(double x, double y) { return pow(x, y); }
 
 // the double of bits (hi, lo) plus k * unit ulps: the low part of a two-float seed enters as
 // an integer, read off a float sum with `magic` (1.5 * 2^e, so that the sum's last bit is
@@ -139,6 +131,12 @@ __device__ __forceinline__ double dsqrt(double x) {
   const double hy = __hiloint2double(__double2hiint(y) - 0x00100000, __double2loint(y));   // y/2
   return fma(fma(-s, s, x), hy, s);
 }
+
+#ifndef SALSA_MATH_PLAIN_FUNCTIONS
+__device__ __noinline__ double fm_cbrt_slow(double x) { return cbrt(x); }
+__device__ __noinline__ double fm_exp_slow(double x) { return exp(x); }
+__device__ __noinline__ double fm_log_slow(double x) { return log(x); }
+__device__ __noinline__ double fm_pow_slow(double x, double y) { return pow(x, y); }
 
 // cbrt(x), x positive and normal, or zero
 __device__ __forceinline__ double dcbrt(double x) {
@@ -295,7 +293,15 @@ __device__ __forceinline__ double dpow(double x, double y) {
   return fm_pow_slow(x, y);
 }
 
+#endif  // SALSA_MATH_PLAIN_FUNCTIONS
 #endif  // SALSA_MATH_PLAIN
+
+#if defined(SALSA_MATH_PLAIN) || defined(SALSA_MATH_PLAIN_FUNCTIONS)
+__device__ __forceinline__ double dcbrt(double x) { return cbrt(x); }
+__device__ __forceinline__ double dexp(double x) { return exp(x); }
+__device__ __forceinline__ double dlog(double x) { return log(x); }
+__device__ __forceinline__ double dpow(double x, double y) { return pow(x, y); }
+#endif
 
 // the float forms of templates written for both types
 __device__ __forceinline__ float ddiv(float n, float d) { return n / d; }
