@@ -4,22 +4,23 @@
 // One launch advances every interior grid cell by one SALSA call
 // (UCLALES-SALSA src/src_salsa/mo_salsa_driver.f90:180-427 -> mo_salsa.f90:45-153).
 //
-// Execution model
-//   * block = SALSA_CPG warps = SALSA_CPG interior cells ("group");
-//     the block stages the group's bin-major input rows into shared memory with
-//     sector-complete loads (SALSA_CPG consecutive doubles per row), every warp
-//     advances its own cell out of shared memory, and the block writes the
-//     tendency rows back with read-modify-write of SALSA_CPG-cell segments.
-//   * inside a cell, lanes split bins (diameters, condensation, activation,
-//     freezing) and bin pairs (collision kernels); the Gauss-Seidel bin sweep of
-//     the coagulation update stays ordered, each target bin's partner sums are
+// Execution model: two forms of the same templates (LS lanes advance one cell)
+//   * warp form (LS = 32, salsa_step_kernel): block = SALSA_CPG warps = SALSA_CPG interior
+//     cells ("group"); the block stages the group's bin-major input rows into shared memory
+//     with sector-complete loads, every warp advances its own cell out of shared memory,
+//     lanes split bins (diameters, condensation, activation, freezing) and bin pairs
+//     (collision kernels), and the block writes the tendency rows back.  The Gauss-Seidel
+//     bin sweep of the coagulation update stays ordered; each target bin's partner sums are
 //     lane-parallel and reduced with warp shuffles.
+//   * lane form (LS = 1, salsa_lane_kernel): every lane advances a cell of its own out of a
+//     workspace in global memory, for calls with enough cells to fill the lanes.  The FP64
+//     pipe, which bounds both forms, takes as long for one lane as for 32.
 //   * KT is the arithmetic type of the collision kernels and of the condensation
 //     mass-transfer coefficients: double for the parity form, float for the mixed
 //     form (whose partner sums are compensated float sums; denominators, the water
 //     budget and all state updates stay double).
-//   * a pre-pass orders the cells so that the cells of one block share a class
-//     (all-clear or cloudy); a block's cells are then not always neighbours.
+//   * a pre-pass orders the cells so that the cells of one block or warp share a class
+//     (dry clear, moist clear or cloudy); they are then not always neighbours.
 #pragma once
 #include "salsa_device.cuh"
 #include "salsa_math.cuh"
@@ -152,7 +153,8 @@ __device__ __forceinline__ KT kget(const WS<KT, LS> &w, int i, int j) {
 // With limit set, dnsp = MIN(dwet, dlim) overwrites the non-spherical diameter (:149-150),
 // so getDiameter's value never survives a type="all" update and is not evaluated here.
 // ----------------------------------------------------------------------------------------
-template <typename KT, int LS>
+// CUDA_ROOT: the wet diameter by CUDA's cbrt (see the condensation coefficients).
+template <bool CUDA_ROOT = false, typename KT, int LS>
 __device__ __forceinline__ void updateDiameterAll(const DevParams &P, const WS<KT, LS> &w, const double *dmid, int b) {
   int ph = phase_of(P, b);
   double n = w.numc[b];
@@ -164,7 +166,7 @@ __device__ __forceinline__ void updateDiameterAll(const DevParams &P, const WS<K
     for (int k = 0; k < P.ninsoluble; k++) vi += w.v(P.ind_insoluble[k], b);
     // (v / numc / pi6)^(1/3) with one division for the three diameters
     const double q = drcp(n * K_PI6);
-    dw = dcbrt(vs * q);
+    dw = CUDA_ROOT ? ::cbrt(vs * q) : dcbrt(vs * q);
     dd = dcbrt(vd * q);
     di = dcbrt(vi * q);
   } else {
@@ -2866,9 +2868,12 @@ __device__ void gpparth2o(const DevParams &P, const WS<KT, LS> &w, const double 
   (void)NB;
   const double sfl = divc(prs * rhoair, K_MWA), sfi = divc(prsi * rhoair, K_MWA);   // saturation, liquid and ice
   const double adt = 2.e-2;                                                         // substep [s]
-  // diameters and densities (:819-822), then per-bin coefficients (:826-955)
+  // diameters and densities (:819-822), then per-bin coefficients (:826-955).  The explicit
+  // substeps magnify a last-bit difference of the diameter or the Kelvin term of the
+  // smallest wet aerosol to as much as 1e-3 of the bin's water in a few cells in 1e5, so both
+  // come from CUDA's functions (once per bin and step: no measurable time).
   for (int b = lane; b < ntot; b += LS) {
-    updateDiameterAll(P, w, dmid, b);
+    updateDiameterAll<true>(P, w, dmid, b);
     int ph = phase_of(P, b);
     w.rhomean[b] = rhomean_of(P, ph, w.numc[b], w.v(iwa, b), w.v(irim, b));
     double n = w.numc[b];
@@ -2884,7 +2889,7 @@ __device__ void gpparth2o(const DevParams &P, const WS<KT, LS> &w, const double 
         double dwet = w.dwet[b];
         double znw = ddiv(w.v(iwa, b) * P.rholiq[iwa], P.MM[iwa]);
         double zact = acth2o_w(znw, ns_);
-        k_ = dexp(ddiv(4. * K_SURFW0 * K_MWA, K_RG * T * K_RHOWA * dwet));
+        k_ = ::exp(ddiv(4. * K_SURFW0 * K_MWA, K_RG * T * K_RHOWA * dwet));
         const double sf = sfl;
         ws = zact * k_;
         KT zknud = ddiv((KT)2. * (KT)zmfph2o, (KT)dwet);
@@ -2896,7 +2901,7 @@ __device__ void gpparth2o(const DevParams &P, const WS<KT, LS> &w, const double 
       } else {
         double dwet = w.dnsp[b];
         double cap = 0.5 * dwet;
-        k_ = dexp(ddiv(4. * K_SURFI0 * K_MWA, K_RG * T * K_RHOWA * dwet));
+        k_ = ::exp(ddiv(4. * K_SURFI0 * K_MWA, K_RG * T * K_RHOWA * dwet));
         const double sf = sfi;
         ws = 1.0 * k_;
         KT zknud = ddiv((KT)2. * (KT)zmfph2o, (KT)dwet);
@@ -4619,9 +4624,10 @@ __global__ void __launch_bounds__(SALSA_THREADS, 2) salsa_step_kernel(const DevP
 // spare (they are 5-15 % busy).  Blocks take four tiles of 32 cells from a counter, the cloudy
 // end of the list first (its cells take several times as long as clear ones).
 // FP64 instructions per cell of grid384x384x160: 6,190 in the warp form, about 1,000 here; a
-// 1.1 M cell block takes 78 ms, where the warp form took 299 ms.  Four blocks of 128 threads
+// 1.1 M cell block takes 76 ms, where the warp form took 299 ms.  Four blocks of 128 threads
 // per SM (128 registers) measured better than three (164 registers): clear cells 39.3
-// against 43.9 ns a cell, cloudy ones 397 against 455; the FP64 pipe is 71-80 % busy.
+// against 43.9 ns a cell, cloudy ones 397 against 455 (372 since); the FP64 pipe is 71-80 %
+// busy.
 template <typename KT, bool SIP>
 __global__ void __launch_bounds__(32 * SALSA_LANE_WARPS, SALSA_LANE_MINBLOCKS) salsa_lane_kernel(const DevParams P) {
   extern __shared__ double smem[];
