@@ -27,7 +27,7 @@
 // 417 -> 299 ms; FP64 instructions per cell 9,620 -> 6,190) and the sedimentation 1.26 times.
 //
 // Arguments outside the fast range (zero, subnormal, infinite, NaN, extreme exponents) take
-// the plain operation, out of line.  A unit that defines SALSA_MATH_PLAIN gets the plain
+// the plain operation, out of line (divc: see there).  A unit that defines SALSA_MATH_PLAIN gets the plain
 // operations throughout, one that defines SALSA_MATH_PLAIN_FUNCTIONS CUDA's cbrt, exp, log and pow.
 #pragma once
 #include <cstdint>
@@ -89,8 +89,11 @@ __device__ __forceinline__ double drcp(double d) {
   return fma(fma(-d, r, 1.), r, r);
 }
 
-// n/d with r = drcp(d) at hand (several quotients by one denominator)
+// n/d with r = drcp(d) at hand (several quotients by one denominator).  Exponents within
+// +-500; n = 0 too.
 __device__ __forceinline__ double ddiv_r(double n, double d, double r) {
+  const unsigned hi = (unsigned)__double2hiint(d), hn = (unsigned)__double2hiint(n);
+  if (!(fm_mid(hi) && (fm_mid(hn) || ((hn << 1) | (unsigned)__double2loint(n)) == 0u))) return fm_div_slow(n, d);
   const double q = n * r;
   return fma(fma(-d, q, n), r, q);
 }
@@ -104,11 +107,16 @@ __device__ __forceinline__ double ddiv(double n, double d) {
   return fma(fma(-d, q, n), r, q);
 }
 
-// x / c for a constant c: the product with 1/c as a sum of two doubles, folded at compile
-// time (exact when c is a power of two)
+// x / c for a positive constant c: the product with 1/c as a sum of two doubles, folded at
+// compile time (exact when c is a power of two).  The low product is left out, by a selection
+// on integers, where it cannot be formed (x zero, subnormal, above 2^877, infinite or NaN: an
+// infinite x against a negative low part gave NaN): one ulp there.
 __device__ __forceinline__ double divc(double x, double c) {
   const double r = 1. / c, l = fma(-c, r, 1.) * r;
-  return l == 0. ? x * r : fma(x, r, x * l);
+  if (l == 0.) return x * r;
+  const unsigned hi = (unsigned)__double2hiint(x);
+  const bool low = (hi & 0x7fffffffu) - (1u << 20) < (1899u << 20);
+  return fma(x, r, low ? x * l : __hiloint2double((int)(hi & 0x80000000u), 0));
 }
 // sqrt(x), x's exponent within +-500, or zero
 __device__ __forceinline__ double dsqrt(double x) {
