@@ -134,10 +134,11 @@ __device__ __forceinline__ double pos_part(double x) {
 }
 // fmax(c, x) of x >= 0 (or NaN: c)
 __device__ __forceinline__ double max_pos(double c, double x) { return num_gt(x, c) ? x : c; }
-// fmin(fmax(x, -t), t) of t >= 0
+// fmin(fmax(x, -t), t) of t >= 0 (NaN x: -t)
 __device__ __forceinline__ double limit_pos(double x, double t) {
   const long long b = __double_as_longlong(x), m = b & 0x7fffffffffffffffll, bt = __double_as_longlong(t);
-  return m > bt ? __longlong_as_double(bt | (b ^ m)) : x;
+  const long long sign = m > FM_INF ? (long long)0x8000000000000000ull : b ^ m;
+  return m > bt ? __longlong_as_double(bt | sign) : x;
 }
 __device__ __forceinline__ int tri(int i, int j, int NB) {  // i <= j
   return i * NB - (i * (i - 1)) / 2 + (j - i);
