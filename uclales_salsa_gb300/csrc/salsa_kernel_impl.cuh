@@ -3629,6 +3629,22 @@ __device__ void ice_nucl_SE(const DevParams &P, const WS<KT, LS> &w, const doubl
   const auto rec = row_cast<double>(w.K);
   enum { R_MODE = 0, R_THMIN, R_DIN, R_AE, R_SIG, R_DG, R_FHOM, R_FINT };
   const double Si = ddiv(prv, prsi);
+  // The lane form's short cuts leave out bins that cannot freeze.  A bin that freezes by nothing
+  // still sets negative values of the crystal bin of its size to zero (fmax of the sum), so
+  // they are for cells without negative ice: every cell, unless coagulation is off and
+  // advection left some.
+  bool quick = LS == 1;
+  if constexpr (LS == 1) {
+    auto ok = [](double x) {   // zero, positive or infinite
+      const unsigned long long b = (unsigned long long)__double_as_longlong(x);
+      return b <= (unsigned long long)FM_INF || b << 1 == 0ull;
+    };
+    if (P.st_icenucl)
+      for (int g = nl; g < P.ntotal; g++) {
+        quick = quick && ok(w.numc[g]);
+        for (int s = 0; s < P.nused; s++) quick = quick && ok(w.v(s, g));
+      }
+  }
   // pass A
   for (int kk = lane; kk < nl; kk += LS) {
     const auto st = stage + kk * 10;
@@ -3638,7 +3654,7 @@ __device__ void ice_nucl_SE(const DevParams &P, const WS<KT, LS> &w, const doubl
       // no scheme can freeze this bin (dry aerosol with immersion freezing alone, empty bins)
       const int ph = phase_of(P, kk);
       const bool cnt = !(T > 273.15) && !num_lt(w.numc[kk], nlim_of(ph));
-      if (!((P.lsicehom && T < tmax_homog) || (cnt && ph > 1 && P.lsiceimm) || (cnt && ph == 1 && P.lsicedep))) {
+      if (quick && !((P.lsicehom && T < tmax_homog) || (cnt && ph > 1 && P.lsiceimm) || (cnt && ph == 1 && P.lsicedep))) {
         r[R_FHOM] = 0.;
         r[R_MODE] = 0.;
         continue;
@@ -3743,7 +3759,6 @@ __device__ void ice_nucl_SE(const DevParams &P, const WS<KT, LS> &w, const doubl
   }
   // pass C: iceNucleation (:421-538)
   double dh = 0., dd = 0., di = 0.;
-  bool any0 = false;
   for (int kk = lane; kk < nl; kk += LS) {
     const auto st = stage + kk * 10;
     const auto r = rec + kk * 8;
@@ -3751,14 +3766,13 @@ __device__ void ice_nucl_SE(const DevParams &P, const WS<KT, LS> &w, const doubl
     const double n = w.numc[kk];
     const int ph = phase_of(P, kk);
     if constexpr (LS == 1) {
-      if ((__double_as_longlong(r[R_MODE]) | __double_as_longlong(r[R_FHOM])) == 0) {
+      if (quick && (__double_as_longlong(r[R_MODE]) | __double_as_longlong(r[R_FHOM])) == 0) {
         // nothing freezes: what is left of the update below are its limits, and an IN deficit
         // of 0/0 -> 0 without dust
         if (num_lt(n, nlim_of(ph))) continue;
         double vins = 0.;
         for (int k = 0; k < P.ninsoluble; k++) vins += w.v(P.ind_insoluble[k], kk);
         if (num_lt(vins, minVin)) continue;
-        any0 = true;
         w.indef[kk] = __double_as_longlong(w.v(idu, kk)) << 1 == 0 ? 0. : min_pos(pos_part(w.indef[kk]), 1.);
         for (int s = 0; s < P.nwet; s++) w.v(s, kk) = pos_part(w.v(s, kk));
         w.numc[kk] = pos_part(n);
@@ -3817,14 +3831,7 @@ __device__ void ice_nucl_SE(const DevParams &P, const WS<KT, LS> &w, const doubl
       w.misc[M_DIAG + DG_ICEIMM] += di;
     }
   }
-  if (P.st_icenucl) {
-    ice_apply_staged(P, w, stage, nl, lane);
-    if (any0)
-      for (int g = P.nliquid; g < P.ntotal; g++) {
-        for (int s = 0; s < P.nused; s++) w.v(s, g) = pos_part(w.v(s, g));
-        w.numc[g] = pos_part(w.numc[g]);
-      }
-  }
+  if (P.st_icenucl) ice_apply_staged(P, w, stage, nl, lane);
 }
 
 // classic ice nucleation (mo_salsa_cloud_ice.f90:26-140 with calc_Jhet/Jdep/Jhf :146-291)
