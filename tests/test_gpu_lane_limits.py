@@ -9,6 +9,7 @@ from parity import interior
 
 pytestmark = pytest.mark.gpu
 BINS = ("naerot", "ncloudt", "nprecpt", "nicet", "maerot", "mcloudt", "mprecpt", "micet")
+CELLS = ((2, 2, 1), (5, 9, 14), (20, 33, 27), (32, 17, 3))   # y, x, z
 
 
 def _run(inp, fields):
@@ -62,3 +63,26 @@ def test_negative_ice_without_coagulation(precision):
         stay = [(old < 0) & (old + o[key] * inp.dt <= 0.5 * old) for o in (a, b)]
         assert torch.equal(stay[0], stay[1]), (key, int((stay[0] != stay[1]).sum()))
         assert bool(stay[1].any()) and bool(((old < 0) & ~stay[1]).any())
+
+
+@pytest.mark.parametrize("coag", [0, 1])
+@pytest.mark.parametrize("value", [float("nan"), float("inf"), 0.0])
+def test_density_that_is_not_a_positive_number(value, coag):
+    """0 dn and 0 / dn are NaN then: the empty bins of such a cell show it too, and no other
+    cell does."""
+    inp = make_inputs("grid384x384x160", "cuda", X=32, Y=31, Z=27, overrides=dict(cloudy=0.0))   # 26,784 cells
+    inp.cfg.lscoag.sw = coag
+    for j, i, k in CELLS:
+        inp.fields["dn"][j, i, k] = value
+    a, b, na, nb = _both(inp)
+    assert na == nb
+    for key in BINS:
+        assert torch.equal(torch.isnan(a[key]), torch.isnan(b[key])), key
+    # (coagulation sets infinite numbers to zero, and 1/dn is zero: nothing is left to see)
+    ok = torch.ones(b["naerot"].shape[1:], dtype=torch.bool, device="cuda")
+    for j, i, k in CELLS:
+        assert bool(torch.isnan(a["naerot"][:, j - 2, i - 2, k - 1]).any()) == (not (coag and value > 0.0))
+        ok[j - 2, i - 2, k - 1] = False
+    for key in BINS:
+        d = (a[key] - b[key])[:, ok].abs()
+        assert float(d.max()) <= 1e-6 * float(b[key][:, ok].abs().max()), key

@@ -4260,15 +4260,17 @@ template <int LS> __device__ __forceinline__ void stage_sync() {
 }
 // ---- the lane form's unit conversion, straight between the fields and the workspace ----
 // x a and x a b, without FP64 products for the zeros of unpopulated bins (rounded as in the
-// warp form: the substeps magnify last-bit differences of the water)
-__device__ __forceinline__ double scaled(double x, double a) { return __double_as_longlong(x) == 0 ? 0. : x * a; }
-__device__ __forceinline__ double scaled(double x, double a, double b) {
-  return __double_as_longlong(x) == 0 ? 0. : x * a * b;
+// warp form: the substeps magnify last-bit differences of the water); z = 0 a, NaN when a is
+// not finite
+__device__ __forceinline__ double scaled(double x, double a, double z) { return __double_as_longlong(x) == 0 ? z : x * a; }
+__device__ __forceinline__ double scaled(double x, double a, double b, double z) {
+  return __double_as_longlong(x) == 0 ? z : x * a * b;
 }
 
 // (mo_salsa_driver.f90:196-283) the cell's bins in particles and volume per m3 of air
 template <typename KT>
 __device__ __forceinline__ void lane_unpack(const DevParams &P, const WS<KT, 1> &w, const double *dmid, double dn) {
+  const double zero = 0. * dn;
   int b0 = 0;
 #pragma unroll 1
   for (int c = 0; c < 4; c++) {
@@ -4287,7 +4289,7 @@ __device__ __forceinline__ void lane_unpack(const DevParams &P, const WS<KT, 1> 
       w.ddry[g] = 0.;
       w.dins[g] = 0.;
       w.dnsp[g] = 0.;
-      w.numc[g] = scaled(n, dn);
+      w.numc[g] = absent ? 0. : scaled(n, dn, zero);
       w.indef[g] = d;
       w.ctime[g] = t;
     }
@@ -4298,7 +4300,7 @@ __device__ __forceinline__ void lane_unpack(const DevParams &P, const WS<KT, 1> 
       const double irho = c < 3 ? P.irholiq[s] : (s < P.nwet ? P.irhoice[s] : 1. / K_RHORI);
       const double *f = s < ns ? fm + P.plane * ((long long)s * nb) : nullptr;
 #pragma unroll 8
-      for (int b = 0; b < nb; b++) w.v(s, b0 + b) = f ? scaled(__ldg(f + P.plane * b), dn, irho) : 0.;
+      for (int b = 0; b < nb; b++) w.v(s, b0 + b) = f ? scaled(__ldg(f + P.plane * b), dn, irho, zero) : 0.;
     }
     for (int b = 0; b < nb; b++) {
       const int g = b0 + b;
@@ -4313,8 +4315,9 @@ __device__ __forceinline__ void lane_unpack(const DevParams &P, const WS<KT, 1> 
 template <typename KT>
 __device__ __forceinline__ bool lane_output(const DevParams &P, const WS<KT, 1> &w, double idn) {
   const double dt = P.dt, idt = P.inv_dt != 0. ? P.inv_dt : drcp(dt);
+  const long long degenerate = (__double_as_longlong(idn) & FM_INF) == FM_INF;   // no finite 1/dn: 0/dn is NaN
   auto add = [&](double *f, double x, double v, double rho) {   // f += (v rho / dn - x) / dt
-    if ((__double_as_longlong(v) | __double_as_longlong(x)) == 0 || !w.live) return;
+    if ((__double_as_longlong(v) | __double_as_longlong(x) | degenerate) == 0 || !w.live) return;
     const double d = (v * rho * idn) - x;
     *f = *f + (P.inv_dt != 0. ? d * idt : ddiv_r(d, dt, idt));
   };
