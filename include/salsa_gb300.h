@@ -222,6 +222,13 @@ int salsa_gb300_last_launches(const salsa_handle_t *h);
 /* Device time in ms of the last run's kernels (cell-order pre-pass and step kernel). */
 double salsa_gb300_last_kernel_ms(const salsa_handle_t *h);
 
+/* Cells of the last step that were advanced one cell per lane (the lane form; the others one
+ * cell per warp), once that step's stream has been waited for.  No counterpart in the
+ * reference: the two forms round differently, and the lane form needs workspaces of up to
+ * about 2 GB, which the handle keeps; a large call that cannot have at least half of them
+ * takes the warp form, several times slower, and this tells. */
+long long salsa_gb300_last_lane_cells(const salsa_handle_t *h);
+
 void salsa_gb300_finalize(salsa_handle_t *h);
 
 const char *salsa_gb300_version(void);

@@ -47,6 +47,8 @@ def library():
     L.salsa_gb300_last_launches.restype = C.c_int
     L.salsa_gb300_last_kernel_ms.argtypes = [C.c_void_p]
     L.salsa_gb300_last_kernel_ms.restype = C.c_double
+    L.salsa_gb300_last_lane_cells.argtypes = [C.c_void_p]
+    L.salsa_gb300_last_lane_cells.restype = C.c_longlong
     L.salsa_gb300_tend_constrain.argtypes = [C.c_void_p, C.c_int, C.c_int, C.c_int, C.c_double,
                                              C.POINTER(PostFields), C.c_void_p]
     L.salsa_gb300_tend_constrain.restype = C.c_int
@@ -63,7 +65,7 @@ def library():
 
 
 EXPORTED = ["salsa_gb300_default_config", "salsa_gb300_init", "salsa_gb300_run", "salsa_gb300_run_async",
-            "salsa_gb300_layout", "salsa_gb300_last_launches", "salsa_gb300_last_kernel_ms",
+            "salsa_gb300_layout", "salsa_gb300_last_launches", "salsa_gb300_last_kernel_ms", "salsa_gb300_last_lane_cells",
             "salsa_gb300_finalize", "salsa_gb300_version", "salsa_gb300_run_noalloc", "salsa_gb300_chain_state_size",
             "salsa_gb300_chain_adjoint_bytes",
             "salsa_gb300_chain_forward", "salsa_gb300_chain_tlm", "salsa_gb300_chain_adjoint",
@@ -135,6 +137,10 @@ class SalsaStep:
 
     def last_kernel_ms(self):
         return library().salsa_gb300_last_kernel_ms(self.h)
+
+    def last_lane_cells(self):
+        """Cells of the last (synchronised) step that the lane form advanced; 0 in the warp form."""
+        return library().salsa_gb300_last_lane_cells(self.h)
 
     def close(self):
         if getattr(self, "h", None) and self.h.value:

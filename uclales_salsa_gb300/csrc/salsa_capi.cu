@@ -19,6 +19,7 @@
 #include "../../include/salsa_gb300.h"
 #include "salsa_device.cuh"
 #include "salsa_internal.h"
+#include "salsa_space.h"
 
 namespace salsa {
 cudaError_t launch_d1(const DevParams &, cudaStream_t, int);
@@ -192,8 +193,7 @@ struct salsa_handle {
   size_t kcache_bytes = 0;
   cudaStream_t s_in = nullptr, s_out = nullptr;     // copy streams of the host-buffer pipeline
   cudaEvent_t pev[3 * SALSA_PIPE_SLOTS + 2] = {};   // its slot and start/end events
-  double *lane_ws = nullptr;    // workspaces of the lane form, one per resident warp
-  size_t lane_ws_bytes = 0;
+  salsa::Space lane_ws;         // workspaces of the lane form, one per resident warp
   int *d_order = nullptr;       // cell order lists (salsa_order_kernel), order_cap entries each
   long long order_cap = 0;
   int *na_order = nullptr;      // module scratch of salsa_gb300_run_noalloc on this handle's device
@@ -603,6 +603,7 @@ int salsa_gb300_init(const salsa_config_t *cfg, salsa_handle_t **out) {
             // fields), as a synchronous call should
             cudaStreamCreate(&h->stream) == cudaSuccess &&
             cudaEventCreate(&h->ev0) == cudaSuccess && cudaEventCreate(&h->ev1) == cudaSuccess;
+  if (ok) memset(h->h_status, 0, salsa::ST_N * sizeof(unsigned long long));
   if (ok)
     ok = cudaMemcpy(h->d_tables, tab.data(), tab.size() * sizeof(double), cudaMemcpyHostToDevice) == cudaSuccess &&
          cudaMemcpy(h->d_rows, rows.data(), rows.size() * sizeof(Row), cudaMemcpyHostToDevice) == cudaSuccess &&
@@ -659,7 +660,7 @@ void salsa_gb300_finalize(salsa_handle_t *h) {
   if (h->d_rows) cudaFree(h->d_rows);
   if (h->d_pairs) cudaFree(h->d_pairs);
   if (h->d_order) cudaFree(h->d_order);
-  if (h->lane_ws) cudaFree(h->lane_ws);
+  if (h->lane_ws.p) cudaFree(h->lane_ws.p);
   for (int i = 0; i < 4; i++)
     if (h->scratch[i]) cudaFree(h->scratch[i]);
   if (h->d_status) cudaFree(h->d_status);
@@ -690,6 +691,9 @@ int salsa_gb300_layout(const salsa_handle_t *h, int *nbins, int *ncld, int *nprc
 
 int salsa_gb300_last_launches(const salsa_handle_t *h) { return h ? h->last_launches : 0; }
 double salsa_gb300_last_kernel_ms(const salsa_handle_t *h) { return h ? h->last_kernel_ms : 0.; }
+long long salsa_gb300_last_lane_cells(const salsa_handle_t *h) {
+  return h ? (long long)h->h_status[salsa::ST_LANE_CELLS] : 0;
+}
 
 }  // extern "C"
 
@@ -877,19 +881,18 @@ int run_impl(salsa_handle_t *h, int nzp, int nxp, int nyp, int ns, double tstep,
       const long long need = ((Q.ncells + 31) / 32 + SALSA_LANE_WARPS - 1) / SALSA_LANE_WARPS;
       lane_grid = (int)std::min((long long)lbps * h->nsm, need);
       Q.lane_rows = Q.ws_doubles + (prec == 0 ? 0 : SALSA_LEAF_ROWS);
-      const size_t bytes = (size_t)lane_grid * SALSA_LANE_WARPS * 32 * (size_t)Q.lane_rows * sizeof(double);
-      if (lane_grid > 0 && bytes > h->lane_ws_bytes) {
-        if (h->lane_ws) cudaFree(h->lane_ws);
-        h->lane_ws = nullptr;
-        h->lane_ws_bytes = 0;
-        if (cudaMalloc(&h->lane_ws, bytes) == cudaSuccess) {
-          h->lane_ws_bytes = bytes;
-        } else {
-          cudaGetLastError();   // no memory: the warp form needs none
-          lane_grid = 0;
-        }
-      }
-      Q.lane_ws = h->lane_ws;
+      cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;   // no allocation while a graph is captured
+      if (cudaStreamIsCapturing(s, &cap) != cudaSuccess) cudaGetLastError();
+      lane_grid = salsa::lane_blocks(
+          h->lane_ws, lane_grid, (size_t)SALSA_LANE_WARPS * 32 * (size_t)Q.lane_rows * sizeof(double),
+          [&](size_t bytes) -> void * {
+            void *p = nullptr;
+            if (cap == cudaStreamCaptureStatusNone && cudaMalloc(&p, bytes) == cudaSuccess) return p;
+            cudaGetLastError();
+            return nullptr;
+          },
+          [](void *p) { cudaFree(p); });
+      Q.lane_ws = static_cast<double *>(h->lane_ws.p);
     }
     int *moist = order && !noalloc ? order + h->order_cap : nullptr;   // the second half of the list's memory
     Q.order = order;
@@ -1034,7 +1037,7 @@ int run_impl(salsa_handle_t *h, int nzp, int nxp, int nyp, int ns, double tstep,
   salsa_status_t loc;
   memset(&loc, 0, sizeof loc);
   if (P.ncells > 0) {
-    loc.n_cells = (long long)h->h_status[salsa::ST_CELLS];
+    loc.n_cells = (long long)(h->h_status[salsa::ST_CELLS] + h->h_status[salsa::ST_LANE_CELLS]);
     loc.n_equil_nonconv = (long long)h->h_status[salsa::ST_EQUIL];
     loc.n_distr_nonconv = (long long)h->h_status[salsa::ST_DISTR];
     loc.n_distr_negfrac = (long long)h->h_status[salsa::ST_NEGFRAC];

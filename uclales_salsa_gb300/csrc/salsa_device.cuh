@@ -77,7 +77,8 @@ enum {
 };
 
 // status counters
-enum { ST_CELLS = 0, ST_EQUIL, ST_DISTR, ST_NEGFRAC, ST_COND, ST_NEG, ST_NONFINITE,
+enum { ST_CELLS = 0, ST_LANE_CELLS,      // cells advanced by the warp form, by the lane form
+       ST_EQUIL, ST_DISTR, ST_NEGFRAC, ST_COND, ST_NEG, ST_NONFINITE,
        ST_ORDER_CLEAR, ST_ORDER_CLOUDY, ST_ORDER_MOIST,   // fill counters of the cell order lists
        ST_TILE,                           // the lane form's next tile of 32 cells
        ST_N };

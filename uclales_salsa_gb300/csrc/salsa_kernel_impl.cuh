@@ -4694,7 +4694,7 @@ __global__ void __launch_bounds__(32 * SALSA_LANE_WARPS, SALSA_LANE_MINBLOCKS) s
       }
     }
     const unsigned nlive = __popc(__ballot_sync(0xffffffffu, w.live));
-    if (lane == 0) atomicAdd(P.status + ST_CELLS, (unsigned long long)nlive);
+    if (lane == 0) atomicAdd(P.status + ST_LANE_CELLS, (unsigned long long)nlive);
   }
 }
 
