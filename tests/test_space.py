@@ -64,3 +64,26 @@ def serve(prog, budget, calls):
 ])
 def test_blocks_served_when_memory_is_short(prog, budget, calls, served):
     assert serve(prog, budget, calls) == served
+
+
+LISTS = r"""
+#include <cstdio>
+#include "salsa_space.h"
+int main() {
+  size_t n, budget;
+  while (std::scanf("%zu %zu", &n, &budget) == 2) {
+    void *p = nullptr;
+    const int k = salsa::order_lists(n, &p, [&](size_t b) -> void * { return b <= budget ? (void *)1 : nullptr; });
+    std::printf("%d %d\n", k, p ? 1 : 0);
+  }
+}
+"""
+
+
+def test_order_lists_when_memory_is_short(tmp_path):
+    """One list serves a call whose two do not fit, as before there were two."""
+    (tmp_path / "l.cpp").write_text(LISTS)
+    subprocess.run(["g++", "-std=c++17", "-Wall", "-Werror", "-I", CSRC, str(tmp_path / "l.cpp"), "-o", str(tmp_path / "l")],
+                   check=True)
+    r = subprocess.run([str(tmp_path / "l")], input="100 800 100 799 100 400 100 399", text=True, capture_output=True, check=True)
+    assert r.stdout.split() == ["2", "1", "1", "1", "1", "1", "0", "0"]

@@ -196,6 +196,7 @@ struct salsa_handle {
   salsa::Space lane_ws;         // workspaces of the lane form, one per resident warp
   int *d_order = nullptr;       // cell order lists (salsa_order_kernel), order_cap entries each
   long long order_cap = 0;
+  int order_lists = 0;          // 2, or 1 when memory was short
   int *na_order = nullptr;      // module scratch of salsa_gb300_run_noalloc on this handle's device
   unsigned long long *na_status = nullptr;
   void *scratch[4] = {nullptr, nullptr, nullptr, nullptr};   // gradient-chain buffers
@@ -894,7 +895,7 @@ int run_impl(salsa_handle_t *h, int nzp, int nxp, int nyp, int ns, double tstep,
           [](void *p) { cudaFree(p); });
       Q.lane_ws = static_cast<double *>(h->lane_ws.p);
     }
-    int *moist = order && !noalloc ? order + h->order_cap : nullptr;   // the second half of the list's memory
+    int *moist = order && !noalloc && h->order_lists == 2 ? order + h->order_cap : nullptr;   // the second list
     Q.order = order;
     Q.order_moist = moist;
     if (order) {
@@ -921,7 +922,15 @@ int run_impl(salsa_handle_t *h, int nzp, int nxp, int nyp, int ns, double tstep,
       if (h->d_order) cudaFree(h->d_order);
       h->d_order = nullptr;
       h->order_cap = 0;
-      if (cudaMalloc(&h->d_order, 2 * (size_t)n * sizeof(int)) != cudaSuccess) return nullptr;
+      void *p = nullptr;
+      h->order_lists = salsa::order_lists((size_t)n, &p, [](size_t bytes) -> void * {
+        void *q = nullptr;
+        if (cudaMalloc(&q, bytes) == cudaSuccess) return q;
+        cudaGetLastError();
+        return nullptr;
+      });
+      if (!p) return nullptr;
+      h->d_order = static_cast<int *>(p);
       h->order_cap = n;
     }
     return h->d_order;

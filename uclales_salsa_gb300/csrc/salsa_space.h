@@ -32,4 +32,13 @@ int lane_blocks(Space &s, int grid, size_t per_block, Alloc alloc, Release relea
   return have >= (size_t)grid ? grid : (have >= (size_t)least ? (int)have : 0);
 }
 
+// Cell order lists of n entries: two of them (the second one for moist clear cells), or, when
+// memory is short, one, with those cells among the dry ones.  Returns how many, 0 for none.
+template <typename Alloc>
+int order_lists(size_t n, void **p, Alloc alloc) {
+  for (int lists = 2; lists > 0; lists--)
+    if ((*p = alloc((size_t)lists * n * sizeof(int)))) return lists;
+  return 0;
+}
+
 }  // namespace salsa
