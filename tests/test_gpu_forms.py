@@ -31,3 +31,43 @@ def test_last_lane_cells(size, lane):
                                          C.byref(cf), C.c_void_p(s.cuda_stream), 1, C.byref(st)) == 0
         assert st.n_cells == inp.ncells and step.last_lane_cells() == 0
     step.close()
+
+
+def _scattered(cells, cloudy, precision, sip):
+    """`cells` of grid384x384x160, a share of them in cloud with ice."""
+    inp = make_inputs("grid384x384x160", "cuda", X=16, Y=cells // 512, Z=32, precision=precision, gases=sip,
+                      overrides=dict(cloudy=cloudy, pattern="random"))
+    if sip:
+        for sw in (inp.cfg.lssecice, inp.cfg.lssiprimespln, inp.cfg.lssipdropfrac, inp.cfg.lssipicecollbreak):
+            sw.sw, sw.mode = 1, 1
+        for name in ("sipdrfr", "siprmspl", "sipiibr"):
+            inp.fields[name] = inp.fields["nice"] * 0.02
+    return inp
+
+
+@pytest.mark.parametrize("cells,cloudy,precision,sip,lane", [
+    (24576, 0.0, 0, False, True), (24576, 0.02, 0, False, False), (24576, 0.1, 0, False, False),
+    (24576, 1.0, 0, False, True), (61440, 0.02, 0, False, True), (24064, 1.0, 0, False, False),
+    (40960, 0.02, 1, False, False), (40960, 1.0, 1, False, True), (81920, 0.02, 1, False, True),
+    (8192, 0.0, 0, True, True), (8192, 0.02, 0, True, False), (8192, 1.0, 0, True, True), (24576, 0.02, 0, True, True),
+    (8192, 0.1, 1, True, False), (8192, 1.0, 1, True, True)])
+def test_few_cloudy_cells_take_the_warp_form(cells, cloudy, precision, sip, lane):
+    """The form follows the kinds of cells; a large call that takes the warp form gives every
+    cell what smaller calls give it, bit for bit."""
+    inp = _scattered(cells, cloudy, precision, sip)
+    outs = {k: v for k, v in make_outputs(inp).items()}
+    step = api.SalsaStep(inp.cfg)
+    f = {k: v.clone() for k, v in inp.fields.items()}
+    rc, st = step.run(inp, f, outs, time=1.0)
+    assert rc == 0 and st.n_cells == cells
+    assert step.last_lane_cells() == (cells if lane else 0)
+    if not lane:
+        n = inp.nyp // 3
+        sub = type(inp)(**{**inp.__dict__, "nyp": n})
+        sub.fields = {k: v[..., :n, :, :].contiguous() for k, v in inp.fields.items()}
+        part = make_outputs(sub)
+        rc, st = step.run(sub, {k: v.clone() for k, v in sub.fields.items()}, part, time=1.0)
+        assert rc == 0 and step.last_lane_cells() == 0
+        for k, v in part.items():
+            assert torch.equal(v[..., 2:-2, 2:-2, 1:-1], outs[k][..., 2:n - 2, 2:-2, 1:-1]), k
+    step.close()

@@ -57,18 +57,25 @@ const Form FORMS[2][2] = {
 const Form &form_of(bool sip, int precision) { return FORMS[sip ? 1 : 0][precision]; }
 }  // namespace
 
-// Calls of at least this many cells take the lane form (one cell per lane); smaller ones
-// take the warp form, whose latency per cell is lower: a tile of 32 cells takes the lane form
-// 4 (warm cells) to 12 ms (cloudy ones), and that is what a call takes while every sub-core
-// holds at most one tile.  At 24,576 cells of grid16x16x40, grid256x256x128 and
-// grid384x384x160 the FP64 forms take 5.4 / 5.6, 9.3 / 11.2 and 10.5 / 10.8 ms (lane / warp
-// form); the mixed ones, whose warp form is faster, 5.4 / 4.3, 9.8 / 9.1 and 10.8 / 9.2 ms, and
-// 7.2 / 8.6, 15.8 / 19.5 and 17.1 / 13.0 ms at 49,152.  With secondary ice the warp form holds
-// one block per SM and runs the schemes on one lane: 12.8 / 47 ms at 13,824 cells, even at
-// about 4,000.
+// Calls of at least this many cells can take the lane form (one cell per lane); smaller ones
+// take the warp form, whose latency per cell is lower.
 #define SALSA_LANE_MINCELLS 24576
 #define SALSA_LANE_MINCELLS_MIXED 40960
 #define SALSA_LANE_MINCELLS_SIP 4096
+
+// Above that the slowest kind of cell decides.  A tile of 32 cells takes the lane form lane_ns,
+// and that is what a call takes while every sub-core holds one tile of that kind at most; the
+// warp form takes warp_ns a cell on all SMs together.  So a few cloudy cells among clear ones
+// are better off in the warp form: grid384x384x160 with 2 % of 24,576 cells cloudy takes 4.6 ms
+// there and 9.6 in the lane form, with 30 % 9.7 in both, with all 23.1 against 12.2; with
+// secondary ice, 2 % of 8,192 cells 5.9 against 11.3, 30 % 11.4 against 11.8, all 27.6 against
+// 11.4.  The order pre-pass has counted the kinds when the kernels start: while the call's
+// answer depends on them, both are launched and one of them returns at once (20 to 40 us).
+// The times are of 152 SMs, for dry clear, moist clear and cloudy cells of grid384x384x160 and
+// grid256x256x128; [secondary ice][FP64, mixed].
+const struct { int warp_ns[3], lane_ns[3]; } FORM_NS[2][2] = {
+    {{{170, 390, 950}, {2200000, 4800000, 9500000}}, {{140, 300, 850}, {2200000, 5000000, 9900000}}},
+    {{{560, 880, 3370}, {2050000, 4850000, 10500000}}, {{360, 540, 2250}, {2050000, 4850000, 10000000}}}};
 
 using salsa::DevParams;
 using salsa::Row;
@@ -909,9 +916,21 @@ int run_impl(salsa_handle_t *h, int nzp, int nxp, int nyp, int ns, double tstep,
       if (cudaGetLastError() != cudaSuccess) return SALSA_E_CUDA;
       launches++;
     }
-    const cudaError_t e = lane_grid > 0 ? form.lane(Q, s, lane_grid) : form.warp(Q, s, (int)grid);
-    if (e != cudaSuccess) return SALSA_E_CUDA;
-    launches++;
+    const auto &t = FORM_NS[sip ? 1 : 0][prec];
+    // the lane form alone when even dry cells would take the warp form longer than a cloudy tile
+    Q.choose = lane_grid > 0 && Q.ncells * t.warp_ns[0] < t.lane_ns[2];
+    for (int c = 0; c < 3; c++) {
+      Q.warp_ns[c] = t.warp_ns[c];
+      Q.lane_ns[c] = t.lane_ns[c];
+    }
+    if (lane_grid > 0) {
+      if (form.lane(Q, s, lane_grid) != cudaSuccess) return SALSA_E_CUDA;
+      launches++;
+    }
+    if (lane_grid <= 0 || Q.choose) {
+      if (form.warp(Q, s, (int)grid) != cudaSuccess) return SALSA_E_CUDA;
+      launches++;
+    }
     return SALSA_OK;
   };
   // the cell order lists for up to n cells

@@ -144,6 +144,9 @@ struct DevParams {
   // offset of the tally region inside each warp's workspace (doubles)
   int st_secice, st_siprs, st_sipdf, st_sipib;
   int sip_rs_mode, sip_df_mode, sip_ib_mode, sip_splbin, sip_off;
+  // both forms are launched and the counts of the order lists choose (lane_pays): the warp
+  // form's time per cell, the lane form's for a tile, of a dry clear, moist clear and cloudy cell [ns]
+  int choose, warp_ns[3], lane_ns[3];
   double *lane_ws;   // workspaces of the lane form, one of 32 * lane_rows doubles per resident warp
   int lane_rows;     // ws_doubles, and in the mixed form the leaves of its partner sums
   int raw_sip;   // first of the 3 x nice tracer rows (sipdrfr, siprmspl, sipiibr), or -1
@@ -181,6 +184,19 @@ __device__ __forceinline__ long long cell_at(const DevParams &P, long long i) {
   if (!P.order_moist) return P.order[i];
   const long long nd = (long long)P.status[ST_ORDER_CLEAR], nm = (long long)P.status[ST_ORDER_MOIST];
   return i < nd ? P.order[i] : (i < nd + nm ? P.order_moist[i - nd] : P.order[P.ncells - 1 - (i - nd - nm)]);
+}
+
+// whether the call's cells take the lane form: the warp form's time grows with their number and
+// kind, the lane form's is that of the slowest tile while every sub-core has one
+__device__ __forceinline__ bool lane_pays(const DevParams &P) {
+  const int counter[3] = {ST_ORDER_CLEAR, ST_ORDER_MOIST, ST_ORDER_CLOUDY};
+  long long warp = 0, lane = 0;
+  for (int c = 0; c < 3; c++) {
+    const long long n = (long long)P.status[counter[c]];
+    warp += n * P.warp_ns[c];
+    if (n) lane = P.lane_ns[c];
+  }
+  return warp >= lane;
 }
 
 }  // namespace salsa

@@ -4584,6 +4584,7 @@ __device__ __forceinline__ WS<KT, LS> make_ws(const DevParams &P, Ptr<double, LS
 template <typename KT, bool SIP>
 __global__ void __launch_bounds__(SALSA_THREADS, 2) salsa_step_kernel(const DevParams P) {
   extern __shared__ double smem[];
+  if (P.choose && lane_pays(P)) return;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   double *tb = smem;
   for (int i = tid; i < P.tab_doubles; i += SALSA_THREADS) tb[i] = P.tables[i];
@@ -4646,6 +4647,7 @@ __global__ void __launch_bounds__(SALSA_THREADS, 2) salsa_step_kernel(const DevP
 template <typename KT, bool SIP>
 __global__ void __launch_bounds__(32 * SALSA_LANE_WARPS, SALSA_LANE_MINBLOCKS) salsa_lane_kernel(const DevParams P) {
   extern __shared__ double smem[];
+  if (P.choose && !lane_pays(P)) return;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   double *tb = smem;
   for (int i = tid; i < P.tab_doubles; i += 32 * SALSA_LANE_WARPS) tb[i] = P.tables[i];
