@@ -20,7 +20,7 @@ pytestmark = pytest.mark.gpu
 SIP_SIZE = {0: dict(X=20, Y=22, Z=21), 1: dict(X=21, Y=26, Z=23)}
 
 
-def _outputs(inp, fields, noalloc):
+def _outputs(inp, fields, noalloc, initialize=0):
     out = {k: v.cuda() for k, v in make_outputs(inp).items()}
     f = {k: v.clone().cuda() for k, v in fields.items()}
     step = api.SalsaStep(inp.cfg)
@@ -29,11 +29,11 @@ def _outputs(inp, fields, noalloc):
         L.salsa_gb300_run_noalloc.argtypes = L.salsa_gb300_run_async.argtypes
         cf, st, s = capi.make_fields(f, out), capi.Status(), torch.cuda.Stream()
         s.wait_stream(torch.cuda.current_stream())
-        rc = L.salsa_gb300_run_noalloc(step.h, inp.nzp, inp.nxp, inp.nyp, inp.ns, inp.dt, 1.0, 1, inp.level, 0, 0,
+        rc = L.salsa_gb300_run_noalloc(step.h, inp.nzp, inp.nxp, inp.nyp, inp.ns, inp.dt, 1.0, 1, inp.level, 0, initialize,
                                        C.byref(cf), C.c_void_p(s.cuda_stream), 1, C.byref(st))
         torch.cuda.synchronize()
     else:
-        rc, st = step.run(inp, f, out, time=1.0)
+        rc, st = step.run(inp, f, out, time=1.0, initialize=initialize)
     assert rc == 0 and st.n_cells == inp.ncells, (rc, st.as_dict())
     assert step.last_lane_cells() == (0 if noalloc else inp.ncells)
     step.close()
@@ -89,9 +89,19 @@ def test_secondary_ice_lane_form_against_the_oracle():
     _parity(inp, 1e-10, 2.2e-16)
 
 
-def test_large_noalloc_call_differs_from_run_by_rounding():
-    inp = make_inputs("grid384x384x160", "cuda", X=32, Y=31, Z=27)
-    _compare(inp, _outputs(inp, inp.fields, False), _outputs(inp, inp.fields, True), False)
+@pytest.mark.parametrize("precision", [0, 1])
+@pytest.mark.parametrize("kind", ["plain", "dt", "initialize", "kappa"])
+def test_noalloc_differs_from_a_large_run_by_rounding(kind, precision):
+    """The configured call; a step length without an exact reciprocal; the initial equilibration
+    of the aerosol water; kappa and supersaturation per cell."""
+    if kind == "kappa":
+        inp = make_inputs("batch65536", "cuda", X=1, Y=1, Z=41001, precision=precision)
+    else:
+        inp = make_inputs("grid384x384x160", "cuda", X=32, Y=43, Z=31, precision=precision)
+    if kind == "dt":
+        inp.dt = 0.7
+    init = int(kind == "initialize")
+    _compare(inp, _outputs(inp, inp.fields, False, init), _outputs(inp, inp.fields, True, init), False)
 
 
 @pytest.mark.parametrize("precision", [0, 1])
