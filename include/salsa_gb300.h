@@ -174,7 +174,17 @@ void salsa_gb300_default_config(salsa_config_t *cfg);
 int salsa_gb300_init(const salsa_config_t *cfg, salsa_handle_t **out);
 
 /* Replaces run_SALSA(Diag, Prog, nzp, nxp, nyp, ns, wp, pa_nactd, pa_vactd,
- * tstep, time, istp, level, lcharge, initialize)  (mo_salsa_driver.f90:112-435). */
+ * tstep, time, istp, level, lcharge, initialize)  (mo_salsa_driver.f90:112-435).
+ *
+ * Two forms of the kernel serve it: one warp per cell, and one lane per cell for calls with
+ * enough cells (from 24,576, FP32-mixed 40,960, with secondary ice 4,096; there the kinds of
+ * cells in the call choose).  They agree to rounding, which the scheme magnifies where it is
+ * ill-conditioned (Aitken water in supersaturation, new ice): a grid in one call and the same
+ * grid in parts can differ by that.  The lane form's workspaces, up to about 2 GB of device
+ * memory, are allocated by the first call that takes it, kept with the handle and released by
+ * salsa_gb300_finalize; when they are not to be had the call runs with fewer blocks or in the
+ * warp form (salsa_gb300_last_lane_cells tells).  Calls on one handle share its scratch: the
+ * caller serialises them. */
 int salsa_gb300_run(salsa_handle_t *h, int nzp, int nxp, int nyp, int ns,
                     double tstep, double time, int istp, int level, int lcharge,
                     int initialize, const salsa_fields_t *f, salsa_status_t *st);
@@ -192,8 +202,11 @@ int salsa_gb300_run_async(salsa_handle_t *h, int nzp, int nxp, int nyp, int ns,
  * memory: a model that gives all free device memory to its own pool at start-up (a
  * later cudaMalloc then fails), or one whose time loop cannot afford the
  * device-wide synchronisation that cudaMalloc and cudaFree imply.  Same arguments
- * and results as salsa_gb300_run_async (device pointers only), but the scratch the
- * step needs -- the cell-order list and the status counters -- sits in a static
+ * as salsa_gb300_run_async (device pointers only), and its results: bit for bit where that
+ * takes the warp form (one warp per cell), to rounding where it takes the lane form, whose
+ * workspaces this call cannot have.  It always runs the warp form, which takes three to four
+ * times as long on large calls (196,608 cells of grid384x384x160, 10 % cloudy: 49 against
+ * 16 ms).  The scratch the step needs -- the cell-order list and the status counters -- sits in a static
  * device array of the library: 8 MiB, enough for SALSA_NOALLOC_MAXCELLS =
  * 2,097,152 interior cells (larger grids return SALSA_E_ARG).  Every GPU that loads
  * the library holds that array until the process exits.  The array keeps the last
@@ -202,8 +215,8 @@ int salsa_gb300_run_async(salsa_handle_t *h, int nzp, int nxp, int nyp, int ns,
  * kernel modules on the handle's device (the array is part of one of them: with lazy
  * module loading a module's device memory is taken when it loads) and looks up the
  * array's device address there (cudaGetSymbolAddress); so create the handle before
- * the caller's pool takes the free memory.  All calls on one device share the array: calls that overlap
- * on the GPU (other streams, other handles on that device) race on it, so the
+ * the caller's pool takes the free memory.  All calls on one device share the array: calls
+ * that overlap on the GPU (other streams, other handles on that device) race on it, so the
  * caller must serialise them. */
 #define SALSA_NOALLOC_MAXCELLS 2097152
 int salsa_gb300_run_noalloc(salsa_handle_t *h, int nzp, int nxp, int nyp, int ns,

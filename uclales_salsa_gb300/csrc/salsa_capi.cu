@@ -95,9 +95,9 @@ static __device__ __align__(256) unsigned long long g_na_status[salsa::ST_N];
 // path.  Clear cells at 98 % relative humidity and more, where water condenses on the
 // aerosol in substeps, go to a list of their own where there is one: in two classes most
 // warps of the lane form ran the substeps for a few lanes (a grid256x256x128 block of 152 k
-// cells, whose clear cells lie at 90-101 %: 27.7 ms in two classes, 19.7 in three).  Each warp claims its slots with one atomic per
-// class; the order of the claims does not affect any result, since every cell is computed
-// independently.
+// cells, whose clear cells lie at 90-101 %: 27.7 ms in two classes, 19.7 in three; 17.4 now).
+// Each warp claims its slots with one atomic per class; the order of the claims does not affect
+// any result, since every cell is computed independently.
 __global__ void salsa_order_kernel(const DevParams P, int *order, int *moist) {
   const unsigned F = 0xffffffffu;
   const int lane = threadIdx.x & 31;
@@ -906,8 +906,8 @@ int run_impl(salsa_handle_t *h, int nzp, int nxp, int nyp, int ns, double tstep,
     Q.order = order;
     Q.order_moist = moist;
     if (order) {
-      // the order list's fill counters and the lane form's tile counter start at zero for every launch (a call may launch
-      // several, one per slab)
+      // the order lists' fill counters and the lane form's tile counter start at zero for every
+      // launch (a call may launch several, one per slab)
       if (cudaMemsetAsync(Q.status + salsa::ST_ORDER_CLEAR, 0, 4 * sizeof(unsigned long long), s) != cudaSuccess)
         return SALSA_E_CUDA;
       long long og = (Q.ncells + 255) / 256;

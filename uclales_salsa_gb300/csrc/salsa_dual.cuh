@@ -4,9 +4,11 @@
 // templates (bin_props, coag_pair, terminal_vel) instantiate with Dual<2> to give
 // dK/d(d_i) and dK/d(d_j) for the adjoint, and the chain step instantiates with
 // Dual<1> for the tangent-linear model.  Derivatives follow the elementary rules;
-// min/max/abs take the branch of the value (one-sided at ties).  The value parts round
-// exactly as the plain FP64 code (no contraction); the tangent parts use fused
-// multiply-adds, which only changes their last bits.
+// min/max/abs take the branch of the value (one-sided at ties).  The value parts take the
+// operations of the plain FP64 code without contraction; divisions and functions are those of
+// salsa_math.cuh, as far as the unit takes them (the kernels that advance the state: none; the
+// taped step: divisions and roots, within 0.501 ulp; the reverse step: all).  The tangent parts
+// use fused multiply-adds, which only changes their last bits.
 #pragma once
 #include <cuda_runtime.h>
 #include "salsa_math.cuh"

@@ -115,8 +115,8 @@ __device__ __forceinline__ double dlim_of(int ph) {
 }
 // Comparisons of a number with a positive constant, and minima and maxima of non-negative
 // ones, on the bit patterns: an FP64 comparison occupies the FP64 pipe as long as a sum
-// does.  The results equal the FP64 ones for every x that arithmetic produces (NaNs are
-// positive quiet ones here).
+// does.  The results equal the FP64 ones over the stated ranges, infinities and the positive
+// quiet NaN of the GPU's arithmetic included (-0 counts as 0).
 #define FM_INF 0x7ff0000000000000ll
 __device__ __forceinline__ bool num_ge(double x, double c) {
   const long long b = __double_as_longlong(x);
@@ -4640,7 +4640,7 @@ __global__ void __launch_bounds__(SALSA_THREADS, 2) salsa_step_kernel(const DevP
 // them all: grid384x384x160 with 10 % of the cells cloudy, scattered, took 13.1 ms at 24,576
 // cells and 18.3 at 49,152 (the warp form 6.1 and 12.4); now 9.6 and 10.5.
 // FP64 instructions per cell of grid384x384x160: 6,190 in the warp form, about 1,000 here; a
-// 1.1 M cell block takes 76 ms, where the warp form took 299 ms.  Four blocks of 128 threads
+// 1.1 M cell block takes 76 ms, where the warp form took 299 ms (FP32-mixed: 69 and 226 ms).  Four blocks of 128 threads
 // per SM (128 registers) measured better than three (164 registers): clear cells 39.3
 // against 43.9 ns a cell, cloudy ones 397 against 455 (372 since); the FP64 pipe is 71-80 %
 // busy.

@@ -39,12 +39,10 @@ namespace {
 typedef unsigned long long fm_u64;
 typedef unsigned __int128 fm_u128;
 
-#ifndef SALSA_MATH_HOST
 __device__ __forceinline__ float fm_rcp32(float x) { float r; asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x)); return r; }
 __device__ __forceinline__ float fm_rsqrt32(float x) { float r; asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x)); return r; }
 __device__ __forceinline__ float fm_lg2_32(float x) { float r; asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x)); return r; }
 __device__ __forceinline__ float fm_ex2_32(float x) { float r; asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x)); return r; }
-#endif
 
 #ifdef SALSA_MATH_PLAIN
 __device__ __forceinline__ double drcp(double d) { return 1. / d; }

@@ -26,13 +26,14 @@ namespace {
 //     and marks the levels it changes; pass B gathers, for every marked level, the
 //     contributions of the sources in the order the reference adds them (sources from
 //     the top down, a level's removal of its own parcel before its re-deposit).
-// The FP64 pipe bounds it: a full pass over a million points moves bytes for 1.2 ms.  So the surface level's dry deposition (two powers and six
-// quotients) is taken for 32 bins at a time, one per lane, before their loop, where one lane
-// of the first round did it for every bin; the flux divergence is two products per species
-// with the level's coefficients; the shares of a falling parcel are taken once per source;
-// the number limits are compared as integers; an ice crystal's shape and dimension share their
-// limits.  grid256x256x128, 96 x 96 columns, all four parts: 13.7 ms before the fast division
-// and roots, 10.8 with them, 7.9 with these, 7.7 with four blocks of 55 KB per SM instead of three of 66.
+// The FP64 pipe bounds it: a full pass over a million points moves bytes for 1.2 ms.  So the
+// surface level's dry deposition (two powers and six quotients) is taken for 32 bins at a time,
+// one per lane, before their loop, where one lane did it for every bin in turn; the flux
+// divergence is two products per species with the level's coefficients; the shares of a falling
+// parcel are taken once per source; the number limits are compared as integers; an ice crystal's
+// shape and dimension share their limits.  grid256x256x128, 96 x 96 columns, all four parts:
+// 13.7 ms before the fast division and roots, 10.8 with them, 7.9 with these, 7.7 with four
+// blocks of 55 KB per SM instead of three of 66.
 // Levels and bins that the reference visits only to add a zero are skipped.  The sums
 // over bins (rrate, tlt, the surface rates) run in the reference's index order,
 // including the range (ns-1)*nb:ns*nb of its water sums, which starts at the last bin
